@@ -91,6 +91,13 @@ struct Scene {
   size_t n_node4 = 0, n_tri4 = 0, n_shade4 = 0;   // float4 records of the repacked arrays
 };
 
+// the device copy of a scene's lights (yc::prepare_light)
+std::vector<yc_quad_light> prepared_lights(const yc_quad_light* lights, int n) {
+  std::vector<yc_quad_light> out(lights, lights + n);
+  for (yc_quad_light& l : out) yc::prepare_light(l);
+  return out;
+}
+
 struct Accum {
   DevBuf<float4> buf;
   DevBuf<float4> ldr;   // tonemapped image
@@ -672,7 +679,9 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
   if (n_mat > 0)
     YC_CUDA(cudaMemcpyAsync(s->mats.p, mats, n_mat * sizeof(yc_material), cudaMemcpyHostToDevice, c->stream));
   YC_CUDA(cudaMemcpyAsync(s->on_ab.p, on_ab.data(), on_ab.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
-  YC_CUDA(cudaMemcpyAsync(s->lights.p, lights, n_light * sizeof(yc_quad_light), cudaMemcpyHostToDevice, c->stream));
+  const std::vector<yc_quad_light> dev_lights = prepared_lights(lights, n_light);
+  YC_CUDA(cudaMemcpyAsync(s->lights.p, dev_lights.data(), n_light * sizeof(yc_quad_light), cudaMemcpyHostToDevice,
+                          c->stream));
   YC_CUDA(cudaStreamSynchronize(c->stream));
   yc::DevScene& d = s->dev;
   d.nodes = s->nodes.p;
@@ -776,7 +785,9 @@ int yc_set_lights(yc_ctx* c, int scene_id, const yc_quad_light* lights, int n_li
   Scene* s = find_scene(c, scene_id);
   if (!s) return fail(YC_E_NOTFOUND, "unknown scene");
   if (n_light < 1 || n_light > yc::MAX_LIGHTS || !lights) return fail(YC_E_INVALID, "need 1..16 lights");
-  YC_CUDA(cudaMemcpyAsync(s->lights.p, lights, n_light * sizeof(yc_quad_light), cudaMemcpyHostToDevice, c->stream));
+  const std::vector<yc_quad_light> dev_lights = prepared_lights(lights, n_light);
+  YC_CUDA(cudaMemcpyAsync(s->lights.p, dev_lights.data(), n_light * sizeof(yc_quad_light), cudaMemcpyHostToDevice,
+                          c->stream));
   YC_CUDA(cudaStreamSynchronize(c->stream));
   s->dev.n_lights = n_light;
   return YC_OK;

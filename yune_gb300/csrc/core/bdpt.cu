@@ -27,13 +27,10 @@ namespace yc {
 
 enum : int { BF_GLOSSY = 1, BF_OCCLUDED = 2 };
 
-// The BRDF and Phong-lobe helpers of the logic kernel, inlined or called (BDPT_HELPER).
+// The BRDF helper of the logic kernel, inlined or called (BDPT_HELPER).
 #define BDPT_HELPER __forceinline__
 __device__ BDPT_HELPER f4 brdf_bk(f4 w_i, f4 w_o, f4 n, const yc_material& m, bool glossy, float rr_prob) {
   return brdf_b(w_i, w_o, n, m, glossy, rr_prob);
-}
-__device__ BDPT_HELPER f4 sample_phong_bk(const Vtx& v, const yc_material& m, f4 w_i, uint32_t& seed, float& pdf) {
-  return sample_phong_b(v, m, w_i, seed, pdf);
 }
 
 struct BCount {
@@ -119,8 +116,7 @@ __global__ void __launch_bounds__(256) k_raygen_bdpt(PassParams pp, PathState ps
     v0.hp = (A + B) + ld4(L.pos);
     v0.n = ld4(L.normal);
     v0.mat = -1;
-    const float area = ym::mul(ym::length(ld4(L.edge_l)), ym::length(ld4(L.edge_w)));
-    const float fwd = ym::div(1.0f, area);
+    const float fwd = ym::rcp(light_area(L));
     const f4 c0 = ld4(L.ke) / fwd;
     lv.at(0, 0) = make_float4(v0.hp.x, v0.hp.y, v0.hp.z, __int_as_float(-1));
     lv.at(0, 1) = make_float4(v0.n.x, v0.n.y, v0.n.z, v0.n.w);
@@ -276,7 +272,7 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
             const bool g = sample_glossy_b(m, seed, prob);
             if (prob == 0.0f) { phase = Q_EYE_START; break; }
             float pdf = 1.0f;
-            const f4 nd = g ? sample_phong_bk(pv, m, -lv.dir(cnt.i - 1), seed, pdf) : sample_cosine(pv, seed, pdf);
+            const f4 nd = sample_lobe_b(pv, m, g, -lv.dir(cnt.i - 1), seed, pdf);
             flags = g ? (flags | BF_GLOSSY) : (flags & ~BF_GLOSSY);
             pend_pdf = pdf;
             pend_prob = prob;
@@ -333,7 +329,7 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
             const bool g = sample_glossy_b(m, seed, prob);
             if (prob == 0.0f) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
             float pdf = 1.0f;
-            const f4 nd = g ? sample_phong_bk(pv, m, -ev.dir(cnt.i - 1), seed, pdf) : sample_cosine(pv, seed, pdf);
+            const f4 nd = sample_lobe_b(pv, m, g, -ev.dir(cnt.i - 1), seed, pdf);
             if (pdf <= 0.0f) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
             flags = g ? (flags | BF_GLOSSY) : (flags & ~BF_GLOSSY);
             pend_pdf = pdf;

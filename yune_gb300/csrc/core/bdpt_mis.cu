@@ -105,14 +105,10 @@ __device__ __forceinline__ bool sample_dir(const Vtx& v, const yc_material& m, f
   const float u = draw(seed);
   const float pd = diffuse_prob(m);
   float pdf = 0.0f;
-  if (pd >= 1.0f || u < pd) w_next = sample_cosine(v, seed, pdf);
-  else w_next = sample_phong_b(v, m, w_prev, seed, pdf);
+  w_next = sample_lobe_b(v, m, !(pd >= 1.0f || u < pd), w_prev, seed, pdf);
   return ym::dot(w_next, v.n) > 0.0f;
 }
 
-__device__ __forceinline__ float light_area(const yc_quad_light& L) {
-  return ym::mul(ym::length(ld4(L.edge_l)), ym::length(ld4(L.edge_w)));
-}
 __device__ __forceinline__ float light_weight(const yc_quad_light& L) {
   return ym::mul(ym::add(ym::add(L.ke.x, L.ke.y), L.ke.z), light_area(L));
 }

@@ -168,12 +168,13 @@ __global__ void __launch_bounds__(ENGINE_TB) k_batch_logic(const BatchJob* __res
     int p = -1;
     bool need_task = false;
     LogicCounts lc;
+    const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
       p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
       const int4 jp = job_pass[p];
       const BatchJob& J = jobs[jp.x];
       const int reset = (jp.y == 0) ? J.reset_first : 0;
-      emit = logic_path(J.pp, reset, ps, p, lc);
+      emit = logic_path(J.pp, reset, ps, p, lc, mask);
       if (emit == 0) {
         if (jp.y + 1 < J.n_pass && !J.cancelled) {   // next pass of the same pixel
           start_pass(J, jp.x, ps.misc[p].y, jp.y + 1, p, ps, job_pass);

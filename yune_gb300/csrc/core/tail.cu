@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
         ps.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
         ++rays_e;
       }
-      const int emit = logic_path(pp, pp.reset, ps, p, lc);
+      const int emit = logic_path(pp, pp.reset, ps, p, lc, __activemask());
       if (emit == 0) break;
       any = emit == 2;
     }

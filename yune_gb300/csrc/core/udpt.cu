@@ -85,9 +85,10 @@ __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps,
     int emit = 0;
     int p = -1;
     LogicCounts lc;
+    const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
       p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
-      emit = logic_path(pp, pp.reset, ps, p, lc);
+      emit = logic_path(pp, pp.reset, ps, p, lc, mask);
     }
     // compaction: ballot + popc prefix per queue, one atomic per warp and queue
     const unsigned mc = __ballot_sync(0xffffffffu, emit == 1);

@@ -32,6 +32,20 @@ struct Vtx {
   int mat;
 };
 
+// The device copy of a quad light carries in its padding three values that depend on the
+// light alone, computed once on the host by the same operations (prepare_light): the
+// lengths of its edges and of its emission.
+inline void prepare_light(yc_quad_light& L) {
+  auto f = [](const yc_float4& v) { return ym::mk(v.x, v.y, v.z, v.w); };
+  L.pad[0] = ym::length(f(L.edge_l));
+  L.pad[1] = ym::length(f(L.edge_w));
+  L.pad[2] = ym::length(f(L.ke));
+}
+__device__ __forceinline__ float light_len_l(const yc_quad_light& L) { return L.pad[0]; }
+__device__ __forceinline__ float light_len_w(const yc_quad_light& L) { return L.pad[1]; }
+__device__ __forceinline__ float light_len_ke(const yc_quad_light& L) { return L.pad[2]; }
+__device__ __forceinline__ float light_area(const yc_quad_light& L) { return ym::mul(light_len_l(L), light_len_w(L)); }
+
 // the analytic quad-light loop of traceRay (udpt.cl:244-276); updates len and the hit light
 __device__ __forceinline__ void light_test(const DevScene& sc, f4 o, f4 d, float& len, int& light) {
   for (int i = 0; i < sc.n_lights; ++i) {
@@ -47,7 +61,7 @@ __device__ __forceinline__ void light_test(const DevScene& sc, f4 o, f4 d, float
         const f4 el = ld4(L.edge_l), ew = ld4(L.edge_w);
         float p1 = ym::dot(temp, el);
         float p2 = ym::dot(temp, ew);
-        const float la = ym::length(el), lb = ym::length(ew);
+        const float la = light_len_l(L), lb = light_len_w(L);
         p1 = ym::div(p1, la);
         p2 = ym::div(p2, lb);
         if ((p1 >= 0.0f && p2 >= 0.0f) && (p1 <= la && p2 <= lb)) {
@@ -110,38 +124,40 @@ __device__ __forceinline__ f4 to_world(f4 Nx, f4 Ny, f4 Nz, f4 p, f4 d) {
   return ym::normalize(o);
 }
 
-// phongSampleHemisphere, udpt.cl:700-771 (direction and pdf; origin = hp + dir * EPS)
-__device__ __forceinline__ f4 sample_phong(const Vtx& v, const yc_material& m, f4 w_i, uint32_t& seed, float& pdf) {
-  const f4 Nz = ym::normalize(reflect(w_i, v.n));
+// A direction around the axis Nz (phongSampleHemisphere, udpt.cl:700-771, and
+// cosineWeightedHemisphere, udpt.cl:843-910, differ in the axis, the polar angle and the
+// density): one code for both, so that lanes with either lobe run it together. `lobe`: the
+// modified Phong lobe of exponent pe around Nz; otherwise the cosine lobe, Nz = v.n.
+__device__ __forceinline__ f4 sample_around(const Vtx& v, f4 Nz, bool lobe, int pe, uint32_t& seed, float& pdf) {
   f4 Nx, Ny;
   frame(Nz, Nx, Ny);
   const float r1 = draw(seed);
   const float r2 = draw(seed);
-  const int pe = (int)ym::add(m.px, m.py);
   const float phi = ym::mul(ym::mul(2.0f, PI_F), r2);
-  const float ct = ym::pow(r1, ym::div(1.0f, (float)(pe + 1)));
-  float st = ym::sub(1.0f, ym::pow(r1, ym::div(2.0f, (float)(pe + 1))));
-  st = ym::sqrt(st);
-  const f4 d = ym::mk(ym::mul(st, ym::cos(phi)), ym::mul(st, ym::sin(phi)), ct, 0.0f);
-  const f4 dir = to_world(Nx, Ny, Nz, v.hp, d);
-  if (ym::dot(dir, v.n) < 0.0f) pdf = 0.0f;
+  float st, ct;
+  if (lobe) {
+    ct = ym::pow(r1, ym::rcp((float)(pe + 1)));
+    st = ym::sqrt(ym::sub(1.0f, ym::pow(r1, ym::div(2.0f, (float)(pe + 1)))));
+  } else {
+    st = ym::sqrt(r1);
+    ct = ym::sqrt(ym::sub(1.0f, r1));
+  }
+  float sn, cs;
+  ym::sincos(phi, sn, cs);
+  const f4 dir = to_world(Nx, Ny, Nz, v.hp, ym::mk(ym::mul(st, cs), ym::mul(st, sn), ct, 0.0f));
+  if (!lobe) pdf = ym::mul(ct, INV_PI_F);
+  else if (ym::dot(dir, v.n) < 0.0f) pdf = 0.0f;
   else pdf = (float)((double)(pe + 1) * 0.5 * (double)INV_PI_F * (double)ym::pow(ct, (float)pe));
   return dir;
 }
-
-// cosineWeightedHemisphere, udpt.cl:843-910
 __device__ __forceinline__ f4 sample_cosine(const Vtx& v, uint32_t& seed, float& pdf) {
-  f4 Nx, Ny;
-  frame(v.n, Nx, Ny);
-  const float r1 = draw(seed);
-  const float r2 = draw(seed);
-  const float phi = ym::mul(ym::mul(2.0f, PI_F), r2);
-  const float sT = ym::sqrt(r1);
-  const float z = ym::sqrt(ym::sub(1.0f, r1));
-  const f4 d = ym::mk(ym::mul(sT, ym::cos(phi)), ym::mul(sT, ym::sin(phi)), z, 0.0f);
-  const f4 dir = to_world(Nx, Ny, v.n, v.hp, d);
-  pdf = ym::mul(z, INV_PI_F);
-  return dir;
+  return sample_around(v, v.n, false, 0, seed, pdf);
+}
+// the diffuse or the glossy lobe of m seen from w_i (direction and pdf; origin = hp + dir * EPS)
+__device__ __forceinline__ f4 sample_lobe(const Vtx& v, const yc_material& m, bool glossy, f4 w_i, uint32_t& seed,
+                                          float& pdf) {
+  const f4 Nz = glossy ? ym::normalize(reflect(w_i, v.n)) : v.n;
+  return sample_around(v, Nz, glossy, (int)ym::add(m.px, m.py), seed, pdf);
 }
 
 // calcPhongPDF, udpt.cl:1033-1045
@@ -222,11 +238,11 @@ __device__ __forceinline__ f4 oren_nayar(f4 w_i, f4 w_o, const Vtx& v, const yc_
 // brdf_model = 1, udpt-primitives.cl:673-686; on_ab: the scene's per-material A and B)
 __device__ __forceinline__ f4 brdf(f4 w_i, f4 w_o, const Vtx& v, const yc_material& m, bool glossy, float rr_prob,
                                    int brdf_model, const float2* on_ab) {
-  const f4 refl = ym::normalize(reflect(w_i, v.n));
   if (!glossy) {
     if (brdf_model == 1 && rr_prob == 1.0f) return oren_nayar(w_i, w_o, v, m, on_ab[v.mat]);
     return (ld4(m.kd) * INV_PI_F) / rr_prob;
   }
+  const f4 refl = ym::normalize(reflect(w_i, v.n));
   const float ca = ym::pow(ym::fmax(ym::dot(w_o, refl), 0.0f), ym::add(m.px, m.py));
   const int pe = (int)ym::add(m.px, m.py);
   return ((((ld4(m.ks) * ca) * (float)(pe + 2)) * INV_PI_F) * 0.5f) / rr_prob;
@@ -253,14 +269,14 @@ __device__ __forceinline__ int sample_lights(const DevScene& sc, const Vtx& v, u
     const f4 ln = ld4(L.normal);
     const float cf = ym::mul(ym::max(ym::dot(t, v.n), 0.0f), ym::max(ym::dot(-t, ln), 0.0f));
     if (cf <= 0.0f) continue;
-    const float area = ym::mul(ym::length(ld4(L.edge_l)), ym::length(ld4(L.edge_w)));
+    const float area = light_area(L);
     if (n == 1) {
       w_i = ti;
-      light_pdf = ym::div(1.0f, area);
+      light_pdf = ym::rcp(area);
       light_pdf = ym::mul(light_pdf, ym::div(distance, ym::fmax(ym::dot(-t, ln), 0.0f)));
       return i;
     }
-    sum = ym::add(sum, ym::div(ym::mul(ym::mul(ym::length(ld4(L.ke)), cf), area), distance));
+    sum = ym::add(sum, ym::div(ym::mul(ym::mul(light_len_ke(L), cf), area), distance));
   }
   if (sum == 0.0f) return -1;
   const float r1 = draw(seed);
@@ -276,8 +292,8 @@ __device__ __forceinline__ int sample_lights(const DevScene& sc, const Vtx& v, u
     t = ym::normalize(t);
     const f4 ln = ld4(L.normal);
     const float cf = ym::mul(ym::max(ym::dot(t, v.n), 0.0f), ym::max(ym::dot(-t, ln), 0.0f));
-    const float area = ym::mul(ym::length(ld4(L.edge_l)), ym::length(ld4(L.edge_w)));
-    const float weight = cf <= 0.0f ? 0.0f : ym::div(ym::mul(ym::mul(ym::length(ld4(L.ke)), cf), area), distance);
+    const float area = light_area(L);
+    const float weight = cf <= 0.0f ? 0.0f : ym::div(ym::mul(ym::mul(light_len_ke(L), cf), area), distance);
     const float wgt = ym::div(weight, sum);
     if (r1 >= cum && r1 < ym::add(cum, wgt)) {
       w_i = ti;
@@ -301,24 +317,12 @@ __device__ __forceinline__ f4 brdf_b(f4 w_i, f4 w_o, f4 n, const yc_material& m,
   return ((((ld4(m.ks) * ca) * (float)(pe + 2)) * INV_PI_F) * 0.5f) / rr_prob;
 }
 
-// phongSampleHemisphere, bdpt.cl:807-870: lobe axis without the normal flip
-__device__ __forceinline__ f4 sample_phong_b(const Vtx& v, const yc_material& m, f4 w_i, uint32_t& seed, float& pdf) {
-  f4 Nz = ym::mul(2.0f, ym::dot(w_i, v.n)) * v.n - w_i;
-  Nz = ym::normalize(Nz);
-  f4 Nx, Ny;
-  frame(Nz, Nx, Ny);
-  const float r1 = draw(seed);
-  const float r2 = draw(seed);
-  const int pe = (int)ym::add(m.px, m.py);
-  const float phi = ym::mul(ym::mul(2.0f, PI_F), r2);
-  const float ct = ym::pow(r1, ym::div(1.0f, (float)(pe + 1)));
-  float st = ym::sub(1.0f, ym::pow(r1, ym::div(2.0f, (float)(pe + 1))));
-  st = ym::sqrt(st);
-  const f4 d = ym::mk(ym::mul(st, ym::cos(phi)), ym::mul(st, ym::sin(phi)), ct, 0.0f);
-  const f4 dir = to_world(Nx, Ny, Nz, v.hp, d);
-  if (ym::dot(dir, v.n) < 0.0f) pdf = 0.0f;
-  else pdf = (float)((double)(pe + 1) * 0.5 * (double)INV_PI_F * (double)ym::pow(ct, (float)pe));
-  return dir;
+// the diffuse or the glossy lobe (phongSampleHemisphere, bdpt.cl:807-870: lobe axis
+// without the normal flip)
+__device__ __forceinline__ f4 sample_lobe_b(const Vtx& v, const yc_material& m, bool glossy, f4 w_i, uint32_t& seed,
+                                            float& pdf) {
+  const f4 Nz = glossy ? ym::normalize(ym::mul(2.0f, ym::dot(w_i, v.n)) * v.n - w_i) : v.n;
+  return sample_around(v, Nz, glossy, (int)ym::add(m.px, m.py), seed, pdf);
 }
 
 // sampleGlossyPdf, bdpt.cl:1048-1105: probabilities raised by (1 - max)/2, no absorption

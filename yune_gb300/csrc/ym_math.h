@@ -208,6 +208,20 @@ YM_HD float cos(float x) {
   }
 }
 
+// sin(x) and cos(x) of an angle with |x| <= 65536, from one reduction: the values of the
+// two functions above.
+YM_HD void sincos(float x, float& sn, float& cs) {
+  const float k = rint(mul(x, 0.636619746685028076171875f));
+  float r = fma(-k, 1.57079637050628662109375f, x);
+  r = fma(-k, -4.37113882867379300296306610107421875e-08f, r);
+  r = fma(-k, -1.71512451000588185767965542129220217e-15f, r);
+  const float s = sin_poly(r), c = cos_poly(r);
+  const int q = (int)k;
+  const float a = (q & 1) ? c : s, b = (q & 1) ? s : c;
+  sn = (q & 2) ? -a : a;
+  cs = ((q + 1) & 2) ? -b : b;
+}
+
 // ---- log2 / exp2 / pow ------------------------------------------------------------
 // log2(x) = e + 2*atanh(s)/ln2 with s = (m-1)/(m+1), m in [sqrt(1/2), sqrt(2)).
 YM_HD float log2_pos(float x) {      // x finite, > 0
@@ -326,7 +340,7 @@ YM_HD float length3(f4 a) { return sqrt(dot3(a, a)); }
 YM_HD f4 normalize(f4 a) {
   const float l2 = dot(a, a);
   if (l2 == 0.0f) return a;
-  const float inv = div(1.0f, sqrt(l2));
+  const float inv = rcp(sqrt(l2));
   return a * inv;
 }
 // OpenCL cross for float4: w of the result is 0.
