@@ -144,7 +144,10 @@ int yc_bvh_copy_nodes(yc_ctx* ctx, yc_bvh_node* nodes_host, int capacity);
  * links to the host). Synchronous. */
 int yc_refit_scene(yc_ctx* ctx, int scene_id, const yc_triangle* tris_host, int n_tri);
 int yc_release_scene(yc_ctx* ctx, int scene_id);
-/* bytes the scene holds on the device */
+/* bytes of the scene's arrays on the device (yc_scene_layout). Workspaces made from them
+ * beside these are not counted: a refit's, and the walk index of a tree-mode-1 scene (at most
+ * 128 bytes per interior node, usually 57; made when memory allows, the scene renders the same
+ * without it). */
 int yc_scene_bytes(yc_ctx* ctx, int scene_id, uint64_t* bytes);
 /* interior levels of the uploaded hierarchy (a traversal stack needs depth + 2 slots) */
 int yc_scene_depth(yc_ctx* ctx, int scene_id, int* depth);
@@ -465,14 +468,16 @@ enum {
   /* Traversal stack entries a walk may use in yc_render_pass(es) and
    * yc_render_pass_noalloc; 0 (default) = as many as the scene's hierarchy needs (its
    * depth + 2). A smaller bound shrinks the kernels' shared memory; a walk that reaches it
-   * fails the call with YC_E_OVERFLOW. Otherwise >= 3. */
+   * fails the call with YC_E_OVERFLOW. Otherwise >= 3. With a bound set the scene's own nodes
+   * are walked, not its walk index (whose walks stack other numbers of entries). */
   YC_OPT_STACK_LIMIT = 8,
   /* Walk-stack entries kept in shared memory by yc_render_pass(es)'s traversal (one launch
    * per round, YC_OPT_MIXED_TRACE); the deeper entries go to a spill area of the context in
    * global memory (allocated by the first pass that needs it). Fewer entries leave more of
    * each SM's L1 to the node and triangle fetches and more blocks per SM. 0 = 12 (the
-   * default); a value at or above the scene's stack depth keeps the whole stack in shared
-   * memory. yc_render_pass_noalloc keeps the whole stack there (it allocates nothing). The
+   * default); a value at or above the entries a walk can need (yc_scene_depth + 2 over the
+   * scene's own nodes, up to half as many more over its walk index) keeps the whole stack in
+   * shared memory. yc_render_pass_noalloc keeps the whole stack there (it allocates nothing). The
    * batch engine has its own setting (yc_batch_cfg.stack_smem). */
   YC_OPT_STACK_SMEM = 9,
   /* Where yc_upload_scene repacks a scene for YC_OPT_TREE 1: 1 (default) on the device

@@ -25,7 +25,7 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off,-fno-fa
 
 CU_SOURCES = ["core/api.cu", "core/trace.cu", "core/udpt.cu", "core/bench_kernels.cu", "core/noalloc.cu", "core/bdpt.cu",
               "core/engine.cu", "core/tail.cu", "core/raysort.cu", "core/bvh_build.cu", "core/bdpt_mis.cu", "core/refit.cu",
-              "core/repack_dev.cu"]
+              "core/repack_dev.cu", "core/widen.cu"]
 CXX_SOURCES = ["core/repack.cpp", "core/serve.cpp", "core/walk_host.cpp", "core/tune.cpp", "host/yh_bvh.cpp", "host/yh_camera.cpp", "host/yh_scene.cpp", "host/yh_image.cpp",
                "host/yh_cache.cpp", "host/yh_threads.cpp"]
 HEADERS = ["ym_math.h", "core/yc_scene.h", "core/yc_internal.h", "core/yc_traverse.cuh", "core/yc_shade.cuh",

@@ -89,7 +89,23 @@ struct Scene {
   DevBuf<yc_triangle> refit_tris;
   DevBuf<float4> refit_root;
   size_t n_node4 = 0, n_tri4 = 0, n_shade4 = 0;   // float4 records of the repacked arrays
+  // the four-child walk index over dev's two-child nodes (widen.cu); none for scenes without
+  // interior nodes, in the other tree modes, and when there was no memory for it. It is a
+  // derived array like the refit's: `bytes` does not count it.
+  DevBuf<float4> windex;
+  int windex_nodes = 0, windex_depth = 0;   // its nodes; stack entries a walk over it can need
 };
+
+// the scene as the traversal kernels walk it: over its index where it has one
+yc::DevScene walk_scene(const Scene& s) {
+  yc::DevScene d = s.dev;
+  if (s.windex.p) {
+    d.nodes = s.windex.p;
+    d.wide = 1;
+    d.depth = s.windex_depth;
+  }
+  return d;
+}
 
 // the device copy of a scene's lights (yc::prepare_light)
 std::vector<yc_quad_light> prepared_lights(const yc_quad_light* lights, int n) {
@@ -314,6 +330,52 @@ Accum* find_accum(yc_ctx* c, int id) {
   return it == c->accums.end() ? nullptr : it->second.get();
 }
 
+// The walk index of a scene uploaded in tree mode 1. Hierarchies whose index would need more
+// stack than kWalkIndexMaxStack entries (chains of far deeper levels than a SAH tree has) keep
+// their two-child walk, and so do scenes the device has no memory left to index.
+constexpr int kWalkIndexMaxStack = 128;
+// Two steps around the upload's last synchronisation, which a small scene's index (one
+// launch) shares.
+int queue_walk_index(yc_ctx* c, Scene* s) {
+  const int n = (int)(s->n_node4 / 4);
+  if (!yc::widen_in_one_launch(n)) return 0;
+  cudaError_t e = s->windex.alloc((size_t)n * 8);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();   // not an error of the upload
+    return 0;
+  }
+  if (e == cudaSuccess) e = yc::widen_small(s->nodes.p, n, s->windex.p, c->q_work.p, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c->rc_host, c->q_work.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  YC_CUDA(e);
+  return 0;
+}
+int finish_walk_index(yc_ctx* c, Scene* s) {
+  const int n = (int)(s->n_node4 / 4);
+  int n_wide = 0, need = 0;
+  if (yc::widen_in_one_launch(n)) {
+    need = reinterpret_cast<const int*>(c->rc_host)[0];
+    n_wide = reinterpret_cast<const int*>(c->rc_host)[1];
+  } else {
+    DevBuf<int> tmp;
+    cudaError_t e = tmp.alloc(yc::widen_tmp_ints(n));
+    if (e == cudaSuccess) e = yc::widen_plan(s->nodes.p, n, tmp.p, n_wide, need, c->stream);
+    if (e == cudaSuccess) e = s->windex.alloc((size_t)n_wide * 8);
+    if (e == cudaSuccess) e = yc::widen_write(s->nodes.p, n, tmp.p, s->windex.p, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      s->windex.release();
+      return 0;
+    }
+    YC_CUDA(e);
+  }
+  if (need + 2 > kWalkIndexMaxStack) s->windex.release();
+  s->windex_nodes = n_wide;
+  s->windex_depth = need;
+  return 0;
+}
+
 int validate_cfg(const yc_pass_cfg* cfg) {
   if (!cfg) return fail(YC_E_INVALID, "cfg is NULL");
   if (cfg->integrator != YC_UDPT && cfg->integrator != YC_BDPT && cfg->integrator != YC_BDPT_MIS)
@@ -328,11 +390,13 @@ int validate_cfg(const yc_pass_cfg* cfg) {
 // accumulator, the tile of cfg->block (udpt.cl:166-167, src/RendererCore.cpp:146-150) and
 // the options the reference bakes into its kernel text. yc_render_pass and
 // yc_render_pass_noalloc both build their passes here. The scene's traversal depth is
-// capped by YC_OPT_STACK_LIMIT (a deeper walk then overflows and the call fails).
+// capped by YC_OPT_STACK_LIMIT (a deeper walk then overflows and the call fails); the limit
+// counts the entries of a walk over the scene's own nodes, so with one set those are walked,
+// as they are where the kernels keep the whole stack in shared memory (`indexed` false).
 yc::PassParams pass_params(const yc_ctx* c, const Scene* sc, const Accum* ac, uint32_t rand_seed, int reset,
-                           int gi_check, const yc_pass_cfg* cfg) {
+                           int gi_check, const yc_pass_cfg* cfg, bool indexed) {
   yc::PassParams pp{};
-  pp.sc = sc->dev;
+  pp.sc = indexed && c->stack_limit == 0 ? walk_scene(*sc) : sc->dev;
   if (c->stack_limit > 0) pp.sc.depth = std::min(pp.sc.depth, c->stack_limit - 2);
   pp.cam = c->cam;
   pp.accum = ac->buf.p;
@@ -385,7 +449,8 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
   const int W = ac->w, H = ac->h;
   int rc_ = ensure_paths(c, (size_t)W * H);
   if (rc_) return rc_;
-  const yc::PassParams pp = pass_params(c, sc, ac, rand_seed, reset, gi_check, cfg);
+  const bool mixed = c->mixed_trace != 0;
+  const yc::PassParams pp = pass_params(c, sc, ac, rand_seed, reset, gi_check, cfg, mixed);
   const yc::DevScene& dsc = pp.sc;   // the scene as the kernels walk it (stack limit applied)
   const yc::PathState ps = path_state(c);
   yc::BdptBuffers bb{};
@@ -413,7 +478,6 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
     else yc::launch_raygen(pp, ps, c->q[0].p, rc + 0, c->stats.p, c->stream);
   }
   YC_CUDA(cudaPeekAtLastError());
-  const bool mixed = c->mixed_trace != 0;
   // (a walk through a scene of a few thousand triangles is a handful of boxes: sorting
   // its rays costs more than it saves)
   const bool raysort = mixed && (c->rs_ob + c->rs_db) > 0 && c->rs_threshold > 0 &&
@@ -440,21 +504,23 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
                                                     : std::max((size_t)c->ss_threshold, kShadeSortMinPixels));
   if (shadesort)
     if (int e = ensure_shadesort(c, (size_t)W * H)) return e;
-  const int grid_c = yc::trace_grid_blocks(false, dsc.depth, dsc.wide != 0);
-  const int grid_a = yc::trace_grid_blocks(true, dsc.depth, dsc.wide != 0);
+  const int own_depth = c->stack_limit > 0 ? std::min(sc->dev.depth, c->stack_limit - 2) : sc->dev.depth;
+  const int grid_c = yc::trace_grid_blocks(false, own_depth, sc->dev.wide != 0);
+  const int grid_a = yc::trace_grid_blocks(true, own_depth, sc->dev.wide != 0);
   // the mixed trace's walk stacks: c->stack_smem entries in shared memory, the rest spilled
   const int cap = yc::trace_stack_cap(dsc.depth);
   const int n_smem = (mixed && c->stack_smem < cap) ? c->stack_smem : 0;   // 0: the whole stack
   const int grid_m = mixed ? yc::trace_mixed_grid_blocks(dsc.depth, dsc.wide != 0, n_smem) : 1;
-  if (n_smem > 0 && grid_m > 0)
-    if (int e = ensure_pass_spill(c, (size_t)grid_m * yc::TRACE_TB_PASS * 2 * (size_t)(cap - n_smem))) return e;
   if (grid_c <= 0 || grid_a <= 0 || grid_m <= 0)
     return fail(YC_E_LAUNCH, "trace kernel cannot be resident (stack too deep)");
   int tail_grid = 0, tail_at = 0;
   if (!bdpt && c->tail_paths != 0) {
-    const int capacity = yc::tail_capacity(dsc, &tail_grid);
+    const int capacity = yc::tail_capacity(dsc, n_smem, &tail_grid);
     tail_at = c->tail_paths < 0 ? capacity : std::min(c->tail_paths, capacity);
   }
+  if (n_smem > 0)
+    if (int e = ensure_pass_spill(c, (size_t)std::max(grid_m, tail_grid) * yc::TRACE_TB_PASS * 2 * (size_t)(cap - n_smem)))
+      return e;
   int cur = 0;
   const int check_every = 6;
   bool finished = false;
@@ -527,7 +593,8 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
     }
     if (tail_at > 0) {
       KTimer kt(c, K_TAIL);
-      if (yc::launch_tail(pp, ps, out_c, out_a, rout, tail_at, c->stats.p, tail_grid, c->stream))
+      if (yc::launch_tail(pp, ps, out_c, out_a, rout, tail_at, c->stats.p, tail_grid, c->stream, n_smem,
+                          n_smem > 0 ? c->pass_spill.p : nullptr))
         return fail(YC_E_LAUNCH, std::string("tail kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }
     YC_CUDA(cudaPeekAtLastError());
@@ -572,7 +639,7 @@ int yc_create(int device, yc_ctx** out) {
   if (e == cudaSuccess) e = c->stats.alloc(1);
   if (e == cudaSuccess) e = cudaMallocHost(&c->rc_host, sizeof(yc::RoundCounters));
   if (e == cudaSuccess) e = cudaMallocHost(&c->overflow_host, sizeof(unsigned long long));
-  if (e == cudaSuccess) e = c->q_work.alloc(1);
+  if (e == cudaSuccess) e = c->q_work.alloc(2);
   if (e == cudaSuccess) e = cudaMemset(c->stats.p, 0, sizeof(yc::DevStats));
   if (e != cudaSuccess) {
     yc_destroy(c);
@@ -682,7 +749,12 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
   const std::vector<yc_quad_light> dev_lights = prepared_lights(lights, n_light);
   YC_CUDA(cudaMemcpyAsync(s->lights.p, dev_lights.data(), n_light * sizeof(yc_quad_light), cudaMemcpyHostToDevice,
                           c->stream));
+  const bool index = c->tree_mode == yc::TREE_SAH_OVER_LEAVES && rp.root_link == 0 && rp.root_test != 0;
+  if (index)
+    if (int r = queue_walk_index(c, s.get())) return r;
   YC_CUDA(cudaStreamSynchronize(c->stream));
+  if (index)
+    if (int r = finish_walk_index(c, s.get())) return r;
   yc::DevScene& d = s->dev;
   d.nodes = s->nodes.p;
   d.tris = s->tris.p;
@@ -874,6 +946,7 @@ int yc_refit_scene(yc_ctx* c, int scene_id, const yc_triangle* tris, int n_tri) 
   if (yc::launch_refit(plan, s->refit_tris.p, n_tri, s->nodes.p, s->tris.p, n_slots, s->shade.p, s->dev.wide != 0,
                        s->dev.root_link, refit_nodes, s->refit_root.p, c->stream))
     return fail(YC_E_LAUNCH, std::string("refit: ") + cudaGetErrorString(cudaGetLastError()));
+  if (s->windex.p) YC_CUDA(yc::widen_boxes(s->nodes.p, s->windex.p, s->windex_nodes, c->stream));
   float4 root[2];
   if (refit_nodes && s->dev.root_link != yc::LINK_NONE)
     YC_CUDA(cudaMemcpyAsync(root, s->refit_root.p, sizeof root, cudaMemcpyDeviceToHost, c->stream));
@@ -1024,7 +1097,7 @@ int yc_render_pass_noalloc(yc_ctx* c, int scene_id, int accum_id, uint32_t rand_
   if (!c->have_cam) return fail(YC_E_INVALID, "no camera set");
   YC_CUDA(cudaSetDevice(c->device));
   yc::NoallocPass a{};
-  a.pp = pass_params(c, sc, ac, rand_seed, reset, gi_check, cfg);
+  a.pp = pass_params(c, sc, ac, rand_seed, reset, gi_check, cfg, false);
   a.stream = c->stream;
   a.stats = c->stats.p;
   a.rc_host = c->rc_host;
@@ -1059,11 +1132,20 @@ int yc_trace_device(yc_ctx* c, int scene_id, const float* rays_dev, int n, int a
   Scene* s = find_scene(c, scene_id);
   if (!s) return fail(YC_E_NOTFOUND, "unknown scene");
   if (n == 0) return YC_OK;
+  // (an any-hit query also reports the t of the triangle it met: the first one of the walk
+  // over the scene's own nodes)
+  const yc::DevScene sc = any_hit ? s->dev : walk_scene(*s);
+  const int cap = yc::trace_stack_cap(sc.depth), n_smem = c->stack_smem < cap ? c->stack_smem : 0;
+  const int grid = yc::trace_rays_grid_blocks(any_hit != 0, sc.depth, sc.wide != 0, n_smem);
+  if (grid <= 0) return fail(YC_E_LAUNCH, "trace kernel cannot be resident (stack too deep)");
+  if (n_smem > 0)
+    if (int r = ensure_pass_spill(c, (size_t)grid * yc::TRACE_TB_PASS * 2 * (size_t)(cap - n_smem))) return r;
   YC_CUDA(cudaMemsetAsync(c->q_work.p, 0, sizeof(int), c->stream));
   int e;
   {
     KTimer kt(c, any_hit ? K_OCCL : K_EXTEND);
-    e = yc::launch_trace_rays(s->dev, any_hit != 0, rays_dev, n, tri_dev, t_dev, c->q_work.p, c->stats.p, c->stream);
+    e = yc::launch_trace_rays(sc, any_hit != 0, rays_dev, n, tri_dev, t_dev, c->q_work.p, c->stats.p, grid, c->stream,
+                              n_smem, n_smem > 0 ? c->pass_spill.p : nullptr);
   }
   if (e) return fail(YC_E_LAUNCH, std::string("trace kernel: ") + cudaGetErrorString(cudaGetLastError()));
   return YC_OK;
@@ -1283,6 +1365,13 @@ struct yc_batch {
   int stack_smem = 0;   // walk stack entries in shared memory (the rest spill to BatchGroup::spill)
   size_t spill_slot = 0;   // ints of one launch's spill columns
   int wide = -1;   // node layout of the batch's scenes (-1: no job yet)
+  // Whether the kernels walk the scenes' four-child nodes: their own (layout 1), or, while
+  // every scene has one and fits stack_cap, their walk indexes. walk_cap: the entries of the
+  // walks' stacks (stack_cap bounds a walk over the scenes' own nodes).
+  bool indexed = true;
+  int walk_cap = 0, index_cap = 0;   // index_cap: the deepest index of the jobs so far, + 2
+  std::vector<yc::DevScene> job_dev;   // each job's scene with its own nodes
+  bool walks_wide() const { return wide == 1 || indexed; }
   int grid_c = 0, grid_a = 0, grid_m = 0, logic_grid = 0;
   bool mixed = true;   // YC_OPT_MIXED_TRACE of the context when the batch was created
   bool raysort = false;   // YC_OPT_RAY_SORT / _MIN of the context when the batch was created
@@ -1338,8 +1427,8 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
       yc::launch_raysort_batch(b->jobs.p, batch_state(b).job, in_c, in_a, rin, ps.ro, ps.rd, rsb, b->logic_grid, sm);
     }
     KTimer kt(c, K_TRACE, timed);
-    yc::launch_batch_trace_mixed(b->wide == 1, b->jobs.p, batch_state(b).job, in_c, in_a, rin, ps.ro, ps.rd, ps.hit,
-                                 c->stats.p, b->stack_cap, b->stack_smem, g.spill.p, b->grid_m, b->cfg.trace_block, sm,
+    yc::launch_batch_trace_mixed(b->walks_wide(), b->jobs.p, batch_state(b).job, in_c, in_a, rin, ps.ro, ps.rd, ps.hit,
+                                 c->stats.p, b->walk_cap, b->stack_smem, g.spill.p, b->grid_m, b->cfg.trace_block, sm,
                                  b->raysort ? rsb.sorted : nullptr,
                                  b->raysort ? rsb.ctl : nullptr);
   } else {
@@ -1350,14 +1439,14 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
     }
     {
       KTimer kt(c, K_EXTEND, timed);
-      yc::launch_batch_trace(false, b->wide == 1, b->jobs.p, batch_state(b).job, in_c, &rin->n_closest,
-                             &rin->work_closest, ps.ro, ps.rd, ps.hit, c->stats.p, b->stack_cap, b->stack_smem,
+      yc::launch_batch_trace(false, b->walks_wide(), b->jobs.p, batch_state(b).job, in_c, &rin->n_closest,
+                             &rin->work_closest, ps.ro, ps.rd, ps.hit, c->stats.p, b->walk_cap, b->stack_smem,
                              g.spill.p, b->grid_c, b->cfg.trace_block, sm);
     }
     {
       KTimer kt(c, K_OCCL, timed);
-      yc::launch_batch_trace(true, b->wide == 1, b->jobs.p, batch_state(b).job, in_a, &rin->n_any, &rin->work_any, ps.ro,
-                             ps.rd, ps.hit, c->stats.p, b->stack_cap, b->stack_smem,
+      yc::launch_batch_trace(true, b->walks_wide(), b->jobs.p, batch_state(b).job, in_a, &rin->n_any, &rin->work_any, ps.ro,
+                             ps.rd, ps.hit, c->stats.p, b->walk_cap, b->stack_smem,
                              g.spill.p ? g.spill.p + b->spill_slot : nullptr, b->grid_a, b->cfg.trace_block, sa);
     }
     if (!serial) {
@@ -1409,6 +1498,48 @@ int batch_body(yc_batch* b, bool timed) {
   return 0;
 }
 
+// launch shapes and stack spill areas of the traversal kernels for the nodes they walk
+int batch_shape(yc_batch* b) {
+  yc_ctx* c = b->ctx;
+  const bool wide = b->walks_wide();
+  // (walks over indexes: room for scenes added later, as deep as stack_cap admits)
+  b->walk_cap = b->indexed && b->wide != 1 ? std::max(b->index_cap, b->stack_cap + b->stack_cap / 2) : b->stack_cap;
+  b->stack_smem = std::min(b->walk_cap, b->cfg.stack_smem);
+  b->grid_c = yc::batch_trace_grid(false, b->stack_smem, wide, b->cfg.trace_block);
+  b->grid_a = yc::batch_trace_grid(true, b->stack_smem, wide, b->cfg.trace_block);
+  b->grid_m = yc::batch_trace_mixed_grid(b->stack_smem, wide, b->cfg.trace_block);
+  // trace_share: a persistent grid of that share of the resident blocks (at least one per
+  // SM) leaves each SM room for the other groups' kernels
+  if (b->cfg.trace_share < 100 && b->grid_m > 0)
+    b->grid_m = std::max(c->sm_count, (int)((int64_t)b->grid_m * b->cfg.trace_share / 100));
+  if (b->grid_c <= 0 || b->grid_a <= 0 || b->grid_m <= 0)
+    return fail(YC_E_LAUNCH, "batch trace kernel cannot be resident");
+  if (b->stack_smem < b->walk_cap) {
+    const size_t threads = (size_t)std::max({b->grid_c, b->grid_a, b->grid_m}) * b->cfg.trace_block;
+    b->spill_slot = threads * 2 * (size_t)(b->walk_cap - b->stack_smem);
+    for (auto& g : b->groups) YC_CUDA(g->spill.alloc(2 * b->spill_slot));
+  }
+  return 0;
+}
+
+// From here on the batch walks its scenes' own nodes: a scene without an index was added, one
+// deeper than the stacks of a running batch hold, or one that stack_cap does not hold. Called
+// between launches.
+int batch_unindex(yc_batch* b) {
+  yc_ctx* c = b->ctx;
+  b->indexed = false;
+  for (size_t i = 0; i < b->host_jobs.size(); ++i) b->host_jobs[i].pp.sc = b->job_dev[i];
+  if (!b->host_jobs.empty())
+    YC_CUDA(cudaMemcpyAsync(b->jobs.p, b->host_jobs.data(), b->host_jobs.size() * sizeof(yc::BatchJob),
+                            cudaMemcpyHostToDevice, c->stream));
+  YC_CUDA(cudaStreamSynchronize(c->stream));
+  if (b->exec) cudaGraphExecDestroy(b->exec);
+  if (b->graph) cudaGraphDestroy(b->graph);
+  b->exec = nullptr;
+  b->graph = nullptr;
+  return b->started ? batch_shape(b) : 0;
+}
+
 int batch_launch(yc_batch* b) {
   yc_ctx* c = b->ctx;
   if (b->cfg.use_graph) {
@@ -1440,6 +1571,7 @@ int yc_batch_create(yc_ctx* c, const yc_batch_cfg* cfg, yc_batch** out) {
   if (!b) return fail(YC_E_NOMEM, "host allocation failed");
   b->ctx = c;
   b->mixed = c->mixed_trace != 0;
+  b->indexed = b->mixed;   // (one launch per ray kind keeps walking the scenes' own nodes)
   b->rs_ob = c->rs_ob;
   b->rs_db = c->rs_db;
   b->rs_threshold = c->rs_threshold;
@@ -1550,11 +1682,21 @@ int yc_batch_add_job(yc_batch* b, int scene_id, int accum_id, const yc_cam* cam,
   if (!b->started) b->stack_cap = std::max(b->stack_cap, b->cfg.stack_cap > 0 ? b->cfg.stack_cap : need_cap);
   else if (need_cap > b->stack_cap)
     return fail(YC_E_INVALID, "scene BVH deeper than the running batch's traversal stack");
+  if (b->indexed && sc->dev.wide == 0) {
+    // (a scene without interior nodes is walked alike by both kernels)
+    const bool has = sc->windex.p || sc->dev.root_link < 0 || sc->dev.root_link == yc::LINK_NONE;
+    const int index_cap = sc->windex.p ? yc::trace_stack_cap(sc->windex_depth) : 0;
+    if (!has || need_cap > b->stack_cap || (b->started && index_cap > b->walk_cap)) {
+      if (int r = batch_unindex(b)) return r;
+    } else if (!b->started) {
+      b->index_cap = std::max(b->index_cap, index_cap);
+    }
+  }
   std::unique_ptr<DevBuf<uint32_t>> sd(new DevBuf<uint32_t>);
   YC_CUDA(sd->alloc(n_pass));
   YC_CUDA(cudaMemcpyAsync(sd->p, seeds, n_pass * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
   yc::BatchJob j{};
-  j.pp.sc = sc->dev;
+  j.pp.sc = b->indexed && sc->dev.wide == 0 ? walk_scene(*sc) : sc->dev;
   j.pp.cam = *cam;
   j.pp.accum = ac->buf.p;
   j.pp.width = ac->w;
@@ -1589,6 +1731,7 @@ int yc_batch_add_job(yc_batch* b, int scene_id, int accum_id, const yc_cam* cam,
   YC_CUDA(cudaMemcpyAsync(&b->tasks.p->task_total, &tt, sizeof(tt), cudaMemcpyHostToDevice, c->stream));
   YC_CUDA(cudaStreamSynchronize(c->stream));
   b->host_jobs.push_back(j);
+  b->job_dev.push_back(sc->dev);
   b->seeds.push_back(std::move(sd));
   b->wide = sc->dev.wide;
   *job_id = id;
@@ -1601,21 +1744,7 @@ int yc_batch_run(yc_batch* b, int max_launches, int* unfinished) {
   YC_CUDA(cudaSetDevice(c->device));
   if (!b->started) {
     if (b->stack_cap <= 0) b->stack_cap = b->cfg.stack_cap > 0 ? b->cfg.stack_cap : 32;
-    b->stack_smem = std::min(b->stack_cap, b->cfg.stack_smem);
-    b->grid_c = yc::batch_trace_grid(false, b->stack_smem, b->wide == 1, b->cfg.trace_block);
-    b->grid_a = yc::batch_trace_grid(true, b->stack_smem, b->wide == 1, b->cfg.trace_block);
-    b->grid_m = yc::batch_trace_mixed_grid(b->stack_smem, b->wide == 1, b->cfg.trace_block);
-    // trace_share: a persistent grid of that share of the resident blocks (at least one per
-    // SM) leaves each SM room for the other groups' kernels
-    if (b->cfg.trace_share < 100 && b->grid_m > 0)
-      b->grid_m = std::max(c->sm_count, (int)((int64_t)b->grid_m * b->cfg.trace_share / 100));
-    if (b->grid_c <= 0 || b->grid_a <= 0 || b->grid_m <= 0)
-      return fail(YC_E_LAUNCH, "batch trace kernel cannot be resident");
-    if (b->stack_smem < b->stack_cap) {
-      const size_t threads = (size_t)std::max({b->grid_c, b->grid_a, b->grid_m}) * b->cfg.trace_block;
-      b->spill_slot = threads * 2 * (size_t)(b->stack_cap - b->stack_smem);
-      for (auto& g : b->groups) YC_CUDA(g->spill.alloc(2 * b->spill_slot));
-    }
+    if (int r = batch_shape(b)) return r;
     b->started = true;
   }
   if (int r = begin_call_checks(c)) return r;

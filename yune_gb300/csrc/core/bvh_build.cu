@@ -472,6 +472,13 @@ struct Buf {
 
 }  // namespace
 
+void launch_exclusive_scan(const int* in, int* out, int* tile_sum, int n, cudaStream_t s) {
+  const int tiles = (n + 1023) / 1024;
+  k_scan_tiles<<<tiles, 1024, 0, s>>>(in, out, tile_sum, n);
+  k_scan_sums<<<1, 1024, 0, s>>>(tile_sum, tiles);
+  k_scan_add<<<tiles, 1024, 0, s>>>(out, tile_sum, n);
+}
+
 cudaError_t bvh_build_device(const yc_triangle* tris_dev, int n, int bins, int leaf_max, cudaStream_t s,
                              std::vector<yc_bvh_node>& out, int& depth, bool& too_deep) {
   out.clear();

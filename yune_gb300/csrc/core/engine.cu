@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(TRACE_TB_MAX) k_batch_trace(const BatchJob* jo
                                                           SF<float4> rd, SF<float4> hit, int stack_cap,
                                                           DevStats* st, int n_smem, int* spill) {
   BatchSrc<ANY> src{jobs, job_pass, queue, ro, rd, hit};
-  trace_loop<ANY, WIDE>(src, *count, work, stack_cap, st, n_smem, spill);
+  trace_loop<ANY, WIDE, false>(src, *count, work, stack_cap, st, n_smem, spill);
 }
 
 // both queues of a round: closest-hit entries first, then any-hit (or the sorted list,
@@ -481,9 +481,11 @@ struct BatchMixedSrc {
 // At most 64 registers a thread (four blocks of 256 or eight of 128 threads per SM): with
 // the walk stack mostly outside shared memory (stack_smem) the traversal is bound by the
 // latency of its node and triangle fetches, and the extra warps hide more of it than the
-// few spilled registers cost (measured on the mixed workload: +4% over 78 registers).
+// few spilled registers cost (measured on the mixed workload: +4% over 78 registers). Over
+// four-child nodes 72 to 80 registers (seven or six blocks of 128): at 64 the kernel spills
+// 72 bytes a thread in its inner loops (a batch of eight mixed jobs 82.7 against 78.9 ms).
 template <bool WIDE>
-__global__ void __launch_bounds__(TRACE_TB_MAX, 4) k_batch_trace_mixed(const BatchJob* jobs, SF<int4> job_pass,
+__global__ void __launch_bounds__(TRACE_TB_MAX, WIDE ? 3 : 4) k_batch_trace_mixed(const BatchJob* jobs, SF<int4> job_pass,
                                                                 const int* __restrict__ q_closest,
                                                                 const int* __restrict__ q_any,
                                                                 RoundCounters* rc, SF<float4> ro,

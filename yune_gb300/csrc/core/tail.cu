@@ -3,9 +3,17 @@
 // A pass's last rounds carry few paths (long glass and mirror paths survive Russian
 // roulette), and a round of the wavefront then lasts as long as its slowest ray: the GPU
 // waits on one latency-bound walk per round while almost all of it idles. Once the paths
-// left fit in one resident launch, k_tail gives each of them a thread that runs the same
+// left fit in one resident launch, k_tail gives each of them a lane that runs the same
 // steps in turn -- walk the pending ray, store the hit, advance the state machine
-// (logic_path) -- until the path writes its pixel. Every path computes exactly what the
+// (logic_path) -- until the path writes its pixel. A warp's lanes walk together, the kind of
+// step more of them can take at a time, and run their state machines together once every
+// lane's ray is answered: the state machine's time is that of its code, whose phases a warp
+// runs one after another whatever the lanes in them (25-65 thousand cycles a step), so the
+// fewer runs the better (run when half the lanes wait: 1.65 ms against 1.40 ms on the glass
+// sphere). With each lane on its own the kernel ran 3.5 lanes per instruction: 1.74 ms
+// there, 1.10 ms now; 1.10 against 0.57 ms for a 256x256 frame of the Cornell box. What
+// bounds it is the longest chain of rays in a warp (12-25), at 600-1600 cycles a step of a
+// walk. Every path computes exactly what the
 // round-by-round wavefront computes (same state, same operations), so the pass's result
 // is unchanged; paths no longer wait for each other between rays.
 // The kernel is launched after every round's logic kernel on that round's output
@@ -15,7 +23,7 @@
 #include <cuda_runtime.h>
 
 #include "yc_internal.h"
-#include "yc_traverse.cuh"
+#include "yc_trace_loop.cuh"
 #include "yc_udpt.cuh"
 
 namespace yc {
@@ -25,65 +33,82 @@ constexpr int TAIL_TB = 128;
 // path that reaches it is left unfinished and counted in DevStats::stack_overflow
 constexpr int TAIL_MAX_RAYS = 1 << 22;
 
-template <bool ANY, bool WIDE>
-__device__ __forceinline__ HitOut walk_full(const DevScene& sc, const float4& o, const float4& d, int* stack,
-                                            int stack_cap, WalkCount& wc, unsigned& overflow) {
-  const RayIn r{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
-  Walk w;
-  walk_begin(sc, r, w);
-  bool of = false;
-  bool done = w.link == LINK_NONE;
-  const WalkStack ws{stack, nullptr, TAIL_TB, 0, stack_cap, stack_cap};
-  while (!done) done = walk_step<ANY, WIDE>(w, ws, wc, of);
-  if (of) ++overflow;
-  HitOut h;
-  h.t = w.best; h.u = w.bu; h.v = w.bv; h.tri = w.best_tri;
-  return h;
-}
-
 // three blocks per SM: up to 170 registers a thread, which the kernel needs without spills
 template <bool WIDE>
 __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps, const int* __restrict__ in_closest,
                                                   const int* __restrict__ in_any, RoundCounters* rc_in,
-                                                  int threshold, int stack_cap, DevStats* st) {
-  extern __shared__ int smem[];
-  int* stack = smem + threadIdx.x;
+                                                  int threshold, int stack_cap, DevStats* st, int n_smem, int* spill) {
   __shared__ unsigned long long s_cnt[13];
   __shared__ bool s_last;
   const int nc = rc_in->n_closest, n = nc + rc_in->n_any;
   if (n == 0 || n > threshold) return;   // uniform over the grid
   if (threadIdx.x < 13) s_cnt[threadIdx.x] = 0;
   __syncthreads();
+  const WalkStack stack = thread_stack(stack_cap, n_smem, spill);
+  const int lane = threadIdx.x & 31;
+  const int warps = (int)(gridDim.x * (TAIL_TB / 32));
+  const int quota = min(32, (n + warps - 1) / warps);   // lanes of a warp that take paths
   LogicCounts lc;
-  WalkCount wce, wca;
-  unsigned rays_e = 0, rays_a = 0, overflow = 0;
+  WalkCount wc;              // the current ray's walk
+  unsigned overflow = 0;
+  Walk w;
+  w.link = LINK_NONE;
+  w.leaf = 0;
+  int p = -1, rays = 0;      // this lane's path, and the rays it has walked
+  bool any = false;
+  bool more = true;          // the queues may still hold paths (warp-uniform)
   for (;;) {
-    const int e = atomicAdd(&rc_in->work_logic, 1);
-    if (e >= n) break;
-    const int p = e < nc ? in_closest[e] : in_any[e - nc];
-    bool any = e >= nc;
-    for (int k = 0;; ++k) {
-      if (k == TAIL_MAX_RAYS) { ++overflow; break; }
-      const float4 o = ps.ro[p], d = ps.rd[p];
-      if (any) {
-        const HitOut h = walk_full<true, WIDE>(pp.sc, o, d, stack, stack_cap, wca, overflow);
-        ps.hit[p] = make_float4(h.tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f);
-        ++rays_a;
-      } else {
-        const HitOut h = walk_full<false, WIDE>(pp.sc, o, d, stack, stack_cap, wce, overflow);
-        ps.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
-        ++rays_e;
-      }
-      const int emit = logic_path(pp, pp.reset, ps, p, lc, __activemask());
-      if (emit == 0) break;
-      any = emit == 2;
+    const unsigned nodes = __ballot_sync(0xffffffffu, walk_wants_node(w));
+    const unsigned tris = __ballot_sync(0xffffffffu, walk_wants_tri(w));
+    const unsigned have = __ballot_sync(0xffffffffu, p >= 0);
+    const unsigned waiting = have & ~(nodes | tris);   // paths whose ray is answered
+    if (waiting != have) {
+      bool of = false;
+      warp_walk_step<WIDE>(w, any, stack, wc, of, nodes, tris);
+      if (of) ++overflow;
+      continue;
     }
+    bool ray = false;
+    if ((waiting >> lane) & 1u) {
+      unsigned long long* t = s_cnt + (any ? 9 : 6);
+      atomicAdd(t, 1ull);
+      atomicAdd(t + 1, (unsigned long long)wc.nodes);
+      atomicAdd(t + 2, (unsigned long long)wc.tris);
+      wc.nodes = 0; wc.tris = 0;
+      ps.hit[p] = any ? make_float4(w.best_tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f)
+                      : make_float4(w.best, w.bu, w.bv, __int_as_float(w.best_tri));
+      const int emit = logic_path(pp, pp.reset, ps, p, lc, waiting);
+      any = emit == 2;
+      ray = emit != 0;
+      if (ray && ++rays == TAIL_MAX_RAYS) { ++overflow; ray = false; }
+      if (!ray) p = -1;
+    }
+    if (more) {
+      const bool want = p < 0 && lane < quota;
+      const unsigned m = __ballot_sync(0xffffffffu, want);
+      int base = 0;
+      if (lane == 0 && m) base = atomicAdd(&rc_in->work_logic, __popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (m && base + __popc(m) >= n) more = false;
+      const int e = base + __popc(m & ((1u << lane) - 1));
+      if (want && e < n) {
+        p = e < nc ? in_closest[e] : in_any[e - nc];
+        any = e >= nc;
+        rays = 0;
+        ray = true;
+      }
+    }
+    if (ray) {
+      const float4 o = ps.ro[p], d = ps.rd[p];
+      walk_begin(pp.sc, RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z}, w);
+    }
+    if (!more && __ballot_sync(0xffffffffu, p >= 0) == 0) break;
   }
-  const unsigned long long v[13] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples,
-                                    rays_e, wce.nodes, wce.tris, rays_a, wca.nodes, wca.tris, overflow};
+  const unsigned long long v[6] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples};
 #pragma unroll
-  for (int q = 0; q < 13; ++q)
+  for (int q = 0; q < 6; ++q)
     if (v[q]) atomicAdd(&s_cnt[q], v[q]);
+  if (overflow) atomicAdd(&s_cnt[12], (unsigned long long)overflow);
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long* dst[13] = {&st->rays, &st->extension, &st->shadow, &st->mis, &st->traversed, &st->samples,
@@ -104,7 +129,8 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
   }
 }
 
-static size_t tail_smem(int cap) { return (size_t)TAIL_TB * 2 * cap * sizeof(int); }
+static size_t tail_smem(int n) { return (size_t)TAIL_TB * n * sizeof(int2); }
+static int tail_entries(int depth, int n_smem) { return n_smem > 0 && n_smem < depth + 2 ? n_smem : depth + 2; }
 
 template <class K>
 static int tail_grid_of(K kernel, size_t smem) {
@@ -116,21 +142,22 @@ static int tail_grid_of(K kernel, size_t smem) {
   return per_sm > 0 ? per_sm * sms : -1;
 }
 
-int tail_capacity(const DevScene& sc, int* grid_out) {
-  const size_t smem = tail_smem(sc.depth + 2);
+int tail_capacity(const DevScene& sc, int n_smem, int* grid_out) {
+  const size_t smem = tail_smem(tail_entries(sc.depth, n_smem));
   const int grid = sc.wide ? tail_grid_of(k_tail<true>, smem) : tail_grid_of(k_tail<false>, smem);
   if (grid_out) *grid_out = grid;
   return grid > 0 ? grid * TAIL_TB : 0;
 }
 
 int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_any,
-                RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s) {
+                RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s, int n_smem, int* spill) {
   const int cap = pp.sc.depth + 2;
-  const size_t smem = tail_smem(cap);
+  n_smem = tail_entries(pp.sc.depth, spill ? n_smem : 0);
+  const size_t smem = tail_smem(n_smem);
   if (pp.sc.wide)
-    k_tail<true><<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_any, rc_in, threshold, cap, st);
+    k_tail<true><<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_any, rc_in, threshold, cap, st, n_smem, spill);
   else
-    k_tail<false><<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_any, rc_in, threshold, cap, st);
+    k_tail<false><<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_any, rc_in, threshold, cap, st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -181,6 +181,20 @@ int launch_refit(const RefitPlan& plan, const yc_triangle* tris_dev, int n_tri, 
                  int n_slots, float4* shade, bool wide, int root_link, bool refit_nodes, float4* root_out,
                  cudaStream_t s);
 
+// widen.cu: the four-child walk index of a two-child hierarchy whose root is node 0. The
+// plan finds the wide nodes (their number, and the stack entries a walk over them can need)
+// in `tmp` (widen_tmp_ints ints), the write fills them in (8 float4 each), and after a refit of
+// the two-child nodes widen_boxes copies their boxes over again. A small hierarchy's index is
+// one launch: `wide` takes n_nodes nodes at most, ctl[0] the stack entries, ctl[1] the nodes.
+bool widen_in_one_launch(int n_nodes);
+cudaError_t widen_small(const float4* n2, int n_nodes, float4* wide, int* ctl, cudaStream_t s);
+size_t widen_tmp_ints(int n_nodes);
+cudaError_t widen_plan(const float4* n2, int n_nodes, int* tmp, int& n_wide, int& need, cudaStream_t s);
+cudaError_t widen_write(const float4* n2, int n_nodes, const int* tmp, float4* wide, cudaStream_t s);
+cudaError_t widen_boxes(const float4* n2, float4* wide, int n_wide, cudaStream_t s);
+// bvh_build.cu: exclusive scan of n ints; tile_sum: one int per 1024
+void launch_exclusive_scan(const int* in, int* out, int* tile_sum, int n, cudaStream_t s);
+
 // launchers (udpt.cu / trace.cu)
 void launch_raygen(const PassParams& pp, const PathState& ps, int* q_closest, RoundCounters* rc, DevStats* st,
                    cudaStream_t s);
@@ -195,12 +209,15 @@ int launch_trace(const DevScene& sc, bool any_hit, const int* queue, const int* 
                  cudaStream_t s);
 void launch_tonemap(const float4* in, float4* out, int n, cudaStream_t s);
 // tail.cu: finish a pass's paths one thread each once at most `threshold` are left
-int tail_capacity(const DevScene& sc, int* grid_out);
+int tail_capacity(const DevScene& sc, int n_smem, int* grid_out);
+// n_smem, spill: as for launch_trace_mixed (grid * TAIL_TB columns)
 int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_any,
-                RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s);
+                RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s, int n_smem, int* spill);
 // direct query: rays as 9 floats each
+// (n_smem, spill: as for launch_trace_mixed)
 int launch_trace_rays(const DevScene& sc, bool any_hit, const float* rays9, int n, int* tri_out, float* t_out,
-                      int* work, DevStats* st, cudaStream_t s);
+                      int* work, DevStats* st, int grid_blocks, cudaStream_t s, int n_smem, int* spill);
+int trace_rays_grid_blocks(bool any_hit, int depth, bool wide, int n_smem);
 int trace_grid_blocks(bool any_hit, int depth, bool wide);
 // one launch over both queues of a round (closest-hit entries, then any-hit); the work
 // cursor is rc->work_closest. n_smem (< the stack depth, with spill): walk-stack entries in

@@ -16,7 +16,8 @@
 //           udpt.cl:316).
 //           four-child layout (wide = 1): 8 x float4 (128 B) per node, the boxes of
 //           its four children as lo.x[4], hi.x[4], lo.y[4], hi.y[4], lo.z[4], hi.z[4],
-//           then the four links (LINK_NONE for an empty slot) and 16 unused bytes.
+//           then the four links (LINK_NONE for an empty slot) and 16 bytes that no walk
+//           reads (a walk index, widen.cu, keeps there where each box came from).
 //   tris    3 x float4 (48 B) per stream slot, leaves' triangles contiguous:
 //             (v1.xyz, original index), (e1 = v2 - v1, tie-break rank), (e2 = v3 - v1, 0)
 //           with the index and rank as int bits; the rank orders triangles at equal t

@@ -169,11 +169,9 @@ __device__ __forceinline__ bool tri_test(float ox, float oy, float oz, float dx,
   const float v = __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(qx, dx), __fmul_rn(qy, dy)), __fmul_rn(qz, dz)), 0.0f), inv_det);
   if (v < 0.0f || __fadd_rn(u, v) > 1.0f) return false;
   const float t = __fmul_rn(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(c.x, qx), __fmul_rn(c.y, qy)), __fmul_rn(c.z, qz)), 0.0f), inv_det);
-  if (t > 0.0f && (t < best || (t == best && __float_as_int(b.w) < best_rank))) {
-    out.t = t; out.u = u; out.v = v;
-    return true;
-  }
-  return false;
+  out.t = t; out.u = u; out.v = v;
+  const bool outside = (u < 0.0f) | (u > 1.0f) | (v < 0.0f) | (__fadd_rn(u, v) > 1.0f);
+  return !outside & (t > 0.0f) & ((t < best) | ((t == best) & (__float_as_int(b.w) < best_rank)));
 }
 
 // Cull factor for the distance test: a child is skipped when its entry distance exceeds
@@ -188,7 +186,9 @@ __device__ __forceinline__ float cull_up(float best) {
 // ---- resumable walk for the persistent kernels ----
 // The state of one ray's walk, so a warp can run its lanes' walks step by step and hand
 // a lane a new ray as soon as its walk ends (the replenishing persistent warps of Aila
-// and Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009).
+// and Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009). A walk
+// holds at most two pending subtrees beside its stack: `link`, the next one, and `leaf`,
+// a leaf met on the way whose triangles are still to be tested.
 struct Walk {
   const float4* nodes;   // the scene of this ray (lanes of one warp may walk different scenes)
   const float4* tris;
@@ -211,8 +211,9 @@ struct Walk {
   float best, bu, bv;
   float best_up;         // cull_up(best)
   int best_tri, best_rank;
-  int link, sp;
-  float link_t;          // entry distance of the subtree `link` (checked again before it is opened)
+  int link, sp;          // LINK_NONE: nothing left to open, LINK_POP: the stack's next; a leaf link waits for `leaf`
+  float link_t;          // entry distance of the subtree `link` (checked again when a hit shortens the ray)
+  int leaf;              // (stream slot << 4) | triangles left of the pending leaf; 0 in the low bits: none
   bool exact;
 };
 
@@ -229,6 +230,7 @@ __device__ __forceinline__ void walk_begin(const DevScene& sc, const RayIn& r, W
   w.best_up = cull_up(r.tmax);
   w.best_tri = -1; w.best_rank = -1;
   w.sp = 0;
+  w.leaf = 0;
   w.link = sc.root_link;
   w.link_t = -__int_as_float(0x7f800000);
   if (w.link != LINK_NONE && sc.root_test) {
@@ -239,82 +241,40 @@ __device__ __forceinline__ void walk_begin(const DevScene& sc, const RayIn& r, W
                                       sc.root_hi.y, sc.root_lo.z, sc.root_hi.z, __int_as_float(0x7f800000), false, te);
     if (!h) w.link = LINK_NONE;
   }
-}
-
-// Triangles of one leaf (the reference's vert_list run, yc_scene.h); returns true when
-// an any-hit walk (any = true) has found its hit.
-__device__ __forceinline__ bool walk_leaf(Walk& w, int link, WalkCount& wc, bool any) {
-  const int enc = ~link;
-  const int count = enc & 15;
-  const float4* tp = w.tris + 3 * (size_t)(enc >> 4);
-  for (int k = 0; k < count; ++k) {
-    ++wc.tris;
-    const float4 a = __ldg(tp + 3 * k + 0);
-    const float4 b = __ldg(tp + 3 * k + 1);
-    const float4 c = __ldg(tp + 3 * k + 2);
-    TriHit th;
-    if (tri_test(w.ox(), w.oy(), w.oz(), w.dx, w.dy, w.dz, a, b, c, w.best, w.best_rank, th)) {
-      w.best = th.t;
-      w.best_up = cull_up(th.t);
-      w.bu = th.u;
-      w.bv = th.v;
-      w.best_tri = __float_as_int(a.w);
-      w.best_rank = __float_as_int(b.w);
-      if (any) return true;
-    }
+  if (w.link < 0) {   // the whole scene is one leaf
+    w.leaf = ~w.link;
+    w.link = LINK_NONE;
   }
-  return false;
 }
 
 // A walk's stack of (subtree link, entry distance) pairs, at most `cap` deep: entries
 // [0, n_smem) in this thread's column of the block's shared memory (stride: the block
-// size), deeper ones in its column of a global spill area (stride: the grid's threads).
+// size), deeper ones in its column of a global spill area (stride: the grid's threads),
+// each entry one 64-bit word.
 // A short shared part leaves more of the SM's unified L1 and shared memory to the node
 // and triangle fetches; n_smem == cap (g unused) keeps the whole stack in shared memory.
 struct WalkStack {
-  int* s;
-  int* g;
+  int2* s;
+  int2* g;
   int stride, gstride, n_smem, cap;
   __device__ __forceinline__ void put(int i, int link, float t) const {
-    if (i < n_smem) {
-      s[(2 * i) * stride] = link;
-      s[(2 * i + 1) * stride] = __float_as_int(t);
-    } else {
-      const size_t j = (size_t)(2 * (i - n_smem)) * gstride;
-      g[j] = link;
-      g[j + gstride] = __float_as_int(t);
-    }
+    const int2 e = make_int2(link, __float_as_int(t));
+    if (i < n_smem) s[i * stride] = e;
+    else g[(size_t)(i - n_smem) * gstride] = e;
   }
-  __device__ __forceinline__ float t_at(int i) const {
-    return __int_as_float(i < n_smem ? s[(2 * i + 1) * stride] : g[(size_t)(2 * (i - n_smem) + 1) * gstride]);
-  }
-  __device__ __forceinline__ int link_at(int i) const {
-    return i < n_smem ? s[(2 * i) * stride] : g[(size_t)(2 * (i - n_smem)) * gstride];
+  __device__ __forceinline__ int2 at(int i) const {
+    return i < n_smem ? s[i * stride] : g[(size_t)(i - n_smem) * gstride];
   }
 };
 
-// pops the next subtree whose entry is still within reach (LINK_NONE: the walk ends)
-__device__ __forceinline__ int walk_pop(Walk& w, const WalkStack& st) {
-  while (w.sp > 0) {
-    --w.sp;
-    const float te = st.t_at(w.sp);
-    if (!(te > cull_bound(w.best))) {
-      w.link_t = te;
-      return st.link_at(w.sp);
-    }
-  }
-  return LINK_NONE;
-}
-
-// the pending subtree, unless a hit found since it was chosen puts it out of reach
-__device__ __forceinline__ int walk_recheck(Walk& w, int link, const WalkStack& st) {
-  if (link != LINK_NONE && w.link_t > cull_bound(w.best)) return walk_pop(w, st);
-  return link;
-}
+// The link of a walk that has to take its next subtree from the stack. Popping is left to
+// the next node step, so that a step has one place where lanes pop, together.
+constexpr int LINK_POP = LINK_NONE - 1;
+__device__ __forceinline__ int pop_link(const Walk& w) { return w.sp > 0 ? LINK_POP : LINK_NONE; }
 
 // One interior node of the two-child layout: returns the next node (the nearer child
-// hit, the other one pushed), or the next subtree popped from the stack when neither
-// child is hit. LINK_NONE: the walk is over (or the stack bound was reached).
+// hit, the other one pushed), or pop_link when neither child is hit. LINK_NONE: nothing
+// left to open (or the stack bound was reached).
 __device__ __forceinline__ int visit2(Walk& w, bool any, int link, const WalkStack& st, WalkCount& wc,
                                       bool& overflow) {
   const float4* nd = w.nodes + 4 * (size_t)link;
@@ -345,17 +305,16 @@ __device__ __forceinline__ int visit2(Walk& w, bool any, int link, const WalkSta
   }
   h0 = h0 && n3.x != LINK_NONE;
   h1 = h1 && n3.y != LINK_NONE;
-  if (h0 && h1) {
-    const bool swap = t1 < t0;
+  if (!(h0 || h1)) return pop_link(w);
+  const bool both = h0 && h1;
+  const bool second = both ? t1 < t0 : h1;   // the child to open next
+  if (both) {
     if (w.sp >= st.cap) { overflow = true; w.sp = 0; return LINK_NONE; }
-    st.put(w.sp, swap ? n3.x : n3.y, swap ? t0 : t1);
+    st.put(w.sp, second ? n3.x : n3.y, second ? t0 : t1);
     ++w.sp;
-    w.link_t = swap ? t1 : t0;
-    return swap ? n3.y : n3.x;
   }
-  if (h0) { w.link_t = t0; return n3.x; }
-  if (h1) { w.link_t = t1; return n3.y; }
-  return walk_pop(w, st);
+  w.link_t = second ? t1 : t0;
+  return second ? n3.y : n3.x;
 }
 
 // (t, link) compare-exchange: the smaller entry distance first
@@ -367,41 +326,51 @@ __device__ __forceinline__ void cx(float& ta, int& la, float& tb, int& lb) {
 }
 
 // One interior node of the four-child layout (yc_scene.h, wide nodes): the four child
-// boxes are tested with the reference's slab arithmetic, the hits sorted by entry
-// distance, the nearest returned and the others pushed farthest first.
+// boxes are tested with the reference's slab arithmetic, two children per packed
+// operation, the hits sorted by entry distance, the nearest returned and the others
+// pushed farthest first (pushed in any order, the walk visited more nodes: 3.97 against
+// 3.59 ms per 1080p pass of a 260K-triangle scene).
 __device__ __forceinline__ int visit4(Walk& w, bool any, int link, const WalkStack& st, WalkCount& wc,
                                       bool& overflow) {
   const float INF = __int_as_float(0x7f800000);
   const float4* nd = w.nodes + 8 * (size_t)link;
-  const float4 lx = __ldg(nd + 0), hx = __ldg(nd + 1);
-  const float4 ly = __ldg(nd + 2), hy = __ldg(nd + 3);
-  const float4 lz = __ldg(nd + 4), hz = __ldg(nd + 5);
-  const int4 ln = __ldg(reinterpret_cast<const int4*>(nd + 6));
+  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(nd);
   wc.nodes += 4;
-  const float cb = cull_bound(w.best);
   float t[4];
   int l[4];
-  const float clx[4] = {lx.x, lx.y, lx.z, lx.w}, chx[4] = {hx.x, hx.y, hx.z, hx.w};
-  const float cly[4] = {ly.x, ly.y, ly.z, ly.w}, chy[4] = {hy.x, hy.y, hy.z, hy.w};
-  const float clz[4] = {lz.x, lz.y, lz.z, lz.w}, chz[4] = {hz.x, hz.y, hz.z, hz.w};
-  const int cl[4] = {ln.x, ln.y, ln.z, ln.w};
+  const int4 ln = __ldg(reinterpret_cast<const int4*>(nd + 6));
+  l[0] = ln.x; l[1] = ln.y; l[2] = ln.z; l[3] = ln.w;
+  float a[3][4], b[3][4];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const ulonglong2 lo = __ldg(q + 2 * k), hi = __ldg(q + 2 * k + 1);
+    const f32x2 o = k == 0 ? w.ox2() : k == 1 ? w.oy2() : w.oz2();
+    const f32x2 i = k == 0 ? w.ix2() : k == 1 ? w.iy2() : w.iz2();
+    up2(mul2(sub2(lo.x, o), i), a[k][0], a[k][1]);
+    up2(mul2(sub2(lo.y, o), i), a[k][2], a[k][3]);
+    up2(mul2(sub2(hi.x, o), i), b[k][0], b[k][1]);
+    up2(mul2(sub2(hi.y, o), i), b[k][2], b[k][3]);
+  }
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     float te;
-    bool h = !w.exact ? box_fast(w.ox(), w.oy(), w.oz(), w.ix(), w.iy(), w.iz(), clx[c], chx[c], cly[c], chy[c], clz[c], chz[c],
-                                 w.best_up, !any, te)
-                      : box_ref(w.ox(), w.oy(), w.oz(), w.ix(), w.iy(), w.iz(), clx[c], chx[c], cly[c], chy[c], clz[c], chz[c], te);
-    h = h && cl[c] != LINK_NONE && !(te > cb);
+    bool h;
+    if (!w.exact) {
+      h = box_fast_ab(a[0][c], b[0][c], a[1][c], b[1][c], a[2][c], b[2][c], w.best_up, !any, te);
+    } else {
+      h = box_ref_ab(a[0][c], b[0][c], a[1][c], b[1][c], a[2][c], b[2][c], te);
+      h = h && !(te >= w.best_up);
+    }
+    h = h && l[c] != LINK_NONE;
     t[c] = h ? te : INF;
-    l[c] = h ? cl[c] : LINK_NONE;
+    l[c] = h ? l[c] : LINK_NONE;
   }
-  // sorting network for four entries; misses (t = inf, LINK_NONE) end up last
   cx(t[0], l[0], t[1], l[1]);
   cx(t[2], l[2], t[3], l[3]);
   cx(t[0], l[0], t[2], l[2]);
   cx(t[1], l[1], t[3], l[3]);
   cx(t[1], l[1], t[2], l[2]);
-  if (l[0] == LINK_NONE) return walk_pop(w, st);
+  if (l[0] == LINK_NONE) return pop_link(w);
   const int extra = (l[1] != LINK_NONE) + (l[2] != LINK_NONE) + (l[3] != LINK_NONE);
   if (w.sp + extra > st.cap) { overflow = true; w.sp = 0; return LINK_NONE; }
 #pragma unroll
@@ -415,50 +384,100 @@ __device__ __forceinline__ int visit4(Walk& w, bool any, int link, const WalkSta
   return l[0];
 }
 
-// One step of the walk, the while-while loop with postponed leaves of Aila and Laine
-// ("Understanding the Efficiency of Ray Traversal on GPUs", 2009, and its 2012
-// addendum): interior nodes are visited until every lane of the warp still walking has
-// reached a leaf; a lane that meets its first leaf keeps it aside and goes on with the
-// next subtree, so the lanes test triangles together instead of one after another.
-// Returns true when the walk has ended (w.link == LINK_NONE); `overflow` is set when the
-// stack bound was reached (the walk then ends early). Leaves are kept aside before the
-// hits inside them lower the culling distance, so the walk may open a few more boxes
-// than a leaf-first order would; it never skips one that can hold a closer hit.
-// `any` selects the any-hit walk (it stops at the first hit); callers that know the kind
-// at compile time use walk_step<ANY, WIDE>, the mixed trace loop passes it per lane.
-template <bool WIDE>
-__device__ __forceinline__ bool walk_step_k(Walk& w, bool any, const WalkStack& st, WalkCount& wc, bool& overflow) {
-  // (an any-hit walk keeps its segment length until it stops: nothing to check again)
-  int link = any ? w.link : walk_recheck(w, w.link, st);
-  int leaf = LINK_NONE;
-  while (link >= 0 && link != LINK_NONE) {
-    link = WIDE ? visit4(w, any, link, st, wc, overflow) : visit2(w, any, link, st, wc, overflow);
-    if (link < 0 && link != LINK_NONE && leaf == LINK_NONE) {
-      leaf = link;
-      link = walk_pop(w, st);
-    }
-    if (!__any_sync(__activemask(), leaf == LINK_NONE)) break;
+// ---- steps of a walk ----
+// A walk is a sequence of two kinds of step, opening an interior node and testing a leaf's
+// triangles, and any order of a ray's pending steps gives its result (above). A lane that
+// meets a leaf keeps it aside and goes on opening nodes (the postponed leaves of Aila and
+// Laine) until it meets a second one. The warp takes one kind of step at a time, for all
+// lanes that can take it (walk_wants_node, walk_wants_tri): the kind more of them can. Left to
+// themselves (nodes until every lane has a leaf, then leaves until every lane has none)
+// the lanes of a warp ran 12.8 at a time in nodes and 7.3 in triangles on the glass sphere's
+// path rays, 8.2 and 3.1 on incoherent ones; with the vote 17.5 and 16.5, 16.3 and 14.7. The
+// vote is two ballots a step, which four-child nodes (half as many steps) pay for: a
+// million incoherent rays through the glass sphere 588 -> 448 us.
+__device__ __forceinline__ bool walk_wants_node(const Walk& w) { return w.link >= 0 && w.link != LINK_NONE; }
+__device__ __forceinline__ bool walk_wants_tri(const Walk& w) { return (w.leaf & 15) != 0; }
+
+// a leaf met while none is pending is kept aside
+__device__ __forceinline__ void walk_keep_leaf(Walk& w) {
+  if (w.link < 0 && (w.leaf & 15) == 0) {
+    w.leaf = ~w.link;
+    w.link = pop_link(w);
   }
-  if (leaf == LINK_NONE && link < 0 && link != LINK_NONE) {
-    leaf = link;
-    link = walk_pop(w, st);
-  }
-  while (leaf != LINK_NONE) {
-    if (walk_leaf(w, leaf, wc, any)) { w.sp = 0; w.link = LINK_NONE; return true; }
-    leaf = LINK_NONE;
-    if (!any) link = walk_recheck(w, link, st);
-    if (link < 0 && link != LINK_NONE) {   // a second leaf met by the speculative walk
-      leaf = link;
-      link = walk_pop(w, st);
-    }
-  }
-  w.link = link;
-  return link == LINK_NONE;
 }
 
-template <bool ANY, bool WIDE>
-__device__ __forceinline__ bool walk_step(Walk& w, const WalkStack& st, WalkCount& wc, bool& overflow) {
-  return walk_step_k<WIDE>(w, ANY, st, wc, overflow);
+// The next subtree from the stack where one is due, then one interior node
+// (walk_wants_node). `any` selects the any-hit rule, `overflow` is set when the stack
+// bound was reached (the walk then ends early).
+template <bool WIDE>
+__device__ __forceinline__ void walk_node_step(Walk& w, bool any, const WalkStack& st, WalkCount& wc, bool& overflow) {
+  while (w.link == LINK_POP) {
+    --w.sp;
+    const int2 e = st.at(w.sp);
+    const float te = __int_as_float(e.y);
+    w.link_t = te;
+    w.link = te >= w.best_up ? pop_link(w) : e.x;   // (beyond the cull bound: the next one)
+    walk_keep_leaf(w);
+  }
+  if (walk_wants_node(w)) {
+    w.link = WIDE ? visit4(w, any, w.link, st, wc, overflow) : visit2(w, any, w.link, st, wc, overflow);
+    walk_keep_leaf(w);
+  }
+}
+
+// the triangles of the pending leaf (walk_wants_tri); an any-hit walk ends at its first hit
+__device__ __forceinline__ void walk_leaf(Walk& w, bool any, WalkCount& wc) {
+  const float4* tp = w.tris + 3 * (size_t)(w.leaf >> 4);
+  int left = w.leaf & 15;
+  w.leaf = 0;
+  do {
+    const float4 a = __ldg(tp + 0);
+    const float4 b = __ldg(tp + 1);
+    const float4 c = __ldg(tp + 2);
+    tp += 3;
+    ++wc.tris;
+    TriHit th;
+    if (tri_test(w.ox(), w.oy(), w.oz(), w.dx, w.dy, w.dz, a, b, c, w.best, w.best_rank, th)) {
+      w.best = th.t;
+      w.bu = th.u;
+      w.bv = th.v;
+      w.best_tri = __float_as_int(a.w);
+      w.best_rank = __float_as_int(b.w);
+      if (any) {
+        w.link = LINK_NONE;
+        return;
+      }
+    }
+  } while (--left);
+  w.best_up = cull_up(w.best);
+  // the pending subtree, unless a hit put it out of reach
+  if (w.link < LINK_POP && w.link_t >= w.best_up) w.link = pop_link(w);
+  walk_keep_leaf(w);
+}
+
+// One step for the lanes of a warp that can take the kind more of them wait for; `nodes`
+// and `tris` are the warp's ballots of walk_wants_node and walk_wants_tri, at least one of
+// them not empty.
+template <bool WIDE>
+__device__ __forceinline__ void warp_walk_step(Walk& w, bool any, const WalkStack& st, WalkCount& wc, bool& overflow,
+                                               unsigned nodes, unsigned tris) {
+  if (__popc(nodes) >= __popc(tris)) {
+    if (walk_wants_node(w)) walk_node_step<WIDE>(w, any, st, wc, overflow);
+  } else {
+    if (walk_wants_tri(w)) walk_leaf(w, any, wc);
+  }
+}
+
+// The while-while loop of Aila and Laine without a vote: every lane with a step to take opens
+// nodes until each of them has a leaf, then tests its leaf's triangles. Any-hit queries use
+// it where the votes cost more than the lanes they bring together (trace.cu, rays_by_lane).
+template <bool WIDE>
+__device__ __forceinline__ void lane_walk_step(Walk& w, bool any, const WalkStack& st, WalkCount& wc, bool& overflow) {
+  while (walk_wants_node(w)) {
+    walk_node_step<WIDE>(w, any, st, wc, overflow);
+    if (!__any_sync(__activemask(), !walk_wants_tri(w))) break;
+  }
+  while (walk_wants_tri(w)) walk_leaf(w, any, wc);
 }
 
 }  // namespace yc
