@@ -107,10 +107,10 @@ yc::DevScene walk_scene(const Scene& s) {
   return d;
 }
 
-// the device copy of a scene's lights (yc::prepare_light)
+// the device copy of a scene's lights (yc::prepare_lights)
 std::vector<yc_quad_light> prepared_lights(const yc_quad_light* lights, int n) {
   std::vector<yc_quad_light> out(lights, lights + n);
-  for (yc_quad_light& l : out) yc::prepare_light(l);
+  yc::prepare_lights(out.data(), n);
   return out;
 }
 

@@ -40,7 +40,7 @@ namespace yc {
 
 namespace {
 
-enum : int { M_EYE_START = 8, M_VERTEX = 9, M_CONN = 10, M_CONT = 11, M_FINISH = 12 };
+enum : int { M_EYE_START = 8, M_VERTEX = 9, M_CONN = 10, M_CONT = 11, M_FINISH = 12, M_LIGHT_CONT = 13 };
 
 struct MCount {
   int j, m, nl;   // light vertex index, eye vertex index, stored light vertices
@@ -64,38 +64,47 @@ __device__ __forceinline__ float diffuse_prob(const yc_material& m) {
 
 __device__ __forceinline__ f4 mirror(f4 w, f4 n) { return ym::normalize(ym::mul(2.0f, ym::dot(w, n)) * n - w); }
 
-// BRDF at v between the direction toward the previous subpath vertex and the next one.
-// f_eval and pdf_dir are called, not inlined: the logic kernel's lanes run different
-// states, and one copy of each keeps the code within the instruction cache (measured
-// 1024x1024: 797 against 651 Mrays/s inlined, despite the call's register spills).
-__device__ __noinline__ f4 f_eval(const Vtx& v, const yc_material& m, f4 w_prev, f4 w_next, int brdf_model,
-                                  const float2* on_ab) {
-  const bool glossy = ym::length3(ld4(m.ks)) != 0.0f;
+// What a step of the weights needs at vertex v between the directions a, toward the previous
+// subpath vertex, and b, toward the next one: the solid-angle densities with which
+// sample_dir picks b arriving from a and a arriving from b, and the BRDF.
+struct VtxEval {
+  float fwd, rev;
   f4 f;
-  if (brdf_model == 1 && !glossy) f = oren_nayar(w_next, w_prev, v, m, on_ab[v.mat]);
-  else f = ld4(m.kd) * INV_PI_F;
-  if (glossy) {
-    const float ca = ym::pow(ym::fmax(ym::dot(w_next, mirror(w_prev, v.n)), 0.0f), ym::add(m.px, m.py));
-    const int pe = (int)ym::add(m.px, m.py);
-    f = f + (((ld4(m.ks) * ca) * (float)(pe + 2)) * INV_PI_F) * 0.5f;
-  }
-  f.w = 0.0f;
-  return f;
-}
-
-// solid-angle density with which sample_dir picks w_next at v after arriving from w_prev
-__device__ __noinline__ float pdf_dir(const Vtx& v, const yc_material& m, f4 w_prev, f4 w_next) {
-  const float cn = ym::dot(w_next, v.n);
+};
+__device__ __forceinline__ float pdf_at(const yc_material& m, float pd, float cn, float ca) {
   if (!(cn > 0.0f)) return 0.0f;
-  const float pd = diffuse_prob(m);
   float p = ym::mul(pd, ym::mul(cn, INV_PI_F));
   if (pd < 1.0f) {
     const int pe = (int)ym::add(m.px, m.py);
-    const float ca = ym::fmax(ym::dot(w_next, mirror(w_prev, v.n)), 0.0f);
     const float lobe = ym::mul(ym::mul(ym::mul((float)(pe + 1), 0.5f), INV_PI_F), ym::pow(ca, (float)pe));
     p = ym::add(p, ym::mul(ym::sub(1.0f, pd), lobe));
   }
   return p;
+}
+__device__ __forceinline__ VtxEval eval_at(const Vtx& v, const yc_material& m, f4 a, f4 b, int brdf_model,
+                                           const float2* on_ab) {
+  const bool glossy = ym::length3(ld4(m.ks)) != 0.0f;
+  const float pd = diffuse_prob(m);
+  VtxEval r;
+  float c[2] = {0.0f, 0.0f};   // the lobes' cosines, of b about a's mirror direction and the other way
+  if (pd < 1.0f || glossy) {
+    c[0] = ym::fmax(ym::dot(b, mirror(a, v.n)), 0.0f);
+    c[1] = ym::fmax(ym::dot(a, mirror(b, v.n)), 0.0f);
+  }
+  float p[2];
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) p[k] = pdf_at(m, pd, ym::dot(k ? a : b, v.n), k ? c[1] : c[0]);
+  r.fwd = p[0];
+  r.rev = p[1];
+  if (brdf_model == 1 && !glossy) r.f = oren_nayar(b, a, v, m, on_ab[v.mat]);
+  else r.f = ld4(m.kd) * INV_PI_F;
+  if (glossy) {
+    const float ca = ym::pow(c[0], ym::add(m.px, m.py));
+    const int pe = (int)ym::add(m.px, m.py);
+    r.f = r.f + (((ld4(m.ks) * ca) * (float)(pe + 2)) * INV_PI_F) * 0.5f;
+  }
+  r.f.w = 0.0f;
+  return r;
 }
 
 // lobe (1 number), then a cosine or Phong-lobe direction (2 numbers); false when the
@@ -109,31 +118,16 @@ __device__ __forceinline__ bool sample_dir(const Vtx& v, const yc_material& m, f
   return ym::dot(w_next, v.n) > 0.0f;
 }
 
-__device__ __forceinline__ float light_weight(const yc_quad_light& L) {
-  return ym::mul(ym::add(ym::add(L.ke.x, L.ke.y), L.ke.z), light_area(L));
-}
-__device__ __forceinline__ float light_total(const DevScene& sc) {
-  float t = 0.0f;
-  for (int i = 0; i < sc.n_lights; ++i) t = ym::add(t, light_weight(sc.lights[i]));
-  return t;
-}
-// area density of the point a light sample lands on, on light i
-__device__ __forceinline__ float light_point_pdf(const DevScene& sc, int i) {
-  const yc_quad_light& L = sc.lights[i];
-  return ym::div(ym::div(light_weight(L), light_total(sc)), light_area(L));
-}
 // picks a light (1 number) with probability proportional to (ke.r + ke.g + ke.b) * area
 __device__ __forceinline__ int pick_light(const DevScene& sc, uint32_t& seed) {
   const float u = draw(seed);
-  const float total = light_total(sc);
-  if (!(total > 0.0f)) return -1;
+  if (!(light_total(sc.lights[0]) > 0.0f)) return -1;
   float cum = 0.0f;
   int last = -1;
   for (int i = 0; i < sc.n_lights; ++i) {
-    const float w = light_weight(sc.lights[i]);
-    if (!(w > 0.0f)) continue;
+    if (!(light_weight(sc.lights[i]) > 0.0f)) continue;
     last = i;
-    const float p = ym::div(w, total);
+    const float p = light_share(sc.lights[i]);
     if (u < ym::add(cum, p)) return i;
     cum = ym::add(cum, p);
   }
@@ -211,7 +205,7 @@ __global__ void __launch_bounds__(256) k_raygen_bdpt_mis(PassParams pp, PathStat
     float p0 = 0.0f, c0 = 0.0f;
     if (lk >= 0) {
       const yc_quad_light& L = sc.lights[lk];
-      p0 = light_point_pdf(sc, lk);
+      p0 = light_point_pdf(L);
       Vtx v0;
       v0.hp = light_point(L, seed);
       v0.n = ld4(L.normal);
@@ -260,7 +254,11 @@ void launch_raygen_bdpt_mis(const PassParams& pp, const PathState& ps, const Bdp
 }
 
 // ---- logic: advance each path to its next ray ----
-__global__ void __launch_bounds__(256) k_logic_bdpt_mis(PassParams pp, PathState ps, BdptBuffers bb,
+// Bound by the latency of a long dependent chain at few warps: 163 registers in three blocks
+// of 128 per SM measured best (unbounded, 210 in two: 2.98 ms per two 512x512 passes; three:
+// 2.70; four, 386 B spilled: 2.87; five, 768 B: 3.22).
+constexpr int MIS_TB = 128;
+__global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, PathState ps, BdptBuffers bb,
                                                         const int* __restrict__ in_closest,
                                                         const int* __restrict__ in_any, const RoundCounters* rc_in,
                                                         int* out_closest, int* out_any, RoundCounters* rc_out,
@@ -286,6 +284,7 @@ __global__ void __launch_bounds__(256) k_logic_bdpt_mis(PassParams pp, PathState
     int emit = 0;
     int p = -1;
     unsigned c[7] = {0, 0, 0, 0, 0, 0, 0};
+    const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
       p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
       const MisRec lv{bb.lv + (size_t)p * bb.bounces * 4};
@@ -342,282 +341,256 @@ __global__ void __launch_bounds__(256) k_logic_bdpt_mis(PassParams pp, PathState
       const float4 hit = ps.hit[p];
       bool moved = false;    // the eye vertex changed
       bool w_color = false, w_eye = false, w_pend = false, w_bounce = false;   // fields to write back
-      bool done = false;
 
-      for (int guard = 0; guard < 8192 && !done; ++guard) {
-        switch (phase) {
-          case B_LIGHT: {   // light vertex j reached (or the light subpath ends)
-            const int tri = __float_as_int(hit.w);
-            if (tri < 0) { phase = M_EYE_START; break; }
-            const Vtx v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-            const float cv = -ym::dot(rd, v.n);
-            if (!(cv > 0.0f)) { phase = M_EYE_START; break; }
+      // ---- the result of the ray the path waited for ----
+      Vtx x;                        // the light vertex just made, where the light subpath goes on
+      x.hp = x.n = ym::splat(0.0f);
+      x.mat = 0;
+      f4 lp = ym::splat(0.0f);      // toward the vertex before it
+      float r_x = 0.0f, s_x = 0.0f;
+      if (shadow) {
+        if (hit.x == 0.0f) {
+          color = color + pend;
+          w_color = true;
+        }
+        phase = M_CONN;
+      } else {
+        const int tri = __float_as_int(hit.w);
+        const bool eye0 = phase == B_EYE0, light = phase == B_LIGHT;
+        const bool met = tri >= 0;
+        if (met) x = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
+        lp = -rd;
+        const float cv = ym::dot(lp, x.n);   // (-dot(rd, n), and dot(-rd, n) for the camera ray: the same bits)
+        const bool faces = met && cv > 0.0f;
+        if (faces && !eye0) {
+          const Vtx pv = light ? lv.vtx(cnt.j - 1) : y;
+          const f4 dv = x.hp - pv.hp;
+          const float d2 = ym::dot(dv, dv);
+          r_x = mis(ym::div(d2, ym::mul(w_f, cv)));
+          s_x = mul0(ym::mul(r_x, mis(ym::div(c_out, d2))), acc);
+        }
+        if (light) {   // light vertex j reached (or the light subpath ends)
+          phase = M_EYE_START;
+          if (faces) {
             const int j = cnt.j;
-            const Vtx pv = lv.vtx(j - 1);
-            const f4 dv = v.hp - pv.hp;
-            const float d2 = ym::dot(dv, dv);
-            const float r = mis(ym::div(d2, ym::mul(w_f, cv)));
-            const float s = mul0(ym::mul(r, mis(ym::div(c_out, d2))), acc);
-            lv.at(j, 0) = make_float4(v.hp.x, v.hp.y, v.hp.z, __int_as_float(v.mat));
-            lv.at(j, 1) = make_float4(v.n.x, v.n.y, v.n.z, r);
-            lv.at(j, 2) = make_float4(rd.x, rd.y, rd.z, s);
+            lv.at(j, 0) = make_float4(x.hp.x, x.hp.y, x.hp.z, __int_as_float(x.mat));
+            lv.at(j, 1) = make_float4(x.n.x, x.n.y, x.n.z, r_x);
+            lv.at(j, 2) = make_float4(rd.x, rd.y, rd.z, s_x);
             lv.at(j, 3) = make_float4(bnext.x, bnext.y, bnext.z, 0.0f);
             cnt.nl = j;
-            if (j + 1 > KMAX - 2) { phase = M_EYE_START; break; }
-            const yc_material& m = sc.mats[v.mat];
-            f4 cont = bnext;
-            if (j > RR) {
-              const float q = ym::min(luminance(bnext), 0.95f);
-              if (!(draw(seed) < q)) { phase = M_EYE_START; break; }
-              cont = bnext / q;
-            }
-            const f4 lp = -rd;
-            f4 wn;
-            if (!sample_dir(v, m, lp, seed, wn)) { phase = M_EYE_START; break; }
-            w_f = pdf_dir(v, m, lp, wn);
-            if (!(w_f > 0.0f)) { phase = M_EYE_START; break; }
-            const float w_r = pdf_dir(v, m, wn, lp);
-            c_out = ym::dot(wn, v.n);
-            acc = ym::add(r, mul0(s, mis(w_r)));
-            bnext = ((cont * f_eval(v, m, lp, wn, pp.brdf_model, sc.on_ab)) * c_out) / w_f;
-            w_bounce = true;
-            ro = v.hp + wn * EPS_F;
-            rd = wn;
-            tmax = INF;
-            k = -1;
-            light_test(sc, ro, rd, tmax, k);
-            cnt.j = j + 1;
-            count_ray(c, 2);
-            c[5]++;
-            emit = 1;
-            done = true;
-            break;
+            if (j + 1 <= KMAX - 2) phase = M_LIGHT_CONT;
           }
-          case M_EYE_START: {   // the camera ray
-            ro = ym::mk(pp.cam.r1.w, pp.cam.r2.w, pp.cam.r3.w, pp.cam.r4.w);
-            const float4 d = ps.wi[p];
-            rd = ym::mk(d.x, d.y, d.z, d.w);
-            tmax = INF;
-            k = -1;
-            light_test(sc, ro, rd, tmax, k);
-            cnt.m = 0;
-            count_ray(c, 1);
-            c[5]++;
-            phase = B_EYE0;
-            emit = 1;
-            done = true;
-            break;
-          }
-          case B_EYE0: {
-            const int tri = __float_as_int(hit.w);
-            if (tri < 0) {
-              if (k >= 0) {
-                color = (ym::dot(rd, ld4(sc.lights[k].normal)) < 0.0f) ? ym::mk(1.0f, 1.0f, 1.0f, 1.0f)
-                                                                       : ym::mk(0.1f, 0.1f, 0.1f, 1.0f);
-              } else {
-                color = ym::mk(0.4f, 0.4f, 0.4f, 1.0f);
-              }
-              phase = M_FINISH;
-              break;
-            }
-            color = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
-            w_color = true;
-            y = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-            wp = -rd;
-            if (!(ym::dot(wp, y.n) > 0.0f)) { phase = M_FINISH; break; }
-            beta = ym::mk(1.0f, 1.0f, 1.0f, 0.0f);
-            r_y = 0.0f;
-            s_y = 0.0f;
-            cnt.m = 1;
-            moved = w_eye = w_pend = true;
-            phase = M_VERTEX;
-            break;
-          }
-          case M_VERTEX: {   // emission, then the next-event estimate at eye vertex m
-            const yc_material& m = sc.mats[y.mat];
-            color = color + beta * rgb(m.ke);
-            w_color = true;
-            if (cnt.m + 1 > KMAX) { phase = M_FINISH; break; }
-            if (lk < 0) { phase = M_CONT; break; }
-            cnt.j = 1;
-            phase = M_CONN;
-            const int kl = pick_light(sc, seed);
-            if (kl < 0) break;
-            const yc_quad_light& L = sc.lights[kl];
-            const float pk = light_point_pdf(sc, kl);
-            const f4 x = light_point(L, seed);
-            const f4 v = x - y.hp;
-            const float d2 = ym::dot(v, v);
-            const float dist = ym::sqrt(d2);
-            const f4 dir = v * ym::div(1.0f, dist);
-            const float cy = ym::dot(dir, y.n);
-            const float cl = -ym::dot(dir, ld4(L.normal));
-            if (!(cy > 0.0f) || !(cl > 0.0f)) break;
-            const float wf = pdf_dir(y, m, wp, dir);
-            const float wr = pdf_dir(y, m, dir, wp);
-            const float ls = mis(ym::div(ym::mul(wf, cl), ym::mul(d2, pk)));
-            const float es = mul0(mis(ym::div(ym::mul(ym::mul(cl, INV_PI_F), cy), d2)), ym::add(r_y, mul0(s_y, mis(wr))));
-            const float w = ym::div(1.0f, ym::add(ym::add(1.0f, ls), es));
-            const float g = ym::div(ym::mul(cy, cl), ym::mul(d2, pk));
-            pend = ((beta * f_eval(y, m, wp, dir, pp.brdf_model, sc.on_ab)) * rgb(L.ke)) * ym::mul(g, w);
-            w_pend = true;
-            ro = y.hp + dir * EPS_F;
-            rd = dir;
-            tmax = ym::sub(dist, ym::mul(EPS_F, 1.5f));
-            count_ray(c, 3);
-            int lh = -1;
-            float tl = tmax;
-            light_test(sc, ro, rd, tl, lh);
-            if (lh >= 0) break;   // a light closes the segment: occluded
-            c[5]++;
-            phase = B_NEE;
-            emit = 2;
-            done = true;
-            break;
-          }
-          case B_NEE: {
-            if (hit.x == 0.0f) {
-              color = color + pend;
-              w_color = true;
-            }
-            phase = M_CONN;
-            break;
-          }
-          case M_CONN: {   // connection of eye vertex m to light vertex j
-            const int j = cnt.j;
-            if (j > cnt.nl || cnt.m + j + 1 > KMAX) { phase = M_CONT; break; }
-            cnt.j = j + 1;
-            const Vtx lvx = lv.vtx(j);
-            const f4 v = lvx.hp - y.hp;
-            const float d2 = ym::dot(v, v);
-            const float dist = ym::sqrt(d2);
-            const f4 dir = v * ym::div(1.0f, dist);
-            const float cy = ym::dot(dir, y.n);
-            const float cl = -ym::dot(dir, lvx.n);
-            if (!(cy > 0.0f) || !(cl > 0.0f)) break;
-            const float4 f2 = lv.at(j, 2), f3 = lv.at(j, 3);
-            const float lr = lv.at(j, 1).w, lsv = f2.w;
-            const f4 lp = ym::mk(-f2.x, -f2.y, -f2.z, -0.0f);
-            const f4 wl = -dir;
-            const yc_material& my = sc.mats[y.mat];
-            const yc_material& ml = sc.mats[lvx.mat];
-            const float wy_f = pdf_dir(y, my, wp, dir);
-            const float wy_r = pdf_dir(y, my, dir, wp);
-            const float wl_f = pdf_dir(lvx, ml, lp, wl);
-            const float wl_r = pdf_dir(lvx, ml, wl, lp);
-            const float ls = mul0(mis(ym::div(ym::mul(wy_f, cl), d2)), ym::add(lr, mul0(lsv, mis(wl_r))));
-            const float es = mul0(mis(ym::div(ym::mul(wl_f, cy), d2)), ym::add(r_y, mul0(s_y, mis(wy_r))));
-            const float w = ym::div(1.0f, ym::add(ym::add(1.0f, ls), es));
-            const float g = ym::div(ym::mul(cy, cl), d2);
-            const f4 le = rgb(sc.lights[lk].ke) * ym::div(PI_F, p0);
-            pend = ((((beta * f_eval(y, my, wp, dir, pp.brdf_model, sc.on_ab)) * f_eval(lvx, ml, lp, wl, pp.brdf_model, sc.on_ab)) *
-                     ym::mk(f3.x, f3.y, f3.z, 0.0f)) * le) * ym::mul(g, w);
-            w_pend = true;
-            ro = y.hp + dir * EPS_F;
-            rd = dir;
-            tmax = ym::sub(dist, ym::mul(EPS_F, 2.0f));
-            count_ray(c, 4);
-            int lh = -1;
-            float tl = tmax;
-            light_test(sc, ro, rd, tl, lh);
-            if (lh >= 0) break;
-            c[5]++;
-            phase = B_CONN;
-            emit = 2;
-            done = true;
-            break;
-          }
-          case B_CONN: {
-            if (hit.x == 0.0f) {
-              color = color + pend;
-              w_color = true;
-            }
-            phase = M_CONN;
-            break;
-          }
-          case M_CONT: {   // the next eye ray from vertex m
-            const yc_material& m = sc.mats[y.mat];
-            f4 cont = beta;
-            if (cnt.m > RR) {
-              const float q = ym::min(luminance(beta), 0.95f);
-              if (!(draw(seed) < q)) { phase = M_FINISH; break; }
-              cont = beta / q;
-            }
-            f4 wn;
-            if (!sample_dir(y, m, wp, seed, wn)) { phase = M_FINISH; break; }
-            w_f = pdf_dir(y, m, wp, wn);
-            if (!(w_f > 0.0f)) { phase = M_FINISH; break; }
-            const float w_r = pdf_dir(y, m, wn, wp);
-            c_out = ym::dot(wn, y.n);
-            acc = ym::add(r_y, mul0(s_y, mis(w_r)));
-            bnext = ((cont * f_eval(y, m, wp, wn, pp.brdf_model, sc.on_ab)) * c_out) / w_f;
-            w_bounce = true;
-            ro = y.hp + wn * EPS_F;
-            rd = wn;
-            tmax = INF;
-            k = -1;
-            light_test(sc, ro, rd, tmax, k);
-            count_ray(c, 2);
-            c[5]++;
-            phase = B_EYE;
-            emit = 1;
-            done = true;
-            break;
-          }
-          case B_EYE: {   // eye vertex m + 1 reached, or a light (strategy s = 0)
-            const int tri = __float_as_int(hit.w);
-            if (tri < 0) {
-              if (k >= 0) {
-                const yc_quad_light& L = sc.lights[k];
-                const float cl = -ym::dot(rd, ld4(L.normal));
-                if (cl > 0.0f) {
-                  const f4 z = ro + rd * tmax;
-                  const f4 dv = z - y.hp;
-                  const float d2 = ym::dot(dv, dv);
-                  const float r2 = mis(ym::div(d2, ym::mul(w_f, cl)));
-                  const float s2 = mul0(ym::mul(r2, mis(ym::div(c_out, d2))), acc);
-                  const float es = ym::mul(mis(light_point_pdf(sc, k)), ym::add(r2, mul0(s2, mis(ym::mul(cl, INV_PI_F)))));
-                  const float w = ym::div(1.0f, ym::add(1.0f, es));
-                  color = color + (bnext * rgb(L.ke)) * w;
-                }
-              }
-              phase = M_FINISH;
-              break;
-            }
-            const Vtx v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-            const float cv = -ym::dot(rd, v.n);
-            if (!(cv > 0.0f)) { phase = M_FINISH; break; }
-            const f4 dv = v.hp - y.hp;
-            const float d2 = ym::dot(dv, dv);
-            r_y = mis(ym::div(d2, ym::mul(w_f, cv)));
-            s_y = mul0(ym::mul(r_y, mis(ym::div(c_out, d2))), acc);
-            beta = bnext;
-            y = v;
-            wp = -rd;
-            cnt.m += 1;
-            moved = w_eye = w_pend = true;
-            phase = M_VERTEX;
-            break;
-          }
-          case M_FINISH:
-          default: {
-            if (ym::any_nan(color)) color = ym::mk(0.988f, 0.0588f, 0.7529f, 1.0f);
-            const float4 prev = pp.accum[pix];
-            f4 cc = color;
-            if (pp.reset == 1) {
-              cc.w = 1.0f;
+        } else if (faces) {   // an eye vertex: the first one, or vertex m + 1
+          beta = eye0 ? ym::mk(1.0f, 1.0f, 1.0f, 0.0f) : bnext;
+          r_y = r_x;
+          s_y = s_x;
+          cnt.m = eye0 ? 1 : cnt.m + 1;
+          if (eye0) color = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
+          y = x;
+          wp = lp;
+          moved = w_eye = w_pend = true;
+          phase = M_VERTEX;
+        } else {
+          phase = M_FINISH;
+          if (eye0) {
+            if (met) {
+              color = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
+            } else if (k >= 0) {
+              color = (ym::dot(rd, ld4(sc.lights[k].normal)) < 0.0f) ? ym::mk(1.0f, 1.0f, 1.0f, 1.0f)
+                                                                     : ym::mk(0.1f, 0.1f, 0.1f, 1.0f);
             } else {
-              const int np = (int)prev.w;
-              cc = cc + f4of(prev) * (float)np;
-              cc = cc / (float)(np + 1);
-              cc.w = (float)(np + 1);
+              color = ym::mk(0.4f, 0.4f, 0.4f, 1.0f);
             }
-            pp.accum[pix] = make_float4(cc.x, cc.y, cc.z, cc.w);
-            c[6]++;
-            done = true;
-            break;
+          } else if (!met && k >= 0) {   // the eye subpath met a light (strategy s = 0)
+            const yc_quad_light& L = sc.lights[k];
+            const float cl = -ym::dot(rd, ld4(L.normal));
+            if (cl > 0.0f) {
+              const f4 z = ro + rd * tmax;
+              const f4 dv = z - y.hp;
+              const float d2 = ym::dot(dv, dv);
+              const float r2 = mis(ym::div(d2, ym::mul(w_f, cl)));
+              const float s2 = mul0(ym::mul(r2, mis(ym::div(c_out, d2))), acc);
+              const float es = ym::mul(mis(light_point_pdf(L)), ym::add(r2, mul0(s2, mis(ym::mul(cl, INV_PI_F)))));
+              const float w = ym::div(1.0f, ym::add(1.0f, es));
+              color = color + (bnext * rgb(L.ke)) * w;
+            }
           }
         }
+      }
+      // ---- an eye vertex's emission, and its light sample ----
+      int cand = 0;             // a segment to a light or a light vertex: B_NEE or B_CONN
+      f4 dir = ym::splat(0.0f); //   its direction, squared length, length and end cosines
+      float d2 = 0.0f, dist = 0.0f, cy = 0.0f, cl = 0.0f, pk = 0.0f;
+      int at = 0;               //   the light, or the light vertex, at its end
+      __syncwarp(mask);
+      if (phase == M_VERTEX) {
+        color = color + beta * rgb(sc.mats[y.mat].ke);
+        w_color = true;
+        if (cnt.m + 1 > KMAX) {
+          phase = M_FINISH;
+        } else if (lk < 0) {
+          phase = M_CONT;
+        } else {
+          cnt.j = 1;
+          phase = M_CONN;
+          at = pick_light(sc, seed);
+          if (at >= 0) {
+            const yc_quad_light& L = sc.lights[at];
+            pk = light_point_pdf(L);
+            const f4 v = light_point(L, seed) - y.hp;
+            d2 = ym::dot(v, v);
+            dist = ym::sqrt(d2);
+            dir = v * ym::rcp(dist);
+            cy = ym::dot(dir, y.n);
+            cl = -ym::dot(dir, ld4(L.normal));
+            if (cy > 0.0f && cl > 0.0f) cand = B_NEE;
+          }
+        }
+      }
+      // Each pass over the stages below takes the path to a ray: the next segment of the eye
+      // vertex worth a shadow ray, or the subpath's next direction. The evaluation at a vertex
+      // (two densities and the BRDF), which is most of the work, appears once, for the
+      // segments, for the light vertex at a connection's other end and for the new
+      // directions alike, so that lanes in different states run it together. With one copy of
+      // the stages per state and the evaluation in called functions the kernel ran 8-9 of 32
+      // lanes (loops over rejected segments among them) at 195 registers; two 512x512 passes
+      // of the four-light Cornell box took 5.75 ms of shading, now 2.70 ms.
+      for (;;) {
+        __syncwarp(mask);
+        if (phase == M_CONN && !cand) {   // the next light vertex both ends of whose segment face each other
+          while (cnt.j <= cnt.nl && cnt.m + cnt.j + 1 <= KMAX && !cand) {
+            at = cnt.j++;
+            const float4 h4 = lv.at(at, 0), n4 = lv.at(at, 1);
+            const f4 v = ym::mk(h4.x, h4.y, h4.z, 1.0f) - y.hp;
+            d2 = ym::dot(v, v);
+            dist = ym::sqrt(d2);
+            dir = v * ym::rcp(dist);
+            cy = ym::dot(dir, y.n);
+            cl = -ym::dot(dir, ym::mk(n4.x, n4.y, n4.z, 0.0f));
+            if (cy > 0.0f && cl > 0.0f) cand = B_CONN;
+          }
+          if (!cand) phase = M_CONT;
+        }
+        __syncwarp(mask);
+        const bool light = phase == M_LIGHT_CONT;
+        bool go = light || (phase == M_CONT && !emit);   // a subpath's next direction is drawn
+        f4 cont = light ? bnext : beta;
+        if (go) {
+          const Vtx v = light ? x : y;
+          if ((light ? cnt.j : cnt.m) > RR) {
+            const float q = ym::min(luminance(cont), 0.95f);
+            go = draw(seed) < q;
+            if (go) cont = cont / q;
+          }
+          if (go) go = sample_dir(v, sc.mats[v.mat], light ? lp : wp, seed, dir);
+          if (!go) phase = light ? M_EYE_START : M_FINISH;
+        }
+        __syncwarp(mask);
+        // at the vertex: of a segment y, then for a connection the light vertex; of a new
+        // direction the vertex it leaves
+        VtxEval ev{0.0f, 0.0f, ym::splat(0.0f)}, el{0.0f, 0.0f, ym::splat(0.0f)};
+        Vtx lx = x;
+        float lr = 0.0f, lsv = 0.0f;
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+          if (side == 0 ? cand || go : cand == B_CONN) {
+            f4 a = light ? lp : wp, b = dir;
+            Vtx v = light ? x : y;
+            if (side) {
+              const float4 f2 = lv.at(at, 2);
+              v = lv.vtx(at);
+              lr = lv.at(at, 1).w;
+              lsv = f2.w;
+              a = ym::mk(-f2.x, -f2.y, -f2.z, -0.0f);
+              b = -dir;
+            }
+            const VtxEval r = eval_at(v, sc.mats[v.mat], a, b, pp.brdf_model, sc.on_ab);
+            if (side) el = r;
+            else ev = r;
+          }
+          if (!__any_sync(mask, cand == B_CONN)) break;
+        }
+        if (cand) {
+          const bool conn = cand == B_CONN;
+          float ls, es, g;
+          f4 c3;
+          if (conn) {
+            ls = mul0(mis(ym::div(ym::mul(ev.fwd, cl), d2)), ym::add(lr, mul0(lsv, mis(el.rev))));
+            es = mul0(mis(ym::div(ym::mul(el.fwd, cy), d2)), ym::add(r_y, mul0(s_y, mis(ev.rev))));
+            g = ym::div(ym::mul(cy, cl), d2);
+            const float4 f3 = lv.at(at, 3);
+            const f4 le = rgb(sc.lights[lk].ke) * ym::div(PI_F, p0);
+            c3 = (((beta * ev.f) * el.f) * ym::mk(f3.x, f3.y, f3.z, 0.0f)) * le;
+          } else {
+            ls = mis(ym::div(ym::mul(ev.fwd, cl), ym::mul(d2, pk)));
+            es = mul0(mis(ym::div(ym::mul(ym::mul(cl, INV_PI_F), cy), d2)), ym::add(r_y, mul0(s_y, mis(ev.rev))));
+            g = ym::div(ym::mul(cy, cl), ym::mul(d2, pk));
+            c3 = (beta * ev.f) * rgb(sc.lights[at].ke);
+          }
+          const float w = ym::div(1.0f, ym::add(ym::add(1.0f, ls), es));
+          pend = c3 * ym::mul(g, w);
+          w_pend = true;
+        } else if (go) {
+          if (ev.fwd > 0.0f) {
+            const Vtx v = light ? x : y;
+            w_f = ev.fwd;
+            c_out = ym::dot(dir, v.n);
+            acc = ym::add(light ? r_x : r_y, mul0(light ? s_x : s_y, mis(ev.rev)));
+            bnext = ((cont * ev.f) * c_out) / w_f;
+            w_bounce = true;
+          } else {
+            go = false;
+            phase = light ? M_EYE_START : M_FINISH;
+          }
+        }
+        // the ray: its light loop, and whether the hierarchy has to settle it
+        __syncwarp(mask);
+        const bool start = phase == M_EYE_START && !emit;   // the camera ray
+        if (cand || go || start) {
+          ro = (light && go ? x.hp : y.hp) + dir * EPS_F;
+          rd = dir;
+          tmax = INF;
+          if (start) {
+            const float4 d = ps.wi[p];
+            ro = ym::mk(pp.cam.r1.w, pp.cam.r2.w, pp.cam.r3.w, pp.cam.r4.w);
+            rd = ym::mk(d.x, d.y, d.z, d.w);
+            cnt.m = 0;
+          } else if (cand) {
+            tmax = ym::sub(dist, ym::mul(EPS_F, cand == B_CONN ? 2.0f : 1.5f));
+          }
+          float tl = tmax;
+          int lh = -1;
+          light_test(sc, ro, rd, tl, lh);
+          count_ray(c, start ? 1 : go ? 2 : cand == B_NEE ? 3 : 4);
+          if (!cand) {
+            k = lh;
+            tmax = tl;
+            if (go && light) ++cnt.j;
+            phase = start ? B_EYE0 : light ? B_LIGHT : B_EYE;
+            emit = 1;
+          } else if (lh < 0) {   // (a light that closes the segment occludes it)
+            phase = cand;
+            emit = 2;
+          }
+          if (emit) c[5]++;
+          cand = 0;
+        }
+        if (!__any_sync(mask, !emit && phase != M_FINISH)) break;
+      }
+      if (!emit) {   // the running mean of the pixel
+        if (ym::any_nan(color)) color = ym::mk(0.988f, 0.0588f, 0.7529f, 1.0f);
+        const float4 prev = pp.accum[pix];
+        f4 cc = color;
+        if (pp.reset == 1) {
+          cc.w = 1.0f;
+        } else {
+          const int np = (int)prev.w;
+          cc = cc + f4of(prev) * (float)np;
+          cc = cc / (float)(np + 1);
+          cc.w = (float)(np + 1);
+        }
+        pp.accum[pix] = make_float4(cc.x, cc.y, cc.z, cc.w);
+        c[6]++;
       }
       if (emit) {
         ps.misc[p] = make_int4((int)seed, pix, pack_ms(phase, lk, k), pack_mc(cnt));
@@ -674,8 +647,9 @@ void launch_logic_bdpt_mis(const PassParams& pp, const PathState& ps, const Bdpt
                            const int* in_any, const RoundCounters* rc_in, int* out_closest, int* out_any,
                            RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted,
                            const SortCtl* sctl) {
-  k_logic_bdpt_mis<<<grid, 256, 0, s>>>(pp, ps, bb, in_closest, in_any, rc_in, out_closest, out_any, rc_out, st,
-                                        sorted, sctl);
+  // (grid counts blocks of 256)
+  k_logic_bdpt_mis<<<grid * (256 / MIS_TB), MIS_TB, 0, s>>>(pp, ps, bb, in_closest, in_any, rc_in, out_closest, out_any,
+                                                            rc_out, st, sorted, sctl);
 }
 
 }  // namespace yc

@@ -32,19 +32,36 @@ struct Vtx {
   int mat;
 };
 
-// The device copy of a quad light carries in its padding three values that depend on the
-// light alone, computed once on the host by the same operations (prepare_light): the
-// lengths of its edges and of its emission.
-inline void prepare_light(yc_quad_light& L) {
+// The device copies of a scene's quad lights carry, in fields the kernels do not read otherwise,
+// values that depend on the lights alone, computed once on the host by the same operations
+// (prepare_lights): in the padding the lengths of a light's edges and of its emission, in kd
+// the power-proportional choice among the lights: the sum of the weights
+// (ke.r + ke.g + ke.b) * area, this light's weight, its share, and the area density of a point
+// sampled on it.
+inline void prepare_lights(yc_quad_light* L, int n) {
   auto f = [](const yc_float4& v) { return ym::mk(v.x, v.y, v.z, v.w); };
-  L.pad[0] = ym::length(f(L.edge_l));
-  L.pad[1] = ym::length(f(L.edge_w));
-  L.pad[2] = ym::length(f(L.ke));
+  float total = 0.0f;
+  for (int i = 0; i < n; ++i) {
+    L[i].pad[0] = ym::length(f(L[i].edge_l));
+    L[i].pad[1] = ym::length(f(L[i].edge_w));
+    L[i].pad[2] = ym::length(f(L[i].ke));
+    L[i].kd.y = ym::mul(ym::add(ym::add(L[i].ke.x, L[i].ke.y), L[i].ke.z), ym::mul(L[i].pad[0], L[i].pad[1]));
+    total = ym::add(total, L[i].kd.y);
+  }
+  for (int i = 0; i < n; ++i) {
+    L[i].kd.x = total;
+    L[i].kd.z = ym::div(L[i].kd.y, total);
+    L[i].kd.w = ym::div(L[i].kd.z, ym::mul(L[i].pad[0], L[i].pad[1]));
+  }
 }
 __device__ __forceinline__ float light_len_l(const yc_quad_light& L) { return L.pad[0]; }
 __device__ __forceinline__ float light_len_w(const yc_quad_light& L) { return L.pad[1]; }
 __device__ __forceinline__ float light_len_ke(const yc_quad_light& L) { return L.pad[2]; }
 __device__ __forceinline__ float light_area(const yc_quad_light& L) { return ym::mul(light_len_l(L), light_len_w(L)); }
+__device__ __forceinline__ float light_total(const yc_quad_light& L) { return L.kd.x; }
+__device__ __forceinline__ float light_weight(const yc_quad_light& L) { return L.kd.y; }
+__device__ __forceinline__ float light_share(const yc_quad_light& L) { return L.kd.z; }
+__device__ __forceinline__ float light_point_pdf(const yc_quad_light& L) { return L.kd.w; }
 
 // the analytic quad-light loop of traceRay (udpt.cl:244-276); updates len and the hit light
 __device__ __forceinline__ void light_test(const DevScene& sc, f4 o, f4 d, float& len, int& light) {
