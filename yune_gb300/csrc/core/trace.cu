@@ -10,8 +10,6 @@
 // the stack is counted in DevStats::stack_overflow instead of writing out of bounds.
 #include <cuda_runtime.h>
 
-#include <algorithm>
-
 #include "yc_internal.h"
 #include "yc_shade.cuh"
 #include "yc_trace_loop.cuh"
@@ -201,19 +199,19 @@ int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_an
 // the 82K-triangle glass sphere 43.8 us against 49.5 us voted, 20,000 98.8 against 106.3, a
 // million 367 against 315; a million through the 34 triangles of the Cornell box 149 against
 // 162 us.
-constexpr int TINY_SCENE = 512;   // triangles
-static bool rays_by_lane(const DevScene& sc, bool any_hit, int n, int grid) {
-  return any_hit && !sc.wide && (sc.n_tri < TINY_SCENE || n < grid * (TRACE_TB / 2));
+constexpr int TINY_SCENE = 512;        // triangles
+constexpr int SHORT_LIST = 1 << 16;    // rays, less than half of the lanes of eight blocks on each of 152 SMs
+
+using RaysKernel = void (*)(DevScene, const float*, int, int*, int*, float*, int, DevStats*, int, int*);
+static RaysKernel rays_kernel(const DevScene& sc, bool any_hit, int n) {
+  if (!any_hit) return sc.wide ? k_trace_rays<false, true, false> : k_trace_rays<false, false, false>;
+  if (sc.wide) return k_trace_rays<true, true, false>;
+  return sc.n_tri < TINY_SCENE || n < SHORT_LIST ? k_trace_rays<true, false, true> : k_trace_rays<true, false, false>;
 }
 
-int trace_rays_grid_blocks(bool any_hit, int depth, bool wide, int n_smem) {
-  const int cap = stack_cap_for(depth);
-  const size_t smem = smem_for(n_smem > 0 && n_smem < cap ? n_smem : cap);
-  if (any_hit) return wide ? resident_grid(k_trace_rays<true, true, false>, smem)
-                           : std::min(resident_grid(k_trace_rays<true, false, false>, smem),
-                                      resident_grid(k_trace_rays<true, false, true>, smem));
-  return wide ? resident_grid(k_trace_rays<false, true, false>, smem)
-              : resident_grid(k_trace_rays<false, false, false>, smem);
+int trace_rays_grid_blocks(const DevScene& sc, bool any_hit, int n, int n_smem) {
+  const int cap = stack_cap_for(sc.depth);
+  return resident_grid(rays_kernel(sc, any_hit, n), smem_for(n_smem > 0 && n_smem < cap ? n_smem : cap));
 }
 
 int launch_trace_rays(const DevScene& sc, bool any_hit, const float* rays9, int n, int* tri_out, float* t_out,
@@ -221,10 +219,7 @@ int launch_trace_rays(const DevScene& sc, bool any_hit, const float* rays9, int 
   const int cap = stack_cap_for(sc.depth);
   if (!(n_smem > 0 && n_smem < cap && spill)) n_smem = cap;
   const size_t smem = smem_for(n_smem);
-  const bool wide = sc.wide != 0;
-  const auto kernel = rays_by_lane(sc, any_hit, n, grid) ? k_trace_rays<true, false, true>
-                      : any_hit ? (wide ? k_trace_rays<true, true, false> : k_trace_rays<true, false, false>)
-                                : (wide ? k_trace_rays<false, true, false> : k_trace_rays<false, false, false>);
+  const RaysKernel kernel = rays_kernel(sc, any_hit, n);
   kernel<<<grid, TRACE_TB, smem, s>>>(sc, rays9, n, work, tri_out, t_out, cap, st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

@@ -217,7 +217,7 @@ int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest
 // (n_smem, spill: as for launch_trace_mixed)
 int launch_trace_rays(const DevScene& sc, bool any_hit, const float* rays9, int n, int* tri_out, float* t_out,
                       int* work, DevStats* st, int grid_blocks, cudaStream_t s, int n_smem, int* spill);
-int trace_rays_grid_blocks(bool any_hit, int depth, bool wide, int n_smem);
+int trace_rays_grid_blocks(const DevScene& sc, bool any_hit, int n, int n_smem);
 int trace_grid_blocks(bool any_hit, int depth, bool wide);
 // one launch over both queues of a round (closest-hit entries, then any-hit); the work
 // cursor is rc->work_closest. n_smem (< the stack depth, with spill): walk-stack entries in
