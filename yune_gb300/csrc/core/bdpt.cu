@@ -25,13 +25,8 @@
 
 namespace yc {
 
-enum : int { BF_GLOSSY = 1, BF_OCCLUDED = 2 };
-
-// The BRDF helper of the logic kernel, inlined or called (BDPT_HELPER).
-#define BDPT_HELPER __forceinline__
-__device__ BDPT_HELPER f4 brdf_bk(f4 w_i, f4 w_o, f4 n, const yc_material& m, bool glossy, float rr_prob) {
-  return brdf_b(w_i, w_o, n, m, glossy, rr_prob);
-}
+enum : int { BF_GLOSSY = 1 };
+constexpr int CAST = 1;   // a pending cast holds its state + CAST (0: none)
 
 struct BCount {
   int i, j, lp, ep;
@@ -187,12 +182,13 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
   const bool use_sorted = sctl && sctl->use;
 
   for (int wbase = warp_global * 32; wbase < n; wbase += warps_total * 32) {
-    const int e = wbase + lane;
+    const int entry = wbase + lane;
     int emit = 0;
     int p = -1;
     unsigned c[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (e < n) {
-      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
+    const unsigned mask = __ballot_sync(0xffffffffu, entry < n);
+    if (entry < n) {
+      p = use_sorted ? sorted[entry] : (entry < nc ? in_closest[entry] : in_any[entry - nc]);
       const VertexRef lv{bb.lv + (size_t)p * bb.bounces * 4};
       const VertexRef ev{bb.ev + (size_t)p * bb.bounces * 4};
       const int4 misc = ps.misc[p];
@@ -232,279 +228,259 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
         rd = ym::mk(rd4.x, rd4.y, rd4.z, rd4.w);
       }
       const float4 hit = ps.hit[p];
-      bool done = false;
 
-      for (int guard = 0; guard < 8192 && !done; ++guard) {
-        switch (phase) {
-          case B_LIGHT: {   // createLightPath, bdpt.cl:458-510
-            const int tri = __float_as_int(hit.w);
-            if (tri < 0 || pend_pdf <= 0.0f) { phase = Q_EYE_START; break; }
-            const Vtx v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-            f4 contrib;
-            if (cnt.i == 1) {
+      // ---- the result of the ray the path waited for ----
+      // Its BRDFs: at the vertex a subpath ray left, at the eye vertex of a light sample, or at
+      // the eye vertex and then the light vertex of a connection; one copy of the lobe choice and
+      // the BRDF for all of them.
+      const bool light = phase == B_LIGHT, subpath = phase == B_LIGHT || phase == B_EYE;
+      const int tri = __float_as_int(hit.w);
+      const bool made = building && tri >= 0 && !(light && pend_pdf <= 0.0f);   // a vertex is made
+      const bool seen = !building && hit.x == 0.0f;                             // a segment is free
+      Vtx v, e;           // the vertex made; the eye vertex of the connection stage
+      v.hp = v.n = e.hp = e.n = ym::splat(0.0f);
+      v.mat = e.mat = 0;
+      if (made) v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
+      if (!building) e = ev.vtx(cnt.i);
+      f4 f0 = ym::splat(0.0f), f1 = ym::splat(0.0f), pn = ym::splat(0.0f);
+      float prob0 = 0.0f;
+      __syncwarp(mask);
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
+        if (side == 0 ? (made && subpath && !(light && cnt.i == 1)) || seen : seen && phase == B_CONN) {
+          Vtx at = e;
+          f4 w_in = phase == B_NEE ? w_i : rd, w_out = ym::splat(0.0f);
+          bool g = (flags & BF_GLOSSY) != 0;
+          float prob = pend_prob;
+          if (subpath) {
+            const VertexRef& sv = light ? lv : ev;
+            const f4 back = -sv.dir(cnt.i - 1);
+            at = sv.vtx(cnt.i - 1);
+            pn = at.n;
+            w_in = light ? back : rd;
+            w_out = light ? rd : back;
+          } else {
+            if (side) {
+              at = lv.vtx(cnt.j);
+              w_in = -lv.dir(cnt.j);
+              w_out = -rd;
+            } else {
+              w_out = -ev.dir(cnt.i);
+            }
+            g = sample_glossy_b(sc.mats[at.mat], seed, prob);
+            if (side == 0) prob0 = prob;
+          }
+          const f4 f = brdf_b(w_in, w_out, at.n, sc.mats[at.mat], g, prob);
+          if (side) f1 = f;
+          else f0 = f;
+        }
+        if (!__any_sync(mask, seen && phase == B_CONN)) break;
+      }
+      if (building) {
+        if (!made) {
+          if (light) {
+            phase = Q_EYE_START;
+          } else if (phase == B_EYE) {
+            phase = Q_CONNECT;
+          } else {   // the camera ray met a light or nothing
+            color = ym::mk(0.4f, 0.4f, 0.4f, 1.0f);
+            if (k >= 0)
+              color = (ym::dot(rd, ld4(sc.lights[k].normal)) < 0.0f) ? ym::mk(1.0f, 1.0f, 1.0f, 1.0f)
+                                                                     : ym::mk(0.1f, 0.1f, 0.1f, 1.0f);
+            phase = Q_FINISH;
+          }
+        } else {   // createLightPath (bdpt.cl:458-510), createEyePath (bdpt.cl:517-558)
+          f4 contrib = ym::mk(1.0f, 1.0f, 1.0f, 1.0f);
+          bool stop = false;
+          const VertexRef& sv = light ? lv : ev;
+          if (subpath) {
+            if (light && cnt.i == 1) {
               const float c1 = ym::div(ym::max(0.0f, ym::dot(lv.vtx(0).n, rd)), pend_pdf);
               contrib = ym::splat(c1) * lv.contrib(0);
             } else {
-              const Vtx pv = lv.vtx(cnt.i - 1);
-              contrib = brdf_bk(-lv.dir(cnt.i - 1), rd, pv.n, sc.mats[pv.mat], (flags & BF_GLOSSY) != 0, pend_prob) *
-                        ym::fmax(0.0f, ym::dot(rd, pv.n));
+              const float cosine = ym::dot(rd, pn);
+              contrib = f0 * (light ? ym::fmax(0.0f, cosine) : ym::max(0.0f, cosine));
               contrib = contrib / pend_pdf;
-              contrib = contrib * lv.contrib(cnt.i - 1);
+              contrib = contrib * sv.contrib(cnt.i - 1);
             }
-            cnt.lp = cnt.i + 1;
-            bool stop = false;
-            if (cnt.i >= 2 && cnt.i > RR) {
-              const float r = draw(seed);
-              const float pr = ym::min(luminance(contrib), 0.95f);
-              if (r >= pr) stop = true;
-              else contrib = contrib * ym::div(1.0f, pr);
-            }
-            lv.store(cnt.i, v, rd, contrib);
-            if (stop || cnt.i + 1 >= BOUNCES) { phase = Q_EYE_START; break; }
-            cnt.i += 1;
-            phase = Q_LIGHT_SAMPLE;
-            break;
-          }
-          case Q_LIGHT_SAMPLE: {   // sample from light vertex i - 1 (bdpt.cl:473-484)
-            const Vtx pv = lv.vtx(cnt.i - 1);
-            const yc_material& m = sc.mats[pv.mat];
-            float prob = 0.0f;
-            const bool g = sample_glossy_b(m, seed, prob);
-            if (prob == 0.0f) { phase = Q_EYE_START; break; }
-            float pdf = 1.0f;
-            const f4 nd = sample_lobe_b(pv, m, g, -lv.dir(cnt.i - 1), seed, pdf);
-            flags = g ? (flags | BF_GLOSSY) : (flags & ~BF_GLOSSY);
-            pend_pdf = pdf;
-            pend_prob = prob;
-            // the reference traces before it tests the pdf (bdpt.cl:486)
-            ro = pv.hp + nd * EPS_F;
-            rd = nd;
-            tmax = INF;
-            k = -1;
-            light_test(sc, ro, rd, tmax, k);
-            c[0]++; c[2]++; c[5]++;
-            phase = B_LIGHT;
-            emit = 1;
-            done = true;
-            break;
-          }
-          case Q_EYE_START: {   // createEyePath: the camera ray (bdpt.cl:517-519)
-            ro = ym::mk(pp.cam.r1.w, pp.cam.r2.w, pp.cam.r3.w, pp.cam.r4.w);
-            const float4 d = ev.at(0, 2);
-            rd = ym::mk(d.x, d.y, d.z, d.w);
-            tmax = INF;
-            k = -1;
-            light_test(sc, ro, rd, tmax, k);
-            cnt.i = 0;
-            c[0]++; c[1]++; c[5]++;
-            phase = B_EYE0;
-            emit = 1;
-            done = true;
-            break;
-          }
-          case B_EYE0: {
-            const int tri = __float_as_int(hit.w);
-            if (tri < 0) {
-              if (k >= 0) {
-                color = (ym::dot(rd, ld4(sc.lights[k].normal)) < 0.0f) ? ym::mk(1.0f, 1.0f, 1.0f, 1.0f)
-                                                                       : ym::mk(0.1f, 0.1f, 0.1f, 1.0f);
-              } else {
-                color = ym::mk(0.4f, 0.4f, 0.4f, 1.0f);
-              }
-              phase = Q_FINISH;
-              break;
-            }
-            const Vtx v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-            ev.store(0, v, rd, ym::mk(1.0f, 1.0f, 1.0f, 1.0f));
-            cnt.ep = 1;
-            cnt.i = 1;
-            phase = Q_EYE_SAMPLE;
-            break;
-          }
-          case Q_EYE_SAMPLE: {   // bdpt.cl:527-535
-            if (cnt.i >= BOUNCES) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
-            const Vtx pv = ev.vtx(cnt.i - 1);
-            const yc_material& m = sc.mats[pv.mat];
-            float prob = 0.0f;
-            const bool g = sample_glossy_b(m, seed, prob);
-            if (prob == 0.0f) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
-            float pdf = 1.0f;
-            const f4 nd = sample_lobe_b(pv, m, g, -ev.dir(cnt.i - 1), seed, pdf);
-            if (pdf <= 0.0f) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
-            flags = g ? (flags | BF_GLOSSY) : (flags & ~BF_GLOSSY);
-            pend_pdf = pdf;
-            pend_prob = prob;
-            ro = pv.hp + nd * EPS_F;
-            rd = nd;
-            tmax = INF;
-            k = -1;
-            light_test(sc, ro, rd, tmax, k);
-            c[0]++; c[2]++; c[5]++;
-            phase = B_EYE;
-            emit = 1;
-            done = true;
-            break;
-          }
-          case B_EYE: {   // bdpt.cl:537-558
-            const int tri = __float_as_int(hit.w);
-            if (tri < 0) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
-            const Vtx v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-            const Vtx pv = ev.vtx(cnt.i - 1);
-            f4 contrib = brdf_bk(rd, -ev.dir(cnt.i - 1), pv.n, sc.mats[pv.mat], (flags & BF_GLOSSY) != 0, pend_prob) *
-                         ym::max(0.0f, ym::dot(rd, pv.n));
-            contrib = contrib / pend_pdf;
-            contrib = contrib * ev.contrib(cnt.i - 1);
-            cnt.ep = cnt.i + 1;
-            bool stop = false;
             if (cnt.i > RR) {
               const float r = draw(seed);
               const float pr = ym::min(luminance(contrib), 0.95f);
               if (r >= pr) stop = true;
               else contrib = contrib * ym::div(1.0f, pr);
             }
-            ev.store(cnt.i, v, rd, contrib);
-            if (stop) { phase = Q_CONNECT; cnt.i = 0; cnt.j = 0; flags = 0; break; }
-            cnt.i += 1;
-            phase = Q_EYE_SAMPLE;
-            break;
+          } else {
+            cnt.i = 0;
           }
-          case Q_CONNECT: {   // shading, bdpt.cl:578-595: start eye vertex i
-            if (cnt.i == 0 && cnt.j == 0 && !(flags & 8)) {
-              color = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
-              weight = 1.0f;
-              ks = 0.0f;
-              conn_live = true;
-              flags = 8;   // connection stage started
-            }
-            if (cnt.i >= cnt.ep || weight == 0.0f) { phase = Q_FINISH; break; }
-            phase = Q_VERTEX;
-            break;
-          }
-          case Q_VERTEX: {   // emission + next-event estimate at eye vertex i (bdpt.cl:591-597, 642-660)
-            const Vtx v = ev.vtx(cnt.i);
-            const yc_material& m = sc.mats[v.mat];
-            sub = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
-            ks = ym::max(ym::max(m.ks.x, ym::max(m.ks.y, m.ks.z)), 0.1f);
-            f4 wi_raw;
-            lj = sample_lights(sc, v, seed, light_pdf, wi_raw);
-            if (lj == -1 || light_pdf <= 0.0f) {
-              // DL = emission
-              color = color + (ev.contrib(cnt.i) * (ld4(m.ke) + ld4(m.ke))) * weight;
-              cnt.j = cnt.lp - 1;
-              phase = Q_CONNECT + 16;   // connections
-              break;
-            }
-            float len = ym::length(wi_raw);
-            len = ym::sub(len, ym::mul(EPS_F, 1.5f));
-            w_i = ym::normalize(wi_raw);
-            ro = v.hp + w_i * EPS_F;
-            rd = w_i;
-            tmax = len;
-            c[0]++; c[3]++;
-            int lk = -1;
-            float tl = len;
-            light_test(sc, ro, rd, tl, lk);
-            if (lk >= 0) { flags |= BF_OCCLUDED; phase = B_NEE; break; }
-            flags &= ~BF_OCCLUDED;
-            c[5]++;
-            phase = B_NEE;
-            emit = 2;
-            done = true;
-            break;
-          }
-          case B_NEE: {   // bdpt.cl:662-671 (MIS off, as shipped)
-            if (hit.x != 0.0f) flags |= BF_OCCLUDED;
-            const Vtx v = ev.vtx(cnt.i);
-            const yc_material& m = sc.mats[v.mat];
-            const f4 em = ld4(m.ke);
-            f4 dl = ym::splat(0.0f) + em;   // light_sample (0) + emission
-            if (!(flags & BF_OCCLUDED)) {
-              float prob = 0.0f;
-              const bool g = sample_glossy_b(m, seed, prob);
-              if (prob == 0.0f) {
-                dl = em;
-              } else {
-                f4 ls = (brdf_bk(w_i, -ev.dir(cnt.i), v.n, m, g, prob) * ld4(sc.lights[lj].ke)) *
-                        ym::fmax(ym::dot(w_i, v.n), 0.0f);
-                ls = ls * ym::div(1.0f, light_pdf);
-                dl = ls + em;
-              }
-            }
-            flags &= ~BF_OCCLUDED;
-            color = color + (ev.contrib(cnt.i) * (em + dl)) * weight;
-            cnt.j = cnt.lp - 1;
-            phase = Q_CONNECT + 16;
-            break;
-          }
-          case Q_CONNECT + 16: {   // next connection j (bdpt.cl:598-615)
-            if (cnt.j <= 0) {
-              color = color + sub * ym::mul(weight, ym::sub(1.0f, ks));
-              weight = ym::mul(weight, ks);
-              cnt.i += 1;
-              phase = Q_CONNECT;
-              break;
-            }
-            const Vtx e_v = ev.vtx(cnt.i);
-            const Vtx l_v = lv.vtx(cnt.j);
-            const f4 dir = ym::normalize(l_v.hp - e_v.hp);
-            const f4 org = e_v.hp + dir * EPS_F;
-            if (ym::dot(dir, e_v.n) <= 0.0f || ym::dot(-dir, l_v.n) <= 0.0f) { cnt.j -= 1; break; }
-            ro = org;
-            rd = dir;
-            tmax = ym::length(l_v.hp - org);
-            c[0]++; c[4]++;
-            int lk = -1;
-            float tl = tmax;
-            light_test(sc, ro, rd, tl, lk);
-            if (lk >= 0) { cnt.j -= 1; break; }   // a light closes the segment: occluded
-            c[5]++;
-            phase = B_CONN;
-            emit = 2;
-            done = true;
-            break;
-          }
-          case B_CONN: {   // bdpt.cl:616-634
-            if (hit.x == 0.0f) {
-              const Vtx e_v = ev.vtx(cnt.i);
-              const Vtx l_v = lv.vtx(cnt.j);
-              float dist = ym::length(l_v.hp - e_v.hp);
-              dist = ym::mul(dist, dist);
-              const f4 wi = rd;
-              const f4 wo = -ev.dir(cnt.i);
-              const float gf = ym::div(ym::mul(ym::max(ym::dot(wi, e_v.n), 0.0f), ym::max(ym::dot(-wi, l_v.n), 0.0f)), dist);
-              float prob = 0.0f;
-              bool g = sample_glossy_b(sc.mats[e_v.mat], seed, prob);
-              const f4 e2l = brdf_bk(wi, wo, e_v.n, sc.mats[e_v.mat], g, prob);
-              g = sample_glossy_b(sc.mats[l_v.mat], seed, prob);
-              const f4 l2e = brdf_bk(-lv.dir(cnt.j), -wi, l_v.n, sc.mats[l_v.mat], g, prob);
-              f4 tlp = lv.contrib(cnt.j);
-              tlp = tlp * ((gf * e2l) * l2e);
-              tlp = tlp * ev.contrib(cnt.i);
-              sub = sub + tlp;
-            }
-            cnt.j -= 1;
-            phase = Q_CONNECT + 16;
-            break;
-          }
-          case Q_FINISH:
-          default: {
-            if (ym::any_nan(color)) color = ym::mk(0.988f, 0.0588f, 0.7529f, 1.0f);
-            const float4 prev = pp.accum[pix];
-            f4 cc = color;
-            if (pp.reset == 1) {
-              cc.w = 1.0f;
-            } else {
-              const int np = (int)prev.w;
-              cc = cc + f4of(prev) * (float)np;
-              cc = cc / (float)(np + 1);
-              cc.w = (float)(np + 1);
-            }
-            pp.accum[pix] = make_float4(cc.x, cc.y, cc.z, cc.w);
-            c[6]++;
-            done = true;
-            break;
+          sv.store(cnt.i, v, rd, contrib);
+          cnt.i += 1;
+          if (light) cnt.lp = cnt.i;
+          else cnt.ep = cnt.i;
+          const bool full = cnt.i >= BOUNCES;
+          phase = light ? (stop || full ? Q_EYE_START : Q_LIGHT_SAMPLE) : (stop || full ? Q_CONNECT : Q_EYE_SAMPLE);
+        }
+      } else if (phase == B_NEE) {   // bdpt.cl:662-671 (MIS off, as shipped)
+        const f4 em = ld4(sc.mats[e.mat].ke);
+        f4 dl = ym::splat(0.0f) + em;   // light_sample (0) + emission
+        if (seen) {
+          if (prob0 == 0.0f) {
+            dl = em;
+          } else {
+            f4 ls = (f0 * ld4(sc.lights[lj].ke)) * ym::fmax(ym::dot(w_i, e.n), 0.0f);
+            ls = ls * ym::div(1.0f, light_pdf);
+            dl = ls + em;
           }
         }
+        color = color + (ev.contrib(cnt.i) * (em + dl)) * weight;
+        cnt.j = cnt.lp - 1;
+        phase = Q_SEGMENTS;
+      } else {   // B_CONN, bdpt.cl:616-634
+        if (seen) {
+          const Vtx l_v = lv.vtx(cnt.j);
+          float dist = ym::length(l_v.hp - e.hp);
+          dist = ym::mul(dist, dist);
+          const float gf = ym::div(ym::mul(ym::max(ym::dot(rd, e.n), 0.0f), ym::max(ym::dot(-rd, l_v.n), 0.0f)), dist);
+          f4 tlp = lv.contrib(cnt.j);
+          tlp = tlp * ((gf * f0) * f1);
+          tlp = tlp * ev.contrib(cnt.i);
+          sub = sub + tlp;
+        }
+        cnt.j -= 1;
+        phase = Q_SEGMENTS;
+      }
+      // ---- a subpath's next direction, from the vertex just made (bdpt.cl:473-484, 527-535) ----
+      int cast = 0;           // the state the next ray will be waited for in
+      f4 org = v.hp, dir = ym::splat(0.0f);
+      float limit = INF;
+      __syncwarp(mask);
+      if (phase == Q_LIGHT_SAMPLE || phase == Q_EYE_SAMPLE) {
+        const yc_material& m = sc.mats[v.mat];
+        const bool on_light = phase == Q_LIGHT_SAMPLE;
+        float prob = 0.0f, pdf = 1.0f;
+        const bool g = sample_glossy_b(m, seed, prob);
+        phase = on_light ? Q_EYE_START : Q_CONNECT;   // unless a direction is drawn
+        if (prob != 0.0f) {
+          dir = sample_lobe_b(v, m, g, -ym::mk(rd.x, rd.y, rd.z, 0.0f), seed, pdf);
+          // (of the light subpath the reference traces before it tests the density, bdpt.cl:486)
+          if (on_light || !(pdf <= 0.0f)) {
+            flags = g ? (flags | BF_GLOSSY) : (flags & ~BF_GLOSSY);
+            pend_pdf = pdf;
+            pend_prob = prob;
+            cast = on_light ? B_LIGHT + CAST : B_EYE + CAST;
+          }
+        }
+      }
+      if (phase == Q_EYE_START && !cast) {   // the camera ray (bdpt.cl:517-519)
+        org = ym::mk(pp.cam.r1.w, pp.cam.r2.w, pp.cam.r3.w, pp.cam.r4.w);
+        const float4 d = ev.at(0, 2);
+        dir = ym::mk(d.x, d.y, d.z, d.w);
+        cnt.i = 0;
+        cast = B_EYE0 + CAST;
+      }
+      if (phase == Q_CONNECT && !cast) {   // shading starts (bdpt.cl:578-595)
+        color = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
+        weight = 1.0f;
+        ks = 0.0f;
+        cnt.i = cnt.j = 0;
+        flags = 8;
+        conn_live = true;
+        phase = cnt.ep > 0 ? Q_VERTEX : Q_FINISH;
+      }
+      // ---- the connection stage until its next ray ----
+      // Each pass takes the path to a segment worth a ray: the light sample of an eye vertex, or
+      // the next light vertex whose segment both ends face. The light loop appears once, for
+      // every kind of ray; a segment a light closes sends the path round again. With one copy
+      // of the stages per state (a switch that looped over rejected segments while other lanes
+      // shaded) a 1280x720 pass over 758K triangles took 4.63 ms of shading, now 3.61 ms.
+      for (;;) {
+        __syncwarp(mask);
+        if (phase == Q_VERTEX) {   // emission + next-event estimate at eye vertex i (bdpt.cl:591-597, 642-660)
+          e = ev.vtx(cnt.i);
+          const yc_material& m = sc.mats[e.mat];
+          sub = ym::mk(0.0f, 0.0f, 0.0f, 1.0f);
+          ks = ym::max(ym::max(m.ks.x, ym::max(m.ks.y, m.ks.z)), 0.1f);
+          f4 wi_raw;
+          lj = sample_lights(sc, e, seed, light_pdf, wi_raw);
+          if (lj == -1 || light_pdf <= 0.0f) {
+            color = color + (ev.contrib(cnt.i) * (ld4(m.ke) + ld4(m.ke))) * weight;   // DL = emission
+            cnt.j = cnt.lp - 1;
+            phase = Q_SEGMENTS;
+          } else {
+            limit = ym::sub(ym::length(wi_raw), ym::mul(EPS_F, 1.5f));
+            w_i = ym::normalize(wi_raw);
+            org = e.hp;
+            dir = w_i;
+            cast = B_NEE + CAST;
+          }
+        }
+        __syncwarp(mask);
+        if (phase == Q_SEGMENTS && !cast) {   // the next connection j (bdpt.cl:598-615)
+          while (cnt.j > 0 && !cast) {
+            const float4 h4 = lv.at(cnt.j, 0), n4 = lv.at(cnt.j, 1);
+            const f4 l_hp = ym::mk(h4.x, h4.y, h4.z, 1.0f), l_n = ym::mk(n4.x, n4.y, n4.z, 0.0f);
+            dir = ym::normalize(l_hp - e.hp);
+            if (ym::dot(dir, e.n) <= 0.0f || ym::dot(-dir, l_n) <= 0.0f) { cnt.j -= 1; continue; }
+            org = e.hp;
+            limit = ym::length(l_hp - (e.hp + dir * EPS_F));
+            cast = B_CONN + CAST;
+          }
+          if (!cast) {
+            color = color + sub * ym::mul(weight, ym::sub(1.0f, ks));
+            weight = ym::mul(weight, ks);
+            cnt.i += 1;
+            phase = cnt.i >= cnt.ep || weight == 0.0f ? Q_FINISH : Q_VERTEX;
+          }
+        }
+        __syncwarp(mask);
+        if (cast) {   // traceRay's light loop (udpt.cl:244-276)
+          const int to = cast - CAST;
+          const bool segment = to == B_NEE || to == B_CONN;
+          ro = to == B_EYE0 ? org : org + dir * EPS_F;
+          rd = dir;
+          tmax = limit;
+          float tl = tmax;
+          int lh = -1;
+          light_test(sc, ro, rd, tl, lh);
+          c[0]++;
+          c[1] += to == B_EYE0;
+          c[2] += to == B_LIGHT || to == B_EYE;
+          c[3] += to == B_NEE;
+          c[4] += to == B_CONN;
+          cast = 0;
+          if (!segment) {
+            k = lh;
+            tmax = tl;
+            phase = to;
+            emit = 1;
+          } else if (lh < 0) {
+            phase = to;
+            emit = 2;
+          } else if (to == B_CONN) {   // a light closes the segment: occluded
+            cnt.j -= 1;
+          } else {
+            const f4 em = ld4(sc.mats[e.mat].ke);
+            color = color + (ev.contrib(cnt.i) * (em + (ym::splat(0.0f) + em))) * weight;
+            cnt.j = cnt.lp - 1;
+            phase = Q_SEGMENTS;
+          }
+          if (emit) c[5]++;
+        }
+        if (!__any_sync(mask, !emit && phase != Q_FINISH)) break;
+      }
+      if (!emit) {   // the running mean of the pixel
+        if (ym::any_nan(color)) color = ym::mk(0.988f, 0.0588f, 0.7529f, 1.0f);
+        const float4 prev = pp.accum[pix];
+        f4 cc = color;
+        if (pp.reset == 1) {
+          cc.w = 1.0f;
+        } else {
+          const int np = (int)prev.w;
+          cc = cc + f4of(prev) * (float)np;
+          cc = cc / (float)(np + 1);
+          cc.w = (float)(np + 1);
+        }
+        pp.accum[pix] = make_float4(cc.x, cc.y, cc.z, cc.w);
+        c[6]++;
       }
       if (emit) {
         ps.misc[p] = make_int4((int)seed, pix, pack_st(phase, flags & 15, lj, k), pack_cnt(cnt));

@@ -152,11 +152,6 @@ struct MisRec {
   }
 };
 
-__device__ __forceinline__ void count_ray(unsigned* c, int kind) {
-  c[0]++;
-  c[kind]++;
-}
-
 }  // namespace
 
 // ---- raygen: pixel prologue, camera ray kept, light point and the first light ray ----
@@ -561,7 +556,11 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
           float tl = tmax;
           int lh = -1;
           light_test(sc, ro, rd, tl, lh);
-          count_ray(c, start ? 1 : go ? 2 : cand == B_NEE ? 3 : 4);
+          c[0]++;
+          c[1] += start;
+          c[2] += go;
+          c[3] += cand == B_NEE;
+          c[4] += cand == B_CONN;
           if (!cand) {
             k = lh;
             tmax = tl;

@@ -21,7 +21,8 @@ enum : int {
   Q_EYE_SAMPLE = 10,
   Q_VERTEX = 11,
   Q_CONNECT = 12,
-  Q_FINISH = 13
+  Q_SEGMENTS = 13,
+  Q_FINISH = 14
 };
 
 // subpath vertices, one 64-byte record (4 float4 fields) per vertex: vertex k of path p,
