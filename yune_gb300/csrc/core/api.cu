@@ -181,7 +181,10 @@ struct yc_ctx {
   yc_kernel_times ktimes{};
   DevBuf<char> flush_buf;
   // BDPT subpath vertices
-  DevBuf<float4> bd_lv, bd_ev;
+  DevBuf<float4> bd_lv, bd_ev, bd_seg;
+  DevBuf<int> bd_q_seg;
+  int bd_shift = yc::FAN_SHIFT;       // segments a path sends at once, for frames of bd_paths paths (log2)
+  size_t bd_paths = 0;
   size_t bd_cap = 0, bd_ev_cap = 0;   // light / eye vertex records (the MIS tracer has no eye records)
   // direct queries
   DevBuf<float> q_rays;
@@ -257,6 +260,36 @@ int ensure_raysort(yc_ctx* c, size_t n) {
     c->rs_cap = n;
   }
   return 0;
+}
+
+// The segments of a bidirectional pass over n paths, and the ray sort's lists for them: 2^FAN_SHIFT
+// a path (180 bytes with the sort's), fewer where an entry would not fit the queues' 32 bits or
+// the device's memory.
+int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
+  for (int shift = c->bd_paths == n ? c->bd_shift : yc::FAN_SHIFT;; --shift) {
+    const size_t m = n << shift;
+    if (shift > 0 && m > ((size_t)1 << 30)) continue;
+    cudaError_t e = cudaSuccess;
+    if (c->bd_seg.n < m) e = c->bd_seg.alloc(m);
+    if (e == cudaSuccess && c->bd_q_seg.n < m) e = c->bd_q_seg.alloc(m);
+    if (e == cudaSuccess && raysort && c->rs_cap < m) {
+      c->rs_cap = 0;
+      e = c->rs_keys.alloc(m);
+      if (e == cudaSuccess) e = c->rs_sorted.alloc(m);
+      if (e == cudaSuccess) c->rs_cap = m;
+    }
+    if (e == cudaSuccess) {
+      c->bd_shift = shift;
+      c->bd_paths = n;
+      return 0;
+    }
+    cudaGetLastError();
+    c->bd_seg.release();
+    c->bd_q_seg.release();
+    if (shift == 0)
+      return fail(e == cudaErrorMemoryAllocation ? YC_E_NOMEM : YC_E_LAUNCH,
+                  std::string("segments of a bidirectional pass: ") + cudaGetErrorString(e));
+  }
 }
 
 // key and sorted-list buffers of the per-pass shade-queue sort, for n paths
@@ -487,8 +520,6 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
   yc::RaySortBufs rsb{};
   if (raysort) {
     if (int e = ensure_raysort(c, (size_t)W * H)) return e;
-    rsb = yc::RaySortBufs{c->rs_keys.p, nullptr, c->rs_hist.p, c->rs_cursor.p, c->rs_blk.p, c->rs_sorted.p, c->rs_ctl.p,
-                          c->rs_ob, c->rs_db, 0, c->rs_threshold};
   }
   // shade-queue sort by phase and material class before the logic kernel (unidirectional
   // passes whose frame can fill a sorted queue, in scenes with a mirror or dielectric:
@@ -523,6 +554,14 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
   if (n_smem > 0)
     if (int e = ensure_pass_spill(c, (size_t)std::max(grid_m, tail_grid) * yc::TRACE_TB_PASS * 2 * (size_t)(cap - n_smem)))
       return e;
+  if (bdpt) {
+    if (int e = ensure_segments(c, (size_t)W * H, raysort)) return e;
+    bb.sg = yc::Segments{c->bd_seg.p, c->bd_shift};
+    bb.q_seg = c->bd_q_seg.p;
+  }
+  if (raysort)
+    rsb = yc::RaySortBufs{c->rs_keys.p, nullptr, c->rs_hist.p, c->rs_cursor.p, c->rs_blk.p, c->rs_sorted.p, c->rs_ctl.p,
+                          c->rs_ob, c->rs_db, 0, c->rs_threshold};
   int cur = 0;
   const int check_every = 6;
   bool finished = false;
@@ -537,13 +576,17 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
     if (mixed) {   // both ray kinds of the round in one launch
       if (raysort) {
         KTimer kt(c, K_RAYSORT);
-        if (yc::launch_raysort(dsc, in_c, in_a, rin, ps.ro, ps.rd, rsb, c->logic_grid, c->stream))
+        if (yc::launch_raysort(dsc, in_c, bdpt ? bb.q_seg : in_a, rin, ps.ro, ps.rd, rsb, c->logic_grid, c->stream, bb.sg))
           return fail(YC_E_LAUNCH, std::string("ray sort: ") + cudaGetErrorString(cudaGetLastError()));
       }
       KTimer kt(c, K_TRACE);
-      if (yc::launch_trace_mixed(dsc, in_c, in_a, rin, ps.ro, ps.rd, ps.hit, c->stats.p, grid_m, c->stream,
-                                 raysort ? rsb.sorted : nullptr, raysort ? rsb.ctl : nullptr, n_smem,
-                                 n_smem > 0 ? c->pass_spill.p : nullptr))
+      const int* sorted = raysort ? rsb.sorted : nullptr;
+      const yc::RaySortCtl* rctl = raysort ? rsb.ctl : nullptr;
+      int* spill = n_smem > 0 ? c->pass_spill.p : nullptr;
+      if (bdpt ? yc::launch_trace_fans(dsc, in_c, bb.q_seg, rin, ps, bb.sg, c->stats.p, grid_m, c->stream, sorted, rctl,
+                                       n_smem, spill)
+               : yc::launch_trace_mixed(dsc, in_c, in_a, rin, ps.ro, ps.rd, ps.hit, c->stats.p, grid_m, c->stream,
+                                        sorted, rctl, n_smem, spill))
         return fail(YC_E_LAUNCH, std::string("trace kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }
     // otherwise the two traces of a round are independent: the any-hit one runs on the
@@ -564,8 +607,9 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
       if (e1) return fail(YC_E_LAUNCH, std::string("extend kernel: ") + cudaGetErrorString(cudaGetLastError()));
       {
         KTimer kt(c, K_OCCL);
-        e2 = yc::launch_trace(dsc, true, in_a, &rin->n_any, &rin->work_any, ps.ro, ps.rd, ps.hit, c->stats.p,
-                              grid_a, s_any);
+        e2 = bdpt ? yc::launch_trace_segments(dsc, bb.q_seg, rin, ps, bb.sg, c->stats.p, grid_a, s_any)
+                  : yc::launch_trace(dsc, true, in_a, &rin->n_any, &rin->work_any, ps.ro, ps.rd, ps.hit, c->stats.p,
+                                     grid_a, s_any);
       }
       if (e2) return fail(YC_E_LAUNCH, std::string("occlusion kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }

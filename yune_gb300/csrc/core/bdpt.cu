@@ -5,11 +5,11 @@
 // an eye subpath (createEyePath, bdpt.cl:513-560), then for every eye vertex adds its
 // emission and next-event estimate and connects it to every light vertex j >= 1 with a
 // shadow ray (shading, bdpt.cl:562-640). Here each path is a state machine like the
-// unidirectional one (udpt.cu): the logic kernel advances it to its next ray, the extend
-// and occlusion kernels trace the queues, and the subpath vertices live in HBM as one
-// 64-byte record per vertex (two full 32-byte sectors: a connection reads two vertices of
-// a path whose neighbours in the queue are unrelated), vertex k of path p at
-// [(p * bounces + k) * 4 + field]:
+// unidirectional one (udpt.cu): the logic kernel advances it to its next subpath ray, or to
+// all shadow rays of one eye vertex, the trace kernel settles both queues, and the subpath
+// vertices live in HBM as one 64-byte record per vertex (two full 32-byte sectors: a
+// connection reads two vertices of a path whose neighbours in the queue are unrelated),
+// vertex k of path p at [(p * bounces + k) * 4 + field]:
 //   field 0: hit point xyz, material index (int bits)
 //   field 1: shading normal xyz
 //   field 2: direction of the ray that reached the vertex xyz
@@ -26,7 +26,8 @@
 namespace yc {
 
 enum : int { BF_GLOSSY = 1 };
-constexpr int CAST = 1;   // a pending cast holds its state + CAST (0: none)
+constexpr int CAST = 1;                         // a ray about to be sent: its state + CAST (0: none),
+constexpr int TO_LIGHT = 8, TO_VERTEX = 9;      // or a segment's kind
 
 struct BCount {
   int i, j, lp, ep;
@@ -163,14 +164,14 @@ void launch_raygen_bdpt(const PassParams& pp, const PathState& ps, const BdptBuf
 
 // ---- logic: advance each path to its next ray ----
 __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps, BdptBuffers bb,
-                                                    const int* __restrict__ in_closest, const int* __restrict__ in_any,
-                                                    const RoundCounters* rc_in, int* out_closest, int* out_any,
+                                                    const int* __restrict__ in_closest, const int* __restrict__ in_fan,
+                                                    const RoundCounters* rc_in, int* out_closest, int* out_fan,
                                                     RoundCounters* rc_out, DevStats* st, const int* __restrict__ sorted,
                                                     const SortCtl* sctl) {
   __shared__ unsigned long long s_cnt[8];   // rays, primary, extension, shadow, connection, traversed, samples
   if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
   __syncthreads();
-  const int nc = rc_in->n_closest, na = rc_in->n_any;
+  const int nc = rc_in->n_closest, na = rc_in->n_fan;
   const int n = nc + na;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -185,10 +186,11 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
     const int entry = wbase + lane;
     int emit = 0;
     int p = -1;
+    FanOut out;   // the segments to send
     unsigned c[7] = {0, 0, 0, 0, 0, 0, 0};
     const unsigned mask = __ballot_sync(0xffffffffu, entry < n);
     if (entry < n) {
-      p = use_sorted ? sorted[entry] : (entry < nc ? in_closest[entry] : in_any[entry - nc]);
+      p = use_sorted ? sorted[entry] : (entry < nc ? in_closest[entry] : in_fan[entry - nc]);
       const VertexRef lv{bb.lv + (size_t)p * bb.bounces * 4};
       const VertexRef ev{bb.ev + (size_t)p * bb.bounces * 4};
       const int4 misc = ps.misc[p];
@@ -200,81 +202,114 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
       int k = ((misc.z >> 13) & 31) - 1;
       BCount cnt = unpack_cnt(misc.w);
       // While the subpaths are built (B_LIGHT, B_EYE0, B_EYE) the connection stage's
-      // fields (colour, sub-sum, NEE direction) are dead: Q_CONNECT initialises them.
+      // fields (colour, sub-sum, density of the light sample) are dead: Q_CONNECT initialises them.
       // They are loaded in the connection states only and stored once the stage has
       // started; the ray origin is read only where a hit point is built from it.
       const bool building = phase == B_LIGHT || phase == B_EYE0 || phase == B_EYE;
       bool conn_live = !building;
-      f4 color = ym::splat(0.0f), sub = ym::splat(0.0f), w_i = ym::splat(0.0f);
+      f4 color = ym::splat(0.0f), sub = ym::splat(0.0f);
       float light_pdf = 0.0f;
       if (!building) {
         color = f4of(ps.thr[p]);
         sub = f4of(ps.thr_next[p]);
-        const float4 nee = ps.indirect[p];
-        w_i = ym::mk(nee.x, nee.y, nee.z, 0.0f);
-        light_pdf = nee.w;
+        light_pdf = ps.indirect[p].x;
       }
       float4 dv = ps.direct[p];
       float weight = dv.x, ks = dv.y, pend_pdf = dv.z, pend_prob = dv.w;
       f4 ro = ym::splat(0.0f), rd = ym::splat(0.0f);
       float tmax = 0.0f;
       if (building) {
-        const float4 ro4 = ps.ro[p];
+        const float4 ro4 = ps.ro[p], rd4 = ps.rd[p];
         ro = ym::mk(ro4.x, ro4.y, ro4.z, 1.0f);
-        tmax = ro4.w;
-      }
-      if (building || phase == B_CONN) {
-        const float4 rd4 = ps.rd[p];
         rd = ym::mk(rd4.x, rd4.y, rd4.z, rd4.w);
+        tmax = ro4.w;
       }
       const float4 hit = ps.hit[p];
 
-      // ---- the result of the ray the path waited for ----
-      // Its BRDFs: at the vertex a subpath ray left, at the eye vertex of a light sample, or at
-      // the eye vertex and then the light vertex of a connection; one copy of the lobe choice and
-      // the BRDF for all of them.
+      // ---- the result of the ray, or of the segments, the path waited for ----
+      // A subpath ray's vertex takes the BRDF at the vertex the ray left; a free segment to a
+      // light the BRDF at the eye vertex, a free one to a light vertex those at both ends, in
+      // the order the reference connects them. One evaluation (lobe choice, BRDF) a pass for
+      // each lane that has one left, so that one copy of the code serves them all.
       const bool light = phase == B_LIGHT, subpath = phase == B_LIGHT || phase == B_EYE;
       const int tri = __float_as_int(hit.w);
       const bool made = building && tri >= 0 && !(light && pend_pdf <= 0.0f);   // a vertex is made
-      const bool seen = !building && hit.x == 0.0f;                             // a segment is free
       Vtx v, e;           // the vertex made; the eye vertex of the connection stage
       v.hp = v.n = e.hp = e.n = ym::splat(0.0f);
       v.mat = e.mat = 0;
+      FanIn fan{0, 0};
       if (made) v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
-      if (!building) e = ev.vtx(cnt.i);
-      f4 f0 = ym::splat(0.0f), f1 = ym::splat(0.0f), pn = ym::splat(0.0f);
-      float prob0 = 0.0f;
-      __syncwarp(mask);
-#pragma unroll 1
-      for (int side = 0; side < 2; ++side) {
-        if (side == 0 ? (made && subpath && !(light && cnt.i == 1)) || seen : seen && phase == B_CONN) {
+      if (!building) {
+        e = ev.vtx(cnt.i);
+        fan.load(ps.job[p]);
+        if (fan.vertex(0) == 0 && !(fan.free & 1u)) {   // the light sample is occluded: DL = emission
+          const f4 em = ld4(sc.mats[e.mat].ke);
+          color = color + (ev.contrib(cnt.i) * (em + (ym::splat(0.0f) + em))) * weight;
+        }
+      }
+      f4 f0 = ym::splat(0.0f), pn = ym::splat(0.0f);
+      bool left = made && subpath && !(light && cnt.i == 1);   // the BRDF where the subpath ray left
+      bool far_end = false;                                    // of the first free segment
+      for (;;) {
+        const bool has = left || fan.free;
+        if (!__any_sync(mask, has)) break;
+        if (has) {
           Vtx at = e;
-          f4 w_in = phase == B_NEE ? w_i : rd, w_out = ym::splat(0.0f);
+          f4 w_in = rd, w_out = rd, dir = ym::splat(0.0f);
           bool g = (flags & BF_GLOSSY) != 0;
           float prob = pend_prob;
-          if (subpath) {
+          int j = 0;
+          if (left) {
             const VertexRef& sv = light ? lv : ev;
             const f4 back = -sv.dir(cnt.i - 1);
             at = sv.vtx(cnt.i - 1);
             pn = at.n;
-            w_in = light ? back : rd;
-            w_out = light ? rd : back;
+            if (light) w_in = back;
+            else w_out = back;
           } else {
-            if (side) {
-              at = lv.vtx(cnt.j);
-              w_in = -lv.dir(cnt.j);
-              w_out = -rd;
+            const int sg = __ffs(fan.free) - 1;
+            const float4 d4 = bb.sg.seg[((size_t)p << bb.sg.shift) + sg];
+            dir = ym::mk(d4.x, d4.y, d4.z, 0.0f);
+            j = fan.vertex(sg);
+            if (far_end) {
+              at = lv.vtx(j);
+              w_in = -lv.dir(j);
+              w_out = -dir;
             } else {
+              w_in = dir;
               w_out = -ev.dir(cnt.i);
             }
             g = sample_glossy_b(sc.mats[at.mat], seed, prob);
-            if (side == 0) prob0 = prob;
           }
           const f4 f = brdf_b(w_in, w_out, at.n, sc.mats[at.mat], g, prob);
-          if (side) f1 = f;
-          else f0 = f;
+          if (left) {
+            f0 = f;
+            left = false;
+          } else if (j == 0) {   // the light sample, bdpt.cl:662-671 (MIS off, as shipped)
+            const f4 em = ld4(sc.mats[e.mat].ke);
+            f4 dl = em;
+            if (prob != 0.0f) {
+              f4 ls = (f * ld4(sc.lights[lj].ke)) * ym::fmax(ym::dot(dir, e.n), 0.0f);
+              ls = ls * ym::div(1.0f, light_pdf);
+              dl = ls + em;
+            }
+            color = color + (ev.contrib(cnt.i) * (em + dl)) * weight;
+            fan.free &= fan.free - 1u;
+          } else if (!far_end) {
+            f0 = f;
+            far_end = true;
+          } else {               // a connection, bdpt.cl:616-634
+            float dist = ym::length(at.hp - e.hp);
+            dist = ym::mul(dist, dist);
+            const float gf = ym::div(ym::mul(ym::max(ym::dot(dir, e.n), 0.0f), ym::max(ym::dot(-dir, at.n), 0.0f)), dist);
+            f4 tlp = lv.contrib(j);
+            tlp = tlp * ((gf * f0) * f);
+            tlp = tlp * ev.contrib(cnt.i);
+            sub = sub + tlp;
+            far_end = false;
+            fan.free &= fan.free - 1u;
+          }
         }
-        if (!__any_sync(mask, seen && phase == B_CONN)) break;
       }
       if (building) {
         if (!made) {
@@ -319,37 +354,11 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
           const bool full = cnt.i >= BOUNCES;
           phase = light ? (stop || full ? Q_EYE_START : Q_LIGHT_SAMPLE) : (stop || full ? Q_CONNECT : Q_EYE_SAMPLE);
         }
-      } else if (phase == B_NEE) {   // bdpt.cl:662-671 (MIS off, as shipped)
-        const f4 em = ld4(sc.mats[e.mat].ke);
-        f4 dl = ym::splat(0.0f) + em;   // light_sample (0) + emission
-        if (seen) {
-          if (prob0 == 0.0f) {
-            dl = em;
-          } else {
-            f4 ls = (f0 * ld4(sc.lights[lj].ke)) * ym::fmax(ym::dot(w_i, e.n), 0.0f);
-            ls = ls * ym::div(1.0f, light_pdf);
-            dl = ls + em;
-          }
-        }
-        color = color + (ev.contrib(cnt.i) * (em + dl)) * weight;
-        cnt.j = cnt.lp - 1;
-        phase = Q_SEGMENTS;
-      } else {   // B_CONN, bdpt.cl:616-634
-        if (seen) {
-          const Vtx l_v = lv.vtx(cnt.j);
-          float dist = ym::length(l_v.hp - e.hp);
-          dist = ym::mul(dist, dist);
-          const float gf = ym::div(ym::mul(ym::max(ym::dot(rd, e.n), 0.0f), ym::max(ym::dot(-rd, l_v.n), 0.0f)), dist);
-          f4 tlp = lv.contrib(cnt.j);
-          tlp = tlp * ((gf * f0) * f1);
-          tlp = tlp * ev.contrib(cnt.i);
-          sub = sub + tlp;
-        }
-        cnt.j -= 1;
-        phase = Q_SEGMENTS;
+      } else {
+        phase = Q_SEGMENTS;   // the vertex's light vertices not tried yet, if any
       }
       // ---- a subpath's next direction, from the vertex just made (bdpt.cl:473-484, 527-535) ----
-      int cast = 0;           // the state the next ray will be waited for in
+      int cast = 0;           // the next ray: the state it will be waited for in + CAST, or a segment's kind
       f4 org = v.hp, dir = ym::splat(0.0f);
       float limit = INF;
       __syncwarp(mask);
@@ -386,12 +395,15 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
         conn_live = true;
         phase = cnt.ep > 0 ? Q_VERTEX : Q_FINISH;
       }
-      // ---- the connection stage until its next ray ----
-      // Each pass takes the path to a segment worth a ray: the light sample of an eye vertex, or
-      // the next light vertex whose segment both ends face. The light loop appears once, for
-      // every kind of ray; a segment a light closes sends the path round again. With one copy
-      // of the stages per state (a switch that looped over rejected segments while other lanes
-      // shaded) a 1280x720 pass over 758K triangles took 4.63 ms of shading, now 3.61 ms.
+      // ---- the connection stage until its next rays ----
+      // The segments of an eye vertex, to the light sample and to every light vertex where both
+      // ends face each other and no light is in between, are sent in one round (they depend on
+      // no random number that a result draws): a path goes through as many rounds as it has
+      // vertices, not segments. Each pass of the loop takes a lane past one light loop, which
+      // serves every kind of ray. A round costs its launches and the chains of loads of its
+      // last lanes, so fewer and larger ones pay in every kernel: a 1280x720 pass over 758K
+      // triangles took 66 rounds and 15.3 ms with one segment a round, 24 rounds and 9.6 ms
+      // with eight (trace 8.6 -> 5.2 ms, shading 3.6 -> 2.7, sorts 3.0 -> 1.7).
       for (;;) {
         __syncwarp(mask);
         if (phase == Q_VERTEX) {   // emission + next-event estimate at eye vertex i (bdpt.cl:591-597, 642-660)
@@ -401,69 +413,71 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
           ks = ym::max(ym::max(m.ks.x, ym::max(m.ks.y, m.ks.z)), 0.1f);
           f4 wi_raw;
           lj = sample_lights(sc, e, seed, light_pdf, wi_raw);
+          cnt.j = cnt.lp - 1;
+          phase = Q_SEGMENTS;
+          org = e.hp;
           if (lj == -1 || light_pdf <= 0.0f) {
             color = color + (ev.contrib(cnt.i) * (ld4(m.ke) + ld4(m.ke))) * weight;   // DL = emission
-            cnt.j = cnt.lp - 1;
-            phase = Q_SEGMENTS;
           } else {
             limit = ym::sub(ym::length(wi_raw), ym::mul(EPS_F, 1.5f));
-            w_i = ym::normalize(wi_raw);
-            org = e.hp;
-            dir = w_i;
-            cast = B_NEE + CAST;
+            dir = ym::normalize(wi_raw);
+            cast = TO_LIGHT;
           }
         }
         __syncwarp(mask);
         if (phase == Q_SEGMENTS && !cast) {   // the next connection j (bdpt.cl:598-615)
-          while (cnt.j > 0 && !cast) {
+          org = e.hp;
+          while (cnt.j > 0 && !cast && !out.full(bb)) {
             const float4 h4 = lv.at(cnt.j, 0), n4 = lv.at(cnt.j, 1);
             const f4 l_hp = ym::mk(h4.x, h4.y, h4.z, 1.0f), l_n = ym::mk(n4.x, n4.y, n4.z, 0.0f);
             dir = ym::normalize(l_hp - e.hp);
             if (ym::dot(dir, e.n) <= 0.0f || ym::dot(-dir, l_n) <= 0.0f) { cnt.j -= 1; continue; }
-            org = e.hp;
             limit = ym::length(l_hp - (e.hp + dir * EPS_F));
-            cast = B_CONN + CAST;
+            cast = TO_VERTEX;
           }
           if (!cast) {
-            color = color + sub * ym::mul(weight, ym::sub(1.0f, ks));
-            weight = ym::mul(weight, ks);
-            cnt.i += 1;
-            phase = cnt.i >= cnt.ep || weight == 0.0f ? Q_FINISH : Q_VERTEX;
+            if (out.n > 0) {
+              phase = B_FAN;
+              emit = 2;
+            } else {   // every light vertex tried
+              color = color + sub * ym::mul(weight, ym::sub(1.0f, ks));
+              weight = ym::mul(weight, ks);
+              cnt.i += 1;
+              phase = cnt.i >= cnt.ep || weight == 0.0f ? Q_FINISH : Q_VERTEX;
+            }
           }
         }
         __syncwarp(mask);
         if (cast) {   // traceRay's light loop (udpt.cl:244-276)
-          const int to = cast - CAST;
-          const bool segment = to == B_NEE || to == B_CONN;
-          ro = to == B_EYE0 ? org : org + dir * EPS_F;
-          rd = dir;
-          tmax = limit;
-          float tl = tmax;
+          const bool segment = cast >= TO_LIGHT;
+          const f4 from = cast == B_EYE0 + CAST ? org : org + dir * EPS_F;
+          float tl = limit;
           int lh = -1;
-          light_test(sc, ro, rd, tl, lh);
+          light_test(sc, from, dir, tl, lh);
           c[0]++;
-          c[1] += to == B_EYE0;
-          c[2] += to == B_LIGHT || to == B_EYE;
-          c[3] += to == B_NEE;
-          c[4] += to == B_CONN;
-          cast = 0;
+          c[1] += cast == B_EYE0 + CAST;
+          c[2] += cast == B_LIGHT + CAST || cast == B_EYE + CAST;
+          c[3] += cast == TO_LIGHT;
+          c[4] += cast == TO_VERTEX;
           if (!segment) {
+            ro = from;
+            rd = dir;
             k = lh;
             tmax = tl;
-            phase = to;
+            phase = cast - CAST;
             emit = 1;
-          } else if (lh < 0) {
-            phase = to;
-            emit = 2;
-          } else if (to == B_CONN) {   // a light closes the segment: occluded
-            cnt.j -= 1;
+            c[5]++;
           } else {
-            const f4 em = ld4(sc.mats[e.mat].ke);
-            color = color + (ev.contrib(cnt.i) * (em + (ym::splat(0.0f) + em))) * weight;
-            cnt.j = cnt.lp - 1;
-            phase = Q_SEGMENTS;
+            if (lh < 0) {
+              out.add(bb, p, cast == TO_VERTEX ? cnt.j : 0, dir, limit);
+              c[5]++;
+            } else if (cast == TO_LIGHT) {   // a light closes the segment: occluded
+              const f4 em = ld4(sc.mats[e.mat].ke);
+              color = color + (ev.contrib(cnt.i) * (em + (ym::splat(0.0f) + em))) * weight;
+            }
+            if (cast == TO_VERTEX) cnt.j -= 1;
           }
-          if (emit) c[5]++;
+          cast = 0;
         }
         if (!__any_sync(mask, !emit && phase != Q_FINISH)) break;
       }
@@ -487,25 +501,19 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
         if (conn_live) {
           ps.thr[p] = make_float4(color.x, color.y, color.z, color.w);
           ps.thr_next[p] = make_float4(sub.x, sub.y, sub.z, sub.w);
-          ps.indirect[p] = make_float4(w_i.x, w_i.y, w_i.z, light_pdf);
+          ps.indirect[p] = make_float4(light_pdf, 0.0f, 0.0f, 0.0f);
         }
         ps.direct[p] = make_float4(weight, ks, pend_pdf, pend_prob);
-        ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
-        ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
+        if (emit == 2) {
+          ps.ro[p] = make_float4(e.hp.x, e.hp.y, e.hp.z, 0.0f);
+          ps.job[p] = make_int4((int)out.js, (int)(out.js >> 32), 0, out.n);
+        } else {
+          ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
+          ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
+        }
       }
     }
-    const unsigned mc = __ballot_sync(0xffffffffu, emit == 1);
-    const unsigned ma = __ballot_sync(0xffffffffu, emit == 2);
-    int bc = 0, ba = 0;
-    if (lane == 0) {
-      if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
-      if (ma) ba = atomicAdd(&rc_out->n_any, __popc(ma));
-    }
-    bc = __shfl_sync(0xffffffffu, bc, 0);
-    ba = __shfl_sync(0xffffffffu, ba, 0);
-    const unsigned below = (1u << lane) - 1;
-    if (emit == 1) out_closest[bc + __popc(mc & below)] = p;
-    if (emit == 2) out_any[ba + __popc(ma & below)] = p;
+    append_bdpt(bb, emit, p, out.n, out_closest, out_fan, rc_out);
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
       unsigned x = c[q];
@@ -527,10 +535,10 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
 }
 
 void launch_logic_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                       const int* in_any, const RoundCounters* rc_in, int* out_closest, int* out_any,
+                       const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
                        RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted,
                        const SortCtl* sctl) {
-  k_logic_bdpt<<<grid, 256, 0, s>>>(pp, ps, bb, in_closest, in_any, rc_in, out_closest, out_any, rc_out, st, sorted,
+  k_logic_bdpt<<<grid, 256, 0, s>>>(pp, ps, bb, in_closest, in_fan, rc_in, out_closest, out_fan, rc_out, st, sorted,
                                     sctl);
 }
 

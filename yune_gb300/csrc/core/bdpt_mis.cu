@@ -16,7 +16,7 @@
 //   1 / (1 + (w_{Y->L} c_L / d2)^2 (r_L + s_L w_{L,rev}^2) + (w_{L->Y} c_Y / d2)^2 (r_Y + s_Y w_{Y,rev}^2)).
 // The random-number order, the material and light models and the operation order are
 // those of the CPU statement the parity tests compare against; each sample is one state
-// machine as in bdpt.cu (one ray in flight), with the light subpath in 64-byte vertex
+// machine as in bdpt.cu (one subpath ray, or the segments of one eye vertex, in flight), with the light subpath in 64-byte vertex
 // records, vertex k of path p at [(p * bounces + k) * 4 + field]:
 //   field 0: hit point xyz, material index (int bits; -1 for the point on the light)
 //   field 1: shading normal xyz, r
@@ -25,7 +25,7 @@
 // The eye subpath is walked vertex by vertex: next-event estimate, then the connections
 // to every stored light vertex, then the next eye ray. Path slot fields:
 //   thr      pixel colour              thr_next  eye throughput xyz, r of the eye vertex
-//   direct   pending shadow-ray contribution xyz, s of the eye vertex
+//   direct   light sample's contribution if its segment is free xyz, s of the eye vertex
 //   indirect throughput after the pending bounce xyz, its solid-angle density
 //   ls       cosine toward the pending ray at its origin, acc of the origin vertex,
 //            area density of the light subpath's start point
@@ -253,17 +253,18 @@ void launch_raygen_bdpt_mis(const PassParams& pp, const PathState& ps, const Bdp
 // of 128 per SM measured best (unbounded, 210 in two: 2.98 ms per two 512x512 passes; three:
 // 2.70; four, 386 B spilled: 2.87; five, 768 B: 3.22).
 constexpr int MIS_TB = 128;
+constexpr int TO_LIGHT = 1, TO_VERTEX = 2;   // a segment's kind
 __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, PathState ps, BdptBuffers bb,
                                                         const int* __restrict__ in_closest,
-                                                        const int* __restrict__ in_any, const RoundCounters* rc_in,
-                                                        int* out_closest, int* out_any, RoundCounters* rc_out,
+                                                        const int* __restrict__ in_fan, const RoundCounters* rc_in,
+                                                        int* out_closest, int* out_fan, RoundCounters* rc_out,
                                                         DevStats* st, const int* __restrict__ sorted,
                                                         const SortCtl* sctl) {
   // per-warp counts of rays, primary, extension, shadow, connection, traversed, samples,
   // added to the device counters when the warp leaves (no block barrier: warps finish at
   // different times)
   unsigned w_cnt[7] = {0, 0, 0, 0, 0, 0, 0};
-  const int nc = rc_in->n_closest, na = rc_in->n_any;
+  const int nc = rc_in->n_closest, na = rc_in->n_fan;
   const int n = nc + na;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -278,10 +279,11 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
     const int e = wbase + lane;
     int emit = 0;
     int p = -1;
+    FanOut out;   // the segments to send
     unsigned c[7] = {0, 0, 0, 0, 0, 0, 0};
     const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
-      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
+      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_fan[e - nc]);
       const MisRec lv{bb.lv + (size_t)p * bb.bounces * 4};
       const int4 misc = ps.misc[p];
       uint32_t seed = (uint32_t)misc.x;
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
       // shadow ray's own origin and direction are not needed after it is traced
       const bool eye_state = phase >= B_EYE;
       const bool pending = phase == B_LIGHT || phase == B_EYE;
-      const bool shadow = phase == B_NEE || phase == B_CONN;
+      const bool shadow = phase == B_FAN;
       const float4 l4 = ps.ls[p];
       float c_out = l4.x, acc = l4.y;
       const float p0 = l4.z;
@@ -343,10 +345,13 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
       x.mat = 0;
       f4 lp = ym::splat(0.0f);      // toward the vertex before it
       float r_x = 0.0f, s_x = 0.0f;
+      FanIn fan{0, 0};              // the free segments to light vertices
       if (shadow) {
-        if (hit.x == 0.0f) {
+        fan.load(ps.job[p]);
+        w_color = fan.free != 0;
+        if (fan.vertex(0) == 0 && (fan.free & 1u)) {   // the light sample
           color = color + pend;
-          w_color = true;
+          fan.free &= ~1u;
         }
         phase = M_CONN;
       } else {
@@ -413,7 +418,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
         }
       }
       // ---- an eye vertex's emission, and its light sample ----
-      int cand = 0;             // a segment to a light or a light vertex: B_NEE or B_CONN
+      int cand = 0;             // a segment to send: TO_LIGHT or TO_VERTEX
       f4 dir = ym::splat(0.0f); //   its direction, squared length, length and end cosines
       float d2 = 0.0f, dist = 0.0f, cy = 0.0f, cl = 0.0f, pk = 0.0f;
       int at = 0;               //   the light, or the light vertex, at its end
@@ -438,22 +443,37 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
             dir = v * ym::rcp(dist);
             cy = ym::dot(dir, y.n);
             cl = -ym::dot(dir, ld4(L.normal));
-            if (cy > 0.0f && cl > 0.0f) cand = B_NEE;
+            if (cy > 0.0f && cl > 0.0f) cand = TO_LIGHT;
           }
         }
       }
-      // Each pass over the stages below takes the path to a ray: the next segment of the eye
-      // vertex worth a shadow ray, or the subpath's next direction. The evaluation at a vertex
-      // (two densities and the BRDF), which is most of the work, appears once, for the
-      // segments, for the light vertex at a connection's other end and for the new
-      // directions alike, so that lanes in different states run it together. With one copy of
-      // the stages per state and the evaluation in called functions the kernel ran 8-9 of 32
-      // lanes (loops over rejected segments among them) at 195 registers; two 512x512 passes
-      // of the four-light Cornell box took 5.75 ms of shading, now 2.70 ms.
+      // Each pass over the stages below takes the path one step on: a free connection is
+      // evaluated, a segment of the eye vertex is collected, or the subpath's next direction is
+      // drawn. The evaluation at a vertex (two densities and the BRDF), which is most of the
+      // work, appears once, for the light sample, both ends of a connection and the new
+      // directions alike, so that lanes in different states run it together, and the segments
+      // of an eye vertex are traced in one round, before the connections are evaluated (no
+      // random number is drawn between them): only the free ones are. Two 512x512 passes of
+      // the four-light Cornell box took 84 rounds and 6.4 ms with one segment a round, 48 and
+      // 4.9 ms with eight (trace 2.44 -> 1.69 ms, shading 2.69 -> 2.34).
+      // With one copy of the stages per state and the evaluation in called functions the kernel
+      // ran 8-9 of 32 lanes (loops over rejected segments among them) at 195 registers: 5.75 ms
+      // of shading.
       for (;;) {
         __syncwarp(mask);
-        if (phase == M_CONN && !cand) {   // the next light vertex both ends of whose segment face each other
-          while (cnt.j <= cnt.nl && cnt.m + cnt.j + 1 <= KMAX && !cand) {
+        const bool conn = fan.free != 0;
+        if (conn) {   // the next connection
+          const int sg = __ffs(fan.free) - 1;
+          fan.free &= fan.free - 1u;
+          at = fan.vertex(sg);
+          const float4 h4 = lv.at(at, 0), n4 = lv.at(at, 1), s4 = bb.sg.seg[((size_t)p << bb.sg.shift) + sg];
+          const f4 v = ym::mk(h4.x, h4.y, h4.z, 1.0f) - y.hp;
+          d2 = ym::dot(v, v);
+          dir = ym::mk(s4.x, s4.y, s4.z, 0.0f);
+          cy = ym::dot(dir, y.n);
+          cl = -ym::dot(dir, ym::mk(n4.x, n4.y, n4.z, 0.0f));
+        } else if (phase == M_CONN && !cand) {   // the next light vertex both ends of whose segment face each other
+          while (cnt.j <= cnt.nl && cnt.m + cnt.j + 1 <= KMAX && !cand && !out.full(bb)) {
             at = cnt.j++;
             const float4 h4 = lv.at(at, 0), n4 = lv.at(at, 1);
             const f4 v = ym::mk(h4.x, h4.y, h4.z, 1.0f) - y.hp;
@@ -462,9 +482,12 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
             dir = v * ym::rcp(dist);
             cy = ym::dot(dir, y.n);
             cl = -ym::dot(dir, ym::mk(n4.x, n4.y, n4.z, 0.0f));
-            if (cy > 0.0f && cl > 0.0f) cand = B_CONN;
+            if (cy > 0.0f && cl > 0.0f) cand = TO_VERTEX;
           }
-          if (!cand) phase = M_CONT;
+          if (!cand) {
+            phase = out.n > 0 ? (int)B_FAN : (int)M_CONT;
+            if (out.n > 0) emit = 2;
+          }
         }
         __syncwarp(mask);
         const bool light = phase == M_LIGHT_CONT;
@@ -488,7 +511,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
         float lr = 0.0f, lsv = 0.0f;
 #pragma unroll 1
         for (int side = 0; side < 2; ++side) {
-          if (side == 0 ? cand || go : cand == B_CONN) {
+          if (side == 0 ? conn || cand == TO_LIGHT || go : conn) {
             f4 a = light ? lp : wp, b = dir;
             Vtx v = light ? x : y;
             if (side) {
@@ -503,10 +526,9 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
             if (side) el = r;
             else ev = r;
           }
-          if (!__any_sync(mask, cand == B_CONN)) break;
+          if (!__any_sync(mask, conn)) break;
         }
-        if (cand) {
-          const bool conn = cand == B_CONN;
+        if (conn || cand == TO_LIGHT) {
           float ls, es, g;
           f4 c3;
           if (conn) {
@@ -523,8 +545,9 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
             c3 = (beta * ev.f) * rgb(sc.lights[at].ke);
           }
           const float w = ym::div(1.0f, ym::add(ym::add(1.0f, ls), es));
-          pend = c3 * ym::mul(g, w);
-          w_pend = true;
+          const f4 part = c3 * ym::mul(g, w);
+          if (conn) color = color + part;
+          else pend = part;
         } else if (go) {
           if (ev.fwd > 0.0f) {
             const Vtx v = light ? x : y;
@@ -551,7 +574,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
             rd = ym::mk(d.x, d.y, d.z, d.w);
             cnt.m = 0;
           } else if (cand) {
-            tmax = ym::sub(dist, ym::mul(EPS_F, cand == B_CONN ? 2.0f : 1.5f));
+            tmax = ym::sub(dist, ym::mul(EPS_F, cand == TO_VERTEX ? 2.0f : 1.5f));
           }
           float tl = tmax;
           int lh = -1;
@@ -559,8 +582,8 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
           c[0]++;
           c[1] += start;
           c[2] += go;
-          c[3] += cand == B_NEE;
-          c[4] += cand == B_CONN;
+          c[3] += cand == TO_LIGHT;
+          c[4] += cand == TO_VERTEX;
           if (!cand) {
             k = lh;
             tmax = tl;
@@ -568,10 +591,9 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
             phase = start ? B_EYE0 : light ? B_LIGHT : B_EYE;
             emit = 1;
           } else if (lh < 0) {   // (a light that closes the segment occludes it)
-            phase = cand;
-            emit = 2;
+            out.add(bb, p, cand == TO_VERTEX ? at : 0, dir, tmax);
           }
-          if (emit) c[5]++;
+          if (!cand || lh < 0) c[5]++;
           cand = 0;
         }
         if (!__any_sync(mask, !emit && phase != M_FINISH)) break;
@@ -605,22 +627,16 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
           ps.nrm[p] = make_float4(y.n.x, y.n.y, y.n.z, 0.0f);
           ps.wo[p] = make_float4(-wp.x, -wp.y, -wp.z, 0.0f);
         }
-        ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
-        ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
+        if (emit == 2) {
+          ps.ro[p] = make_float4(y.hp.x, y.hp.y, y.hp.z, 0.0f);
+          ps.job[p] = make_int4((int)out.js, (int)(out.js >> 32), 0, out.n);
+        } else {
+          ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
+          ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
+        }
       }
     }
-    const unsigned mc = __ballot_sync(0xffffffffu, emit == 1);
-    const unsigned ma = __ballot_sync(0xffffffffu, emit == 2);
-    int bc = 0, ba = 0;
-    if (lane == 0) {
-      if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
-      if (ma) ba = atomicAdd(&rc_out->n_any, __popc(ma));
-    }
-    bc = __shfl_sync(0xffffffffu, bc, 0);
-    ba = __shfl_sync(0xffffffffu, ba, 0);
-    const unsigned below = (1u << lane) - 1;
-    if (emit == 1) out_closest[bc + __popc(mc & below)] = p;
-    if (emit == 2) out_any[ba + __popc(ma & below)] = p;
+    append_bdpt(bb, emit, p, out.n, out_closest, out_fan, rc_out);
 #pragma unroll
     for (int q = 0; q < 7; ++q) w_cnt[q] += c[q];
   }
@@ -643,11 +659,11 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
 }
 
 void launch_logic_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                           const int* in_any, const RoundCounters* rc_in, int* out_closest, int* out_any,
+                           const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
                            RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted,
                            const SortCtl* sctl) {
   // (grid counts blocks of 256)
-  k_logic_bdpt_mis<<<grid * (256 / MIS_TB), MIS_TB, 0, s>>>(pp, ps, bb, in_closest, in_any, rc_in, out_closest, out_any,
+  k_logic_bdpt_mis<<<grid * (256 / MIS_TB), MIS_TB, 0, s>>>(pp, ps, bb, in_closest, in_fan, rc_in, out_closest, out_fan,
                                                             rc_out, st, sorted, sctl);
 }
 

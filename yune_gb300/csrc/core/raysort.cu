@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(RS_TB) k_rs_key(Box box, const int* __restrict
                                                   const int* __restrict__ q_any, const RoundCounters* rc,
                                                   SF<float4> ro, SF<float4> rd,
                                                   unsigned* keys, unsigned* hist, int threshold, int ob, int db,
-                                                  int jb) {
+                                                  int jb, Segments sg) {
   const int nc = rc->n_closest, n = nc + rc->n_any;
   if (threshold <= 0 || n < threshold) return;   // uniform over the grid
   const int lane = threadIdx.x & 31;
@@ -74,9 +74,10 @@ __global__ void __launch_bounds__(RS_TB) k_rs_key(Box box, const int* __restrict
     float4 o[RS_U], d[RS_U];
 #pragma unroll
     for (int u = 0; u < RS_U; ++u) {
-      const int pc = p[u] >= 0 ? p[u] : 0;   // idle lanes read slot 0 (n > 0 here) and discard it
-      o[u] = __ldg(&ro[pc]);
-      d[u] = __ldg(&rd[pc]);
+      const int e = wbase + u * 32 + lane, pc = e < n ? p[u] : 0;   // idle lanes read slot 0 (n > 0 here) and discard it
+      const bool segment = sg.seg && e >= nc && e < n;
+      o[u] = __ldg(&ro[segment ? pc >> sg.shift : pc]);
+      d[u] = __ldg(segment ? sg.seg + pc : &rd[pc]);
     }
 #pragma unroll
     for (int u = 0; u < RS_U; ++u) {
@@ -206,10 +207,11 @@ int raysort_bins(int ob, int db, int jb) { return 1 << (3 * (ob + db) + jb + 1);
 
 template <class Box>
 static int launch_rs(const Box& box, const int* q_closest, const int* q_any, const RoundCounters* rc,
-                     SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s) {
+                     SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s,
+                     const Segments& sg = Segments{nullptr, 0}) {
   if (!b.keys_any)   // else the keys and the histogram were written as the rays were queued
     k_rs_key<Box><<<grid, RS_TB, 0, s>>>(box, q_closest, q_any, rc, ro, rd, b.keys, b.hist, b.threshold, b.ob, b.db,
-                                          b.jb);
+                                          b.jb, sg);
   const int nbins = raysort_bins(b.ob, b.db, b.jb);
   const int nblk = (nbins + RS_SCAN_TB - 1) / RS_SCAN_TB;
   if (nblk > RS_MAX_TILES) return -1;
@@ -220,8 +222,9 @@ static int launch_rs(const Box& box, const int* q_closest, const int* q_any, con
 }
 
 int launch_raysort(const DevScene& sc, const int* q_closest, const int* q_any, const RoundCounters* rc,
-                   SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s) {
-  return launch_rs(BoxOne{sc.root_lo, sc.root_hi}, q_closest, q_any, rc, ro, rd, b, grid, s);
+                   SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s,
+                   const Segments& sg) {
+  return launch_rs(BoxOne{sc.root_lo, sc.root_hi}, q_closest, q_any, rc, ro, rd, b, grid, s, sg);
 }
 
 int launch_raysort_batch(const BatchJob* jobs, SF<int4> job_pass, const int* q_closest, const int* q_any,

@@ -88,6 +88,68 @@ __global__ void __launch_bounds__(TRACE_TB) k_trace_paths_mixed(DevScene sc, con
   trace_loop_mixed<WIDE>(src, nc, nc + rc->n_any, &rc->work_closest, stack_cap, st, n_smem, spill);
 }
 
+// both queues of a BDPT round: the any-hit entries are segments (yc_internal.h)
+struct FanMixedSrc {
+  const DevScene* sc;
+  const int* __restrict__ q_closest;
+  const int* __restrict__ q_any;
+  const int* __restrict__ sorted;
+  int nc;
+  SF<float4> ro;
+  SF<float4> rd;
+  SF<float4> hit;
+  SF<int4> job;
+  Segments sg;
+  __device__ __forceinline__ int slot(int e, bool any) const {
+    return (sorted ? sorted[e] : (any ? q_any[e - nc] : q_closest[e]));
+  }
+  __device__ __forceinline__ const DevScene& begin(int e, bool any, RayIn& r) {
+    const int q = slot(e, any);
+    const float4 o = __ldg(&ro[any ? q >> sg.shift : q]);
+    if (any) {
+      const float4 d = __ldg(sg.seg + q);
+      r = RayIn{ym::add(o.x, ym::mul(d.x, EPS_F)), ym::add(o.y, ym::mul(d.y, EPS_F)), ym::add(o.z, ym::mul(d.z, EPS_F)),
+                d.w, d.x, d.y, d.z};
+    } else {
+      const float4 d = __ldg(&rd[q]);
+      r = RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
+    }
+    return *sc;
+  }
+  __device__ __forceinline__ void end(int e, bool any, const HitOut& h) {
+    const int q = slot(e, any);
+    if (!any) hit[q] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
+    else if (h.tri >= 0) atomicOr(&job[q >> sg.shift].z, 1 << (q & ((1 << sg.shift) - 1)));
+  }
+};
+
+template <bool WIDE>
+__global__ void __launch_bounds__(TRACE_TB) k_trace_fans(DevScene sc, const int* __restrict__ q_closest,
+                                                         const int* __restrict__ q_any, RoundCounters* rc,
+                                                         PathState ps, Segments sg, int stack_cap,
+                                                         DevStats* st, const int* sorted, const RaySortCtl* rs,
+                                                         int n_smem, int* spill) {
+  const int nc = rc->n_closest;
+  FanMixedSrc src{&sc, q_closest, q_any, (rs && rs->use) ? sorted : nullptr, nc, ps.ro, ps.rd, ps.hit, ps.job, sg};
+  trace_loop_mixed<WIDE>(src, nc, nc + rc->n_any, &rc->work_closest, stack_cap, st, n_smem, spill);
+}
+
+// the segments of a round alone
+struct SegmentSrc {
+  FanMixedSrc fans;
+  __device__ __forceinline__ const DevScene& begin(int e, RayIn& r) { return fans.begin(e, true, r); }
+  __device__ __forceinline__ void end(int e, const HitOut& h) { fans.end(e, true, h); }
+};
+
+template <bool WIDE>
+__global__ void __launch_bounds__(TRACE_TB) k_trace_segments(DevScene sc, const int* __restrict__ q_any,
+                                                             RoundCounters* rc, PathState ps,
+                                                             Segments sg, int stack_cap,
+                                                             DevStats* st) {
+  SegmentSrc src{{&sc, nullptr, q_any, nullptr, 0, ps.ro, ps.rd, ps.hit, ps.job, sg}};
+  trace_loop<true, WIDE, false>(src, rc->n_any, &rc->work_any, stack_cap, st);
+}
+
 // traceRay (udpt.cl:240-286) on explicit rays of 9 floats: light loop, then the BVH.
 template <bool ANY>
 struct RaySrc {
@@ -170,6 +232,16 @@ int launch_trace(const DevScene& sc, bool any_hit, const int* queue, const int* 
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
+int launch_trace_segments(const DevScene& sc, const int* q_any, RoundCounters* rc, const PathState& ps,
+                          const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s) {
+  const int cap = stack_cap_for(sc.depth);
+  const size_t smem = smem_for(cap);
+  const auto kernel = sc.wide ? k_trace_segments<true> : k_trace_segments<false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kernel<<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_any, rc, ps, sg, cap, st);
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+}
+
 static_assert(TRACE_TB == TRACE_TB_PASS, "the host sizes the per-pass spill area by TRACE_TB_PASS");
 int trace_stack_cap(int depth) { return stack_cap_for(depth); }
 
@@ -177,6 +249,18 @@ int trace_mixed_grid_blocks(int depth, bool wide, int n_smem) {
   const int cap = stack_cap_for(depth);
   const size_t smem = smem_for(n_smem > 0 && n_smem < cap ? n_smem : cap);
   return wide ? resident_grid(k_trace_paths_mixed<true>, smem) : resident_grid(k_trace_paths_mixed<false>, smem);
+}
+
+int launch_trace_fans(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,
+                      const PathState& ps, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s,
+                      const int* sorted, const RaySortCtl* rs, int n_smem, int* spill) {
+  const int cap = stack_cap_for(sc.depth);
+  if (!(n_smem > 0 && n_smem < cap && spill)) n_smem = cap;
+  const size_t smem = smem_for(n_smem);
+  const auto kernel = sc.wide ? k_trace_fans<true> : k_trace_fans<false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kernel<<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_closest, q_any, rc, ps, sg, cap, st, sorted, rs, n_smem, spill);
+  return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,

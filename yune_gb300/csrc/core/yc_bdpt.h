@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "yc_internal.h"
+#include "../ym_math.h"
 
 namespace yc {
 
@@ -13,8 +14,7 @@ enum : int {
   B_LIGHT = 0,   // closest hit of the light-subpath ray that makes light vertex i
   B_EYE0 = 1,    // closest hit of the camera ray
   B_EYE = 2,     // closest hit of the eye-subpath ray that makes eye vertex i
-  B_NEE = 3,     // shadow ray of the next-event estimate at eye vertex i
-  B_CONN = 4,    // connection ray between eye vertex i and light vertex j
+  B_FAN = 3,     // segments from eye vertex i: to a light (next-event estimate) and to light vertices
   // transient phases
   Q_LIGHT_SAMPLE = 8,
   Q_EYE_START = 9,
@@ -32,20 +32,77 @@ struct BdptBuffers {
   float4* ev;
   size_t N;
   int bounces;
+  Segments sg;    // the segments of the round
+  int* q_seg;     // and their queue
 };
+
+#ifdef __CUDACC__
+// the segments a path collects in one step
+struct FanOut {
+  unsigned long long js = 0;   // which light vertex each goes to, a byte each (0: a light)
+  int n = 0;
+  __device__ __forceinline__ bool full(const BdptBuffers& bb) const { return n >> bb.sg.shift; }
+  __device__ __forceinline__ void add(const BdptBuffers& bb, int p, int j, const ym::f4& dir, float len) {
+    bb.sg.seg[((size_t)p << bb.sg.shift) + n] = make_float4(dir.x, dir.y, dir.z, len);
+    js |= (unsigned long long)j << (8 * n);
+    ++n;
+  }
+};
+// a path's traced segments: which are free, and the light vertex of each
+struct FanIn {
+  unsigned long long js;
+  unsigned free;
+  __device__ __forceinline__ void load(const int4& job) {
+    js = (unsigned)job.x | ((unsigned long long)(unsigned)job.y << 32);
+    free = ~(unsigned)job.z & ((1u << job.w) - 1u);
+  }
+  __device__ __forceinline__ int vertex(int s) const { return (int)(js >> (8 * s)) & 255; }
+};
+
+// the queue entries of a warp's lanes: paths with a closest-hit ray (emit 1), and paths that wait
+// for `segs` segments (emit 2) with the segments themselves; all 32 lanes call it
+__device__ __forceinline__ void append_bdpt(const BdptBuffers& bb, int emit, int p, int segs, int* out_closest,
+                                            int* out_fan, RoundCounters* rc_out) {
+  const int lane = threadIdx.x & 31;
+  const unsigned mc = __ballot_sync(0xffffffffu, emit == 1), mf = __ballot_sync(0xffffffffu, emit == 2);
+  const unsigned below = (1u << lane) - 1;
+  int incl = emit == 2 ? segs : 0;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += u;
+  }
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  int bc = 0, bf = 0, bs = 0;
+  if (lane == 0) {
+    if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
+    if (mf) bf = atomicAdd(&rc_out->n_fan, __popc(mf));
+    if (total) bs = atomicAdd(&rc_out->n_any, total);
+  }
+  bc = __shfl_sync(0xffffffffu, bc, 0);
+  bf = __shfl_sync(0xffffffffu, bf, 0);
+  bs = __shfl_sync(0xffffffffu, bs, 0);
+  if (emit == 1) out_closest[bc + __popc(mc & below)] = p;
+  if (emit == 2) {
+    out_fan[bf + __popc(mf & below)] = p;
+    int* q = bb.q_seg + (bs + incl - segs);
+    for (int k = 0; k < segs; ++k) q[k] = (p << bb.sg.shift) + k;
+  }
+}
+#endif
 
 void launch_raygen_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, int* q_closest,
                         RoundCounters* rc, DevStats* st, cudaStream_t s);
 void launch_logic_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                       const int* in_any, const RoundCounters* rc_in, int* out_closest, int* out_any,
+                       const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
                        RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted = nullptr,
                        const SortCtl* sctl = nullptr);
 // the bidirectional tracer with multiple importance sampling (bdpt_mis.cu): same buffers,
-// same trace-state numbering (B_LIGHT .. B_CONN), light vertices only
+// same trace-state numbering (B_LIGHT .. B_FAN), light vertices only
 void launch_raygen_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, int* q_closest,
                             RoundCounters* rc, DevStats* st, cudaStream_t s);
 void launch_logic_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                           const int* in_any, const RoundCounters* rc_in, int* out_closest, int* out_any,
+                           const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
                            RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted = nullptr,
                            const SortCtl* sctl = nullptr);
 

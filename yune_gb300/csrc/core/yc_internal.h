@@ -81,8 +81,21 @@ struct RoundCounters {
   int work_closest;   // persistent-kernel work cursors
   int work_any;
   int work_logic;
-  int pad[3];
+  int n_fan;          // BDPT passes: paths that wait for segments (n_any counts the segments)
+  int pad[2];
 };
+
+// The segments of a bidirectional path. An eye vertex sends its shadow rays, to a light and to
+// the light subpath's vertices, in one round. Segment s of path p is at seg[(p << shift) + s] =
+// (direction, length); the common origin of a path's segments, before the offset along the
+// direction, is its ro; the any-hit queue holds (p << shift) + s; a segment found occluded sets
+// bit s of the path's job.z. (A path waits in the fan queue of its round; byte s of job.x, job.y
+// says which light vertex segment s goes to, job.w how many segments there are.)
+struct Segments {
+  float4* seg;
+  int shift;       // 2^shift segments a path at most
+};
+constexpr int FAN_SHIFT = 3;
 
 // Sorting of a round's traversal work list by ray origin and direction (raysort.cu):
 // `use` tells the trace kernel whether this round's list is the sorted one.
@@ -227,11 +240,19 @@ int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_an
                        SF<float4> ro, SF<float4> rd, SF<float4> hit, DevStats* st, int grid_blocks,
                        cudaStream_t s, const int* sorted = nullptr, const RaySortCtl* rs = nullptr, int n_smem = 0,
                        int* spill = nullptr);
+// the same over a BDPT round, whose any-hit queue holds segments, and the segments alone
+// (whole stack in shared memory; trace_grid_blocks' grid)
+int launch_trace_fans(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,
+                      const PathState& ps, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s,
+                      const int* sorted, const RaySortCtl* rs, int n_smem, int* spill);
+int launch_trace_segments(const DevScene& sc, const int* q_any, RoundCounters* rc, const PathState& ps,
+                          const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s);
 // raysort.cu: sorts the round's work list (closest-hit queue, then any-hit queue) into
 // b.sorted when the round has at least b.threshold rays, and sets b.ctl->use
 int raysort_bins(int ob, int db, int jb = 0);
 int launch_raysort(const DevScene& sc, const int* q_closest, const int* q_any, const RoundCounters* rc,
-                   SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s);
+                   SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s,
+                   const Segments& sg = Segments{nullptr, 0});
 int trace_mixed_grid_blocks(int depth, bool wide, int n_smem = 0);
 int trace_stack_cap(int depth);   // walk-stack entries the per-pass kernels give a scene of this depth
 constexpr int TRACE_TB_PASS = 128;   // block of the per-pass trace kernels (TRACE_TB of yc_trace_loop.cuh)
