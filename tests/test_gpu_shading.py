@@ -94,3 +94,26 @@ def test_segments_of_an_eye_vertex(r, tris, integrator, bounces, mixed, sort):
     for o, _, v in opts:
         N.check(r.L.yc_set_option(r.h, o, v), "yc_set_option")
     r.release(sid)
+
+
+# A shadow ray goes with the path's next ray where the lobe is drawn whatever its result
+# (mis_lobe_fix): round by round and in the tail, whose idle lanes walk a path's second ray;
+# in the shared launch, its sorted form, and launches of their own.
+@pytest.mark.parametrize("tail", [0, -1])
+@pytest.mark.parametrize("mixed, sort", [(1, 0), (1, 1), (0, 0)])
+@pytest.mark.parametrize("lobe_fix", [0, 1])
+@pytest.mark.parametrize("tris, max_depth", [(0, 100000), (6000, 2), (6000, 100000)])
+def test_rays_sent_together(r, tris, max_depth, lobe_fix, mixed, sort, tail):
+    cfg = scenes.default_cfg(mis=1, mis_lobe_fix=lobe_fix, max_depth=max_depth)
+    s = workloads.mixed_scene(tris, 9, W, H, 1, cfg) if tris else scenes.c0(W, H)
+    s.cfg = dict(s.cfg, mis_lobe_fix=lobe_fix)
+    if tris:
+        s.lights = _crossing_lights(s.lights)
+    sid = r.upload(s)
+    opts = [(2, tail, -1), (3, mixed, 1), (5, 1 if sort else 65536, 65536)]
+    for o, v, _ in opts:
+        N.check(r.L.yc_set_option(r.h, o, v), "yc_set_option")
+    _same(r, s, sid)
+    for o, _, v in opts:
+        N.check(r.L.yc_set_option(r.h, o, v), "yc_set_option")
+    r.release(sid)

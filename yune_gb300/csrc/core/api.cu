@@ -160,7 +160,8 @@ struct yc_ctx {
   // wavefront buffers, sized for the largest image seen
   size_t cap_paths = 0;
   DevBuf<float4> rec;                // path records, PS_STRIDE float4 per slot
-  DevBuf<int> q[4];                  // closest/any for two rounds
+  DevBuf<int> q[4];                  // closest/waiting for two rounds
+  DevBuf<int> q_any;                 // a round's any-hit rays
   DevBuf<yc::RoundCounters> rc;      // two round-counter blocks
   DevBuf<yc::DevStats> stats;
   yc::RoundCounters* rc_host = nullptr;   // pinned
@@ -182,7 +183,7 @@ struct yc_ctx {
   DevBuf<char> flush_buf;
   // BDPT subpath vertices
   DevBuf<float4> bd_lv, bd_ev, bd_seg;
-  DevBuf<int> bd_q_seg;
+  DevBuf<int> bd_q_any;
   int bd_shift = yc::FAN_SHIFT;       // segments a path sends at once, for frames of bd_paths paths (log2)
   size_t bd_paths = 0;
   size_t bd_cap = 0, bd_ev_cap = 0;   // light / eye vertex records (the MIS tracer has no eye records)
@@ -199,6 +200,7 @@ int ensure_paths(yc_ctx* c, size_t n) {
   if (n <= c->cap_paths) return 0;
   YC_CUDA(c->rec.alloc(n * yc::PS_STRIDE));
   for (auto& b : c->q) YC_CUDA(b.alloc(n));
+  YC_CUDA(c->q_any.alloc(2 * n));
   c->cap_paths = n;
   return 0;
 }
@@ -271,7 +273,7 @@ int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
     if (shift > 0 && m > ((size_t)1 << 30)) continue;
     cudaError_t e = cudaSuccess;
     if (c->bd_seg.n < m) e = c->bd_seg.alloc(m);
-    if (e == cudaSuccess && c->bd_q_seg.n < m) e = c->bd_q_seg.alloc(m);
+    if (e == cudaSuccess && c->bd_q_any.n < m) e = c->bd_q_any.alloc(m);
     if (e == cudaSuccess && raysort && c->rs_cap < m) {
       c->rs_cap = 0;
       e = c->rs_keys.alloc(m);
@@ -285,7 +287,7 @@ int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
     }
     cudaGetLastError();
     c->bd_seg.release();
-    c->bd_q_seg.release();
+    c->bd_q_any.release();
     if (shift == 0)
       return fail(e == cudaErrorMemoryAllocation ? YC_E_NOMEM : YC_E_LAUNCH,
                   std::string("segments of a bidirectional pass: ") + cudaGetErrorString(e));
@@ -519,7 +521,7 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
                        (size_t)W * H >= (size_t)c->rs_threshold && dsc.n_tri >= kRaySortMinTris;
   yc::RaySortBufs rsb{};
   if (raysort) {
-    if (int e = ensure_raysort(c, (size_t)W * H)) return e;
+    if (int e = ensure_raysort(c, (size_t)W * H * 3)) return e;   // a closest-hit ray and two segments a path
   }
   // shade-queue sort by phase and material class before the logic kernel (unidirectional
   // passes whose frame can fill a sorted queue, in scenes with a mirror or dielectric:
@@ -548,16 +550,19 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
     return fail(YC_E_LAUNCH, "trace kernel cannot be resident (stack too deep)");
   int tail_grid = 0, tail_at = 0;
   if (!bdpt && c->tail_paths != 0) {
-    const int capacity = yc::tail_capacity(dsc, n_smem, &tail_grid);
+    const int capacity = yc::tail_capacity(pp, n_smem, &tail_grid);
     tail_at = c->tail_paths < 0 ? capacity : std::min(c->tail_paths, capacity);
   }
   if (n_smem > 0)
     if (int e = ensure_pass_spill(c, (size_t)std::max(grid_m, tail_grid) * yc::TRACE_TB_PASS * 2 * (size_t)(cap - n_smem)))
       return e;
+  yc::Segments sg = yc::record_segments(ps);   // the passes' any-hit rays and their queue
+  int* q_any = c->q_any.p;
   if (bdpt) {
     if (int e = ensure_segments(c, (size_t)W * H, raysort)) return e;
-    bb.sg = yc::Segments{c->bd_seg.p, c->bd_shift};
-    bb.q_seg = c->bd_q_seg.p;
+    bb.sg = sg = yc::Segments{c->bd_seg.p, ps.ro, ps.misc, 1 << c->bd_shift, 1, c->bd_shift, yc::FAN_BIT};
+    bb.seg = c->bd_seg.p;
+    bb.q_any = q_any = c->bd_q_any.p;
   }
   if (raysort)
     rsb = yc::RaySortBufs{c->rs_keys.p, nullptr, c->rs_hist.p, c->rs_cursor.p, c->rs_blk.p, c->rs_sorted.p, c->rs_ctl.p,
@@ -567,26 +572,22 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
   bool finished = false;
   for (int round = 0; round < c->max_rounds; ++round) {
     int* in_c = c->q[2 * cur].p;
-    int* in_a = c->q[2 * cur + 1].p;
+    int* in_w = c->q[2 * cur + 1].p;
     int* out_c = c->q[2 * (1 - cur)].p;
-    int* out_a = c->q[2 * (1 - cur) + 1].p;
+    int* out_w = c->q[2 * (1 - cur) + 1].p;
     yc::RoundCounters* rin = rc + cur;
     yc::RoundCounters* rout = rc + (1 - cur);
     int e1, e2;
     if (mixed) {   // both ray kinds of the round in one launch
       if (raysort) {
         KTimer kt(c, K_RAYSORT);
-        if (yc::launch_raysort(dsc, in_c, bdpt ? bb.q_seg : in_a, rin, ps.ro, ps.rd, rsb, c->logic_grid, c->stream, bb.sg))
+        if (yc::launch_raysort(dsc, in_c, q_any, rin, ps.ro, ps.rd, rsb, c->logic_grid, c->stream, sg))
           return fail(YC_E_LAUNCH, std::string("ray sort: ") + cudaGetErrorString(cudaGetLastError()));
       }
       KTimer kt(c, K_TRACE);
-      const int* sorted = raysort ? rsb.sorted : nullptr;
-      const yc::RaySortCtl* rctl = raysort ? rsb.ctl : nullptr;
-      int* spill = n_smem > 0 ? c->pass_spill.p : nullptr;
-      if (bdpt ? yc::launch_trace_fans(dsc, in_c, bb.q_seg, rin, ps, bb.sg, c->stats.p, grid_m, c->stream, sorted, rctl,
-                                       n_smem, spill)
-               : yc::launch_trace_mixed(dsc, in_c, in_a, rin, ps.ro, ps.rd, ps.hit, c->stats.p, grid_m, c->stream,
-                                        sorted, rctl, n_smem, spill))
+      if (yc::launch_trace_mixed(dsc, in_c, q_any, rin, ps, sg, c->stats.p, grid_m, c->stream,
+                                 raysort ? rsb.sorted : nullptr, raysort ? rsb.ctl : nullptr, n_smem,
+                                 n_smem > 0 ? c->pass_spill.p : nullptr))
         return fail(YC_E_LAUNCH, std::string("trace kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }
     // otherwise the two traces of a round are independent: the any-hit one runs on the
@@ -601,15 +602,12 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
     if (!mixed) {
       {
         KTimer kt(c, K_EXTEND);
-        e1 = yc::launch_trace(dsc, false, in_c, &rin->n_closest, &rin->work_closest, ps.ro, ps.rd, ps.hit,
-                              c->stats.p, grid_c, c->stream);
+        e1 = yc::launch_trace(dsc, in_c, rin, ps, c->stats.p, grid_c, c->stream);
       }
       if (e1) return fail(YC_E_LAUNCH, std::string("extend kernel: ") + cudaGetErrorString(cudaGetLastError()));
       {
         KTimer kt(c, K_OCCL);
-        e2 = bdpt ? yc::launch_trace_segments(dsc, bb.q_seg, rin, ps, bb.sg, c->stats.p, grid_a, s_any)
-                  : yc::launch_trace(dsc, true, in_a, &rin->n_any, &rin->work_any, ps.ro, ps.rd, ps.hit, c->stats.p,
-                                     grid_a, s_any);
+        e2 = yc::launch_trace_segments(dsc, q_any, rin, sg, c->stats.p, grid_a, s_any);
       }
       if (e2) return fail(YC_E_LAUNCH, std::string("occlusion kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }
@@ -621,7 +619,7 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
     if (shadesort) {
       KTimer kt(c, K_SORT);
       YC_CUDA(cudaMemsetAsync(c->ss_ctl.p, 0, sizeof(yc::SortCtl), c->stream));
-      yc::launch_pass_sort(dsc, bdpt, ps, in_c, in_a, rin, c->ss_keys.p, c->ss_sorted.p, c->ss_ctl.p,
+      yc::launch_pass_sort(dsc, bdpt, ps, in_c, in_w, rin, c->ss_keys.p, c->ss_sorted.p, c->ss_ctl.p,
                            c->ss_threshold, c->logic_grid, c->stream);
     }
     {
@@ -629,17 +627,17 @@ int run_pass(yc_ctx* c, Scene* sc, Accum* ac, uint32_t rand_seed, int reset, int
       const int* sorted = shadesort ? c->ss_sorted.p : nullptr;
       const yc::SortCtl* sctl = shadesort ? c->ss_ctl.p : nullptr;
       if (bdpt_mis)
-        yc::launch_logic_bdpt_mis(pp, ps, bb, in_c, in_a, rin, out_c, out_a, rout, c->stats.p, c->logic_grid,
+        yc::launch_logic_bdpt_mis(pp, ps, bb, in_c, in_w, rin, out_c, out_w, rout, c->stats.p, c->logic_grid,
                                   c->stream, sorted, sctl);
       else if (bdpt)
-        yc::launch_logic_bdpt(pp, ps, bb, in_c, in_a, rin, out_c, out_a, rout, c->stats.p, c->logic_grid, c->stream,
+        yc::launch_logic_bdpt(pp, ps, bb, in_c, in_w, rin, out_c, out_w, rout, c->stats.p, c->logic_grid, c->stream,
                               sorted, sctl);
-      else yc::launch_logic(pp, ps, in_c, in_a, rin, out_c, out_a, rout, c->stats.p, c->logic_grid, c->stream,
+      else yc::launch_logic(pp, ps, in_c, in_w, rin, out_c, out_w, q_any, rout, c->stats.p, c->logic_grid, c->stream,
                             sorted, sctl);
     }
     if (tail_at > 0) {
       KTimer kt(c, K_TAIL);
-      if (yc::launch_tail(pp, ps, out_c, out_a, rout, tail_at, c->stats.p, tail_grid, c->stream, n_smem,
+      if (yc::launch_tail(pp, ps, out_c, out_w, rout, tail_at, c->stats.p, tail_grid, c->stream, n_smem,
                           n_smem > 0 ? c->pass_spill.p : nullptr))
         return fail(YC_E_LAUNCH, std::string("tail kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }
@@ -1378,7 +1376,7 @@ int yc_last_pass_ms(yc_ctx* c, float* ms) {
 struct BatchGroup {
   int first = 0, count = 0;
   DevBuf<int> free_stack;
-  DevBuf<int> q[4];
+  DevBuf<int> q[4], q_any;
   DevBuf<int> sort_keys, sorted;
   DevBuf<unsigned> rs_keys, rs_hist, rs_cursor, rs_blk;   // ray sort before the trace (raysort.cu)
   DevBuf<int> rs_sorted;
@@ -1465,9 +1463,9 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
   yc_ctx* c = b->ctx;
   const yc::PathState ps = batch_state(b);
   int* in_c = g.q[2 * cur].p;
-  int* in_a = g.q[2 * cur + 1].p;
+  int* in_w = g.q[2 * cur + 1].p;
   int* out_c = g.q[2 * (1 - cur)].p;
-  int* out_a = g.q[2 * (1 - cur) + 1].p;
+  int* out_w = g.q[2 * (1 - cur) + 1].p;
   yc::RoundCounters* rin = g.rc.p + cur;
   yc::RoundCounters* rout = g.rc.p + (1 - cur);
   cudaStream_t sm = serial ? c->stream : g.main;
@@ -1477,11 +1475,11 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
                         g.rs_ctl.p, b->rs_ob, b->rs_db, b->rs_jb, b->rs_threshold};
     if (b->raysort) {
       KTimer kt(c, K_RAYSORT, timed);
-      yc::launch_raysort_batch(b->jobs.p, batch_state(b).job, in_c, in_a, rin, ps.ro, ps.rd, rsb, b->logic_grid, sm);
+      yc::launch_raysort_batch(b->jobs.p, batch_state(b).job, in_c, g.q_any.p, rin, ps, rsb, b->logic_grid, sm);
     }
     KTimer kt(c, K_TRACE, timed);
-    yc::launch_batch_trace_mixed(b->walks_wide(), b->jobs.p, batch_state(b).job, in_c, in_a, rin, ps.ro, ps.rd, ps.hit,
-                                 c->stats.p, b->walk_cap, b->stack_smem, g.spill.p, b->grid_m, b->cfg.trace_block, sm,
+    yc::launch_batch_trace_mixed(b->walks_wide(), b->jobs.p, batch_state(b).job, in_c, g.q_any.p, rin, ps, c->stats.p,
+                                 b->walk_cap, b->stack_smem, g.spill.p, b->grid_m, b->cfg.trace_block, sm,
                                  b->raysort ? rsb.sorted : nullptr,
                                  b->raysort ? rsb.ctl : nullptr);
   } else {
@@ -1493,13 +1491,13 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
     {
       KTimer kt(c, K_EXTEND, timed);
       yc::launch_batch_trace(false, b->walks_wide(), b->jobs.p, batch_state(b).job, in_c, &rin->n_closest,
-                             &rin->work_closest, ps.ro, ps.rd, ps.hit, c->stats.p, b->walk_cap, b->stack_smem,
+                             &rin->work_closest, ps, c->stats.p, b->walk_cap, b->stack_smem,
                              g.spill.p, b->grid_c, b->cfg.trace_block, sm);
     }
     {
       KTimer kt(c, K_OCCL, timed);
-      yc::launch_batch_trace(true, b->walks_wide(), b->jobs.p, batch_state(b).job, in_a, &rin->n_any, &rin->work_any, ps.ro,
-                             ps.rd, ps.hit, c->stats.p, b->walk_cap, b->stack_smem,
+      yc::launch_batch_trace(true, b->walks_wide(), b->jobs.p, batch_state(b).job, g.q_any.p, &rin->n_any,
+                             &rin->work_any, ps, c->stats.p, b->walk_cap, b->stack_smem,
                              g.spill.p ? g.spill.p + b->spill_slot : nullptr, b->grid_a, b->cfg.trace_block, sa);
     }
     if (!serial) {
@@ -1511,13 +1509,13 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
   YC_CUDA(cudaMemsetAsync(g.sctl.p, 0, sizeof(yc::SortCtl), sm));
   if (b->cfg.sort_threshold > 0) {
     KTimer kt(c, K_SORT, timed);
-    yc::launch_batch_sort(b->jobs.p, batch_state(b).job, ps, in_c, in_a, rin, g.sort_keys.p, g.sorted.p, g.sctl.p,
+    yc::launch_batch_sort(b->jobs.p, batch_state(b).job, ps, in_c, in_w, rin, g.sort_keys.p, g.sorted.p, g.sctl.p,
                           b->cfg.sort_threshold, b->logic_grid, sm);
   }
   {
     KTimer kt(c, K_LOGIC, timed);
-    yc::launch_batch_logic(b->jobs.p, b->tasks.p, g.ctl.p, ps, batch_state(b).job, g.free_stack.p, in_c, in_a, rin, out_c,
-                           out_a, rout, c->stats.p, b->job_done.p, g.sorted.p, g.sctl.p, rs_produce(b, g), b->logic_grid,
+    yc::launch_batch_logic(b->jobs.p, b->tasks.p, g.ctl.p, ps, batch_state(b).job, g.free_stack.p, in_c, in_w, rin, out_c,
+                           out_w, g.q_any.p, rout, c->stats.p, b->job_done.p, g.sorted.p, g.sctl.p, rs_produce(b, g), b->logic_grid,
                            sm);
   }
   c->ktimes.rounds++;
@@ -1674,6 +1672,7 @@ int yc_batch_create(yc_ctx* c, const yc_batch_cfg* cfg, yc_batch** out) {
     const size_t m = (size_t)g->count;
     YC_CUDA(g->free_stack.alloc(m));
     for (auto& q : g->q) YC_CUDA(q.alloc(m));
+    YC_CUDA(g->q_any.alloc(m));
     YC_CUDA(g->sctl.alloc(1));
     if (b->cfg.sort_threshold > 0) {
       YC_CUDA(g->sort_keys.alloc(m));

@@ -164,14 +164,14 @@ void launch_raygen_bdpt(const PassParams& pp, const PathState& ps, const BdptBuf
 
 // ---- logic: advance each path to its next ray ----
 __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps, BdptBuffers bb,
-                                                    const int* __restrict__ in_closest, const int* __restrict__ in_fan,
-                                                    const RoundCounters* rc_in, int* out_closest, int* out_fan,
+                                                    const int* __restrict__ in_closest, const int* __restrict__ in_wait,
+                                                    const RoundCounters* rc_in, int* out_closest, int* out_wait,
                                                     RoundCounters* rc_out, DevStats* st, const int* __restrict__ sorted,
                                                     const SortCtl* sctl) {
   __shared__ unsigned long long s_cnt[8];   // rays, primary, extension, shadow, connection, traversed, samples
   if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
   __syncthreads();
-  const int nc = rc_in->n_closest, na = rc_in->n_fan;
+  const int nc = rc_in->n_closest, na = rc_in->n_wait;
   const int n = nc + na;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
     unsigned c[7] = {0, 0, 0, 0, 0, 0, 0};
     const unsigned mask = __ballot_sync(0xffffffffu, entry < n);
     if (entry < n) {
-      p = use_sorted ? sorted[entry] : (entry < nc ? in_closest[entry] : in_fan[entry - nc]);
+      p = use_sorted ? sorted[entry] : (entry < nc ? in_closest[entry] : in_wait[entry - nc]);
       const VertexRef lv{bb.lv + (size_t)p * bb.bounces * 4};
       const VertexRef ev{bb.ev + (size_t)p * bb.bounces * 4};
       const int4 misc = ps.misc[p];
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
       if (made) v = tri_vertex(sc, ro, rd, hit.x, hit.y, hit.z, tri);
       if (!building) {
         e = ev.vtx(cnt.i);
-        fan.load(ps.job[p]);
+        fan.load(ps.job[p], misc);
         if (fan.vertex(0) == 0 && !(fan.free & 1u)) {   // the light sample is occluded: DL = emission
           const f4 em = ld4(sc.mats[e.mat].ke);
           color = color + (ev.contrib(cnt.i) * (em + (ym::splat(0.0f) + em))) * weight;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
             else w_out = back;
           } else {
             const int sg = __ffs(fan.free) - 1;
-            const float4 d4 = bb.sg.seg[((size_t)p << bb.sg.shift) + sg];
+            const float4 d4 = bb.seg[((size_t)p << bb.sg.shift) + sg];
             dir = ym::mk(d4.x, d4.y, d4.z, 0.0f);
             j = fan.vertex(sg);
             if (far_end) {
@@ -506,14 +506,14 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
         ps.direct[p] = make_float4(weight, ks, pend_pdf, pend_prob);
         if (emit == 2) {
           ps.ro[p] = make_float4(e.hp.x, e.hp.y, e.hp.z, 0.0f);
-          ps.job[p] = make_int4((int)out.js, (int)(out.js >> 32), 0, out.n);
+          ps.job[p] = make_int4((int)out.js, (int)(out.js >> 32), out.n, 0);
         } else {
           ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
           ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
         }
       }
     }
-    append_bdpt(bb, emit, p, out.n, out_closest, out_fan, rc_out);
+    append_bdpt(bb, emit, p, out.n, out_closest, out_wait, rc_out);
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
       unsigned x = c[q];
@@ -535,10 +535,10 @@ __global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps,
 }
 
 void launch_logic_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                       const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
+                       const int* in_wait, const RoundCounters* rc_in, int* out_closest, int* out_wait,
                        RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted,
                        const SortCtl* sctl) {
-  k_logic_bdpt<<<grid, 256, 0, s>>>(pp, ps, bb, in_closest, in_fan, rc_in, out_closest, out_fan, rc_out, st, sorted,
+  k_logic_bdpt<<<grid, 256, 0, s>>>(pp, ps, bb, in_closest, in_wait, rc_in, out_closest, out_wait, rc_out, st, sorted,
                                     sctl);
 }
 

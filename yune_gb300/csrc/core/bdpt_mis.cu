@@ -256,15 +256,15 @@ constexpr int MIS_TB = 128;
 constexpr int TO_LIGHT = 1, TO_VERTEX = 2;   // a segment's kind
 __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, PathState ps, BdptBuffers bb,
                                                         const int* __restrict__ in_closest,
-                                                        const int* __restrict__ in_fan, const RoundCounters* rc_in,
-                                                        int* out_closest, int* out_fan, RoundCounters* rc_out,
+                                                        const int* __restrict__ in_wait, const RoundCounters* rc_in,
+                                                        int* out_closest, int* out_wait, RoundCounters* rc_out,
                                                         DevStats* st, const int* __restrict__ sorted,
                                                         const SortCtl* sctl) {
   // per-warp counts of rays, primary, extension, shadow, connection, traversed, samples,
   // added to the device counters when the warp leaves (no block barrier: warps finish at
   // different times)
   unsigned w_cnt[7] = {0, 0, 0, 0, 0, 0, 0};
-  const int nc = rc_in->n_closest, na = rc_in->n_fan;
+  const int nc = rc_in->n_closest, na = rc_in->n_wait;
   const int n = nc + na;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
     unsigned c[7] = {0, 0, 0, 0, 0, 0, 0};
     const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
-      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_fan[e - nc]);
+      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_wait[e - nc]);
       const MisRec lv{bb.lv + (size_t)p * bb.bounces * 4};
       const int4 misc = ps.misc[p];
       uint32_t seed = (uint32_t)misc.x;
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
       float r_x = 0.0f, s_x = 0.0f;
       FanIn fan{0, 0};              // the free segments to light vertices
       if (shadow) {
-        fan.load(ps.job[p]);
+        fan.load(ps.job[p], misc);
         w_color = fan.free != 0;
         if (fan.vertex(0) == 0 && (fan.free & 1u)) {   // the light sample
           color = color + pend;
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
           const int sg = __ffs(fan.free) - 1;
           fan.free &= fan.free - 1u;
           at = fan.vertex(sg);
-          const float4 h4 = lv.at(at, 0), n4 = lv.at(at, 1), s4 = bb.sg.seg[((size_t)p << bb.sg.shift) + sg];
+          const float4 h4 = lv.at(at, 0), n4 = lv.at(at, 1), s4 = bb.seg[((size_t)p << bb.sg.shift) + sg];
           const f4 v = ym::mk(h4.x, h4.y, h4.z, 1.0f) - y.hp;
           d2 = ym::dot(v, v);
           dir = ym::mk(s4.x, s4.y, s4.z, 0.0f);
@@ -629,14 +629,14 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
         }
         if (emit == 2) {
           ps.ro[p] = make_float4(y.hp.x, y.hp.y, y.hp.z, 0.0f);
-          ps.job[p] = make_int4((int)out.js, (int)(out.js >> 32), 0, out.n);
+          ps.job[p] = make_int4((int)out.js, (int)(out.js >> 32), out.n, 0);
         } else {
           ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
           ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
         }
       }
     }
-    append_bdpt(bb, emit, p, out.n, out_closest, out_fan, rc_out);
+    append_bdpt(bb, emit, p, out.n, out_closest, out_wait, rc_out);
 #pragma unroll
     for (int q = 0; q < 7; ++q) w_cnt[q] += c[q];
   }
@@ -659,11 +659,11 @@ __global__ void __launch_bounds__(MIS_TB, 3) k_logic_bdpt_mis(PassParams pp, Pat
 }
 
 void launch_logic_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                           const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
+                           const int* in_wait, const RoundCounters* rc_in, int* out_closest, int* out_wait,
                            RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted,
                            const SortCtl* sctl) {
   // (grid counts blocks of 256)
-  k_logic_bdpt_mis<<<grid * (256 / MIS_TB), MIS_TB, 0, s>>>(pp, ps, bb, in_closest, in_fan, rc_in, out_closest, out_fan,
+  k_logic_bdpt_mis<<<grid * (256 / MIS_TB), MIS_TB, 0, s>>>(pp, ps, bb, in_closest, in_wait, rc_in, out_closest, out_wait,
                                                             rc_out, st, sorted, sctl);
 }
 

@@ -62,15 +62,16 @@ __device__ __forceinline__ unsigned long long claim_tasks(BatchTasks* tasks, int
 }
 
 // ---- ray-sort keys formed by the kernels that queue the rays ----
-// The queued ray of slot p (ps.ro / ps.rd as just written, the scene box of its job) gets
-// the key of k_rs_key (raysort.cu) at its queue position; the warp's equal keys are
-// counted with one histogram atomic. Every lane of the warp calls it (kind 0: no ray).
+// A queued ray of slot p (its closest-hit ray, kind 1, or its segment `seg`, kind 2, as just
+// written; the scene box of its job) gets the key of k_rs_key (raysort.cu) at its queue
+// position; the warp's equal keys are counted with one histogram atomic. Every lane of the
+// warp calls it (kind 0: no ray).
 __device__ __forceinline__ void produce_key(const RsProduce& rsp, const BatchJob* jobs, const PathState& ps,
-                                            SF<int4> job_pass, int p, int kind, int pos) {
+                                            SF<int4> job_pass, int p, int kind, int seg, int pos) {
   const int lane = threadIdx.x & 31;
   unsigned key = 0xffffffffu - lane;   // lanes without a ray match nobody
   if (kind) {
-    const float4 o = ps.ro[p], d = ps.rd[p];
+    const float4 o = kind == 1 ? ps.ro[p] : ps.hp[p], d = kind == 1 || seg ? ps.rd[p] : ps.wi[p];
     const unsigned job = (unsigned)job_pass[p].x;
     const DevScene& sc = jobs[job].pp.sc;
     key = ray_key(o, d, sc.root_lo, sc.root_hi, rsp.ob, rsp.db) |
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(ENGINE_TB) k_batch_fill(const BatchJob* __rest
     b = __shfl_sync(0xffffffffu, b, 0);
     const int pos = b + __popc(m & ((1u << lane) - 1));
     if (active) q_closest[pos] = p;
-    if (rsp.keys_c) produce_key(rsp, jobs, ps, job_pass, p, active ? 1 : 0, pos);
+    if (rsp.keys_c) produce_key(rsp, jobs, ps, job_pass, p, active ? 1 : 0, 0, pos);
     started += __popc(m);
   }
   if (lane == 0 && started) {
@@ -150,15 +151,16 @@ __global__ void __launch_bounds__(BATCH_LOGIC_TB, 4) k_batch_logic(const BatchJo
                                                            BatchCtl* ctl,
                                                            PathState ps, SF<int4> job_pass, int* free_stack,
                                                            const int* __restrict__ in_closest,
-                                                           const int* __restrict__ in_any, const RoundCounters* rc_in,
-                                                           int* out_closest, int* out_any, RoundCounters* rc_out,
+                                                           const int* __restrict__ in_wait, const RoundCounters* rc_in,
+                                                           int* out_closest, int* out_wait, int* q_any,
+                                                           RoundCounters* rc_out,
                                                            DevStats* st, unsigned long long* job_done,
                                                            const int* __restrict__ sorted, const SortCtl* sctl,
                                                            RsProduce rsp) {
   __shared__ unsigned long long s_cnt[8];
   if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
   __syncthreads();
-  const int nc = rc_in->n_closest, na = rc_in->n_any;
+  const int nc = rc_in->n_closest, na = rc_in->n_wait;
   const int n = nc + na;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -173,15 +175,15 @@ __global__ void __launch_bounds__(BATCH_LOGIC_TB, 4) k_batch_logic(const BatchJo
     LogicCounts lc;
     const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
-      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
+      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_wait[e - nc]);
       const int4 jp = job_pass[p];
       const BatchJob& J = jobs[jp.x];
       const int reset = (jp.y == 0) ? J.reset_first : 0;
-      emit = logic_path(J.pp, reset, ps, p, lc, mask);
+      emit = logic_path<false>(J.pp, reset, ps, p, lc, mask);
       if (emit == 0) {
         if (jp.y + 1 < J.n_pass && !J.cancelled) {   // next pass of the same pixel
           start_pass(J, jp.x, ps.misc[p].y, jp.y + 1, p, ps, job_pass);
-          emit = 1;
+          emit = EMIT_CLOSEST;
           lc.rays++; lc.trav++; lc.prim++;
         } else {
           atomicAdd(&job_done[jp.x], 1ull);
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(BATCH_LOGIC_TB, 4) k_batch_logic(const BatchJo
             atomicAdd(&job_done[job], 1ull);
           } else {
             start_pass(jobs[job], job, (int)(t - (unsigned long long)jobs[job].task_base), 0, p, ps, job_pass);
-            emit = 1;
+            emit = EMIT_CLOSEST;
             lc.rays++; lc.trav++; lc.prim++;
             need_task = false;
           }
@@ -220,20 +222,12 @@ __global__ void __launch_bounds__(BATCH_LOGIC_TB, 4) k_batch_logic(const BatchJo
       }
     }
     if (need_task) free_stack[atomicAdd(&ctl->free_top, 1)] = p;
-    const unsigned mc = __ballot_sync(0xffffffffu, emit == 1);
-    const unsigned ma = __ballot_sync(0xffffffffu, emit == 2);
-    int bc = 0, ba = 0;
-    if (lane == 0) {
-      if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
-      if (ma) ba = atomicAdd(&rc_out->n_any, __popc(ma));
+    RaysOut at;
+    append_rays(emit, p, out_closest, out_wait, q_any, rc_out, at);
+    if (rsp.keys_c) {
+      const int kind = emit & EMIT;   // a path has one ray in flight
+      produce_key(rsp, jobs, ps, job_pass, p, kind, (emit & EMIT_SEG1) != 0, kind == EMIT_CLOSEST ? at.closest : at.any);
     }
-    bc = __shfl_sync(0xffffffffu, bc, 0);
-    ba = __shfl_sync(0xffffffffu, ba, 0);
-    const unsigned below = (1u << lane) - 1;
-    const int pos = emit == 1 ? bc + __popc(mc & below) : ba + __popc(ma & below);
-    if (emit == 1) out_closest[pos] = p;
-    if (emit == 2) out_any[pos] = p;
-    if (rsp.keys_c) produce_key(rsp, jobs, ps, job_pass, p, emit, pos);
     unsigned v[7] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples, lc.prim};
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
@@ -257,12 +251,13 @@ __global__ void __launch_bounds__(BATCH_LOGIC_TB, 4) k_batch_logic(const BatchJo
 
 void launch_batch_logic(const BatchJob* jobs, BatchTasks* tasks, BatchCtl* ctl, const PathState& ps, SF<int4> job_pass,
                         int* free_stack,
-                        const int* in_closest, const int* in_any, const RoundCounters* rc_in, int* out_closest,
-                        int* out_any, RoundCounters* rc_out, DevStats* st, unsigned long long* job_done,
+                        const int* in_closest, const int* in_wait, const RoundCounters* rc_in, int* out_closest,
+                        int* out_wait, int* q_any, RoundCounters* rc_out, DevStats* st,
+                        unsigned long long* job_done,
                         const int* sorted, const SortCtl* sctl, const RsProduce& rsp, int grid, cudaStream_t s) {
   // (grid counts blocks of ENGINE_TB)
-  k_batch_logic<<<grid * (ENGINE_TB / BATCH_LOGIC_TB), BATCH_LOGIC_TB, 0, s>>>(jobs, tasks, ctl, ps, job_pass, free_stack, in_closest, in_any, rc_in,
-                                           out_closest, out_any, rc_out, st, job_done, sorted, sctl, rsp);
+  k_batch_logic<<<grid * (ENGINE_TB / BATCH_LOGIC_TB), BATCH_LOGIC_TB, 0, s>>>(jobs, tasks, ctl, ps, job_pass, free_stack, in_closest, in_wait, rc_in,
+                                           out_closest, out_wait, q_any, rc_out, st, job_done, sorted, sctl, rsp);
 }
 
 // ---- shade-queue sort (counting sort over SORT_KEYS keys) ----
@@ -294,25 +289,19 @@ struct KeyUdpt {
       if (tri < 0) return st * 5 + 4;
       mat = __float_as_int(__ldg(sc.shade + 4 * (size_t)tri + 3).x);
     } else {
-      mat = __float_as_int(ps.wi[p].w);
+      mat = __float_as_int(ps.hp[p].w);
     }
     return st * 5 + material_class(sc.mats[mat]);
   }
 };
-// the second of a round's two queues: any-hit rays, or the paths that wait for segments
-__device__ __forceinline__ int second_count(const RoundCounters* rc, bool fans) { return fans ? rc->n_fan : rc->n_any; }
-
 // BDPT paths: the state, and for a closest-hit result the material of the surface hit
 struct KeyBdpt {
   template <class SceneOf>
   __device__ __forceinline__ int operator()(const SceneOf& so, const PathState& ps, int p) const {
-    const int st = ps.misc[p].z & 15;   // B_LIGHT..B_FAN
+    const int z = ps.misc[p].z, st = z & 15;   // B_LIGHT..B_FAN
     // by the free segments, which are what the step has to evaluate: keys 15..23 (against one
     // key for all: two 512x512 MIS passes 5.19 -> 4.91 ms, a 1280x720 pass 9.85 -> 9.69)
-    if (st == B_FAN) {
-      const int4 fan = ps.job[p];
-      return st * 5 + __popc(~fan.z & ((1 << fan.w) - 1));
-    }
+    if (st == B_FAN) return st * 5 + __popc(~((unsigned)z >> FAN_BIT) & ((1u << ps.job[p].z) - 1u));
     const int tri = __float_as_int(ps.hit[p].w);
     if (tri < 0) return st * 5 + 4;
     const DevScene& sc = so.of(p);
@@ -323,15 +312,15 @@ struct KeyBdpt {
 template <class SceneOf, class Key>
 __global__ void __launch_bounds__(ENGINE_TB) k_sort_hist(SceneOf so, Key key_of, PathState ps,
                                                          const int* __restrict__ in_closest,
-                                                         const int* __restrict__ in_any, const RoundCounters* rc_in,
-                                                         int* keys, SortCtl* sctl, int threshold, bool fans) {
+                                                         const int* __restrict__ in_wait, const RoundCounters* rc_in,
+                                                         int* keys, SortCtl* sctl, int threshold) {
   __shared__ int h[SORT_KEYS];
   if (threadIdx.x < SORT_KEYS) h[threadIdx.x] = 0;
   __syncthreads();
-  const int nc = rc_in->n_closest, n = nc + second_count(rc_in, fans);
+  const int nc = rc_in->n_closest, n = nc + rc_in->n_wait;
   if (n < threshold) return;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const int p = e < nc ? in_closest[e] : in_any[e - nc];
+    const int p = e < nc ? in_closest[e] : in_wait[e - nc];
     const int key = key_of(so, ps, p);
     keys[e] = key;
     atomicAdd(&h[key], 1);
@@ -340,9 +329,9 @@ __global__ void __launch_bounds__(ENGINE_TB) k_sort_hist(SceneOf so, Key key_of,
   if (threadIdx.x < SORT_KEYS && h[threadIdx.x]) atomicAdd(&sctl->count[threadIdx.x], h[threadIdx.x]);
 }
 
-__global__ void k_sort_scan(const RoundCounters* rc_in, SortCtl* sctl, int threshold, bool fans) {
+__global__ void k_sort_scan(const RoundCounters* rc_in, SortCtl* sctl, int threshold) {
   if (threadIdx.x != 0) return;
-  const int n = rc_in->n_closest + second_count(rc_in, fans);
+  const int n = rc_in->n_closest + rc_in->n_wait;
   const int use = (threshold > 0 && n >= threshold) ? 1 : 0;
   if (use) {
     int run = 0;
@@ -361,13 +350,12 @@ __global__ void k_sort_scan(const RoundCounters* rc_in, SortCtl* sctl, int thres
 constexpr int SORT_U = 8;
 
 __global__ void __launch_bounds__(ENGINE_TB) k_sort_scatter(const int* __restrict__ in_closest,
-                                                            const int* __restrict__ in_any, const RoundCounters* rc_in,
-                                                            const int* __restrict__ keys, int* sorted, SortCtl* sctl,
-                                                            bool fans) {
+                                                            const int* __restrict__ in_wait, const RoundCounters* rc_in,
+                                                            const int* __restrict__ keys, int* sorted, SortCtl* sctl) {
   __shared__ int s_cnt[SORT_KEYS];
   __shared__ int s_base[SORT_KEYS];
   if (!sctl->use) return;
-  const int nc = rc_in->n_closest, n = nc + second_count(rc_in, fans);
+  const int nc = rc_in->n_closest, n = nc + rc_in->n_wait;
   const int lane = threadIdx.x & 31;
   const int tile = ENGINE_TB * SORT_U;
   // t0 is the same for every thread of the block, so the barriers below are uniform
@@ -381,7 +369,7 @@ __global__ void __launch_bounds__(ENGINE_TB) k_sort_scatter(const int* __restric
       const int e = wbase + u * 32 + lane;
       const bool active = e < n;
       key[u] = active ? keys[e] : -1 - lane;   // idle lanes match nobody
-      val[u] = active ? (e < nc ? in_closest[e] : in_any[e - nc]) : 0;
+      val[u] = active ? (e < nc ? in_closest[e] : in_wait[e - nc]) : 0;
     }
 #pragma unroll
     for (int u = 0; u < SORT_U; ++u) {
@@ -408,61 +396,29 @@ __global__ void __launch_bounds__(ENGINE_TB) k_sort_scatter(const int* __restric
 }
 
 void launch_batch_sort(const BatchJob* jobs, SF<int4> job_pass, const PathState& ps, const int* in_closest,
-                       const int* in_any, const RoundCounters* rc_in, int* keys, int* sorted, SortCtl* sctl,
+                       const int* in_wait, const RoundCounters* rc_in, int* keys, int* sorted, SortCtl* sctl,
                        int threshold, int grid, cudaStream_t s) {
-  k_sort_hist<<<grid, ENGINE_TB, 0, s>>>(SceneOfBatch{jobs, job_pass}, KeyUdpt{}, ps, in_closest, in_any, rc_in, keys,
-                                         sctl, threshold, false);
-  k_sort_scan<<<1, 32, 0, s>>>(rc_in, sctl, threshold, false);
-  k_sort_scatter<<<grid, ENGINE_TB, 0, s>>>(in_closest, in_any, rc_in, keys, sorted, sctl, false);
+  k_sort_hist<<<grid, ENGINE_TB, 0, s>>>(SceneOfBatch{jobs, job_pass}, KeyUdpt{}, ps, in_closest, in_wait, rc_in, keys,
+                                         sctl, threshold);
+  k_sort_scan<<<1, 32, 0, s>>>(rc_in, sctl, threshold);
+  k_sort_scatter<<<grid, ENGINE_TB, 0, s>>>(in_closest, in_wait, rc_in, keys, sorted, sctl);
 }
 
-void launch_pass_sort(const DevScene& sc, bool bdpt, const PathState& ps, const int* in_closest, const int* in_any,
+void launch_pass_sort(const DevScene& sc, bool bdpt, const PathState& ps, const int* in_closest, const int* in_wait,
                       const RoundCounters* rc_in, int* keys, int* sorted, SortCtl* sctl, int threshold, int grid,
                       cudaStream_t s) {
   if (bdpt)
-    k_sort_hist<<<grid, ENGINE_TB, 0, s>>>(SceneOfOne{sc}, KeyBdpt{}, ps, in_closest, in_any, rc_in, keys, sctl,
-                                           threshold, bdpt);
+    k_sort_hist<<<grid, ENGINE_TB, 0, s>>>(SceneOfOne{sc}, KeyBdpt{}, ps, in_closest, in_wait, rc_in, keys, sctl,
+                                           threshold);
   else
-    k_sort_hist<<<grid, ENGINE_TB, 0, s>>>(SceneOfOne{sc}, KeyUdpt{}, ps, in_closest, in_any, rc_in, keys, sctl,
-                                           threshold, bdpt);
-  k_sort_scan<<<1, 32, 0, s>>>(rc_in, sctl, threshold, bdpt);
-  k_sort_scatter<<<grid, ENGINE_TB, 0, s>>>(in_closest, in_any, rc_in, keys, sorted, sctl, bdpt);
+    k_sort_hist<<<grid, ENGINE_TB, 0, s>>>(SceneOfOne{sc}, KeyUdpt{}, ps, in_closest, in_wait, rc_in, keys, sctl,
+                                           threshold);
+  k_sort_scan<<<1, 32, 0, s>>>(rc_in, sctl, threshold);
+  k_sort_scatter<<<grid, ENGINE_TB, 0, s>>>(in_closest, in_wait, rc_in, keys, sorted, sctl);
 }
 
 // ---- traversal with a scene per ray ----
-template <bool ANY>
-struct BatchSrc {
-  const BatchJob* jobs;
-  SF<int4> job_pass;
-  const int* __restrict__ queue;
-  SF<float4> ro;
-  SF<float4> rd;
-  SF<float4> hit;
-  __device__ __forceinline__ const DevScene& begin(int e, RayIn& r) {
-    const int q = queue[e];
-    const float4 o = __ldg(&ro[q]);
-    const float4 d = __ldg(&rd[q]);
-    r = RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
-    return jobs[job_pass[q].x].pp.sc;
-  }
-  __device__ __forceinline__ void end(int e, const HitOut& h) {
-    const int q = queue[e];
-    if (ANY) hit[q] = make_float4(h.tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f);
-    else hit[q] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
-  }
-};
-
-template <bool ANY, bool WIDE>
-__global__ void __launch_bounds__(TRACE_TB_MAX) k_batch_trace(const BatchJob* jobs, SF<int4> job_pass,
-                                                          const int* __restrict__ queue, const int* __restrict__ count,
-                                                          int* work, SF<float4> ro,
-                                                          SF<float4> rd, SF<float4> hit, int stack_cap,
-                                                          DevStats* st, int n_smem, int* spill) {
-  BatchSrc<ANY> src{jobs, job_pass, queue, ro, rd, hit};
-  trace_loop<ANY, WIDE, false>(src, *count, work, stack_cap, st, n_smem, spill);
-}
-
-// both queues of a round: closest-hit entries first, then any-hit (or the sorted list,
+// both queues of a round: closest-hit entries first, then the segments (or the sorted list,
 // which keeps that split)
 struct BatchMixedSrc {
   const BatchJob* jobs;
@@ -474,22 +430,39 @@ struct BatchMixedSrc {
   SF<float4> ro;
   SF<float4> rd;
   SF<float4> hit;
-  __device__ __forceinline__ int slot(int e, bool any) const {
+  Segments sg;
+  __device__ __forceinline__ int entry(int e, bool any) const {
     return sorted ? sorted[e] : (any ? q_any[e - nc] : q_closest[e]);
   }
   __device__ __forceinline__ const DevScene& begin(int e, bool any, RayIn& r) {
-    const int q = slot(e, any);
-    const float4 o = __ldg(&ro[q]);
-    const float4 d = __ldg(&rd[q]);
-    r = RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
-    return jobs[job_pass[q].x].pp.sc;
+    const int q = entry(e, any);
+    r = any ? segment_ray(sg, q) : path_ray(ro, rd, q);
+    return jobs[job_pass[any ? sg.path(q) : q].x].pp.sc;
   }
   __device__ __forceinline__ void end(int e, bool any, const HitOut& h) {
-    const int q = slot(e, any);
-    hit[q] = any ? make_float4(h.tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f)
-                 : make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
+    const int q = entry(e, any);
+    if (!any) hit[q] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
+    else if (h.tri >= 0) sg.occluded(q);
   }
 };
+
+// one kind alone
+template <bool ANY>
+struct BatchSrc {
+  BatchMixedSrc both;
+  __device__ __forceinline__ const DevScene& begin(int e, RayIn& r) { return both.begin(e, ANY, r); }
+  __device__ __forceinline__ void end(int e, const HitOut& h) { both.end(e, ANY, h); }
+};
+
+template <bool ANY, bool WIDE>
+__global__ void __launch_bounds__(TRACE_TB_MAX) k_batch_trace(const BatchJob* jobs, SF<int4> job_pass,
+                                                          const int* __restrict__ queue, const int* __restrict__ count,
+                                                          int* work, SF<float4> ro, SF<float4> rd, SF<float4> hit,
+                                                          Segments sg, int stack_cap, DevStats* st, int n_smem,
+                                                          int* spill) {
+  BatchSrc<ANY> src{{jobs, job_pass, queue, queue, nullptr, 0, ro, rd, hit, sg}};
+  trace_loop<ANY, WIDE, false>(src, *count, work, stack_cap, st, n_smem, spill);
+}
 
 // At most 64 registers a thread (four blocks of 256 or eight of 128 threads per SM): with
 // the walk stack mostly outside shared memory (stack_smem) the traversal is bound by the
@@ -502,11 +475,11 @@ __global__ void __launch_bounds__(TRACE_TB_MAX, WIDE ? 3 : 4) k_batch_trace_mixe
                                                                 const int* __restrict__ q_closest,
                                                                 const int* __restrict__ q_any,
                                                                 RoundCounters* rc, SF<float4> ro,
-                                                                SF<float4> rd, SF<float4> hit,
+                                                                SF<float4> rd, SF<float4> hit, Segments sg,
                                                                 int stack_cap, DevStats* st, const int* sorted,
                                                                 const RaySortCtl* rs, int n_smem, int* spill) {
   const int nc = rc->n_closest;
-  BatchMixedSrc src{jobs, job_pass, q_closest, q_any, (rs && rs->use) ? sorted : nullptr, nc, ro, rd, hit};
+  BatchMixedSrc src{jobs, job_pass, q_closest, q_any, (rs && rs->use) ? sorted : nullptr, nc, ro, rd, hit, sg};
   trace_loop_mixed<WIDE>(src, nc, nc + rc->n_any, &rc->work_closest, stack_cap, st, n_smem, spill);
 }
 
@@ -536,34 +509,33 @@ int batch_trace_mixed_grid(int n_smem, bool wide, int tb) {
 }
 
 int launch_batch_trace_mixed(bool wide, const BatchJob* jobs, SF<int4> job_pass, const int* q_closest,
-                             const int* q_any, RoundCounters* rc, SF<float4> ro, SF<float4> rd, SF<float4> hit,
-                             DevStats* st, int stack_cap, int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s,
+                             const int* q_any, RoundCounters* rc, const PathState& ps, DevStats* st, int stack_cap, int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s,
                              const int* sorted, const RaySortCtl* rs) {
   const size_t smem = batch_smem(n_smem, tb);
   if (wide)
-    k_batch_trace_mixed<true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, q_closest, q_any, rc, ro, rd, hit,
+    k_batch_trace_mixed<true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit, record_segments(ps),
                                                             stack_cap, st, sorted, rs, n_smem, spill);
   else
-    k_batch_trace_mixed<false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, q_closest, q_any, rc, ro, rd, hit,
+    k_batch_trace_mixed<false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit, record_segments(ps),
                                                              stack_cap, st, sorted, rs, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch_batch_trace(bool any_hit, bool wide, const BatchJob* jobs, SF<int4> job_pass, const int* queue,
-                       const int* count, int* work, SF<float4> ro, SF<float4> rd, SF<float4> hit, DevStats* st,
+                       const int* count, int* work, const PathState& ps, DevStats* st,
                        int stack_cap, int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s) {
   const size_t smem = batch_smem(n_smem, tb);
   if (any_hit && wide)
-    k_batch_trace<true, true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ro, rd, hit,
+    k_batch_trace<true, true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
                                                             stack_cap, st, n_smem, spill);
   else if (any_hit)
-    k_batch_trace<true, false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ro, rd, hit,
+    k_batch_trace<true, false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
                                                              stack_cap, st, n_smem, spill);
   else if (wide)
-    k_batch_trace<false, true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ro, rd, hit,
+    k_batch_trace<false, true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
                                                              stack_cap, st, n_smem, spill);
   else
-    k_batch_trace<false, false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ro, rd, hit,
+    k_batch_trace<false, false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
                                                               stack_cap, st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

@@ -22,8 +22,8 @@
 
 namespace yc {
 
-// per-path bytes: the path record (PS_STRIDE float4, 224) + 4 queue slots (16)
-constexpr size_t NOALLOC_PATH_BYTES = PS_STRIDE * 16 + 4 * 4;
+// per-path bytes: the path record (PS_STRIDE float4, 224) + 4 queue slots + 2 segments (24)
+constexpr size_t NOALLOC_PATH_BYTES = PS_STRIDE * 16 + 6 * 4;
 constexpr size_t NOALLOC_BYTES = (size_t)NOALLOC_MAX_PATHS * NOALLOC_PATH_BYTES + 2 * sizeof(RoundCounters);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_BYTES];
@@ -113,13 +113,15 @@ int noalloc_render(const NoallocPass& a, std::string& err) {
     err = "cudaGetSymbolAddress failed for the render scratch";
     return YC_E_LAUNCH;
   }
-  // carve the scratch: the path records, 4 queues, 2 round-counter blocks
+  // carve the scratch: the path records, 4 queues, the segments' queue, 2 round-counter blocks
   const size_t N = NOALLOC_MAX_PATHS;
   float4* f = reinterpret_cast<float4*>(base);
   const PathState ps = path_state_at(f);
   int* q = reinterpret_cast<int*>(f + PS_STRIDE * N);
   int* qs[4] = {q, q + N, q + 2 * N, q + 3 * N};
-  RoundCounters* rc = reinterpret_cast<RoundCounters*>(q + 4 * N);
+  int* q_any = q + 4 * N;
+  RoundCounters* rc = reinterpret_cast<RoundCounters*>(q + 6 * N);
+  const Segments sg = record_segments(ps);
   cudaStream_t s = a.stream;
   auto launch_failed = [&](const char* what) {
     const cudaError_t e = cudaPeekAtLastError();
@@ -145,10 +147,8 @@ int noalloc_render(const NoallocPass& a, std::string& err) {
   for (int round = 0; round < a.max_rounds; ++round) {
     RoundCounters* rin = rc + cur;
     RoundCounters* rout = rc + (1 - cur);
-    if (launch_trace(a.pp.sc, false, qs[2 * cur], &rin->n_closest, &rin->work_closest, ps.ro, ps.rd, ps.hit, a.stats,
-                     grid_c, s) ||
-        launch_trace(a.pp.sc, true, qs[2 * cur + 1], &rin->n_any, &rin->work_any, ps.ro, ps.rd, ps.hit, a.stats,
-                     grid_a, s)) {
+    if (launch_trace(a.pp.sc, qs[2 * cur], rin, ps, a.stats, grid_c, s) ||
+        launch_trace_segments(a.pp.sc, q_any, rin, sg, a.stats, grid_a, s)) {
       launch_failed("trace kernel");
       if (err.empty()) err = "trace kernel launch failed";
       return YC_E_LAUNCH;
@@ -157,7 +157,7 @@ int noalloc_render(const NoallocPass& a, std::string& err) {
       err = "clearing the round counters failed";
       return YC_E_LAUNCH;
     }
-    launch_logic(a.pp, ps, qs[2 * cur], qs[2 * cur + 1], rin, qs[2 * (1 - cur)], qs[2 * (1 - cur) + 1], rout,
+    launch_logic(a.pp, ps, qs[2 * cur], qs[2 * cur + 1], rin, qs[2 * (1 - cur)], qs[2 * (1 - cur) + 1], q_any, rout,
                  a.stats, a.logic_grid, s);
     if (launch_failed("shading kernel")) return YC_E_LAUNCH;
     cur = 1 - cur;

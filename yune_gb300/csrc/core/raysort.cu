@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(RS_TB) k_rs_key(Box box, const int* __restrict
 #pragma unroll
     for (int u = 0; u < RS_U; ++u) {
       const int e = wbase + u * 32 + lane, pc = e < n ? p[u] : 0;   // idle lanes read slot 0 (n > 0 here) and discard it
-      const bool segment = sg.seg && e >= nc && e < n;
-      o[u] = __ldg(&ro[segment ? pc >> sg.shift : pc]);
-      d[u] = __ldg(segment ? sg.seg + pc : &rd[pc]);
+      const bool segment = e >= nc && e < n;
+      o[u] = __ldg(segment ? &sg.org[sg.path(pc)] : &ro[pc]);
+      d[u] = __ldg(segment ? sg.ray(pc) : &rd[pc]);
     }
 #pragma unroll
     for (int u = 0; u < RS_U; ++u) {
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(RS_TB) k_rs_key(Box box, const int* __restrict
       if (e < n) {
         float4 lo, hi;
         unsigned job;
-        box.of(p[u], lo, hi, job);
+        box.of(e >= nc ? sg.path(p[u]) : p[u], lo, hi, job);
         key = ray_key(o[u], d[u], lo, hi, ob, db) | ((job & job_mask) << (3 * (ob + db))) | (e >= nc ? kind_bit : 0u);
         keys[e] = key;
       }
@@ -208,7 +208,7 @@ int raysort_bins(int ob, int db, int jb) { return 1 << (3 * (ob + db) + jb + 1);
 template <class Box>
 static int launch_rs(const Box& box, const int* q_closest, const int* q_any, const RoundCounters* rc,
                      SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s,
-                     const Segments& sg = Segments{nullptr, 0}) {
+                     const Segments& sg) {
   if (!b.keys_any)   // else the keys and the histogram were written as the rays were queued
     k_rs_key<Box><<<grid, RS_TB, 0, s>>>(box, q_closest, q_any, rc, ro, rd, b.keys, b.hist, b.threshold, b.ob, b.db,
                                           b.jb, sg);
@@ -228,9 +228,8 @@ int launch_raysort(const DevScene& sc, const int* q_closest, const int* q_any, c
 }
 
 int launch_raysort_batch(const BatchJob* jobs, SF<int4> job_pass, const int* q_closest, const int* q_any,
-                         const RoundCounters* rc, SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid,
-                         cudaStream_t s) {
-  return launch_rs(BoxBatch{jobs, job_pass}, q_closest, q_any, rc, ro, rd, b, grid, s);
+                         const RoundCounters* rc, const PathState& ps, const RaySortBufs& b, int grid, cudaStream_t s) {
+  return launch_rs(BoxBatch{jobs, job_pass}, q_closest, q_any, rc, ps.ro, ps.rd, b, grid, s, record_segments(ps));
 }
 
 }  // namespace yc

@@ -11,11 +11,11 @@
 // runs one after another whatever the lanes in them (25-65 thousand cycles a step), so the
 // fewer runs the better (run when half the lanes wait: 1.65 ms against 1.40 ms on the glass
 // sphere). With each lane on its own the kernel ran 3.5 lanes per instruction: 1.74 ms
-// there, 1.10 ms now; 1.10 against 0.57 ms for a 256x256 frame of the Cornell box. What
-// bounds it is the longest chain of rays in a warp (12-25), at 600-1600 cycles a step of a
-// walk. Every path computes exactly what the
-// round-by-round wavefront computes (same state, same operations), so the pass's result
-// is unchanged; paths no longer wait for each other between rays.
+// there against 1.10 ms (one ray at a time), and for a 256x256 frame of the Cornell box 1.10
+// against 0.57 ms, 0.44 ms with its rays sent together. What bounds it is the longest chain
+// of rays in a warp (12-25), at 600-1600 cycles a step of a walk. Every path computes exactly
+// what the round-by-round wavefront computes (same state, same operations), so the pass's
+// result is unchanged; paths no longer wait for each other between rays.
 // The kernel is launched after every round's logic kernel on that round's output
 // queues: above the threshold it returns at once; at or below it, it finishes the pass
 // and its last block to exit empties the queues, so the remaining round launches find
@@ -32,15 +32,19 @@ constexpr int TAIL_TB = 128;
 // far more rays than any path can take (max_depth 100000, three rays per bounce); a
 // path that reaches it is left unfinished and counted in DevStats::stack_overflow
 constexpr int TAIL_MAX_RAYS = 1 << 22;
+// Where a path sends two rays at once (logic_path) idle lanes of its warp walk the second ones, at
+// least HELP_AT at a time while others walk (1, 8, 16 and 32 measured alike): four 512x512 passes
+// of the Cornell box 1.30 ms of tail with both rays walked by the path's own lane, 1.06 ms now.
+constexpr int HELP_AT = 8;
 
 // three blocks per SM: up to 170 registers a thread, which the kernel needs without spills
-template <bool WIDE>
+template <bool WIDE, bool TOGETHER>
 __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps, const int* __restrict__ in_closest,
-                                                  const int* __restrict__ in_any, RoundCounters* rc_in,
+                                                  const int* __restrict__ in_wait, RoundCounters* rc_in,
                                                   int threshold, int stack_cap, DevStats* st, int n_smem, int* spill) {
   __shared__ unsigned long long s_cnt[13];
   __shared__ bool s_last;
-  const int nc = rc_in->n_closest, n = nc + rc_in->n_any;
+  const int nc = rc_in->n_closest, n = nc + rc_in->n_wait;
   if (n == 0 || n > threshold) return;   // uniform over the grid
   if (threadIdx.x < 13) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -48,40 +52,79 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
   const int lane = threadIdx.x & 31;
   const int warps = (int)(gridDim.x * (TAIL_TB / 32));
   const int quota = min(32, (n + warps - 1) / warps);   // lanes of a warp that take paths
+  // per warp and lane: the segments of the lane's path found occluded, and the lanes of the
+  // paths in `pend` in order
+  __shared__ int s_occluded[TAIL_TB], s_pending[TAIL_TB];
+  int* occluded = s_occluded + (threadIdx.x & ~31);
+  int* pending = s_pending + (threadIdx.x & ~31);
+  occluded[lane] = 0;
+  const unsigned below = (1u << lane) - 1;
   LogicCounts lc;
   WalkCount wc;              // the current ray's walk
   unsigned overflow = 0;
   Walk w;
   w.link = LINK_NONE;
   w.leaf = 0;
-  int p = -1, rays = 0;      // this lane's path, and the rays it has walked
-  bool any = false;
+  int p = -1, rays = 0;      // this lane's path, and the rays it has sent
+  int todo = 0;              // its rays that no lane walks yet (EMIT_CLOSEST, EMIT_SEG0, EMIT_SEG1)
+  int owner = -1, wp = -1, ray = 0;   // the lane of the path whose ray this lane walks, the path, the ray
+  unsigned pend = 0;         // the lanes with todo (warp-uniform)
   bool more = true;          // the queues may still hold paths (warp-uniform)
+  const auto begin = [&](int from, int path, int which) {
+    owner = from;
+    wp = path;
+    ray = which;
+    const float4 o = which == EMIT_CLOSEST ? ps.ro[path] : ps.hp[path];
+    const float4 d = which == EMIT_SEG0 ? ps.wi[path] : ps.rd[path];
+    if (which == EMIT_CLOSEST)
+      walk_begin(pp.sc, RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z}, w);
+    else
+      walk_begin(pp.sc, RayIn{ym::add(o.x, ym::mul(d.x, EPS_F)), ym::add(o.y, ym::mul(d.y, EPS_F)),
+                              ym::add(o.z, ym::mul(d.z, EPS_F)), d.w, d.x, d.y, d.z}, w);
+  };
   for (;;) {
     const unsigned nodes = __ballot_sync(0xffffffffu, walk_wants_node(w));
     const unsigned tris = __ballot_sync(0xffffffffu, walk_wants_tri(w));
-    const unsigned have = __ballot_sync(0xffffffffu, p >= 0);
-    const unsigned waiting = have & ~(nodes | tris);   // paths whose ray is answered
-    if (waiting != have) {
+    const unsigned idle = ~(nodes | tris);
+    // (idle lanes wait until enough of them can take a ray at once)
+    if (idle != 0xffffffffu && (!TOGETHER || !pend || __popc(idle) < min(HELP_AT, __popc(pend)))) {
       bool of = false;
-      warp_walk_step<WIDE>(w, any, stack, wc, of, nodes, tris);
+      warp_walk_step<WIDE>(w, ray != EMIT_CLOSEST, stack, wc, of, nodes, tris);
       if (of) ++overflow;
       continue;
     }
-    bool ray = false;
-    if ((waiting >> lane) & 1u) {
-      unsigned long long* t = s_cnt + (any ? 9 : 6);
+    if (owner >= 0 && ((idle >> lane) & 1u)) {   // this lane's ray is answered
+      unsigned long long* t = s_cnt + (ray != EMIT_CLOSEST ? 9 : 6);
       atomicAdd(t, 1ull);
       atomicAdd(t + 1, (unsigned long long)wc.nodes);
       atomicAdd(t + 2, (unsigned long long)wc.tris);
       wc.nodes = 0; wc.tris = 0;
-      ps.hit[p] = any ? make_float4(w.best_tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f)
-                      : make_float4(w.best, w.bu, w.bv, __int_as_float(w.best_tri));
-      const int emit = logic_path(pp, pp.reset, ps, p, lc, waiting);
-      any = emit == 2;
-      ray = emit != 0;
-      if (ray && ++rays == TAIL_MAX_RAYS) { ++overflow; ray = false; }
-      if (!ray) p = -1;
+      if (ray == EMIT_CLOSEST) ps.hit[wp] = make_float4(w.best, w.bu, w.bv, __int_as_float(w.best_tri));
+      else if (w.best_tri >= 0) atomicOr(&occluded[owner], ray / EMIT_SEG0);
+      owner = -1;
+    }
+    if (TOGETHER && pend) {   // the r-th idle lane takes a ray of the r-th path that has one left
+      const int r = __popc(idle & below), r_own = __popc(pend & below), k = min(__popc(idle), __popc(pend));
+      if (todo) pending[r_own] = lane;
+      __syncwarp();
+      const bool take = ((idle >> lane) & 1u) && r < k;
+      const int from = take ? pending[r] : lane;
+      const int tp = __shfl_sync(0xffffffffu, p, from), tt = __shfl_sync(0xffffffffu, todo, from);
+      if (take) begin(from, tp, tt & -tt);
+      if (todo && r_own < k) todo &= todo - 1;
+      pend = __ballot_sync(0xffffffffu, todo != 0);
+      continue;
+    }
+    // every ray is answered
+    __syncwarp();
+    const unsigned have = __ballot_sync(0xffffffffu, p >= 0);
+    if (p >= 0) {
+      if (occluded[lane]) ps.misc[p].z |= occluded[lane] << RECORD_BIT;
+      occluded[lane] = 0;
+      todo = logic_path<TOGETHER>(pp, pp.reset, ps, p, lc, have) & ~EMIT_WAIT;
+      rays += __popc(todo);
+      if (todo && rays >= TAIL_MAX_RAYS) { ++overflow; todo = 0; }
+      if (!todo) p = -1;
     }
     if (more) {
       const bool want = p < 0 && lane < quota;
@@ -90,18 +133,18 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
       if (lane == 0 && m) base = atomicAdd(&rc_in->work_logic, __popc(m));
       base = __shfl_sync(0xffffffffu, base, 0);
       if (m && base + __popc(m) >= n) more = false;
-      const int e = base + __popc(m & ((1u << lane) - 1));
+      const int e = base + __popc(m & below);
       if (want && e < n) {
-        p = e < nc ? in_closest[e] : in_any[e - nc];
-        any = e >= nc;
+        p = e < nc ? in_closest[e] : in_wait[e - nc];
+        todo = (e < nc ? EMIT_CLOSEST : 0) | segments_of(ps.misc[p].z);
         rays = 0;
-        ray = true;
       }
     }
-    if (ray) {
-      const float4 o = ps.ro[p], d = ps.rd[p];
-      walk_begin(pp.sc, RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z}, w);
+    if (p >= 0) {   // a path's first ray is walked by its own lane
+      begin(lane, p, todo & -todo);
+      todo &= todo - 1;
     }
+    if (TOGETHER) pend = __ballot_sync(0xffffffffu, todo != 0);
     if (!more && __ballot_sync(0xffffffffu, p >= 0) == 0) break;
   }
   const unsigned long long v[6] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples};
@@ -125,6 +168,7 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
   if (threadIdx.x == 0 && s_last) {
     rc_in->n_closest = 0;
     rc_in->n_any = 0;
+    rc_in->n_wait = 0;
     rc_in->pad[0] = 0;
   }
 }
@@ -142,22 +186,26 @@ static int tail_grid_of(K kernel, size_t smem) {
   return per_sm > 0 ? per_sm * sms : -1;
 }
 
-int tail_capacity(const DevScene& sc, int n_smem, int* grid_out) {
-  const size_t smem = tail_smem(tail_entries(sc.depth, n_smem));
-  const int grid = sc.wide ? tail_grid_of(k_tail<true>, smem) : tail_grid_of(k_tail<false>, smem);
+using TailKernel = void (*)(PassParams, PathState, const int*, const int*, RoundCounters*, int, int, DevStats*, int, int*);
+static TailKernel tail_kernel(const DevScene& sc, bool together) {
+  if (together) return sc.wide ? k_tail<true, true> : k_tail<false, true>;
+  return sc.wide ? k_tail<true, false> : k_tail<false, false>;
+}
+
+int tail_capacity(const PassParams& pp, int n_smem, int* grid_out) {
+  const size_t smem = tail_smem(tail_entries(pp.sc.depth, n_smem));
+  const int grid = tail_grid_of(tail_kernel(pp.sc, rays_together(pp)), smem);
   if (grid_out) *grid_out = grid;
   return grid > 0 ? grid * TAIL_TB : 0;
 }
 
-int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_any,
+int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_wait,
                 RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s, int n_smem, int* spill) {
   const int cap = pp.sc.depth + 2;
   n_smem = tail_entries(pp.sc.depth, spill ? n_smem : 0);
   const size_t smem = tail_smem(n_smem);
-  if (pp.sc.wide)
-    k_tail<true><<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_any, rc_in, threshold, cap, st, n_smem, spill);
-  else
-    k_tail<false><<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_any, rc_in, threshold, cap, st, n_smem, spill);
+  const TailKernel kernel = tail_kernel(pp.sc, rays_together(pp));
+  kernel<<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_wait, rc_in, threshold, cap, st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

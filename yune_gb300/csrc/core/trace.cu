@@ -16,39 +16,7 @@
 
 namespace yc {
 
-// rays of the path state, addressed through the queue
-template <bool ANY>
-struct PathSrc {
-  const DevScene* sc;
-  const int* __restrict__ queue;
-  SF<float4> ro;
-  SF<float4> rd;
-  SF<float4> hit;
-  __device__ __forceinline__ const DevScene& begin(int e, RayIn& r) {
-    const int q = queue[e];
-    const float4 o = __ldg(&ro[q]);
-    const float4 d = __ldg(&rd[q]);
-    r = RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
-    return *sc;
-  }
-  __device__ __forceinline__ void end(int e, const HitOut& h) {
-    const int q = queue[e];
-    if (ANY) hit[q] = make_float4(h.tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f);
-    else hit[q] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
-  }
-};
-
-template <bool ANY, bool WIDE>
-__global__ void __launch_bounds__(TRACE_TB) k_trace_paths(DevScene sc, const int* __restrict__ queue,
-                                                          const int* __restrict__ count, int* work,
-                                                          SF<float4> ro,
-                                                          SF<float4> rd, SF<float4> hit, int stack_cap,
-                                                          DevStats* st) {
-  PathSrc<ANY> src{&sc, queue, ro, rd, hit};
-  trace_loop<ANY, WIDE, false>(src, *count, work, stack_cap, st);
-}
-
-// both queues of a round in one launch: closest-hit entries first, then any-hit (or the
+// both queues of a round in one launch: closest-hit entries first, then the segments (or the
 // sorted list, which keeps that split)
 struct PathMixedSrc {
   const DevScene* sc;
@@ -59,95 +27,49 @@ struct PathMixedSrc {
   SF<float4> ro;
   SF<float4> rd;
   SF<float4> hit;
-  __device__ __forceinline__ int slot(int e, bool any) const {
+  Segments sg;
+  __device__ __forceinline__ int entry(int e, bool any) const {
     return sorted ? sorted[e] : (any ? q_any[e - nc] : q_closest[e]);
   }
   __device__ __forceinline__ const DevScene& begin(int e, bool any, RayIn& r) {
-    const int q = slot(e, any);
-    const float4 o = __ldg(&ro[q]);
-    const float4 d = __ldg(&rd[q]);
-    r = RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
+    const int q = entry(e, any);
+    r = any ? segment_ray(sg, q) : path_ray(ro, rd, q);
     return *sc;
   }
   __device__ __forceinline__ void end(int e, bool any, const HitOut& h) {
-    const int q = slot(e, any);
-    hit[q] = any ? make_float4(h.tri >= 0 ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f)
-                 : make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
+    const int q = entry(e, any);
+    if (!any) hit[q] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
+    else if (h.tri >= 0) sg.occluded(q);
   }
 };
 
 template <bool WIDE>
 __global__ void __launch_bounds__(TRACE_TB) k_trace_paths_mixed(DevScene sc, const int* __restrict__ q_closest,
                                                                 const int* __restrict__ q_any, RoundCounters* rc,
-                                                                SF<float4> ro,
-                                                                SF<float4> rd, SF<float4> hit,
-                                                                int stack_cap, DevStats* st, const int* sorted,
-                                                                const RaySortCtl* rs, int n_smem, int* spill) {
+                                                                SF<float4> ro, SF<float4> rd, SF<float4> hit,
+                                                                Segments sg, int stack_cap, DevStats* st,
+                                                                const int* sorted, const RaySortCtl* rs, int n_smem,
+                                                                int* spill) {
   const int nc = rc->n_closest;
-  PathMixedSrc src{&sc, q_closest, q_any, (rs && rs->use) ? sorted : nullptr, nc, ro, rd, hit};
+  PathMixedSrc src{&sc, q_closest, q_any, (rs && rs->use) ? sorted : nullptr, nc, ro, rd, hit, sg};
   trace_loop_mixed<WIDE>(src, nc, nc + rc->n_any, &rc->work_closest, stack_cap, st, n_smem, spill);
 }
 
-// both queues of a BDPT round: the any-hit entries are segments (yc_internal.h)
-struct FanMixedSrc {
-  const DevScene* sc;
-  const int* __restrict__ q_closest;
-  const int* __restrict__ q_any;
-  const int* __restrict__ sorted;
-  int nc;
-  SF<float4> ro;
-  SF<float4> rd;
-  SF<float4> hit;
-  SF<int4> job;
-  Segments sg;
-  __device__ __forceinline__ int slot(int e, bool any) const {
-    return (sorted ? sorted[e] : (any ? q_any[e - nc] : q_closest[e]));
-  }
-  __device__ __forceinline__ const DevScene& begin(int e, bool any, RayIn& r) {
-    const int q = slot(e, any);
-    const float4 o = __ldg(&ro[any ? q >> sg.shift : q]);
-    if (any) {
-      const float4 d = __ldg(sg.seg + q);
-      r = RayIn{ym::add(o.x, ym::mul(d.x, EPS_F)), ym::add(o.y, ym::mul(d.y, EPS_F)), ym::add(o.z, ym::mul(d.z, EPS_F)),
-                d.w, d.x, d.y, d.z};
-    } else {
-      const float4 d = __ldg(&rd[q]);
-      r = RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
-    }
-    return *sc;
-  }
-  __device__ __forceinline__ void end(int e, bool any, const HitOut& h) {
-    const int q = slot(e, any);
-    if (!any) hit[q] = make_float4(h.t, h.u, h.v, __int_as_float(h.tri));
-    else if (h.tri >= 0) atomicOr(&job[q >> sg.shift].z, 1 << (q & ((1 << sg.shift) - 1)));
-  }
+// one kind alone
+template <bool ANY>
+struct PathSrc {
+  PathMixedSrc both;
+  __device__ __forceinline__ const DevScene& begin(int e, RayIn& r) { return both.begin(e, ANY, r); }
+  __device__ __forceinline__ void end(int e, const HitOut& h) { both.end(e, ANY, h); }
 };
 
-template <bool WIDE>
-__global__ void __launch_bounds__(TRACE_TB) k_trace_fans(DevScene sc, const int* __restrict__ q_closest,
-                                                         const int* __restrict__ q_any, RoundCounters* rc,
-                                                         PathState ps, Segments sg, int stack_cap,
-                                                         DevStats* st, const int* sorted, const RaySortCtl* rs,
-                                                         int n_smem, int* spill) {
-  const int nc = rc->n_closest;
-  FanMixedSrc src{&sc, q_closest, q_any, (rs && rs->use) ? sorted : nullptr, nc, ps.ro, ps.rd, ps.hit, ps.job, sg};
-  trace_loop_mixed<WIDE>(src, nc, nc + rc->n_any, &rc->work_closest, stack_cap, st, n_smem, spill);
-}
-
-// the segments of a round alone
-struct SegmentSrc {
-  FanMixedSrc fans;
-  __device__ __forceinline__ const DevScene& begin(int e, RayIn& r) { return fans.begin(e, true, r); }
-  __device__ __forceinline__ void end(int e, const HitOut& h) { fans.end(e, true, h); }
-};
-
-template <bool WIDE>
-__global__ void __launch_bounds__(TRACE_TB) k_trace_segments(DevScene sc, const int* __restrict__ q_any,
-                                                             RoundCounters* rc, PathState ps,
-                                                             Segments sg, int stack_cap,
-                                                             DevStats* st) {
-  SegmentSrc src{{&sc, nullptr, q_any, nullptr, 0, ps.ro, ps.rd, ps.hit, ps.job, sg}};
-  trace_loop<true, WIDE, false>(src, rc->n_any, &rc->work_any, stack_cap, st);
+template <bool ANY, bool WIDE>
+__global__ void __launch_bounds__(TRACE_TB) k_trace_paths(DevScene sc, const int* __restrict__ queue,
+                                                          RoundCounters* rc, SF<float4> ro, SF<float4> rd,
+                                                          SF<float4> hit, Segments sg, int stack_cap, DevStats* st) {
+  PathSrc<ANY> src{{&sc, queue, queue, nullptr, 0, ro, rd, hit, sg}};
+  trace_loop<ANY, WIDE, false>(src, ANY ? rc->n_any : rc->n_closest, ANY ? &rc->work_any : &rc->work_closest, stack_cap,
+                               st);
 }
 
 // traceRay (udpt.cl:240-286) on explicit rays of 9 floats: light loop, then the BVH.
@@ -216,30 +138,22 @@ int trace_grid_blocks(bool any_hit, int depth, bool wide) {
   return any_hit ? resident_grid(k_trace_paths<true, false>, smem) : resident_grid(k_trace_paths<false, false>, smem);
 }
 
-int launch_trace(const DevScene& sc, bool any_hit, const int* queue, const int* count, int* work, SF<float4> ro,
-                 SF<float4> rd, SF<float4> hit, DevStats* st, int grid_blocks, cudaStream_t s) {
+template <bool ANY>
+static int launch_alone(const DevScene& sc, const int* queue, RoundCounters* rc, SF<float4> ro, SF<float4> rd,
+                        SF<float4> hit, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s) {
   const int cap = stack_cap_for(sc.depth);
   const size_t smem = smem_for(cap);
-  const bool wide = sc.wide != 0;
-  if (any_hit && wide)
-    k_trace_paths<true, true><<<grid_blocks, TRACE_TB, smem, s>>>(sc, queue, count, work, ro, rd, hit, cap, st);
-  else if (any_hit)
-    k_trace_paths<true, false><<<grid_blocks, TRACE_TB, smem, s>>>(sc, queue, count, work, ro, rd, hit, cap, st);
-  else if (wide)
-    k_trace_paths<false, true><<<grid_blocks, TRACE_TB, smem, s>>>(sc, queue, count, work, ro, rd, hit, cap, st);
-  else
-    k_trace_paths<false, false><<<grid_blocks, TRACE_TB, smem, s>>>(sc, queue, count, work, ro, rd, hit, cap, st);
+  if (sc.wide) k_trace_paths<ANY, true><<<grid_blocks, TRACE_TB, smem, s>>>(sc, queue, rc, ro, rd, hit, sg, cap, st);
+  else k_trace_paths<ANY, false><<<grid_blocks, TRACE_TB, smem, s>>>(sc, queue, rc, ro, rd, hit, sg, cap, st);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
-
-int launch_trace_segments(const DevScene& sc, const int* q_any, RoundCounters* rc, const PathState& ps,
-                          const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s) {
-  const int cap = stack_cap_for(sc.depth);
-  const size_t smem = smem_for(cap);
-  const auto kernel = sc.wide ? k_trace_segments<true> : k_trace_segments<false>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kernel<<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_any, rc, ps, sg, cap, st);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+int launch_trace(const DevScene& sc, const int* queue, RoundCounters* rc, const PathState& ps, DevStats* st,
+                 int grid_blocks, cudaStream_t s) {
+  return launch_alone<false>(sc, queue, rc, ps.ro, ps.rd, ps.hit, Segments{}, st, grid_blocks, s);
+}
+int launch_trace_segments(const DevScene& sc, const int* q_any, RoundCounters* rc, const Segments& sg, DevStats* st,
+                          int grid_blocks, cudaStream_t s) {
+  return launch_alone<true>(sc, q_any, rc, {}, {}, {}, sg, st, grid_blocks, s);
 }
 
 static_assert(TRACE_TB == TRACE_TB_PASS, "the host sizes the per-pass spill area by TRACE_TB_PASS");
@@ -251,30 +165,18 @@ int trace_mixed_grid_blocks(int depth, bool wide, int n_smem) {
   return wide ? resident_grid(k_trace_paths_mixed<true>, smem) : resident_grid(k_trace_paths_mixed<false>, smem);
 }
 
-int launch_trace_fans(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,
-                      const PathState& ps, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s,
-                      const int* sorted, const RaySortCtl* rs, int n_smem, int* spill) {
-  const int cap = stack_cap_for(sc.depth);
-  if (!(n_smem > 0 && n_smem < cap && spill)) n_smem = cap;
-  const size_t smem = smem_for(n_smem);
-  const auto kernel = sc.wide ? k_trace_fans<true> : k_trace_fans<false>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kernel<<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_closest, q_any, rc, ps, sg, cap, st, sorted, rs, n_smem, spill);
-  return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
-}
-
 int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,
-                       SF<float4> ro, SF<float4> rd, SF<float4> hit, DevStats* st, int grid_blocks,
-                       cudaStream_t s, const int* sorted, const RaySortCtl* rs, int n_smem, int* spill) {
+                       const PathState& ps, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s,
+                       const int* sorted, const RaySortCtl* rs, int n_smem, int* spill) {
   const int cap = stack_cap_for(sc.depth);
   if (!(n_smem > 0 && n_smem < cap && spill)) n_smem = cap;
   const size_t smem = smem_for(n_smem);
   if (sc.wide)
-    k_trace_paths_mixed<true><<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_closest, q_any, rc, ro, rd, hit, cap, st,
-                                                                  sorted, rs, n_smem, spill);
+    k_trace_paths_mixed<true><<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit, sg, cap,
+                                                                  st, sorted, rs, n_smem, spill);
   else
-    k_trace_paths_mixed<false><<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_closest, q_any, rc, ro, rd, hit, cap, st,
-                                                                   sorted, rs, n_smem, spill);
+    k_trace_paths_mixed<false><<<grid_blocks, TRACE_TB, smem, s>>>(sc, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit, sg,
+                                                                   cap, st, sorted, rs, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

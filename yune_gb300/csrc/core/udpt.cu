@@ -6,11 +6,11 @@
 //   raygen (a)   -> primary rays into the closest-hit queue
 //   trace        -> extend kernel (b) on the closest-hit queue, occlusion kernel on the
 //                   any-hit queue (NEE shadow rays and MIS BRDF rays, (d))
-//   logic        -> advances each path that got a result until it needs its next ray
-//                   (shading (c), light sampling and MIS (d), Russian roulette); the new
-//                   rays are appended to the next round's queues with one warp ballot +
-//                   popc prefix and one atomic per warp (e), so finished paths drop out
-//                   and the queues stay dense.
+//   logic        -> advances each path whose rays are answered until it needs new ones
+//                   (shading (c), light sampling and MIS (d), Russian roulette), up to
+//                   three at once (logic_path); the new rays are appended to the next
+//                   round's queues with warp prefixes and one atomic per warp and queue
+//                   (e), so finished paths drop out and the queues stay dense.
 // A path that finishes writes its colour into the running-mean accumulator
 // (udpt.cl:193-210). The random numbers of a path are drawn in the reference order,
 // from the same per-pixel xorshift stream.
@@ -66,15 +66,17 @@ void launch_raygen(const PassParams& pp, const PathState& ps, int* q_closest, Ro
 
 // ---- logic: one step of every path in the input queues ----
 
+template <bool TOGETHER>
 __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps, const int* __restrict__ in_closest,
-                                                    const int* __restrict__ in_any, const RoundCounters* rc_in,
-                                                    int* out_closest, int* out_any, RoundCounters* rc_out,
+                                                    const int* __restrict__ in_wait, const RoundCounters* rc_in,
+                                                    int* out_closest, int* out_wait, int* q_any,
+                                                    RoundCounters* rc_out,
                                                     DevStats* st, const int* __restrict__ sorted,
                                                     const SortCtl* sctl) {
   __shared__ unsigned long long s_cnt[8];   // rays, extension, shadow, mis, traversed, samples
   if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
   __syncthreads();
-  const int nc = rc_in->n_closest, na = rc_in->n_any;
+  const int nc = rc_in->n_closest, na = rc_in->n_wait;
   const int n = nc + na;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -87,22 +89,11 @@ __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps,
     LogicCounts lc;
     const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
-      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_any[e - nc]);
-      emit = logic_path(pp, pp.reset, ps, p, lc, mask);
+      p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_wait[e - nc]);
+      emit = logic_path<TOGETHER>(pp, pp.reset, ps, p, lc, mask);
     }
-    // compaction: ballot + popc prefix per queue, one atomic per warp and queue
-    const unsigned mc = __ballot_sync(0xffffffffu, emit == 1);
-    const unsigned ma = __ballot_sync(0xffffffffu, emit == 2);
-    int bc = 0, ba = 0;
-    if (lane == 0) {
-      if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
-      if (ma) ba = atomicAdd(&rc_out->n_any, __popc(ma));
-    }
-    bc = __shfl_sync(0xffffffffu, bc, 0);
-    ba = __shfl_sync(0xffffffffu, ba, 0);
-    const unsigned below = (1u << lane) - 1;
-    if (emit == 1) out_closest[bc + __popc(mc & below)] = p;
-    if (emit == 2) out_any[ba + __popc(ma & below)] = p;
+    RaysOut at;
+    append_rays(emit, p, out_closest, out_wait, q_any, rc_out, at);
     // counters
     unsigned v[6] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples};
 #pragma unroll
@@ -124,10 +115,11 @@ __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps,
   }
 }
 
-void launch_logic(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_any,
-                  const RoundCounters* rc_in, int* out_closest, int* out_any, RoundCounters* rc_out, DevStats* st,
-                  int grid, cudaStream_t s, const int* sorted, const SortCtl* sctl) {
-  k_logic<<<grid, LOGIC_TB, 0, s>>>(pp, ps, in_closest, in_any, rc_in, out_closest, out_any, rc_out, st, sorted,
+void launch_logic(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_wait,
+                  const RoundCounters* rc_in, int* out_closest, int* out_wait, int* q_any, RoundCounters* rc_out,
+                  DevStats* st, int grid, cudaStream_t s, const int* sorted, const SortCtl* sctl) {
+  const auto kernel = rays_together(pp) ? k_logic<true> : k_logic<false>;
+  kernel<<<grid, LOGIC_TB, 0, s>>>(pp, ps, in_closest, in_wait, rc_in, out_closest, out_wait, q_any, rc_out, st, sorted,
                                     sctl);
 }
 

@@ -32,8 +32,9 @@ struct BdptBuffers {
   float4* ev;
   size_t N;
   int bounces;
-  Segments sg;    // the segments of the round
-  int* q_seg;     // and their queue
+  Segments sg;    // the segments of the round, at seg[(p << sg.shift) + s],
+  float4* seg;
+  int* q_any;     // and their queue
 };
 
 #ifdef __CUDACC__
@@ -43,7 +44,7 @@ struct FanOut {
   int n = 0;
   __device__ __forceinline__ bool full(const BdptBuffers& bb) const { return n >> bb.sg.shift; }
   __device__ __forceinline__ void add(const BdptBuffers& bb, int p, int j, const ym::f4& dir, float len) {
-    bb.sg.seg[((size_t)p << bb.sg.shift) + n] = make_float4(dir.x, dir.y, dir.z, len);
+    bb.seg[((size_t)p << bb.sg.shift) + n] = make_float4(dir.x, dir.y, dir.z, len);
     js |= (unsigned long long)j << (8 * n);
     ++n;
   }
@@ -52,9 +53,9 @@ struct FanOut {
 struct FanIn {
   unsigned long long js;
   unsigned free;
-  __device__ __forceinline__ void load(const int4& job) {
+  __device__ __forceinline__ void load(const int4& job, const int4& misc) {
     js = (unsigned)job.x | ((unsigned long long)(unsigned)job.y << 32);
-    free = ~(unsigned)job.z & ((1u << job.w) - 1u);
+    free = ~((unsigned)misc.z >> FAN_BIT) & ((1u << job.z) - 1u);
   }
   __device__ __forceinline__ int vertex(int s) const { return (int)(js >> (8 * s)) & 255; }
 };
@@ -62,7 +63,7 @@ struct FanIn {
 // the queue entries of a warp's lanes: paths with a closest-hit ray (emit 1), and paths that wait
 // for `segs` segments (emit 2) with the segments themselves; all 32 lanes call it
 __device__ __forceinline__ void append_bdpt(const BdptBuffers& bb, int emit, int p, int segs, int* out_closest,
-                                            int* out_fan, RoundCounters* rc_out) {
+                                            int* out_wait, RoundCounters* rc_out) {
   const int lane = threadIdx.x & 31;
   const unsigned mc = __ballot_sync(0xffffffffu, emit == 1), mf = __ballot_sync(0xffffffffu, emit == 2);
   const unsigned below = (1u << lane) - 1;
@@ -76,7 +77,7 @@ __device__ __forceinline__ void append_bdpt(const BdptBuffers& bb, int emit, int
   int bc = 0, bf = 0, bs = 0;
   if (lane == 0) {
     if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
-    if (mf) bf = atomicAdd(&rc_out->n_fan, __popc(mf));
+    if (mf) bf = atomicAdd(&rc_out->n_wait, __popc(mf));
     if (total) bs = atomicAdd(&rc_out->n_any, total);
   }
   bc = __shfl_sync(0xffffffffu, bc, 0);
@@ -84,8 +85,8 @@ __device__ __forceinline__ void append_bdpt(const BdptBuffers& bb, int emit, int
   bs = __shfl_sync(0xffffffffu, bs, 0);
   if (emit == 1) out_closest[bc + __popc(mc & below)] = p;
   if (emit == 2) {
-    out_fan[bf + __popc(mf & below)] = p;
-    int* q = bb.q_seg + (bs + incl - segs);
+    out_wait[bf + __popc(mf & below)] = p;
+    int* q = bb.q_any + (bs + incl - segs);
     for (int k = 0; k < segs; ++k) q[k] = (p << bb.sg.shift) + k;
   }
 }
@@ -94,7 +95,7 @@ __device__ __forceinline__ void append_bdpt(const BdptBuffers& bb, int emit, int
 void launch_raygen_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, int* q_closest,
                         RoundCounters* rc, DevStats* st, cudaStream_t s);
 void launch_logic_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                       const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
+                       const int* in_wait, const RoundCounters* rc_in, int* out_closest, int* out_wait,
                        RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted = nullptr,
                        const SortCtl* sctl = nullptr);
 // the bidirectional tracer with multiple importance sampling (bdpt_mis.cu): same buffers,
@@ -102,7 +103,7 @@ void launch_logic_bdpt(const PassParams& pp, const PathState& ps, const BdptBuff
 void launch_raygen_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, int* q_closest,
                             RoundCounters* rc, DevStats* st, cudaStream_t s);
 void launch_logic_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
-                           const int* in_fan, const RoundCounters* rc_in, int* out_closest, int* out_fan,
+                           const int* in_wait, const RoundCounters* rc_in, int* out_closest, int* out_wait,
                            RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted = nullptr,
                            const SortCtl* sctl = nullptr);
 

@@ -39,7 +39,7 @@ struct BatchCtl {
 };
 
 void launch_batch_sort(const BatchJob* jobs, SF<int4> job_pass, const PathState& ps, const int* in_closest,
-                       const int* in_any, const RoundCounters* rc_in, int* keys, int* sorted, SortCtl* sctl,
+                       const int* in_wait, const RoundCounters* rc_in, int* keys, int* sorted, SortCtl* sctl,
                        int threshold, int grid, cudaStream_t s);
 
 // The ray-sort keys of the rays a kernel queues (RaySortBufs: keys of the closest-hit
@@ -55,8 +55,8 @@ void launch_batch_fill(const BatchJob* jobs, BatchTasks* tasks, BatchCtl* ctl, c
                        int* free_stack, int* q_closest, RoundCounters* rc, DevStats* st, const RsProduce& rsp, int grid,
                        cudaStream_t s);
 void launch_batch_logic(const BatchJob* jobs, BatchTasks* tasks, BatchCtl* ctl, const PathState& ps, SF<int4> job_pass,
-                        int* free_stack, const int* in_closest, const int* in_any, const RoundCounters* rc_in,
-                        int* out_closest, int* out_any, RoundCounters* rc_out, DevStats* st,
+                        int* free_stack, const int* in_closest, const int* in_wait, const RoundCounters* rc_in,
+                        int* out_closest, int* out_wait, int* q_any, RoundCounters* rc_out, DevStats* st,
                         unsigned long long* job_done, const int* sorted, const SortCtl* sctl, const RsProduce& rsp,
                         int grid, cudaStream_t s);
 // tb: threads per block of the trace kernels (32..256, a multiple of 32)
@@ -64,23 +64,22 @@ void launch_batch_logic(const BatchJob* jobs, BatchTasks* tasks, BatchCtl* ctl, 
 // in `spill`, one column per thread of the launch (grid_blocks * tb columns of
 // 2 * (stack_cap - n_smem) ints; may be null when n_smem == stack_cap).
 int launch_batch_trace(bool any_hit, bool wide, const BatchJob* jobs, SF<int4> job_pass, const int* queue,
-                       const int* count, int* work, SF<float4> ro, SF<float4> rd, SF<float4> hit, DevStats* st,
+                       const int* count, int* work, const PathState& ps, DevStats* st,
                        int stack_cap, int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s);
 int batch_trace_grid(bool any_hit, int n_smem, bool wide, int tb);
 // one launch over both queues of a round (closest-hit entries, then any-hit); the work
 // cursor is rc->work_closest
 int launch_batch_trace_mixed(bool wide, const BatchJob* jobs, SF<int4> job_pass, const int* q_closest,
-                             const int* q_any, RoundCounters* rc, SF<float4> ro, SF<float4> rd, SF<float4> hit,
-                             DevStats* st, int stack_cap, int n_smem, int* spill, int grid_blocks, int tb,
-                             cudaStream_t s, const int* sorted = nullptr, const RaySortCtl* rs = nullptr);
+                             const int* q_any, RoundCounters* rc, const PathState& ps, DevStats* st, int stack_cap,
+                             int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s,
+                             const int* sorted = nullptr, const RaySortCtl* rs = nullptr);
 // the same shade-queue sort for the per-pass path (one scene)
-void launch_pass_sort(const DevScene& sc, bool bdpt, const PathState& ps, const int* in_closest, const int* in_any,
+void launch_pass_sort(const DevScene& sc, bool bdpt, const PathState& ps, const int* in_closest, const int* in_wait,
                       const RoundCounters* rc_in, int* keys, int* sorted, SortCtl* sctl, int threshold, int grid,
                       cudaStream_t s);
 // raysort.cu, with the scene box of each ray's job
 int launch_raysort_batch(const BatchJob* jobs, SF<int4> job_pass, const int* q_closest, const int* q_any,
-                         const RoundCounters* rc, SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid,
-                         cudaStream_t s);
+                         const RoundCounters* rc, const PathState& ps, const RaySortBufs& b, int grid, cudaStream_t s);
 int batch_trace_mixed_grid(int n_smem, bool wide, int tb);
 
 }  // namespace yc

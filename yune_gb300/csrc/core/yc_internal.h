@@ -16,13 +16,14 @@ namespace yc {
 // The logic kernel reads and writes a path's whole record, and after the shade-queue
 // sort neighbouring threads hold unrelated slots; one contiguous record per path keeps
 // every sector it fetches fully used (a field per array would use half of each). The
-// ray, the batch engine's (job, pass) pair and the hit come first, so the traversal
-// kernels touch the first two sectors only.
+// closest-hit ray shares a sector, so do the batch engine's (job, pass) pair and the hit, and
+// a shadow ray's direction and origin.
 // misc.x seed, misc.y pixel index, misc.z packed (state | flags << 4 | (j+1) << 12 |
-// (k+1) << 20), misc.w bounce index.
+// (k+1) << 20; the trace sets bit 28 when the path's shadow ray is occluded, bit 29 for its
+// MIS ray), misc.w bounce index.
 constexpr int PS_STRIDE = 14;
 enum { PSF_RO = 0, PSF_RD, PSF_JOB, PSF_HIT, PSF_MISC, PSF_THR, PSF_THR_NEXT, PSF_DIRECT, PSF_INDIRECT, PSF_LS,
-       PSF_HP, PSF_NRM, PSF_WO, PSF_WI };
+       PSF_HP, PSF_WI, PSF_WO, PSF_NRM };
 
 // one field of every record: slot i at p[i * PS_STRIDE]
 template <class T>
@@ -37,14 +38,14 @@ struct PathState {
   SF<float4> thr_next;   // throughput after the pending bounce (udpt.cl:504-507)
   SF<float4> direct;     // direct_color (udpt.cl:455)
   SF<float4> indirect;   // indirect_color
-  SF<float4> ls;         // light_sample of the pending NEE (udpt.cl:562-563)
-  SF<float4> hp;         // xyz hit point, w light_pdf
-  SF<float4> nrm;        // xyz shading normal, w brdf_prob of the NEE lobe
-  SF<float4> wo;         // xyz w_o, w brdf_pdf of the MIS sample
-  SF<float4> wi;         // xyz NEE direction, w material index (int bits)
-  SF<float4> ro;         // emitted ray: origin xyz, length
-  SF<float4> rd;         // emitted ray: direction xyz
-  SF<float4> hit;        // trace result: (t, u, v, tri) or (occluded, -, -, -)
+  SF<float4> ls;         // light_sample of the NEE in flight (udpt.cl:562-563)
+  SF<float4> hp;         // xyz hit point, w material index (int bits)
+  SF<float4> nrm;        // xyz shading normal, w light_pdf
+  SF<float4> wo;         // xyz w_o, w brdf_pdf of the MIS ray
+  SF<float4> wi;         // the shadow ray: direction xyz, length
+  SF<float4> ro;         // emitted closest-hit ray: origin xyz, length; or x brdf_prob of the MIS ray
+  SF<float4> rd;         // emitted closest-hit ray: direction xyz; or the MIS ray: direction xyz, length
+  SF<float4> hit;        // its result: (t, u, v, tri)
   SF<int4> job;          // batch engine: (job, pass) of the slot's pixel task
 };
 
@@ -68,12 +69,6 @@ inline PathState path_state_at(float4* rec) {
   return ps;
 }
 
-// queues of one round: path indices for the closest-hit and the any-hit kernels
-struct Queues {
-  int* closest;
-  int* any;
-};
-
 // per-round device counters (cleared by one memset per round)
 struct RoundCounters {
   int n_closest;      // entries appended to the closest queue
@@ -81,21 +76,40 @@ struct RoundCounters {
   int work_closest;   // persistent-kernel work cursors
   int work_any;
   int work_logic;
-  int n_fan;          // BDPT passes: paths that wait for segments (n_any counts the segments)
+  int n_wait;         // paths without a closest-hit ray that wait for segments (n_any counts the segments)
   int pad[2];
 };
 
-// The segments of a bidirectional path. An eye vertex sends its shadow rays, to a light and to
-// the light subpath's vertices, in one round. Segment s of path p is at seg[(p << shift) + s] =
-// (direction, length); the common origin of a path's segments, before the offset along the
-// direction, is its ro; the any-hit queue holds (p << shift) + s; a segment found occluded sets
-// bit s of the path's job.z. (A path waits in the fan queue of its round; byte s of job.x, job.y
-// says which light vertex segment s goes to, job.w how many segments there are.)
+// The segments (any-hit rays) of a path: several may be in flight in one round, beside a
+// closest-hit ray or instead of one. Segment s of path p is entry q = (p << shift) + s of the
+// any-hit queue, its direction and length are at base[p * stride + s * step], its origin is
+// org[p] moved along the direction by EPS_F, and a segment found occluded sets bit (bit + s) of
+// misc[p].z, which the step that sends it writes.
+// A path without a closest-hit ray that waits for segments is in the round's waiting queue.
+//   unidirectional: the shadow and the MIS ray of a vertex, in the record (wi and rd, from hp)
+//   bidirectional: the shadow rays of an eye vertex, to a light and to the light subpath's
+//     vertices, up to 2^shift at once, in an array of their own (from ro); byte s of job.x,
+//     job.y says which light vertex segment s goes to, job.z how many segments there are
 struct Segments {
-  float4* seg;
-  int shift;       // 2^shift segments a path at most
+  const float4* base;
+  SF<float4> org;
+  SF<int4> misc;
+  int stride, step, shift, bit;
+#ifdef __CUDACC__
+  __device__ __forceinline__ int path(int q) const { return q >> shift; }
+  __device__ __forceinline__ int index(int q) const { return q & ((1 << shift) - 1); }
+  __device__ __forceinline__ const float4* ray(int q) const {
+    return base + ((long long)path(q) * stride + index(q) * step);
+  }
+  __device__ __forceinline__ void occluded(int q) const { atomicOr(&misc[path(q)].z, 1 << (bit + index(q))); }
+#endif
 };
 constexpr int FAN_SHIFT = 3;
+constexpr int FAN_BIT = 20, RECORD_BIT = 28;   // `bit` of the two
+// the two segments of a unidirectional path
+inline Segments record_segments(const PathState& ps) {
+  return Segments{ps.wi.p, ps.hp, ps.misc, PS_STRIDE, PSF_RD - PSF_WI, 1, RECORD_BIT};
+}
 
 // Sorting of a round's traversal work list by ray origin and direction (raysort.cu):
 // `use` tells the trace kernel whether this round's list is the sorted one.
@@ -211,20 +225,22 @@ void launch_exclusive_scan(const int* in, int* out, int* tile_sum, int n, cudaSt
 // launchers (udpt.cu / trace.cu)
 void launch_raygen(const PassParams& pp, const PathState& ps, int* q_closest, RoundCounters* rc, DevStats* st,
                    cudaStream_t s);
-// sorted/sctl: the round's shade queue sorted by phase and material class, used when
-// sctl->use is set (null: the queues in order)
-void launch_logic(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_any,
-                  const RoundCounters* rc_in, int* out_closest, int* out_any, RoundCounters* rc_out,
+// sorted/sctl: the round's shade queue (the paths of the closest-hit and the waiting queue) sorted
+// by phase and material class, used when sctl->use is set (null: the queues in order)
+void launch_logic(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_wait,
+                  const RoundCounters* rc_in, int* out_closest, int* out_wait, int* q_any, RoundCounters* rc_out,
                   DevStats* st, int grid, cudaStream_t s, const int* sorted = nullptr,
                   const SortCtl* sctl = nullptr);
-int launch_trace(const DevScene& sc, bool any_hit, const int* queue, const int* count, int* work,
-                 SF<float4> ro, SF<float4> rd, SF<float4> hit, DevStats* st, int grid_blocks,
-                 cudaStream_t s);
+// a round's closest-hit queue alone, and its segments alone (whole stack in shared memory)
+int launch_trace(const DevScene& sc, const int* queue, RoundCounters* rc, const PathState& ps, DevStats* st,
+                 int grid_blocks, cudaStream_t s);
+int launch_trace_segments(const DevScene& sc, const int* q_any, RoundCounters* rc, const Segments& sg, DevStats* st,
+                          int grid_blocks, cudaStream_t s);
 void launch_tonemap(const float4* in, float4* out, int n, cudaStream_t s);
 // tail.cu: finish a pass's paths one thread each once at most `threshold` are left
-int tail_capacity(const DevScene& sc, int n_smem, int* grid_out);
+int tail_capacity(const PassParams& pp, int n_smem, int* grid_out);
 // n_smem, spill: as for launch_trace_mixed (grid * TAIL_TB columns)
-int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_any,
+int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_wait,
                 RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s, int n_smem, int* spill);
 // direct query: rays as 9 floats each
 // (n_smem, spill: as for launch_trace_mixed)
@@ -237,22 +253,15 @@ int trace_grid_blocks(bool any_hit, int depth, bool wide);
 // shared memory, the deeper ones in `spill` (grid_blocks * TRACE_TB columns of
 // 2 * (depth - n_smem) ints); otherwise the whole stack is in shared memory.
 int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,
-                       SF<float4> ro, SF<float4> rd, SF<float4> hit, DevStats* st, int grid_blocks,
-                       cudaStream_t s, const int* sorted = nullptr, const RaySortCtl* rs = nullptr, int n_smem = 0,
+                       const PathState& ps, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s,
+                       const int* sorted = nullptr, const RaySortCtl* rs = nullptr, int n_smem = 0,
                        int* spill = nullptr);
-// the same over a BDPT round, whose any-hit queue holds segments, and the segments alone
-// (whole stack in shared memory; trace_grid_blocks' grid)
-int launch_trace_fans(const DevScene& sc, const int* q_closest, const int* q_any, RoundCounters* rc,
-                      const PathState& ps, const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s,
-                      const int* sorted, const RaySortCtl* rs, int n_smem, int* spill);
-int launch_trace_segments(const DevScene& sc, const int* q_any, RoundCounters* rc, const PathState& ps,
-                          const Segments& sg, DevStats* st, int grid_blocks, cudaStream_t s);
 // raysort.cu: sorts the round's work list (closest-hit queue, then any-hit queue) into
 // b.sorted when the round has at least b.threshold rays, and sets b.ctl->use
 int raysort_bins(int ob, int db, int jb = 0);
 int launch_raysort(const DevScene& sc, const int* q_closest, const int* q_any, const RoundCounters* rc,
                    SF<float4> ro, SF<float4> rd, const RaySortBufs& b, int grid, cudaStream_t s,
-                   const Segments& sg = Segments{nullptr, 0});
+                   const Segments& sg);
 int trace_mixed_grid_blocks(int depth, bool wide, int n_smem = 0);
 int trace_stack_cap(int depth);   // walk-stack entries the per-pass kernels give a scene of this depth
 constexpr int TRACE_TB_PASS = 128;   // block of the per-pass trace kernels (TRACE_TB of yc_trace_loop.cuh)

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "yc_internal.h"
+#include "yc_shade.cuh"
 #include "yc_traverse.cuh"
 
 namespace yc {
@@ -37,6 +38,17 @@ __device__ __forceinline__ void flush_counts(DevStats* st, unsigned rays, const 
       atomicAdd(&st->call_overflow, overflow);
     }
   }
+}
+
+// a path's closest-hit ray, and segment q
+__device__ __forceinline__ RayIn path_ray(const SF<float4>& ro, const SF<float4>& rd, int p) {
+  const float4 o = __ldg(&ro[p]), d = __ldg(&rd[p]);
+  return RayIn{o.x, o.y, o.z, o.w, d.x, d.y, d.z};
+}
+__device__ __forceinline__ RayIn segment_ray(const Segments& sg, int q) {
+  const float4 o = __ldg(&sg.org[sg.path(q)]), d = __ldg(sg.ray(q));
+  return RayIn{ym::add(o.x, ym::mul(d.x, EPS_F)), ym::add(o.y, ym::mul(d.y, EPS_F)), ym::add(o.z, ym::mul(d.z, EPS_F)),
+               d.w, d.x, d.y, d.z};
 }
 
 // Lanes refill when at least this many of a warp's 32 lanes are idle (a round's rays, whose

@@ -9,8 +9,9 @@ namespace yc {
 
 enum : int {
   S_PRIMARY = 0,     // waiting for the closest hit of the camera ray
-  S_NEE_SHADOW = 1,  // waiting for the shadow ray of evaluateDirectLighting
-  S_NEE_MIS = 2,     // waiting for the MIS BRDF ray (any-hit up to the sampled light)
+  S_NEE_SHADOW = 1,  // waiting for the shadow ray of evaluateDirectLighting, to go on from there
+  S_NEE_MIS = 2,     // waiting for the MIS BRDF ray (any-hit up to the sampled light), or only for
+                     // the shadow ray in flight, nothing after it (F_LAST)
   S_EXT = 3,         // waiting for the closest hit of the GI extension ray
   // transient phases
   P_NEE_BEGIN = 8,
@@ -22,14 +23,28 @@ enum : int {
   F_TARGET_INDIRECT = 1,  // NEE result goes to indirect += thr * DL (udpt.cl:527) else direct = DL
   F_NEE_GLOSSY = 2,       // sample_glossy of the NEE (udpt.cl:559)
   F_SPEC = 4,             // the pending extension ray left a specular vertex
-  F_OCCLUDED = 8          // the NEE shadow ray was blocked
+  F_OCCLUDED = 8,         // the NEE shadow ray was blocked
+  F_WAIT = 16,            // a shadow ray is in flight beside the path's next ray (ls: the light sample if it is free)
+  F_OCC_NAN = 32,         //   and if it is occluded the sample is NaN (0 times a weight without a value)
+  F_LAST = 64             //   and it is the path's last ray
 };
+// what a step sends: one closest-hit ray or none (the path then waits for segments), and segments
+enum : int { EMIT_CLOSEST = 1, EMIT_WAIT = 2, EMIT = 3, EMIT_SEG0 = 4, EMIT_SEG1 = 8 };
+// the segments in flight of a path with this misc.z: shadow ray, MIS ray
+__device__ __forceinline__ int segments_of(int state_flags) {
+  const int state = state_flags & 15, flags = state_flags >> 4;
+  return (state == S_NEE_SHADOW || (flags & F_WAIT) ? EMIT_SEG0 : 0) |
+         (state == S_NEE_MIS && !(flags & F_LAST) ? EMIT_SEG1 : 0);
+}
 
 __device__ __forceinline__ int pack_misc(int state, int flags, int j, int k) {
   return state | (flags << 4) | ((j + 1) << 12) | ((k + 1) << 20);
 }
 
 constexpr int LOGIC_TB = 256;
+
+// whether a vertex's shadow ray goes with the path's next ray (TOGETHER of logic_path)
+inline bool rays_together(const PassParams& pp) { return pp.mis != 0 && pp.mis_lobe_fix != 0; }
 
 struct LogicCounts {
   unsigned rays = 0, ext = 0, shadow = 0, mis = 0, trav = 0, samples = 0, prim = 0;
@@ -66,19 +81,54 @@ __device__ __forceinline__ void camera_ray(const PassParams& pp, int px, int py,
 }
 
 // Fields of the path record a step rewrote (stored back when the step emits a ray).
-enum : unsigned {
-  D_THR = 1, D_THR_NEXT = 2, D_DIRECT = 4, D_INDIRECT = 8, D_LS = 16, D_HP = 32, D_NRM = 64, D_WO = 128, D_WI = 256
-};
+enum : unsigned { D_THR = 1, D_DIRECT = 4, D_INDIRECT = 8 };
 
-// One step of path p: runs its state machine from the result of its last ray until it
-// needs the next one. Returns 1 (closest-hit ray written to the path state), 2 (any-hit
-// ray) or 0 (the path finished and its colour went into the accumulator). `mask`: the lanes
-// of the warp that make the call together.
-// The step loads only the record fields its entry state can read before writing them
-// (a camera-ray result reads the ray and the hit; an extension result does not read the
-// last vertex's shading frame, light sample or densities; a shadow or MIS result does not
-// read the ray it traced) and stores only the fields it changed: the record is the same,
-// with fewer bytes moved (pass starts write the misc word and the ray only).
+// The queue entries of a warp's lanes (all 32 call it): paths with a closest-hit ray, paths that
+// only wait for segments, and the segments; where each lane's entries went.
+struct RaysOut {
+  int closest, any;
+};
+__device__ __forceinline__ void append_rays(int emit, int p, int* out_closest, int* out_wait, int* q_any,
+                                            RoundCounters* rc_out, RaysOut& at) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1;
+  const bool closest = (emit & EMIT) == EMIT_CLOSEST, wait = (emit & EMIT) == EMIT_WAIT;
+  const unsigned mc = __ballot_sync(0xffffffffu, closest), mw = __ballot_sync(0xffffffffu, wait);
+  const unsigned m0 = __ballot_sync(0xffffffffu, (emit & EMIT_SEG0) != 0);
+  const unsigned m1 = __ballot_sync(0xffffffffu, (emit & EMIT_SEG1) != 0);
+  int bc = 0, bw = 0, ba = 0;
+  if (lane == 0) {
+    if (mc) bc = atomicAdd(&rc_out->n_closest, __popc(mc));
+    if (mw) bw = atomicAdd(&rc_out->n_wait, __popc(mw));
+    if (m0 | m1) ba = atomicAdd(&rc_out->n_any, __popc(m0) + __popc(m1));
+  }
+  at.closest = __shfl_sync(0xffffffffu, bc, 0) + __popc(mc & below);
+  bw = __shfl_sync(0xffffffffu, bw, 0) + __popc(mw & below);
+  at.any = __shfl_sync(0xffffffffu, ba, 0) + __popc(m0 & below) + __popc(m1 & below);
+  if (closest) out_closest[at.closest] = p;
+  if (wait) out_wait[bw] = p;
+  int a = at.any;
+  if (emit & EMIT_SEG0) q_any[a++] = 2 * p;
+  if (emit & EMIT_SEG1) q_any[a] = 2 * p + 1;
+}
+
+// One step of path p: runs its state machine from the results of its last rays until it needs new
+// ones. Returns what it sends (EMIT_*, the rays are in the path record), or 0 (the path finished
+// and its colour went into the accumulator). `mask`: the lanes of the warp that make the call
+// together.
+// TOGETHER (rays_together): where the lobe is drawn whether the light is visible or not
+// (mis_lobe_fix) no random number depends on the shadow ray's result, so the step goes on as if
+// the ray were free and sends it with the path's next ray: the light sample waits in the record,
+// and the next step takes it or leaves it, with the operations in the reference's order. A bounce
+// is then one round for most paths instead of two or three, and the shading is as much work in
+// fewer launches: four 512x512 passes of the Cornell box 4.77 -> 4.07 ms, a 256x256 frame of it
+// 0.80 -> 0.70 ms, the 1024x1024 glass sphere 5.91 -> 5.60 ms. The MIS ray, which few paths
+// need (most miss the light), stays alone: its share evaluated ahead as well, beside the
+// extension ray, cost the shading kernel another pass of its loop for a few lanes (box 4.38 ms).
+// A batch sends one ray at a time: its slots are always full, so a round less gains nothing.
+// The step loads only the record fields its entry state can read before writing them and stores
+// only the fields a later step reads.
+template <bool TOGETHER>
 __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const PathState& ps, int p, LogicCounts& cnt,
                                           unsigned mask) {
   const DevScene& sc = pp.sc;
@@ -95,31 +145,45 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
   int k = ((misc.z >> 20) & 0xff) - 1;
   int bounce = misc.w;
   const bool enter_cam = phase == S_PRIMARY, enter_ext = phase == S_EXT;
-  const bool enter_nee = phase == S_NEE_SHADOW || phase == S_NEE_MIS;
+  const bool enter_wait = TOGETHER && (flags & F_WAIT), enter_mis = phase == S_NEE_MIS && !(TOGETHER && (flags & F_LAST));
+  const bool enter_nee = phase == S_NEE_SHADOW || enter_mis;
   unsigned dirty = 0;
   const float4 Z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   f4 thr = f4of(enter_cam ? Z4 : ps.thr[p]);
   f4 thr_next = f4of(enter_ext ? ps.thr_next[p] : Z4);
   f4 direct = f4of(enter_cam ? Z4 : ps.direct[p]), indirect = f4of(enter_cam ? Z4 : ps.indirect[p]);
-  f4 ls = f4of(phase == S_NEE_MIS ? ps.ls[p] : Z4);
-  const float4 hp4 = enter_nee ? ps.hp[p] : Z4, n4 = enter_nee ? ps.nrm[p] : Z4;
-  const float4 wo4 = enter_nee ? ps.wo[p] : Z4, wi4 = enter_nee ? ps.wi[p] : Z4;
+  f4 ls = f4of(enter_wait || enter_mis ? ps.ls[p] : Z4);
+  const float4 hp4 = enter_nee || enter_wait ? ps.hp[p] : Z4, n4 = enter_nee ? ps.nrm[p] : Z4;
+  const int occluded = (int)((unsigned)misc.z >> RECORD_BIT);   // bit 0: the shadow ray, bit 1: the MIS ray
+  const float4 wo4 = enter_nee ? ps.wo[p] : Z4;
   Vtx V;
   V.hp = ym::mk(hp4.x, hp4.y, hp4.z, 1.0f);
   V.n = ym::mk(n4.x, n4.y, n4.z, 0.0f);
-  V.mat = __float_as_int(wi4.w);
-  float light_pdf = hp4.w, brdf_prob = n4.w, brdf_pdf = wo4.w;
+  V.mat = __float_as_int(hp4.w);
   f4 wo = ym::mk(wo4.x, wo4.y, wo4.z, -0.0f);
-  f4 w_i = ym::mk(wi4.x, wi4.y, wi4.z, 0.0f);
-  const float4 ro4 = enter_nee ? Z4 : ps.ro[p], rd4 = enter_nee ? Z4 : ps.rd[p];
+  const bool enter_hit = enter_cam || enter_ext;
+  const float4 ro4 = enter_hit || enter_mis ? ps.ro[p] : Z4, hit = enter_hit ? ps.hit[p] : Z4;
+  const float4 rd4 = enter_hit || enter_mis ? ps.rd[p] : enter_nee ? ps.wi[p] : Z4;
+  float light_pdf = n4.w, brdf_prob = ro4.x, brdf_pdf = wo4.w;
+  f4 w_i = ym::mk(rd4.x, rd4.y, rd4.z, 0.0f);   // (of a shadow or MIS ray)
   f4 ro = ym::mk(ro4.x, ro4.y, ro4.z, 1.0f);
   f4 rd = ym::mk(rd4.x, rd4.y, rd4.z, rd4.w);
   float tmax = ro4.w;
-  const float4 hit = ps.hit[p];
   f4 dl = ym::splat(0.0f);   // result of evaluateDirectLighting being delivered
   f4 color = ym::splat(0.0f);
   bool no_surface = false;   // the camera ray met no triangle: its colour is set
 
+  // The light sample of the last vertex, now that its shadow ray is answered.
+  if (enter_wait) {
+    if (occluded & 1) ls = ym::splat(flags & F_OCC_NAN ? __int_as_float(0x7fffffff) : 0.0f);
+    flags &= ~(F_WAIT | F_OCC_NAN);
+    if (!enter_mis) {
+      dl = ls + ld4(sc.mats[V.mat].ke);
+      if (flags & F_TARGET_INDIRECT) { indirect = indirect + thr * dl; dirty |= D_INDIRECT; }
+      else { direct = dl; dirty |= D_DIRECT; }
+      if (!enter_ext) phase = P_FINISH;
+    }
+  }
   // The result of a camera or extension ray: the vertex it met.
   if (enter_cam || enter_ext) {
     const int tri = __float_as_int(hit.w);
@@ -133,7 +197,7 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
         indirect = direct;
         bounce = 0;
         flags = 0;
-        dirty |= D_THR | D_DIRECT | D_INDIRECT | D_HP | D_NRM | D_WO | D_WI;
+        dirty |= D_THR | D_DIRECT | D_INDIRECT;
       } else {
         if (k >= 0) color = (ym::dot(rd, ld4(sc.lights[k].normal)) < 0.0f) ? ym::mk(1.0f, 1.0f, 1.0f, 1.0f)
                                                                            : ym::mk(0.1f, 0.1f, 0.1f, 1.0f);
@@ -145,7 +209,7 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
       if (hit_tri) {
         indirect = indirect + thr * ld4(sc.mats[NV.mat].ke);
         thr = thr_next;
-        dirty |= D_THR | D_INDIRECT | D_HP | D_NRM | D_WO | D_WI;   // new vertex
+        dirty |= D_THR | D_INDIRECT;
         if (bounce > pp.rr_threshold) {
           const float pr = ym::min(luminance(thr), 0.95f);
           const float r = draw(seed);
@@ -185,8 +249,7 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
     } else {
       limit = ym::sub(ym::length(wi_raw), ym::mul(EPS_F, 1.5f));
       w_i = ym::normalize(wi_raw);
-      flags &= ~(F_NEE_GLOSSY | F_OCCLUDED);
-      dirty |= D_WI;
+      flags &= ~(F_NEE_GLOSSY | F_OCCLUDED | (TOGETHER ? F_OCC_NAN : 0));
       dir = w_i;
       cast = S_NEE_SHADOW;
     }
@@ -196,7 +259,8 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
   // is bound by instruction fetch and by its lanes' different phases, so one copy that
   // the lanes of every phase share is worth the loop: a shadow result that goes on to
   // a MIS ray and a path that samples its next bounce run the same instructions). Most
-  // paths leave after one pass; a MIS ray that misses the light takes a second one.
+  // paths leave after one pass; a MIS ray that misses the light takes a second one, and a shadow
+// ray sent with the next ray one or two more.
   // Measured against one copy per phase (a switch over the phases): 2.16 -> 1.69 ms of
   // shading per four 512x512 passes of the Cornell box, whose queue is not sorted, 1.11 ->
   // 0.97 ms per 1024x1024 pass of the glass sphere, whose queue is. The warp barriers keep
@@ -205,8 +269,10 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
   for (;;) {
     __syncwarp(mask);
     if (phase == P_NEE_DELIVER) {
-      if (flags & F_TARGET_INDIRECT) { indirect = indirect + thr * dl; dirty |= D_INDIRECT; }
-      else { direct = dl; dirty |= D_DIRECT; }
+      if (!TOGETHER || !(flags & F_WAIT)) {
+        if (flags & F_TARGET_INDIRECT) { indirect = indirect + thr * dl; dirty |= D_INDIRECT; }
+        else { direct = dl; dirty |= D_DIRECT; }
+      }
       phase = pp.gi_check ? P_GI_SAMPLE : P_FINISH;
     }
     if (phase == P_GI_SAMPLE && bounce >= pp.max_depth) phase = P_FINISH;
@@ -218,13 +284,12 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
       const bool spec = gi && m.is_specular != 0;
       if (shadow) {
         ls = ym::splat(0.0f);   // the light sample of this shadow ray (zero while occluded)
-        dirty |= D_LS | D_NRM | D_WO;   // ls, brdf_prob, brdf_pdf
-        if (hit.x != 0.0f) flags |= F_OCCLUDED;
+        if (enter_nee && (occluded & 1)) flags |= F_OCCLUDED;   // (a ray still in flight counts as free)
         brdf_prob = 0.0f;
       }
-      const bool visible = shadow ? !(flags & F_OCCLUDED) : hit.x == 0.0f;   // of a shadow or MIS result
+      const bool visible = shadow ? !(flags & F_OCCLUDED) : !(occluded & 2);   // of a shadow or MIS result
       // lobe (sampleGlossyPdf): for the light sample and the MIS ray, or for the next bounce
-      const bool draws = shadow ? visible || (pp.mis && pp.mis_lobe_fix) : gi && !spec;
+      const bool draws = shadow ? TOGETHER || visible || (pp.mis && pp.mis_lobe_fix) : gi && !spec;
       bool glossy = mis_result && (flags & F_NEE_GLOSSY);
       float prob = mis_result ? brdf_prob : 0.0f;
       if (draws) glossy = sample_glossy(m, seed, prob);
@@ -256,7 +321,6 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
           phase = P_FINISH;
         } else {
           thr_next = spec ? thr * ior : ((thr * f) * cosine) / pdf;
-          dirty |= D_THR_NEXT;
           flags = spec ? (flags | F_SPEC) : (flags & ~F_SPEC);
           dir = nd;
           limit = INF;
@@ -271,12 +335,13 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
           if (mis) {
             if (glossy) flags |= F_NEE_GLOSSY; else flags &= ~F_NEE_GLOSSY;
             brdf_pdf = glossy ? phong_pdf(w_i, wo, V, m) : cos_pdf(w_i, V.n);
-            ls = ls * ym::div(ym::mul(mw, mw), ym::add(ym::mul(light_pdf, light_pdf), ym::mul(brdf_pdf, brdf_pdf)));
+            const float weight = ym::div(ym::mul(mw, mw), ym::add(ym::mul(light_pdf, light_pdf), ym::mul(brdf_pdf, brdf_pdf)));
+            ls = ls * weight;
+            if (TOGETHER && !(weight < INF)) flags |= F_OCC_NAN;
             brdf_pdf = pdf;
           }
           if (mis && !(pdf <= 0.0f)) {
             w_i = nd;
-            dirty |= D_WI;
             dir = nd;
             limit = INF;
             cast = S_NEE_MIS;
@@ -297,7 +362,7 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
       }
     }
     __syncwarp(mask);
-    if (cast) {   // traceRay's light loop (udpt.cl:244-276); a ray that only the BVH can settle is emitted
+    if (cast) {   // traceRay's light loop (udpt.cl:244-276); a ray that only the BVH can settle is sent
       ro = V.hp + dir * EPS_F;
       rd = dir;
       float tl = limit;
@@ -305,17 +370,22 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
       light_test(sc, ro, rd, tl, lk);
       cnt.rays++;
       phase = cast;
-      emit = cast == S_EXT ? 1 : 2;
+      tmax = tl;
+      emit = EMIT_WAIT;
       if (cast == S_NEE_SHADOW) {
         cnt.shadow++;
         tmax = limit;
         if (lk >= 0) {   // another light closes the segment: blocked without a BVH walk
           flags |= F_OCCLUDED;
           emit = 0;
+        } else if (TOGETHER) {
+          ps.wi[p] = make_float4(dir.x, dir.y, dir.z, limit);
+          flags |= F_WAIT;
+          emit = 0;
+          cnt.trav++;
         }
       } else if (cast == S_NEE_MIS) {   // only light j can satisfy the test
         cnt.mis++;
-        tmax = tl;
         if (lk != j) {
           dl = ls + ld4(sc.mats[V.mat].ke);
           phase = P_NEE_DELIVER;
@@ -323,11 +393,16 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
         }
       } else {
         cnt.ext++;
-        tmax = tl;
         k = lk;
+        emit = EMIT_CLOSEST;
       }
       if (emit) cnt.trav++;
       cast = 0;
+    }
+    if (TOGETHER && phase == P_FINISH && (flags & F_WAIT)) {   // the path ends, its last shadow ray is in flight
+      phase = S_NEE_MIS;
+      flags |= F_LAST;
+      emit = EMIT_WAIT;
     }
     if (!__any_sync(mask, !emit && phase != P_FINISH)) break;
   }
@@ -351,16 +426,22 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
   if (emit) {
     ps.misc[p] = make_int4((int)seed, pix, pack_misc(phase, flags, j, k), bounce);
     if (dirty & D_THR) ps.thr[p] = make_float4(thr.x, thr.y, thr.z, thr.w);
-    if (dirty & D_THR_NEXT) ps.thr_next[p] = make_float4(thr_next.x, thr_next.y, thr_next.z, thr_next.w);
     if (dirty & D_DIRECT) ps.direct[p] = make_float4(direct.x, direct.y, direct.z, direct.w);
     if (dirty & D_INDIRECT) ps.indirect[p] = make_float4(indirect.x, indirect.y, indirect.z, indirect.w);
-    if (dirty & D_LS) ps.ls[p] = make_float4(ls.x, ls.y, ls.z, ls.w);
-    if (dirty & D_HP) ps.hp[p] = make_float4(V.hp.x, V.hp.y, V.hp.z, light_pdf);
-    if (dirty & D_NRM) ps.nrm[p] = make_float4(V.n.x, V.n.y, V.n.z, brdf_prob);
-    if (dirty & D_WO) ps.wo[p] = make_float4(wo.x, wo.y, wo.z, brdf_pdf);
-    if (dirty & D_WI) ps.wi[p] = make_float4(w_i.x, w_i.y, w_i.z, __int_as_float(V.mat));
-    ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
-    ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
+    const bool last = TOGETHER && (flags & F_LAST), wait = TOGETHER && (flags & F_WAIT);
+    if (emit == EMIT_CLOSEST) {
+      ps.thr_next[p] = make_float4(thr_next.x, thr_next.y, thr_next.z, thr_next.w);
+      ps.ro[p] = make_float4(ro.x, ro.y, ro.z, tmax);
+      ps.rd[p] = make_float4(rd.x, rd.y, rd.z, rd.w);
+    } else if (!last) {   // evaluateDirectLighting goes on at this vertex
+      ps.nrm[p] = make_float4(V.n.x, V.n.y, V.n.z, light_pdf);
+      ps.wo[p] = make_float4(wo.x, wo.y, wo.z, brdf_pdf);
+      (phase == S_NEE_MIS ? ps.rd[p] : ps.wi[p]) = make_float4(rd.x, rd.y, rd.z, tmax);
+      if (phase == S_NEE_MIS) ps.ro[p].x = brdf_prob;
+    }
+    if (phase == S_NEE_MIS || wait) ps.ls[p] = make_float4(ls.x, ls.y, ls.z, ls.w);
+    if (emit == EMIT_WAIT || wait) ps.hp[p] = make_float4(V.hp.x, V.hp.y, V.hp.z, __int_as_float(V.mat));
+    emit |= segments_of(phase | (flags << 4));
   }
   return emit;
 }
