@@ -437,9 +437,7 @@ yc::PassParams pass_params(const yc_ctx* c, const Scene* sc, const Accum* ac, ui
   if (c->stack_limit > 0) pp.sc.depth = std::min(pp.sc.depth, c->stack_limit - 2);
   pp.cam = c->cam;
   pp.accum = ac->buf.p;
-  pp.width = ac->w;
-  pp.height = ac->h;
-  pp.aspect = yc::frame_aspect(ac->w, ac->h);
+  yc::frame_size(pp, ac->w, ac->h);
   pp.tile_w = (int)std::ceil((float)ac->w / cfg->block_x);
   pp.tile_h = (int)std::ceil((float)ac->h / cfg->block_y);
   pp.off_x = (int)(std::ceil((float)ac->w / cfg->block_x) * (float)(cfg->block % cfg->block_x));
@@ -1751,9 +1749,7 @@ int yc_batch_add_job(yc_batch* b, int scene_id, int accum_id, const yc_cam* cam,
   j.pp.sc = b->indexed && sc->dev.wide == 0 ? walk_scene(*sc) : sc->dev;
   j.pp.cam = *cam;
   j.pp.accum = ac->buf.p;
-  j.pp.width = ac->w;
-  j.pp.height = ac->h;
-  j.pp.aspect = yc::frame_aspect(ac->w, ac->h);
+  yc::frame_size(j.pp, ac->w, ac->h);
   j.pp.tile_w = ac->w;
   j.pp.tile_h = ac->h;
   j.pp.gi_check = 1;

@@ -62,49 +62,25 @@ struct VertexRef {
 };
 
 // ---- raygen: pixel prologue, eye ray, light vertex 0 and the first light ray ----
-__global__ void __launch_bounds__(256) k_raygen_bdpt(PassParams pp, PathState ps, BdptBuffers bb, int* q_closest,
-                                                     RoundCounters* rc, DevStats* st) {
+__global__ void __launch_bounds__(256) k_raygen_bdpt(PassParams pp, int n, int row, PathState ps,
+                                                     BdptBuffers bb, int* q_closest, RoundCounters* rc, DevStats* st) {
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = pp.tile_w * pp.tile_h;
-  int px = 0, py = 0;
-  bool active = false;
-  if (gid < n) {
-    px = gid % pp.tile_w + pp.off_x;
-    py = gid / pp.tile_w + pp.off_y;
-    active = px < pp.width && py < pp.height;
-  }
-  const int W = pp.width, H = pp.height;
-  const int pix = py * W + px;
+  const bool active = gid < n;
+  const int px = gid % row + pp.off_x, py = gid / row + pp.off_y;
+  const int pix = py * pp.width + px;
   const int slot = pix;
   bool eye_first = false;
   if (active) {
     const DevScene& sc = pp.sc;
-    uint32_t seed = (uint32_t)((py + 1) * W + (px + 1));
-    seed = pp.rand_seed * seed;
-    seed = ym::wang_hash(seed);
-    if (seed == 0) seed = ym::wang_hash(seed);
-    const float r1 = draw(seed);
-    const float r2 = draw(seed);
-    const float fx = ym::add((float)px, r1), fy = ym::add((float)py, r2);
-    const float aspect = pp.aspect;
-    f4 dir;
-    dir.x = (float)((double)aspect * ((2.0 * (double)fx / (double)W) - 1));
-    dir.y = (float)((2.0 * (double)fy / (double)H) - 1);
-    dir.z = -pp.cam.view_plane_dist;
-    dir.w = 0.0f;
-    f4 d;
-    d.x = ym::dot(ld4(pp.cam.r1), dir);
-    d.y = ym::dot(ld4(pp.cam.r2), dir);
-    d.z = ym::dot(ld4(pp.cam.r3), dir);
-    d.w = ym::dot(ld4(pp.cam.r4), dir);
-    d = ym::normalize(d);
+    uint32_t seed;
+    const f4 d = camera_direction(pp, px, py, pp.rand_seed, seed);
     VertexRef ev{bb.ev + (size_t)slot * bb.bounces * 4};
     VertexRef lv{bb.lv + (size_t)slot * bb.bounces * 4};
     ev.at(0, 2) = make_float4(d.x, d.y, d.z, d.w);   // the camera ray, traced after the light subpath
     // light vertex 0 on light 0 (createLightPath, bdpt.cl:435-456)
     const yc_quad_light& L = sc.lights[0];
     seed = ym::xor_shift(seed);
-    const float lr1 = (float)((double)seed / 4294967295.0);   // seed / (double)UINT_MAX
+    const float lr1 = (float)divided((double)seed, 4294967295.0, 1.0 / 4294967295.0);   // seed / (double)UINT_MAX
     const float lr2 = draw(seed);
     const f4 A = ld4(L.edge_l) * lr2;
     const f4 B = ld4(L.edge_w) * lr1;
@@ -141,25 +117,24 @@ __global__ void __launch_bounds__(256) k_raygen_bdpt(PassParams pp, PathState ps
     ps.rd[slot] = make_float4(rdir.x, rdir.y, rdir.z, rdir.w);
     ps.direct[slot] = make_float4(1.0f, 0.0f, pdf, 0.0f);   // weight, ks, pending pdf, pending lobe prob
   }
-  const unsigned m = __ballot_sync(0xffffffffu, active);
-  const int lane = threadIdx.x & 31;
-  int base = 0;
-  if (lane == 0 && m) base = atomicAdd(&rc->n_closest, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (active) q_closest[base + __popc(m & ((1u << lane) - 1))] = slot;
-  const unsigned m_eye = __ballot_sync(0xffffffffu, active && eye_first);
-  if (lane == 0 && m) {
-    atomicAdd(&st->rays, (unsigned long long)__popc(m));
-    atomicAdd(&st->traversed, (unsigned long long)__popc(m));
-    if (m_eye) atomicAdd(&st->primary, (unsigned long long)__popc(m_eye));
-    if (m & ~m_eye) atomicAdd(&st->extension, (unsigned long long)__popc(m & ~m_eye));
+  if (active) q_closest[gid] = slot;
+  const unsigned eye = __ballot_sync(0xffffffffu, eye_first);   // (rare; counted with the light rays below)
+  if (eye && (threadIdx.x & 31) == 0) {
+    atomicAdd(&st->primary, (unsigned long long)__popc(eye));
+    atomicAdd(&st->extension, 0ull - (unsigned long long)__popc(eye));
+  }
+  if (gid == 0) {
+    rc->n_closest = n;
+    atomicAdd(&st->rays, (unsigned long long)n);
+    atomicAdd(&st->traversed, (unsigned long long)n);
+    atomicAdd(&st->extension, (unsigned long long)n);
   }
 }
 
 void launch_raygen_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, int* q_closest,
                         RoundCounters* rc, DevStats* st, cudaStream_t s) {
-  const int n = pp.tile_w * pp.tile_h;
-  k_raygen_bdpt<<<(n + 255) / 256, 256, 0, s>>>(pp, ps, bb, q_closest, rc, st);
+  const int n = tile_pixels(pp);
+  if (n > 0) k_raygen_bdpt<<<(n + 255) / 256, 256, 0, s>>>(pp, n, tile_row(pp), ps, bb, q_closest, rc, st);
 }
 
 // ---- logic: advance each path to its next ray ----

@@ -47,39 +47,15 @@ int scratch_address(unsigned char** out) {
 // pathtracer prologue + createRay (kernels/legacy/udpt.cl:158-189, 213-238) for one
 // tile; the path slot is the pixel's index inside the tile, so the state fits the
 // tile-sized scratch.
-__global__ void __launch_bounds__(256) k_raygen_tile(PassParams pp, PathState ps, int* q_closest, RoundCounters* rc,
-                                                     DevStats* st) {
+__global__ void __launch_bounds__(256) k_raygen_tile(PassParams pp, int n, int row, PathState ps, int* q_closest,
+                                                     RoundCounters* rc, DevStats* st) {
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = pp.tile_w * pp.tile_h;
-  int px = 0, py = 0;
-  bool active = false;
-  if (gid < n) {
-    px = gid % pp.tile_w + pp.off_x;
-    py = gid / pp.tile_w + pp.off_y;
-    active = px < pp.width && py < pp.height;
-  }
-  const int W = pp.width, H = pp.height;
-  const int pix = py * W + px;
+  const bool active = gid < n;
+  const int px = gid % row + pp.off_x, py = gid / row + pp.off_y;
+  const int pix = py * pp.width + px;
   if (active) {
-    uint32_t seed = (uint32_t)((py + 1) * W + (px + 1));
-    seed = pp.rand_seed * seed;
-    seed = ym::wang_hash(seed);
-    if (seed == 0) seed = ym::wang_hash(seed);
-    const float r1 = draw(seed);
-    const float r2 = draw(seed);
-    const float fx = ym::add((float)px, r1), fy = ym::add((float)py, r2);
-    const float aspect = pp.aspect;
-    f4 dir;
-    dir.x = (float)((double)aspect * ((2.0 * (double)fx / (double)W) - 1));
-    dir.y = (float)((2.0 * (double)fy / (double)H) - 1);
-    dir.z = -pp.cam.view_plane_dist;
-    dir.w = 0.0f;
-    f4 d;
-    d.x = ym::dot(ld4(pp.cam.r1), dir);
-    d.y = ym::dot(ld4(pp.cam.r2), dir);
-    d.z = ym::dot(ld4(pp.cam.r3), dir);
-    d.w = ym::dot(ld4(pp.cam.r4), dir);
-    d = ym::normalize(d);
+    uint32_t seed;
+    const f4 d = camera_direction(pp, px, py, pp.rand_seed, seed);
     const f4 o = ym::mk(pp.cam.r1.w, pp.cam.r2.w, pp.cam.r3.w, pp.cam.r4.w);
     float len = __int_as_float(0x7f800000);
     int k = -1;
@@ -88,16 +64,12 @@ __global__ void __launch_bounds__(256) k_raygen_tile(PassParams pp, PathState ps
     ps.ro[gid] = make_float4(o.x, o.y, o.z, len);
     ps.rd[gid] = make_float4(d.x, d.y, d.z, d.w);
   }
-  const unsigned m = __ballot_sync(0xffffffffu, active);
-  const int lane = threadIdx.x & 31;
-  int base = 0;
-  if (lane == 0 && m) base = atomicAdd(&rc->n_closest, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (active) q_closest[base + __popc(m & ((1u << lane) - 1))] = gid;
-  if (lane == 0 && m) {
-    atomicAdd(&st->primary, (unsigned long long)__popc(m));
-    atomicAdd(&st->rays, (unsigned long long)__popc(m));
-    atomicAdd(&st->traversed, (unsigned long long)__popc(m));
+  if (active) q_closest[gid] = gid;
+  if (gid == 0) {
+    rc->n_closest = n;
+    atomicAdd(&st->primary, (unsigned long long)n);
+    atomicAdd(&st->rays, (unsigned long long)n);
+    atomicAdd(&st->traversed, (unsigned long long)n);
   }
 }
 
@@ -134,7 +106,8 @@ int noalloc_render(const NoallocPass& a, std::string& err) {
     err = "clearing the round counters failed";
     return YC_E_LAUNCH;
   }
-  k_raygen_tile<<<(n_paths + 255) / 256, 256, 0, s>>>(a.pp, ps, qs[0], rc, a.stats);
+  if (const int n = tile_pixels(a.pp))
+    k_raygen_tile<<<(n + 255) / 256, 256, 0, s>>>(a.pp, n, tile_row(a.pp), ps, qs[0], rc, a.stats);
   if (launch_failed("ray generation")) return YC_E_LAUNCH;
   const int grid_c = trace_grid_blocks(false, a.pp.sc.depth, a.pp.sc.wide != 0);
   const int grid_a = trace_grid_blocks(true, a.pp.sc.depth, a.pp.sc.wide != 0);

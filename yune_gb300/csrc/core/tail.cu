@@ -162,14 +162,14 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
     if (s_cnt[12]) atomicAdd(&st->call_overflow, s_cnt[12]);
     // the last block to finish empties the queues (every block has read the counts)
     __threadfence();
-    s_last = atomicAdd(&rc_in->pad[0], 1) == (int)gridDim.x - 1;
+    s_last = atomicAdd(&rc_in->tail_exits, 1) == (int)gridDim.x - 1;
   }
   __syncthreads();
   if (threadIdx.x == 0 && s_last) {
     rc_in->n_closest = 0;
     rc_in->n_any = 0;
     rc_in->n_wait = 0;
-    rc_in->pad[0] = 0;
+    rc_in->tail_exits = 0;
   }
 }
 

@@ -55,25 +55,7 @@ struct LogicCounts {
 // along it (the light loop of traceRay runs before the BVH, udpt.cl:244-276)
 __device__ __forceinline__ void camera_ray(const PassParams& pp, int px, int py, uint32_t rand, uint32_t& seed, f4& o, f4& d,
                            float& len, int& k) {
-  const int W = pp.width, H = pp.height;
-  seed = (uint32_t)((py + 1) * W + (px + 1));
-  seed = rand * seed;
-  seed = ym::wang_hash(seed);
-  if (seed == 0) seed = ym::wang_hash(seed);
-  const float r1 = draw(seed);
-  const float r2 = draw(seed);
-  const float fx = ym::add((float)px, r1), fy = ym::add((float)py, r2);
-  const float aspect = pp.aspect;
-  f4 dir;
-  dir.x = (float)((double)aspect * ((2.0 * (double)fx / (double)W) - 1));
-  dir.y = (float)((2.0 * (double)fy / (double)H) - 1);
-  dir.z = -pp.cam.view_plane_dist;
-  dir.w = 0.0f;
-  d.x = ym::dot(ld4(pp.cam.r1), dir);
-  d.y = ym::dot(ld4(pp.cam.r2), dir);
-  d.z = ym::dot(ld4(pp.cam.r3), dir);
-  d.w = ym::dot(ld4(pp.cam.r4), dir);
-  d = ym::normalize(d);
+  d = camera_direction(pp, px, py, rand, seed);
   o = ym::mk(pp.cam.r1.w, pp.cam.r2.w, pp.cam.r3.w, pp.cam.r4.w);
   len = __int_as_float(0x7f800000);
   k = -1;
