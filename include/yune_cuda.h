@@ -206,7 +206,9 @@ int yc_accum_device_ptr(yc_ctx* ctx, int accum_id, void** dptr);
  *      into the accumulator (udpt.cl:196-210). Asynchronous on the context stream. ---- */
 int yc_render_pass(yc_ctx* ctx, int scene_id, int accum_id, uint32_t rand_seed, int reset, int gi_check,
                    const yc_pass_cfg* cfg);
-/* n_pass passes back to back (pass k uses rand_seeds[k]; reset applies to the first). */
+/* n_pass passes (pass k uses rand_seeds[k]; reset applies to the first). Every pixel adds its
+ * passes in order; unidirectional passes may share one wavefront, a pixel a pass ahead of another,
+ * so a call that fails can leave pixels at different passes. */
 int yc_render_passes(yc_ctx* ctx, int scene_id, int accum_id, const uint32_t* rand_seeds_host, int n_pass,
                      int reset_first, int gi_check, const yc_pass_cfg* cfg);
 
@@ -463,7 +465,8 @@ enum {
   YC_OPT_SHADE_SORT_MIN = 6,
   /* Rounds (trace + shade) one pass may take before yc_render_pass(es) and
    * yc_render_pass_noalloc give up with YC_E_TIMEOUT. Default 1,000,000 (the reference's
-   * GI loop bound is 100000 bounces, udpt.cl:463, at most three rays each). */
+   * GI loop bound is 100000 bounces, udpt.cl:463, at most three rays each). Passes that
+   * yc_render_passes runs together may take that many each, counted together. */
   YC_OPT_MAX_ROUNDS = 7,
   /* Traversal stack entries a walk may use in yc_render_pass(es) and
    * yc_render_pass_noalloc; 0 (default) = as many as the scene's hierarchy needs (its

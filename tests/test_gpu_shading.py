@@ -117,3 +117,25 @@ def test_rays_sent_together(r, tris, max_depth, lobe_fix, mixed, sort, tail):
     for o, _, v in opts:
         N.check(r.L.yc_set_option(r.h, o, v), "yc_set_option")
     r.release(sid)
+
+
+@pytest.mark.parametrize("tail", [0, -1])
+@pytest.mark.parametrize("lobe_fix, reset", [(0, 1), (1, 1), (1, 0)])
+@pytest.mark.parametrize("tris, passes", [(0, 3), (6000, 5)])
+def test_passes_of_one_call_equal_a_call_each(r, tris, passes, lobe_fix, reset, tail):
+    s = workloads.mixed_scene(tris, 13, W, H, 1, scenes.default_cfg()) if tris else scenes.c0(W, H)
+    s.cfg = dict(s.cfg, mis_lobe_fix=lobe_fix)
+    sid, seeds = r.upload(s), scenes.pass_seeds(5, passes)
+    r.set_camera(s.cam)
+    N.check(r.L.yc_set_option(r.h, 2, tail), "yc_set_option")
+    got = []
+    for step in (passes, 1):
+        aid = r.alloc_accum(W, H)
+        r.render_passes(sid, aid, seeds[:1], reset_first=1, gi_check=1, cfg=s.cfg)   # something to go on from
+        for k in range(0, passes, step):
+            r.render_passes(sid, aid, seeds[k:k + step], reset_first=reset if k == 0 else 0, gi_check=1, cfg=s.cfg)
+        got.append(r.read_accum(aid))
+        r.free_accum(aid)
+    N.check(r.L.yc_set_option(r.h, 2, -1), "yc_set_option")
+    assert np.array_equal(got[0].view(np.int32), got[1].view(np.int32))
+    r.release(sid)

@@ -38,14 +38,7 @@ __device__ __forceinline__ int job_of_task(const BatchJob* jobs, int n_jobs, uns
 __device__ __forceinline__ void start_pass(const BatchJob& J, int job, int pix, int pass, int p, const PathState& ps,
                                            SF<int4> job_pass) {
   const int W = J.pp.width;
-  uint32_t seed;
-  f4 o, d;
-  float len;
-  int k;
-  camera_ray(J.pp, pix % W, pix / W, J.seeds[pass], seed, o, d, len, k);
-  ps.misc[p] = make_int4((int)seed, pix, pack_misc(S_PRIMARY, 0, -1, k), 0);
-  ps.ro[p] = make_float4(o.x, o.y, o.z, len);
-  ps.rd[p] = make_float4(d.x, d.y, d.z, d.w);
+  start_udpt(J.pp, ps, p, pix % W, pix / W, J.seeds[pass]);
   job_pass[p] = make_int4(job, pass, 0, 0);
 }
 

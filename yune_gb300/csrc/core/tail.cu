@@ -38,15 +38,15 @@ constexpr int TAIL_MAX_RAYS = 1 << 22;
 constexpr int HELP_AT = 8;
 
 // three blocks per SM: up to 170 registers a thread, which the kernel needs without spills
-template <bool WIDE, bool TOGETHER>
+template <bool WIDE, bool TOGETHER, bool MULTI>
 __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps, const int* __restrict__ in_closest,
                                                   const int* __restrict__ in_wait, RoundCounters* rc_in,
                                                   int threshold, int stack_cap, DevStats* st, int n_smem, int* spill) {
-  __shared__ unsigned long long s_cnt[13];
+  __shared__ unsigned long long s_cnt[14];
   __shared__ bool s_last;
   const int nc = rc_in->n_closest, n = nc + rc_in->n_wait;
   if (n == 0 || n > threshold) return;   // uniform over the grid
-  if (threadIdx.x < 13) s_cnt[threadIdx.x] = 0;
+  if (threadIdx.x < 14) s_cnt[threadIdx.x] = 0;
   __syncthreads();
   const WalkStack stack = thread_stack(stack_cap, n_smem, spill);
   const int lane = threadIdx.x & 31;
@@ -121,9 +121,17 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
     if (p >= 0) {
       if (occluded[lane]) ps.misc[p].z |= occluded[lane] << RECORD_BIT;
       occluded[lane] = 0;
-      todo = logic_path<TOGETHER>(pp, pp.reset, ps, p, lc, have) & ~EMIT_WAIT;
+      todo = logic_path<TOGETHER>(pp, MULTI ? pass_reset(pp, ps, p) : pp.reset, ps, p, lc, have) & ~EMIT_WAIT;
       rays += __popc(todo);
       if (todo && rays >= TAIL_MAX_RAYS) { ++overflow; todo = 0; }
+      else if (MULTI && !todo && has_next_pass(pp, ps, p)) {
+        const int pass = ps.job[p].w + 1;
+        ps.job[p].w = pass;
+        start_udpt(pp, ps, p, p % pp.width, p / pp.width, pp.seeds[pass]);
+        lc.rays++; lc.trav++; lc.prim++;
+        todo = EMIT_CLOSEST;
+        rays = 0;
+      }
       if (!todo) p = -1;
     }
     if (more) {
@@ -152,12 +160,13 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
   for (int q = 0; q < 6; ++q)
     if (v[q]) atomicAdd(&s_cnt[q], v[q]);
   if (overflow) atomicAdd(&s_cnt[12], (unsigned long long)overflow);
+  if (lc.prim) atomicAdd(&s_cnt[13], (unsigned long long)lc.prim);
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long* dst[13] = {&st->rays, &st->extension, &st->shadow, &st->mis, &st->traversed, &st->samples,
+    unsigned long long* dst[14] = {&st->rays, &st->extension, &st->shadow, &st->mis, &st->traversed, &st->samples,
                                    &st->ext_rays, &st->ext_boxes, &st->ext_tris, &st->any_rays, &st->any_boxes,
-                                   &st->any_tris, &st->stack_overflow};
-    for (int q = 0; q < 13; ++q)
+                                   &st->any_tris, &st->stack_overflow, &st->primary};
+    for (int q = 0; q < 14; ++q)
       if (s_cnt[q]) atomicAdd(dst[q], s_cnt[q]);
     if (s_cnt[12]) atomicAdd(&st->call_overflow, s_cnt[12]);
     // the last block to finish empties the queues (every block has read the counts)
@@ -187,14 +196,19 @@ static int tail_grid_of(K kernel, size_t smem) {
 }
 
 using TailKernel = void (*)(PassParams, PathState, const int*, const int*, RoundCounters*, int, int, DevStats*, int, int*);
-static TailKernel tail_kernel(const DevScene& sc, bool together) {
-  if (together) return sc.wide ? k_tail<true, true> : k_tail<false, true>;
-  return sc.wide ? k_tail<true, false> : k_tail<false, false>;
+template <bool WIDE>
+static TailKernel tail_kernel_of(bool together, bool multi) {
+  if (together) return multi ? k_tail<WIDE, true, true> : k_tail<WIDE, true, false>;
+  return multi ? k_tail<WIDE, false, true> : k_tail<WIDE, false, false>;
+}
+static TailKernel tail_kernel(const PassParams& pp) {
+  const bool together = rays_together(pp), multi = pp.n_pass > 1;
+  return pp.sc.wide ? tail_kernel_of<true>(together, multi) : tail_kernel_of<false>(together, multi);
 }
 
 int tail_capacity(const PassParams& pp, int n_smem, int* grid_out) {
   const size_t smem = tail_smem(tail_entries(pp.sc.depth, n_smem));
-  const int grid = tail_grid_of(tail_kernel(pp.sc, rays_together(pp)), smem);
+  const int grid = tail_grid_of(tail_kernel(pp), smem);
   if (grid_out) *grid_out = grid;
   return grid > 0 ? grid * TAIL_TB : 0;
 }
@@ -204,7 +218,7 @@ int launch_tail(const PassParams& pp, const PathState& ps, const int* in_closest
   const int cap = pp.sc.depth + 2;
   n_smem = tail_entries(pp.sc.depth, spill ? n_smem : 0);
   const size_t smem = tail_smem(n_smem);
-  const TailKernel kernel = tail_kernel(pp.sc, rays_together(pp));
+  const TailKernel kernel = tail_kernel(pp);
   kernel<<<grid, TAIL_TB, smem, s>>>(pp, ps, in_closest, in_wait, rc_in, threshold, cap, st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }

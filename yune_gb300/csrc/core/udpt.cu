@@ -20,28 +20,42 @@
 #include "yc_udpt.cuh"
 
 namespace yc {
-// The n pixels of the tile in the frame, `row` a row of it, one thread each. Their number is known,
-// so every thread knows its place in the queue: with an append a warp the kernel was bound by its
-// 260,000 atomics to two cache lines (1920x1080: 0.216 ms, now 0.111).
+// The first pass: the n pixels of the tile in the frame, `row` a row of it, one thread each. Their
+// number is known, so every thread knows its place in the queue: with an append a warp the kernel
+// was bound by its 260,000 atomics to two cache lines (1920x1080: 0.216 ms, now 0.111).
 __global__ void __launch_bounds__(256) k_raygen(PassParams pp, int n, int row, PathState ps, int* q_closest,
                                                 RoundCounters* rc, DevStats* st) {
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = gid < n;
-  const int px = gid % row + pp.off_x, py = gid / row + pp.off_y;
-  const int pix = py * pp.width + px;
-  if (active) {
-    uint32_t seed;
-    f4 o, d;
-    float len;
-    int k;
-    camera_ray(pp, px, py, pp.rand_seed, seed, o, d, len, k);
-    ps.misc[pix] = make_int4((int)seed, pix, pack_misc(S_PRIMARY, 0, -1, k), 0);
-    ps.ro[pix] = make_float4(o.x, o.y, o.z, len);
-    ps.rd[pix] = make_float4(d.x, d.y, d.z, d.w);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const int px = i % row + pp.off_x, py = i / row + pp.off_y, pix = py * pp.width + px;
+    start_udpt(pp, ps, pix, px, py, pp.rand_seed);
+    if (pp.n_pass > 1) ps.job[pix].w = 0;
+    q_closest[i] = pix;
   }
-  if (active) q_closest[gid] = pix;
-  if (gid == 0) {
+  if (i == 0) {
     rc->n_closest = n;
+    atomicAdd(&st->primary, (unsigned long long)n);
+    atomicAdd(&st->rays, (unsigned long long)n);
+    atomicAdd(&st->traversed, (unsigned long long)n);
+  }
+}
+
+// the next pass of the paths in pp.q_restart
+__global__ void __launch_bounds__(256) k_raygen_next(PassParams pp, PathState ps, int* q_closest, RoundCounters* rc,
+                                                     DevStats* st) {
+  const int n = rc->n_restart, lane = threadIdx.x & 31;
+  for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x) {
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&rc->n_closest, min(32, n - base));
+    at = __shfl_sync(0xffffffffu, at, 0) + lane;
+    if (base + lane < n) {
+      const int p = pp.q_restart[base + lane], pass = ps.job[p].w + 1;
+      ps.job[p].w = pass;
+      start_udpt(pp, ps, p, p % pp.width, p / pp.width, pp.seeds[pass]);
+      q_closest[at] = p;
+    }
+  }
+  if (n > 0 && blockIdx.x == 0 && threadIdx.x == 0) {
     atomicAdd(&st->primary, (unsigned long long)n);
     atomicAdd(&st->rays, (unsigned long long)n);
     atomicAdd(&st->traversed, (unsigned long long)n);
@@ -53,10 +67,12 @@ void launch_raygen(const PassParams& pp, const PathState& ps, int* q_closest, Ro
   const int n = tile_pixels(pp);
   if (n > 0) k_raygen<<<(n + 255) / 256, 256, 0, s>>>(pp, n, tile_row(pp), ps, q_closest, rc, st);
 }
+void launch_raygen_next(const PassParams& pp, const PathState& ps, int* q_closest, RoundCounters* rc, DevStats* st,
+                        int grid, cudaStream_t s) {
+  k_raygen_next<<<grid, 256, 0, s>>>(pp, ps, q_closest, rc, st);
+}
 
-// ---- logic: one step of every path in the input queues ----
-
-template <bool TOGETHER>
+template <bool TOGETHER, bool MULTI>
 __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps, const int* __restrict__ in_closest,
                                                     const int* __restrict__ in_wait, const RoundCounters* rc_in,
                                                     int* out_closest, int* out_wait, int* q_any,
@@ -80,10 +96,18 @@ __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps,
     const unsigned mask = __ballot_sync(0xffffffffu, e < n);
     if (e < n) {
       p = use_sorted ? sorted[e] : (e < nc ? in_closest[e] : in_wait[e - nc]);
-      emit = logic_path<TOGETHER>(pp, pp.reset, ps, p, lc, mask);
+      emit = logic_path<TOGETHER>(pp, MULTI ? pass_reset(pp, ps, p) : pp.reset, ps, p, lc, mask);
     }
     RaysOut at;
     append_rays(emit, p, out_closest, out_wait, q_any, rc_out, at);
+    if (MULTI) {   // paths that ended a pass and have another
+      const bool again = e < n && !emit && has_next_pass(pp, ps, p);
+      const unsigned m = __ballot_sync(0xffffffffu, again);
+      int first = 0;
+      if (lane == 0 && m) first = atomicAdd(&rc_out->n_restart, __popc(m));
+      first = __shfl_sync(0xffffffffu, first, 0);
+      if (again) pp.q_restart[first + __popc(m & ((1u << lane) - 1))] = p;
+    }
     // counters
     unsigned v[6] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples};
 #pragma unroll
@@ -108,7 +132,9 @@ __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps,
 void launch_logic(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_wait,
                   const RoundCounters* rc_in, int* out_closest, int* out_wait, int* q_any, RoundCounters* rc_out,
                   DevStats* st, int grid, cudaStream_t s, const int* sorted, const SortCtl* sctl) {
-  const auto kernel = rays_together(pp) ? k_logic<true> : k_logic<false>;
+  const bool multi = pp.n_pass > 1;
+  const auto kernel = rays_together(pp) ? (multi ? k_logic<true, true> : k_logic<true, false>)
+                                        : (multi ? k_logic<false, true> : k_logic<false, false>);
   kernel<<<grid, LOGIC_TB, 0, s>>>(pp, ps, in_closest, in_wait, rc_in, out_closest, out_wait, q_any, rc_out, st, sorted,
                                     sctl);
 }

@@ -46,7 +46,8 @@ struct PathState {
   SF<float4> ro;         // emitted closest-hit ray: origin xyz, length; or x brdf_prob of the MIS ray
   SF<float4> rd;         // emitted closest-hit ray: direction xyz; or the MIS ray: direction xyz, length
   SF<float4> hit;        // its result: (t, u, v, tri)
-  SF<int4> job;          // batch engine: (job, pass) of the slot's pixel task
+  SF<int4> job;          // batch engine: x, y = (job, pass) of the slot's pixel task; a call of several
+                         // passes: w = the path's pass
 };
 
 // the path state of the records starting at rec (PS_STRIDE float4 per slot)
@@ -87,6 +88,8 @@ struct RoundCounters {
   int work_logic;
   int tail_exits;     // blocks of the tail kernel that have left
   int pad5_[30];
+  int n_restart;      // paths that ended a pass and have another
+  int pad6_[31];
 };
 
 // The segments (any-hit rays) of a path: several may be in flight in one round, beside a
@@ -200,10 +203,14 @@ struct PassParams {
   double w, h, inv_w, inv_h;   // the frame's size and its reciprocals (frame_size)
   int tile_w, tile_h;      // work-item grid of one block launch
   int off_x, off_y;        // pixel offset of the block (udpt.cl:166-167)
-  uint32_t rand_seed;
-  int reset;
+  uint32_t rand_seed;      // of the first pass
+  int reset;               // whether it starts the accumulator anew
   int gi_check;
   int mis, rr_threshold, max_depth, brdf_model, mis_lobe_fix;
+  // several passes in one wavefront (n_pass > 1): their seeds, and the queue of paths to start again
+  int n_pass;
+  const uint32_t* seeds;
+  int* q_restart;
 };
 
 // the pixels of the launch's tile that lie in the frame: a row of them, and their number
@@ -255,6 +262,9 @@ void launch_exclusive_scan(const int* in, int* out, int* tile_sum, int n, cudaSt
 // launchers (udpt.cu / trace.cu)
 void launch_raygen(const PassParams& pp, const PathState& ps, int* q_closest, RoundCounters* rc, DevStats* st,
                    cudaStream_t s);
+// appends the next passes of the paths in pp.q_restart
+void launch_raygen_next(const PassParams& pp, const PathState& ps, int* q_closest, RoundCounters* rc, DevStats* st,
+                        int grid, cudaStream_t s);
 // sorted/sctl: the round's shade queue (the paths of the closest-hit and the waiting queue) sorted
 // by phase and material class, used when sctl->use is set (null: the queues in order)
 void launch_logic(const PassParams& pp, const PathState& ps, const int* in_closest, const int* in_wait,
