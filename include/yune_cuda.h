@@ -438,10 +438,10 @@ enum {
    * in its parents' bounds and falls back to spatial-median splits below a node area of
    * about 1). */
   YC_OPT_TREE = 1,
-  /* End of a unidirectional pass: once at most this many paths are left, one kernel
-   * finishes them a thread per path (trace and shading in turn) instead of round by
-   * round; the result is the same bits. -1 (default) = as many paths as one resident
-   * launch of that kernel holds; 0 = off. */
+  /* End of a pass: once at most this many paths are left, one kernel finishes them a
+   * thread per path (trace and shading in turn) instead of round by round; the result is
+   * the same bits. -1 (default) = as many paths as one resident launch of that kernel
+   * holds (bidirectional passes: half as many); 0 = off. */
   YC_OPT_TAIL = 2,
   /* Traversal launches of a round: 1 (default) = the closest-hit (extension) and the
    * any-hit (shadow, MIS) rays of a round share one launch; 0 = one launch each, the two

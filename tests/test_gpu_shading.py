@@ -76,18 +76,20 @@ def test_lights_replaced_after_the_upload(r, integrator):
 
 
 # An eye vertex's segments go out in rounds of eight at most: light subpaths that need one
-# round, two and three; in the shared launch, its sorted form, and the launch of their own.
+# round, two and three; in the shared launch, its sorted form, and the launch of their own, and
+# in the tail.
 @pytest.mark.parametrize("mixed, sort", [(1, 0), (1, 1), (0, 0)])
 @pytest.mark.parametrize("bounces", [3, 9, 20])
 @pytest.mark.parametrize("integrator", [1, 2])
 @pytest.mark.parametrize("tris", [0, 6000])
-def test_segments_of_an_eye_vertex(r, tris, integrator, bounces, mixed, sort):
+@pytest.mark.parametrize("tail", [0, -1])
+def test_segments_of_an_eye_vertex(r, tail, tris, integrator, bounces, mixed, sort):
     if sort and not tris:
         pytest.skip("rays are sorted in scenes of at least 4096 triangles")
     s = workloads.mixed_scene(tris, 5, W, H, 1, scenes.default_cfg()) if tris else scenes.c0_bdpt_mis(W, H, lights=4)
     s.cfg = dict(s.cfg, integrator=integrator, bdpt_bounces=bounces, mis=0)
     sid = r.upload(s)
-    opts = [(3, mixed, 1), (5, 1 if sort else 65536, 65536), (6, 1 if sort else 65536, 65536)]
+    opts = [(2, tail, -1), (3, mixed, 1), (5, 1 if sort else 65536, 65536), (6, 1 if sort else 65536, 65536)]
     for o, v, _ in opts:
         N.check(r.L.yc_set_option(r.h, o, v), "yc_set_option")
     _same(r, s, sid)

@@ -213,6 +213,12 @@ constexpr int kTraceStage = 1 << 16;
 constexpr int kRaySortMinTris = 4096;
 // frames with fewer pixels are shaded in queue order by yc_render_pass
 constexpr size_t kShadeSortMinPixels = 1u << 19;
+// The tail of a bidirectional pass begins at one path for so many lanes of its launch: an eye vertex
+// sends up to eight segments, which idle lanes walk. One pass, ms without a tail / at a share of 1,
+// 2, 4, 16: Cornell box 96x64 naive 1.32 / 0.79, 0.80, 0.80, 1.01; 256x192 with MIS 1.33 / 1.40,
+// 1.20, 1.13, 1.13; 640x480 naive 2.56 / 2.88, 2.51, 2.52, 2.52; 60K triangles 160x120 naive 2.40 /
+// 1.51, 1.51, 1.83, 2.15; 820K 1280x720 with MIS 7.69 / 6.91, 6.90, 7.25, 7.34.
+constexpr int kBdptTailShare = 2;
 
 // FNV-1a over the 64-bit words of the repacked node, stream and shading arrays, the root
 // box and the root link and test (yc_scene_layout, yc_scene_digest)
@@ -559,8 +565,14 @@ int run_passes(yc_ctx* c, Scene* sc, Accum* ac, const uint32_t* rands, int n_pas
   if (grid_c <= 0 || grid_a <= 0 || grid_m <= 0)
     return fail(YC_E_LAUNCH, "trace kernel cannot be resident (stack too deep)");
   int tail_grid = 0, tail_at = 0;
-  if (!bdpt && c->tail_paths != 0) {
-    const int capacity = yc::tail_capacity(pp, n_smem, &tail_grid);
+  if (c->tail_paths != 0) {
+    int capacity = 0;
+    if (bdpt) {
+      tail_grid = bdpt_mis ? yc::tail_bdpt_mis_grid(pp, n_smem) : yc::tail_bdpt_grid(pp, n_smem);
+      capacity = tail_grid > 0 ? tail_grid * yc::TRACE_TB_PASS / kBdptTailShare : 0;
+    } else {
+      capacity = yc::tail_capacity(pp, n_smem, &tail_grid);
+    }
     tail_at = c->tail_paths < 0 ? capacity : std::min(c->tail_paths, capacity);
   }
   if (n_smem > 0)
@@ -652,8 +664,13 @@ int run_passes(yc_ctx* c, Scene* sc, Accum* ac, const uint32_t* rands, int n_pas
     }
     if (tail_at > 0) {
       KTimer kt(c, K_TAIL);
-      if (yc::launch_tail(pp, ps, out_c, out_w, rout, tail_at, c->stats.p, tail_grid, c->stream, n_smem,
-                          n_smem > 0 ? c->pass_spill.p : nullptr))
+      int* spill = n_smem > 0 ? c->pass_spill.p : nullptr;
+      if (bdpt_mis ? yc::launch_tail_bdpt_mis(pp, ps, bb, out_c, out_w, rout, tail_at, c->stats.p, tail_grid, c->stream,
+                                              n_smem, spill)
+          : bdpt   ? yc::launch_tail_bdpt(pp, ps, bb, out_c, out_w, rout, tail_at, c->stats.p, tail_grid, c->stream,
+                                          n_smem, spill)
+                   : yc::launch_tail(pp, ps, out_c, out_w, rout, tail_at, c->stats.p, tail_grid, c->stream, n_smem,
+                                     spill))
         return fail(YC_E_LAUNCH, std::string("tail kernel: ") + cudaGetErrorString(cudaGetLastError()));
     }
     YC_CUDA(cudaPeekAtLastError());

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(BATCH_LOGIC_TB, 4) k_batch_logic(const BatchJo
       const int kind = emit & EMIT;   // a path has one ray in flight
       produce_key(rsp, jobs, ps, job_pass, p, kind, (emit & EMIT_SEG1) != 0, kind == EMIT_CLOSEST ? at.closest : at.any);
     }
-    unsigned v[7] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples, lc.prim};
+    unsigned v[7] = {lc.rays, lc.ext, lc.shadow, lc.conn, lc.trav, lc.samples, lc.prim};
 #pragma unroll
     for (int q = 0; q < 7; ++q) {
       unsigned x = v[q];

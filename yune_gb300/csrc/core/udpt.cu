@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps,
       if (again) pp.q_restart[first + __popc(m & ((1u << lane) - 1))] = p;
     }
     // counters
-    unsigned v[6] = {lc.rays, lc.ext, lc.shadow, lc.mis, lc.trav, lc.samples};
+    unsigned v[6] = {lc.rays, lc.ext, lc.shadow, lc.conn, lc.trav, lc.samples};
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
       unsigned x = v[q];

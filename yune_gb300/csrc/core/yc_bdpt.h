@@ -107,4 +107,14 @@ void launch_logic_bdpt_mis(const PassParams& pp, const PathState& ps, const Bdpt
                            RoundCounters* rc_out, DevStats* st, int grid, cudaStream_t s, const int* sorted = nullptr,
                            const SortCtl* sctl = nullptr);
 
+// tail kernels (yc_tail.cuh): blocks of one resident launch, and the launch
+int tail_bdpt_grid(const PassParams& pp, int n_smem);
+int tail_bdpt_mis_grid(const PassParams& pp, int n_smem);
+int launch_tail_bdpt(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
+                     const int* in_wait, RoundCounters* rc_in, int threshold, DevStats* st, int grid, cudaStream_t s,
+                     int n_smem, int* spill);
+int launch_tail_bdpt_mis(const PassParams& pp, const PathState& ps, const BdptBuffers& bb, const int* in_closest,
+                         const int* in_wait, RoundCounters* rc_in, int threshold, DevStats* st, int grid,
+                         cudaStream_t s, int n_smem, int* spill);
+
 }  // namespace yc

@@ -26,6 +26,16 @@ __device__ __forceinline__ f4 ld4(const yc_float4& v) { return ym::mk(v.x, v.y, 
 __device__ __forceinline__ f4 f4of(float4 v) { return ym::mk(v.x, v.y, v.z, v.w); }
 __device__ __forceinline__ float draw(uint32_t& seed) { seed = ym::xor_shift(seed); return ym::u01(seed); }
 
+// What a step of a path sends: one closest-hit ray, or none (the path then waits for segments), and
+// segments (segment s: EMIT_SEG0 << s)
+enum : int { EMIT_CLOSEST = 1, EMIT_WAIT = 2, EMIT = 3, EMIT_SEG0 = 4, EMIT_SEG1 = 8 };
+
+// rays and samples of a thread's steps (conn: MIS rays of unidirectional paths, connections of
+// bidirectional ones)
+struct LogicCounts {
+  unsigned rays = 0, ext = 0, shadow = 0, conn = 0, trav = 0, samples = 0, prim = 0;
+};
+
 // a / b rounded to nearest, from r = 1 / b rounded to nearest: the quotient a * r is within one
 // unit of the last place, and one step along its remainder gives the division's own result
 // (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).

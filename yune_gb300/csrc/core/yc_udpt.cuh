@@ -28,8 +28,6 @@ enum : int {
   F_OCC_NAN = 32,         //   and if it is occluded the sample is NaN (0 times a weight without a value)
   F_LAST = 64             //   and it is the path's last ray
 };
-// what a step sends: one closest-hit ray or none (the path then waits for segments), and segments
-enum : int { EMIT_CLOSEST = 1, EMIT_WAIT = 2, EMIT = 3, EMIT_SEG0 = 4, EMIT_SEG1 = 8 };
 // the segments in flight of a path with this misc.z: shadow ray, MIS ray
 __device__ __forceinline__ int segments_of(int state_flags) {
   const int state = state_flags & 15, flags = state_flags >> 4;
@@ -45,10 +43,6 @@ constexpr int LOGIC_TB = 256;
 
 // whether a vertex's shadow ray goes with the path's next ray (TOGETHER of logic_path)
 inline bool rays_together(const PassParams& pp) { return pp.mis != 0 && pp.mis_lobe_fix != 0; }
-
-struct LogicCounts {
-  unsigned rays = 0, ext = 0, shadow = 0, mis = 0, trav = 0, samples = 0, prim = 0;
-};
 
 // ---- raygen: pathtracer prologue + createRay (udpt.cl:158-189, 213-238) ----
 // seed of pixel (px, py) for pass seed `rand`, the camera ray, and the closest light
@@ -392,7 +386,7 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
           cnt.trav++;
         }
       } else if (cast == S_NEE_MIS) {   // only light j can satisfy the test
-        cnt.mis++;
+        cnt.conn++;
         if (lk != j) {
           dl = ls + ld4(sc.mats[V.mat].ke);
           phase = P_NEE_DELIVER;
