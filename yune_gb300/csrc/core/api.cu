@@ -88,6 +88,7 @@ struct Scene {
   bool refit_ready = false;
   DevBuf<yc_triangle> refit_tris;
   DevBuf<float4> refit_root;
+  DevBuf<int> refit_bad;
   size_t n_node4 = 0, n_tri4 = 0, n_shade4 = 0;   // float4 records of the repacked arrays
   // the four-child walk index over dev's two-child nodes (widen.cu); none for scenes without
   // interior nodes, in the other tree modes, and when there was no memory for it. It is a
@@ -773,29 +774,38 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
   if ((n_tri > 0 && !tris) || (n_mat > 0 && !mats) || (n_node > 0 && !nodes))
     return fail(YC_E_INVALID, "NULL array with non-zero count");
   if (n_light < 1 || n_light > yc::MAX_LIGHTS || !lights) return fail(YC_E_INVALID, "need 1..16 lights");
-  {
-    std::string err;
-    if (yc::check_materials(tris, n_tri, n_mat, err)) return fail(YC_E_INVALID, err);
-  }
-  yc::Repacked rp;
-  yc::DevRepackPlan plan;
-  std::string err;
   // the repack: on the device for tree mode 1 (YC_OPT_REPACK), where a scene has two
   // reachable leaves or more; otherwise (and for the trivial scenes) on the host
+  YC_CUDA(cudaSetDevice(c->device));
+  yc::Repacked rp;
+  yc::DevRepack dev;
+  yc::DevRepackPlan plan;
+  std::string err;
   int on_device = 0;
-  if (c->repack_device && c->tree_mode == yc::TREE_SAH_OVER_LEAVES) {
-    on_device = yc::plan_device_repack(nodes, n_node, n_tri, plan, err);
-    if (on_device < 0) return fail(YC_E_INVALID, err);
+  const bool device_checks = n_tri >= yc::kDeviceCheckTris;
+  if (c->repack_device && c->tree_mode == yc::TREE_SAH_OVER_LEAVES && n_tri > 0 && n_node > 0 && n_node < (1 << 27)) {
+    if (!device_checks && yc::check_materials(tris, n_tri, n_mat, err)) return fail(YC_E_INVALID, err);
+    const int r = yc::repack_copy(tris, n_tri, n_mat, nodes, n_node, device_checks, dev, c->stream, err);
+    if (r < 0) return fail(r == -2 ? YC_E_NOMEM : YC_E_LAUNCH, err);
+    if (dev.bad_tri < n_tri) return fail(YC_E_INVALID, "triangle " + std::to_string(dev.bad_tri) + " has matID out of range");
+    on_device = r && dev.n_leaf >= 2 && dev.slots < (size_t)(1 << 27);
+    if (!on_device) {   // an array the host has to judge
+      on_device = yc::plan_device_repack(nodes, n_node, n_tri, plan, err);
+      if (on_device < 0) return fail(YC_E_INVALID, err);
+      dev.slots = plan.slots;
+      dev.n_leaf = (int)plan.leaf_node.size();
+    }
+  } else if (yc::check_materials(tris, n_tri, n_mat, err)) {
+    return fail(YC_E_INVALID, err);
   }
   if (!on_device && yc::repack_scene(tris, n_tri, nodes, n_node, c->tree_mode, rp, err)) return fail(YC_E_INVALID, err);
-  const size_t n_node4 = on_device ? 4 * (plan.leaf_node.size() - 1) : rp.nodes.size();
-  const size_t n_tri4 = on_device ? 3 * plan.slots : rp.tris.size();
+  const size_t n_node4 = on_device ? 4 * ((size_t)dev.n_leaf - 1) : rp.nodes.size();
+  const size_t n_tri4 = on_device ? 3 * dev.slots : rp.tris.size();
   const size_t n_shade4 = on_device ? 4 * (size_t)n_tri : rp.shade.size();
   std::unique_ptr<Scene> s(new (std::nothrow) Scene);
   if (s)
     for (int i = 0; i < n_mat; ++i) s->has_specular = s->has_specular || mats[i].is_specular != 0;
   if (!s) return fail(YC_E_NOMEM, "host allocation failed");
-  YC_CUDA(cudaSetDevice(c->device));
   YC_CUDA(s->nodes.alloc(std::max<size_t>(n_node4, 4)));
   YC_CUDA(s->tris.alloc(std::max<size_t>(n_tri4, 3)));
   YC_CUDA(s->shade.alloc(std::max<size_t>(n_shade4, 4)));
@@ -807,15 +817,15 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
   s->n_shade4 = n_shade4;
   if (on_device) {
     int depth = 0;
-    const int r = yc::repack_device(tris, n_tri, nodes, n_node, plan, s->nodes.p, s->tris.p, s->shade.p, depth,
-                                    c->stream, err);
+    const int r = yc::repack_device(dev, plan, n_tri, s->nodes.p, s->tris.p, s->shade.p, depth, c->stream, err);
     if (r) return fail(r == -2 ? YC_E_NOMEM : YC_E_LAUNCH, err);
     rp.root_link = 0;   // the root is the first node (two leaves or more)
     rp.root_test = 1;
     rp.depth = depth;
     rp.wide = 0;
-    rp.root_lo = plan.root_lo;
-    rp.root_hi = plan.root_hi;
+    const yc_aabb& box = nodes[0].aabb;
+    rp.root_lo = float4{box.p_min.x, box.p_min.y, box.p_min.z, 0.0f};
+    rp.root_hi = float4{box.p_max.x, box.p_max.y, box.p_max.z, 0.0f};
   }
   if (!rp.nodes.empty())
     YC_CUDA(cudaMemcpyAsync(s->nodes.p, rp.nodes.data(), rp.nodes.size() * sizeof(float4), cudaMemcpyHostToDevice, c->stream));
@@ -994,6 +1004,7 @@ int make_refit_plan(yc_ctx* c, Scene* s) {
     YC_CUDA(cudaMemcpyAsync(s->refit_order.p, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice,
                             c->stream));
   YC_CUDA(s->refit_root.alloc(2));
+  YC_CUDA(s->refit_bad.alloc(1));
   YC_CUDA(cudaStreamSynchronize(c->stream));
   s->refit_ready = true;
   return 0;
@@ -1008,7 +1019,8 @@ int yc_refit_scene(yc_ctx* c, int scene_id, const yc_triangle* tris, int n_tri) 
   Scene* s = find_scene(c, scene_id);
   if (!s) return fail(YC_E_NOTFOUND, "unknown scene");
   if (n_tri != s->dev.n_tri) return fail(YC_E_INVALID, "a refit keeps the scene's triangles: counts differ");
-  {
+  const bool device_checks = n_tri >= yc::kDeviceCheckTris;   // (after the copy, before anything of the scene changes)
+  if (!device_checks) {
     std::string err;
     if (yc::check_materials(tris, n_tri, s->dev.n_mat, err)) return fail(YC_E_INVALID, err);
   }
@@ -1019,6 +1031,10 @@ int yc_refit_scene(yc_ctx* c, int scene_id, const yc_triangle* tris, int n_tri) 
   if (n_tri > 0)
     YC_CUDA(cudaMemcpyAsync(s->refit_tris.p, tris, (size_t)n_tri * sizeof(yc_triangle), cudaMemcpyHostToDevice,
                             c->stream));
+  int bad = n_tri;
+  if (device_checks)
+    YC_CUDA(yc::first_bad_material(s->refit_tris.p, n_tri, s->dev.n_mat, s->refit_bad.p, bad, c->stream));
+  if (bad < n_tri) return fail(YC_E_INVALID, "triangle " + std::to_string(bad) + " has matID out of range");
   yc::RefitPlan plan;
   plan.order = s->refit_order.p;
   plan.level_off = s->refit_levels;

@@ -515,8 +515,6 @@ int plan_device_repack(const yc_bvh_node* nodes, int n_node, int n_tri, DevRepac
   reachable_leaves(nodes, n_node, plan.leaf_node, plan.leaf_first, plan.slots);
   if (plan.leaf_node.size() < 2) return 0;
   if (plan.slots >= (size_t)(1 << 27)) { err = "scene too large for the 27-bit stream index"; return -1; }
-  plan.root_lo = float4{root.aabb.p_min.x, root.aabb.p_min.y, root.aabb.p_min.z, 0.0f};
-  plan.root_hi = float4{root.aabb.p_max.x, root.aabb.p_max.y, root.aabb.p_max.z, 0.0f};
   return 1;
 }
 

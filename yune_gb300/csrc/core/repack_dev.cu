@@ -920,13 +920,134 @@ struct Tmp {
   cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
 };
 
+// The first triangle without a material, a thread per triangle (bound by the stride of the read;
+// starting and joining the host's threads took 1 ms for 330K triangles).
+__global__ void __launch_bounds__(ITEM_TB) k_check_materials(const yc_triangle* tris, int n, int n_mat, int* first) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && (tris[i].matID < 0 || tris[i].matID >= n_mat)) atomicMin(first, i);
+}
+
+// what the copies' checks found
+struct CopyCtl {
+  int bad_tri, irregular, n_leaf, slots;
+};
+__device__ __forceinline__ bool dev_is_leaf(const yc_bvh_node& n) { return n.child_idx == -1 && n.vert_len > 0; }
+__device__ __forceinline__ bool dev_is_queued(const yc_bvh_node& n) { return n.vert_len > 0 || n.child_idx > 0; }
+
+// repack.cpp's node checks, and a mark on every child the reference queues
+__global__ void __launch_bounds__(ITEM_TB) k_check_nodes(const yc_bvh_node* __restrict__ nodes, int n_node, int n_tri,
+                                                         int* child, CopyCtl* ctl) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_node) return;
+  const yc_bvh_node& n = nodes[i];
+  bool bad = n.vert_len > 10;
+  if (!bad && dev_is_leaf(n)) {
+    for (int k = 0; k < n.vert_len; ++k) bad = bad || n.vert_list[k] < 0 || n.vert_list[k] >= n_tri;
+  } else if (!bad && (dev_is_queued(n) || i == 0)) {
+    bad = n.child_idx <= i || n.child_idx >= n_node - 1;
+    if (!bad) child[n.child_idx] = child[n.child_idx + 1] = 1;
+  }
+  if (bad) ctl->irregular = 1;
+}
+
+// With every child after its parent, and every interior node but the root a marked child, a node is
+// reached if it is marked and queued (by induction over the index). Its leaf flag and triangles.
+__global__ void __launch_bounds__(ITEM_TB) k_leaf_flags(const yc_bvh_node* __restrict__ nodes, int n_node,
+                                                        const int* __restrict__ child, int* flag, int* len,
+                                                        CopyCtl* ctl) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_node) return;
+  const yc_bvh_node& n = nodes[i];
+  const bool leaf = dev_is_leaf(n), reached = i == 0 || (child[i] && dev_is_queued(n));
+  if (!reached && !leaf && dev_is_queued(n)) ctl->irregular = 1;
+  flag[i] = reached && leaf;
+  len[i] = reached && leaf ? n.vert_len : 0;
+}
+
+__global__ void __launch_bounds__(ITEM_TB) k_list_leaves(int n_node, const int* __restrict__ flag,
+                                                         const int* __restrict__ len, const int* __restrict__ at,
+                                                         const int* __restrict__ slot, int* leaf, int* first,
+                                                         CopyCtl* ctl) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_node) return;
+  if (flag[i]) {
+    leaf[at[i]] = i;
+    first[at[i]] = slot[i];
+  }
+  if (i == n_node - 1) {
+    ctl->n_leaf = at[i] + flag[i];
+    ctl->slots = slot[i] + len[i];
+  }
+}
+
 }  // namespace
 
-int repack_device(const yc_triangle* tris_host, int n_tri, const yc_bvh_node* nodes_host, int n_node,
-                  const DevRepackPlan& plan, float4* nodes, float4* stream, float4* shade, int& depth, cudaStream_t s,
-                  std::string& err) {
-  const int n_leaf = (int)plan.leaf_node.size();
-  if (n_leaf < 2 || n_tri <= 0 || n_node <= 0) {
+DevRepack::~DevRepack() {
+  cudaFree(tris);
+  cudaFree(nodes);
+  cudaFree(work);
+}
+
+cudaError_t first_bad_material(const yc_triangle* tris, int n, int n_mat, int* first, int& bad, cudaStream_t s) {
+  bad = n;
+  if (n <= 0) return cudaSuccess;
+  cudaError_t e = cudaMemcpyAsync(first, &n, sizeof(int), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) k_check_materials<<<(n + ITEM_TB - 1) / ITEM_TB, ITEM_TB, 0, s>>>(tris, n, n_mat, first);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, first, sizeof(int), cudaMemcpyDeviceToHost, s);
+  return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
+// Listing the leaves of 123K nodes is a dozen passes over a few ints a node; the host's checks and
+// its walk over the nodes in order took 1.7 ms (an upload of 330K triangles 8.7 ms, now 4.6).
+int repack_copy(const yc_triangle* tris_host, int n_tri, int n_mat, const yc_bvh_node* nodes_host, int n_node,
+                bool check, DevRepack& d, cudaStream_t s, std::string& err) {
+  const auto failed = [&](cudaError_t e) {
+    err = std::string("device repack: copy: ") + cudaGetErrorString(e);
+    return e == cudaErrorMemoryAllocation ? -2 : -1;
+  };
+#define YC_COPY_CUDA(call)                        \
+  do {                                            \
+    const cudaError_t e_ = (call);                \
+    if (e_ != cudaSuccess) return failed(e_);     \
+  } while (0)
+  // (the scans take whole tiles of 1024)
+  const size_t N = (size_t)n_node, tiles = (N + 1023) / 1024;
+  YC_COPY_CUDA(cudaMalloc(&d.tris, (size_t)n_tri * sizeof(yc_triangle)));
+  YC_COPY_CUDA(cudaMalloc(&d.nodes, N * sizeof(yc_bvh_node)));
+  YC_COPY_CUDA(cudaMalloc(&d.work, (7 * N + tiles) * sizeof(int) + sizeof(CopyCtl)));
+  d.leaf = d.work;
+  d.first = d.leaf + N;
+  int* child = d.first + N;
+  int *flag = child + N, *len = flag + N, *at = len + N, *slot = at + N, *sums = slot + N;
+  CopyCtl* ctl = reinterpret_cast<CopyCtl*>(sums + tiles);
+  CopyCtl h{n_tri, 0, 0, 0};
+  YC_COPY_CUDA(cudaMemcpyAsync(d.tris, tris_host, (size_t)n_tri * sizeof(yc_triangle), cudaMemcpyHostToDevice, s));
+  YC_COPY_CUDA(cudaMemcpyAsync(d.nodes, nodes_host, N * sizeof(yc_bvh_node), cudaMemcpyHostToDevice, s));
+  d.bad_tri = n_tri;
+  if (!check) return 0;
+  YC_COPY_CUDA(cudaMemcpyAsync(ctl, &h, sizeof h, cudaMemcpyHostToDevice, s));
+  YC_COPY_CUDA(cudaMemsetAsync(child, 0, N * sizeof(int), s));
+  const int g = (n_node + ITEM_TB - 1) / ITEM_TB;
+  k_check_materials<<<(n_tri + ITEM_TB - 1) / ITEM_TB, ITEM_TB, 0, s>>>(d.tris, n_tri, n_mat, &ctl->bad_tri);
+  k_check_nodes<<<g, ITEM_TB, 0, s>>>(d.nodes, n_node, n_tri, child, ctl);
+  k_leaf_flags<<<g, ITEM_TB, 0, s>>>(d.nodes, n_node, child, flag, len, ctl);
+  launch_exclusive_scan(flag, at, sums, n_node, s);
+  launch_exclusive_scan(len, slot, sums, n_node, s);
+  k_list_leaves<<<g, ITEM_TB, 0, s>>>(n_node, flag, len, at, slot, d.leaf, d.first, ctl);
+  YC_COPY_CUDA(cudaPeekAtLastError());
+  YC_COPY_CUDA(cudaMemcpyAsync(&h, ctl, sizeof h, cudaMemcpyDeviceToHost, s));
+  YC_COPY_CUDA(cudaStreamSynchronize(s));
+#undef YC_COPY_CUDA
+  d.bad_tri = h.bad_tri;
+  d.n_leaf = h.n_leaf;
+  d.slots = (size_t)h.slots;
+  return h.irregular ? 0 : 1;
+}
+
+int repack_device(DevRepack& d, const DevRepackPlan& plan, int n_tri, float4* nodes, float4* stream, float4* shade,
+                  int& depth, cudaStream_t s, std::string& err) {
+  const int n_leaf = plan.leaf_node.empty() ? d.n_leaf : (int)plan.leaf_node.size();
+  if (n_leaf < 2 || n_tri <= 0) {
     err = "device repack: the plan has fewer than two leaves";
     return -1;
   }
@@ -941,36 +1062,25 @@ int repack_device(const yc_triangle* tris_host, int n_tri, const yc_bvh_node* no
   } while (0)
   const size_t cap_large = (size_t)n_leaf / (SMALL_MAX + 1) + 1;   // disjoint ranges of more than SMALL_MAX
   const size_t cap_small = (size_t)n_leaf / 2 + 1;                 // disjoint ranges of two leaves or more
-  Tmp<yc_triangle> d_tris;
-  Tmp<yc_bvh_node> d_nodes;
-  Tmp<int> d_leaf, d_first;
   Tmp<SahItem> d_items, d_tmp;
   Tmp<SahTask> d_ta, d_tb, d_small;
   Tmp<SahCtl> d_ctl;
-  YC_REPACK_CUDA(d_tris.alloc(n_tri), "allocation");
-  YC_REPACK_CUDA(d_nodes.alloc(n_node), "allocation");
-  YC_REPACK_CUDA(d_leaf.alloc(n_leaf), "allocation");
-  YC_REPACK_CUDA(d_first.alloc(n_leaf), "allocation");
   YC_REPACK_CUDA(d_items.alloc(n_leaf), "allocation");
   YC_REPACK_CUDA(d_tmp.alloc(n_leaf), "allocation");
   YC_REPACK_CUDA(d_ta.alloc(cap_large), "allocation");
   YC_REPACK_CUDA(d_tb.alloc(cap_large), "allocation");
   YC_REPACK_CUDA(d_small.alloc(cap_small), "allocation");
   YC_REPACK_CUDA(d_ctl.alloc(1), "allocation");
-  YC_REPACK_CUDA(cudaMemcpyAsync(d_tris.p, tris_host, (size_t)n_tri * sizeof(yc_triangle), cudaMemcpyHostToDevice, s),
-                 "copy");
-  YC_REPACK_CUDA(
-      cudaMemcpyAsync(d_nodes.p, nodes_host, (size_t)n_node * sizeof(yc_bvh_node), cudaMemcpyHostToDevice, s), "copy");
-  YC_REPACK_CUDA(cudaMemcpyAsync(d_leaf.p, plan.leaf_node.data(), (size_t)n_leaf * sizeof(int),
-                                 cudaMemcpyHostToDevice, s),
-                 "copy");
-  YC_REPACK_CUDA(cudaMemcpyAsync(d_first.p, plan.leaf_first.data(), (size_t)n_leaf * sizeof(int),
-                                 cudaMemcpyHostToDevice, s),
-                 "copy");
+  if (!plan.leaf_node.empty()) {
+    YC_REPACK_CUDA(cudaMemcpyAsync(d.leaf, plan.leaf_node.data(), (size_t)n_leaf * sizeof(int), cudaMemcpyHostToDevice, s),
+                   "copy");
+    YC_REPACK_CUDA(
+        cudaMemcpyAsync(d.first, plan.leaf_first.data(), (size_t)n_leaf * sizeof(int), cudaMemcpyHostToDevice, s), "copy");
+  }
   // shading records: the refit's kernel alone (no stream slots, no nodes)
-  if (launch_refit(RefitPlan(), d_tris.p, n_tri, nullptr, nullptr, 0, shade, false, LINK_NONE, false, nullptr, s))
+  if (launch_refit(RefitPlan(), d.tris, n_tri, nullptr, nullptr, 0, shade, false, LINK_NONE, false, nullptr, s))
     return cuda_fail(cudaGetLastError(), "shading records");
-  k_leaf_items<<<(n_leaf + ITEM_TB - 1) / ITEM_TB, ITEM_TB, 0, s>>>(d_nodes.p, d_leaf.p, d_first.p, n_leaf, d_tris.p,
+  k_leaf_items<<<(n_leaf + ITEM_TB - 1) / ITEM_TB, ITEM_TB, 0, s>>>(d.nodes, d.leaf, d.first, n_leaf, d.tris,
                                                                    d_items.p, stream);
   YC_REPACK_CUDA(cudaPeekAtLastError(), "leaf items");
   const SahTask root{0, n_leaf, 0, -1, 0};
