@@ -10,10 +10,15 @@
 //   hist     per primitive, its bin (the first plane not below its centroid, when the
 //            centroid lies in the node box) into the node's histogram
 //   decide   one thread per node: leaf, empty, binned SAH split or spatial median
-//   scan     child slots for the splitting nodes, in node order (breadth-first numbering)
-//   flags    per primitive, whether its centroid lies in the first child's box
-//   scan     positions of a stable partition of every node's segment
+//   slots    child slots for the splitting nodes, in node order (breadth-first numbering)
+//   flags    per primitive, whether its centroid lies in the first child's box, and the
+//            scan for a stable partition of every node's segment
+//   children the splitting nodes' children
 //   scatter  primitives into their children's segments
+// A level of a few thousand nodes is bound by its launches and the readback of its splits, so
+// each kernel does what the next would otherwise be launched for, and the buffers start with room
+// for the usual tree (with 14 launches a level, and the buffers grown as the tree grew, 330K
+// triangles took 9.26 ms and 3K 1.92 ms, now 6.17 and 1.19, copies included);
 // then a refit over the levels in reverse. The only liberty taken: a box bound that is
 // zero is stored as +0 (atomics cannot keep "the first of -0 and +0 met", which the
 // sequential builder does); the traversal's arithmetic is the same for either zero.
@@ -106,23 +111,20 @@ struct NodeWork {
   int pad;
 };
 
+__device__ __forceinline__ void open_node(NodeWork& w, int s, int e) {
+  w.s = s;
+  w.e = e;
+  for (int k = 0; k < 3; ++k) { w.box[k] = 0x7fffffff; w.box[3 + k] = (int)0x80000000; }
+  w.split = 0;
+  w.n1 = 0;
+}
+
 __global__ void k_root(yc_bvh_node* nodes, NodeWork* work, const int* root, int n) {
   yc_aabb box;
   box.p_min = yc_float4{unord(root[0]), unord(root[1]), unord(root[2]), 1.0f};
   box.p_max = yc_float4{unord(root[3]), unord(root[4]), unord(root[5]), 1.0f};
   fresh(nodes[0], box);
-  work[0].s = 0;
-  work[0].e = n;
-}
-
-__global__ void k_level_clear(NodeWork* work, int* hist, int a, int b, int bins) {
-  const int i = a + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= b) return;
-  NodeWork& w = work[i];
-  for (int k = 0; k < 3; ++k) { w.box[k] = 0x7fffffff; w.box[3 + k] = (int)0x80000000; }
-  w.split = 0;
-  w.n1 = 0;
-  for (int k = 0; k < bins; ++k) hist[(size_t)(i - a) * bins + k] = 0;
+  open_node(work[0], 0, n);
 }
 
 // primitives of the level's nodes that can split: their node's box union. A node's
@@ -140,14 +142,28 @@ __global__ void k_bounds(const int* __restrict__ perm, const int* __restrict__ p
     nd = pnode[i];
     act = nd >= a && nd < b && work[nd].e - work[nd].s > leaf_max;
   }
+  // a block whose primitives all belong to one node (the top levels) adds one box
+  __shared__ int s_node, s_box[6];
+  if (threadIdx.x == 0) s_node = act ? nd : -1;
+  if (threadIdx.x < 6) s_box[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : (int)0x80000000;
+  __syncthreads();
+  const bool whole = __syncthreads_and(act && nd == s_node);
   const unsigned peers = __match_any_sync(0xffffffffu, act ? nd : -1 - lane);
-  if (!act) return;
+  if (!act) return;   // (of a whole block no thread)
   const float4 l = lo[perm[i]], h = hi[perm[i]];
   const int x0 = __reduce_min_sync(peers, ord(l.x)), y0 = __reduce_min_sync(peers, ord(l.y));
   const int z0 = __reduce_min_sync(peers, ord(l.z));
   const int x1 = __reduce_max_sync(peers, ord(h.x)), y1 = __reduce_max_sync(peers, ord(h.y));
   const int z1 = __reduce_max_sync(peers, ord(h.z));
-  if (lane == __ffs(peers) - 1) {
+  if (whole) {
+    if (lane == 0) {
+      atomicMin(&s_box[0], x0); atomicMin(&s_box[1], y0); atomicMin(&s_box[2], z0);
+      atomicMax(&s_box[3], x1); atomicMax(&s_box[4], y1); atomicMax(&s_box[5], z1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(&work[nd].box[threadIdx.x], s_box[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&work[nd].box[threadIdx.x], s_box[threadIdx.x]);
+  } else if (lane == __ffs(peers) - 1) {
     NodeWork& w = work[nd];
     atomicMin(&w.box[0], x0); atomicMin(&w.box[1], y0); atomicMin(&w.box[2], z0);
     atomicMax(&w.box[3], x1); atomicMax(&w.box[4], y1); atomicMax(&w.box[5], z1);
@@ -280,26 +296,6 @@ __global__ void k_decide(const int* __restrict__ perm, yc_bvh_node* nodes, NodeW
   child_box[2 * (size_t)(nd - a) + 1] = best2;
 }
 
-// membership of each primitive in its node's first child (BVH.cpp:175-216)
-__global__ void k_flags(const int* __restrict__ perm, const int* __restrict__ pnode, const float4* __restrict__ cen,
-                        const NodeWork* work, const yc_aabb* child_box, int* flag, int n, int a, int b) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int nd = pnode[i];
-  int f = 0;
-  if (nd >= a && nd < b && work[nd].split) {
-    const yc_aabb b1 = child_box[2 * (size_t)(nd - a)], b2 = child_box[2 * (size_t)(nd - a) + 1];
-    if (surface_area(b1) == 0.0f) f = 0;
-    else if (surface_area(b2) == 0.0f) f = 1;
-    else {
-      const float4 c = cen[perm[i]];
-      f = (c.x < b1.p_min.x || c.x > b1.p_max.x || c.y < b1.p_min.y || c.y > b1.p_max.y || c.z < b1.p_min.z ||
-           c.z > b1.p_max.z) ? 0 : 1;
-    }
-  }
-  flag[i] = f;
-}
-
 // exclusive scan of n ints in tiles of 1024 (tile sums scanned in one block, then added)
 __global__ void k_scan_tiles(const int* in, int* out, int* tile_sum, int n) {
   __shared__ int s_sum[32];
@@ -324,6 +320,49 @@ __global__ void k_scan_tiles(const int* in, int* out, int* tile_sum, int n) {
   __syncthreads();
   if (i < n) out[i] = incl - v + (warp > 0 ? s_sum[warp - 1] : 0);
   if (threadIdx.x == 1023) tile_sum[blockIdx.x] = s_sum[31];
+}
+
+// Membership of each primitive in its node's first child (BVH.cpp:175-216), and its exclusive scan
+// within the tile: flag in bit 31 of pos, the count before it in the others. (Position of i:
+// pos_of, once the tile sums are scanned.)
+__global__ void __launch_bounds__(1024) k_flag_tiles(const int* __restrict__ perm, const int* __restrict__ pnode,
+                                                     const float4* __restrict__ cen, const NodeWork* work,
+                                                     const yc_aabb* child_box, unsigned* pos, int* tile_sum, int n, int a,
+                                                     int b) {
+  __shared__ int s_sum[32];
+  const int i = blockIdx.x * 1024 + threadIdx.x;
+  int f = 0;
+  if (i < n) {
+    const int nd = pnode[i];
+    if (nd >= a && nd < b && work[nd].split) {
+      const yc_aabb b1 = child_box[2 * (size_t)(nd - a)], b2 = child_box[2 * (size_t)(nd - a) + 1];
+      if (surface_area(b1) == 0.0f) f = 0;
+      else if (surface_area(b2) == 0.0f) f = 1;
+      else {
+        const float4 c = cen[perm[i]];
+        f = (c.x < b1.p_min.x || c.x > b1.p_max.x || c.y < b1.p_min.y || c.y > b1.p_max.y || c.z < b1.p_min.z ||
+             c.z > b1.p_max.z) ? 0 : 1;
+      }
+    }
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned m = __ballot_sync(0xffffffffu, f);
+  if (lane == 0) s_sum[warp] = __popc(m);
+  __syncthreads();
+  if (warp == 0) {
+    int w = s_sum[lane];
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, off);
+      if (lane >= off) w += u;
+    }
+    s_sum[lane] = w;
+  }
+  __syncthreads();
+  if (i < n) pos[i] = ((unsigned)f << 31) | (unsigned)((warp > 0 ? s_sum[warp - 1] : 0) + __popc(m & ((1u << lane) - 1)));
+  if (threadIdx.x == 1023) tile_sum[blockIdx.x] = s_sum[31];
+}
+__device__ __forceinline__ int pos_of(const unsigned* pos, const int* tile_sum, int i) {
+  return (int)(pos[i] & 0x7fffffffu) + tile_sum[i >> 10];
 }
 
 __global__ void k_scan_sums(int* tile_sum, int tiles) {   // one block: exclusive scan in place
@@ -378,28 +417,54 @@ __global__ void k_slots_finish(const int* flag, const int* tile_sum, int* child_
   if (i == count - 1) *total = slot + flag[i];
 }
 
+// A level of at most SLOTS_ONE nodes: the same in one launch of one block, a tile of its threads at a time.
+constexpr int SLOTS_ONE = 4096;
+__global__ void __launch_bounds__(1024) k_slots_small(const NodeWork* work, int a, int count, int* child_of, int* total) {
+  __shared__ int s_sum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int before = 0;
+  for (int base = 0; base < count; base += 1024) {
+    const int i = base + threadIdx.x;
+    const int v = i < count ? work[a + i].split : 0;
+    const unsigned m = __ballot_sync(0xffffffffu, v != 0);
+    if (lane == 0) s_sum[warp] = __popc(m);
+    __syncthreads();
+    if (warp == 0) {
+      int w = s_sum[lane];
+      for (int off = 1; off < 32; off <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, w, off);
+        if (lane >= off) w += u;
+      }
+      s_sum[lane] = w;
+    }
+    __syncthreads();
+    if (i < count) child_of[i] = v ? before + (warp > 0 ? s_sum[warp - 1] : 0) + __popc(m & ((1u << lane) - 1)) : -1;
+    before += s_sum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *total = before;
+}
+
 // per splitting node: the first child's count, the children's nodes and segments
 __global__ void k_children(yc_bvh_node* nodes, NodeWork* work, const yc_aabb* child_box, const int* child_of,
-                           const int* pos, const int* flag, int a, int b, int next) {
+                           const unsigned* pos, const int* tile_sum, int a, int b, int next) {
   const int nd = a + blockIdx.x * blockDim.x + threadIdx.x;
   if (nd >= b) return;
   NodeWork& w = work[nd];
   if (!w.split) return;
   const int e1 = w.e - 1;
-  w.n1 = (pos[e1] + flag[e1]) - pos[w.s];
+  w.n1 = pos_of(pos, tile_sum, e1) + (int)(pos[e1] >> 31) - pos_of(pos, tile_sum, w.s);
   const int c = next + 2 * child_of[nd - a];
   nodes[nd].child_idx = c;
   fresh(nodes[c], child_box[2 * (size_t)(nd - a)]);
   fresh(nodes[c + 1], child_box[2 * (size_t)(nd - a) + 1]);
-  work[c].s = w.s;
-  work[c].e = w.s + w.n1;
-  work[c + 1].s = w.s + w.n1;
-  work[c + 1].e = w.e;
+  open_node(work[c], w.s, w.s + w.n1);
+  open_node(work[c + 1], w.s + w.n1, w.e);
 }
 
 // stable partition of every splitting node's segment; the other primitives stay put
 __global__ void k_scatter(const int* __restrict__ perm, const int* __restrict__ pnode, const NodeWork* work,
-                          const yc_bvh_node* nodes, const int* pos, const int* flag, int* perm_out, int* pnode_out,
+                          const yc_bvh_node* nodes, const unsigned* pos, const int* tile_sum, int* perm_out, int* pnode_out,
                           int n, int a, int b) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -410,10 +475,10 @@ __global__ void k_scatter(const int* __restrict__ perm, const int* __restrict__ 
     return;
   }
   const NodeWork& w = work[nd];
-  const int before1 = pos[i] - pos[w.s];   // first-child members before i in the segment
+  const int before1 = pos_of(pos, tile_sum, i) - pos_of(pos, tile_sum, w.s);   // first-child members before i in the segment
   const int c = nodes[nd].child_idx;
   int dst, child;
-  if (flag[i]) { dst = w.s + before1; child = c; }
+  if (pos[i] >> 31) { dst = w.s + before1; child = c; }
   else { dst = w.s + w.n1 + (i - w.s - before1); child = c + 1; }
   perm_out[dst] = perm[i];
   pnode_out[dst] = child;
@@ -486,13 +551,14 @@ cudaError_t bvh_build_device(const yc_triangle* tris_dev, int n, int bins, int l
   too_deep = false;
   if (n <= 0) return cudaSuccess;
   Buf<float4> cen, lo, hi;
-  Buf<int> perm, perm2, pnode, pnode2, flag, pos, tiles, root, child_of, hist, total, nflag, ntile;
+  Buf<int> perm, perm2, pnode, pnode2, tiles, root, child_of, hist, total, nflag, ntile;
+  Buf<unsigned> pos;
   Buf<yc_bvh_node> nodes;
   Buf<NodeWork> work;
   Buf<yc_aabb> child_box;
   BB_CHECK(cen.need(n, s)); BB_CHECK(lo.need(n, s)); BB_CHECK(hi.need(n, s));
   BB_CHECK(perm.need(n, s)); BB_CHECK(perm2.need(n, s)); BB_CHECK(pnode.need(n, s)); BB_CHECK(pnode2.need(n, s));
-  BB_CHECK(flag.need(n, s)); BB_CHECK(pos.need(n, s));
+  BB_CHECK(pos.need(n, s));
   const int ntiles = (n + 1023) / 1024;
   BB_CHECK(tiles.need(ntiles, s)); BB_CHECK(root.need(6, s)); BB_CHECK(total.need(1, s));
   const int init_root[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000, (int)0x80000000};
@@ -502,7 +568,12 @@ cudaError_t bvh_build_device(const yc_triangle* tris_dev, int n, int bins, int l
   // perm = identity, every primitive in the root
   k_iota<<<gp, BB_TB, 0, s>>>(perm.p, n);
   BB_CHECK(cudaMemsetAsync(pnode.p, 0, n * sizeof(int), s));
-  BB_CHECK(nodes.need(1024, s)); BB_CHECK(work.need(1024, s));
+  // (room for the usual tree, a node to two triangles, so that few levels have to grow the buffers,
+  // which waits for the device)
+  const size_t guess = (size_t)n / 2 + 1024, widest = guess / 4 + 1024;
+  BB_CHECK(nodes.need(guess, s)); BB_CHECK(work.need(guess, s));
+  BB_CHECK(hist.need(widest * bins, s)); BB_CHECK(child_of.need(widest, s)); BB_CHECK(child_box.need(2 * widest, s));
+  BB_CHECK(nflag.need(widest, s)); BB_CHECK(ntile.need(widest / 1024 + 1, s));
   k_root<<<1, 1, 0, s>>>(nodes.p, work.p, root.p, n);
   std::vector<int> level_start = {0};
   int a = 0, b = 1;
@@ -510,11 +581,14 @@ cudaError_t bvh_build_device(const yc_triangle* tris_dev, int n, int bins, int l
     const int cnt = b - a;
     BB_CHECK(hist.need((size_t)cnt * bins, s)); BB_CHECK(child_of.need(cnt, s)); BB_CHECK(child_box.need(2 * (size_t)cnt, s));
     const int gn = (cnt + BB_TB - 1) / BB_TB;
-    k_level_clear<<<gn, BB_TB, 0, s>>>(work.p, hist.p, a, b, bins);
+    if (bins > 2) BB_CHECK(cudaMemsetAsync(hist.p, 0, (size_t)cnt * bins * sizeof(int), s));   // (else no bins are counted)
     k_bounds<<<gp, BB_TB, 0, s>>>(perm.p, pnode.p, lo.p, hi.p, work.p, n, a, b, leaf_max);
     k_hist<<<gp, BB_TB, 0, s>>>(perm.p, pnode.p, cen.p, nodes.p, work.p, hist.p, n, a, b, bins, leaf_max);
     k_decide<<<gn, BB_TB, 0, s>>>(perm.p, nodes.p, work.p, hist.p, child_box.p, a, b, bins, leaf_max);
-    {   // child slots in node order: an exclusive scan of the split flags
+    // child slots in node order: an exclusive scan of the split flags
+    if (cnt <= SLOTS_ONE) {
+      k_slots_small<<<1, 1024, 0, s>>>(work.p, a, cnt, child_of.p, total.p);
+    } else {
       const int ct = (cnt + 1023) / 1024;
       BB_CHECK(nflag.need(cnt, s)); BB_CHECK(ntile.need(ct, s));
       k_split_flags<<<gn, BB_TB, 0, s>>>(work.p, nflag.p, a, b);
@@ -529,12 +603,10 @@ cudaError_t bvh_build_device(const yc_triangle* tris_dev, int n, int bins, int l
     const int next = b;
     BB_CHECK(nodes.need((size_t)b + 2 * splits, s, true));
     BB_CHECK(work.need((size_t)b + 2 * splits, s, true));
-    k_flags<<<gp, BB_TB, 0, s>>>(perm.p, pnode.p, cen.p, work.p, child_box.p, flag.p, n, a, b);
-    k_scan_tiles<<<ntiles, 1024, 0, s>>>(flag.p, pos.p, tiles.p, n);
+    k_flag_tiles<<<ntiles, 1024, 0, s>>>(perm.p, pnode.p, cen.p, work.p, child_box.p, pos.p, tiles.p, n, a, b);
     k_scan_sums<<<1, 1024, 0, s>>>(tiles.p, ntiles);
-    k_scan_add<<<ntiles, 1024, 0, s>>>(pos.p, tiles.p, n);
-    k_children<<<gn, BB_TB, 0, s>>>(nodes.p, work.p, child_box.p, child_of.p, pos.p, flag.p, a, b, next);
-    k_scatter<<<gp, BB_TB, 0, s>>>(perm.p, pnode.p, work.p, nodes.p, pos.p, flag.p, perm2.p, pnode2.p, n, a, b);
+    k_children<<<gn, BB_TB, 0, s>>>(nodes.p, work.p, child_box.p, child_of.p, pos.p, tiles.p, a, b, next);
+    k_scatter<<<gp, BB_TB, 0, s>>>(perm.p, pnode.p, work.p, nodes.p, pos.p, tiles.p, perm2.p, pnode2.p, n, a, b);
     std::swap(perm.p, perm2.p);
     std::swap(pnode.p, pnode2.p);
     BB_CHECK(cudaPeekAtLastError());
