@@ -15,13 +15,13 @@
 //            scan for a stable partition of every node's segment
 //   children the splitting nodes' children
 //   scatter  primitives into their children's segments
-// A level of a few thousand nodes is bound by its launches and the readback of its splits, so
-// each kernel does what the next would otherwise be launched for, and the buffers start with room
-// for the usual tree (with 14 launches a level, and the buffers grown as the tree grew, 330K
-// triangles took 9.26 ms and 3K 1.92 ms, now 6.17 and 1.19, copies included);
 // then a refit over the levels in reverse. The only liberty taken: a box bound that is
 // zero is stored as +0 (atomics cannot keep "the first of -0 and +0 met", which the
 // sequential builder does); the traversal's arithmetic is the same for either zero.
+// A level of a few thousand nodes is bound by its launches and the readback of its splits, so
+// each kernel does what the next would otherwise be launched for, and the buffers start with room
+// for the usual tree (with 14 launches a level, and the buffers grown as the tree grew, 330K
+// triangles took 9.26 ms and 3K 1.92 ms, now 6.17 and 1.19, copies included).
 #include <climits>
 #include <cuda_runtime.h>
 
