@@ -218,7 +218,7 @@ int yc_render_passes(yc_ctx* ctx, int scene_id, int accum_id, const uint32_t* ra
  * stall the frame, or a host whose device memory belongs to its own allocator and that
  * forbids driver allocations after start-up. yc_render_pass sizes its wavefront state
  * to the image on first use; this call keeps that state in a static device array of the
- * library (about 3.9 MB, held by every GPU that loads the library until exit) and so
+ * library (about 4.1 MB, held by every GPU that loads the library until exit) and so
  * renders one tile of at most 16384 pixels (cfg->block / block_x / block_y select it,
  * as for yc_render_pass) with no allocation. The scene and accumulator come from
  * yc_upload_scene / yc_alloc_accum, made beforehand. A larger tile is rejected with

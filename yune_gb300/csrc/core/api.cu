@@ -789,7 +789,7 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
     if (r < 0) return fail(r == -2 ? YC_E_NOMEM : YC_E_LAUNCH, err);
     if (dev.bad_tri < n_tri) return fail(YC_E_INVALID, "triangle " + std::to_string(dev.bad_tri) + " has matID out of range");
     on_device = r && dev.n_leaf >= 2 && dev.slots < (size_t)(1 << 27);
-    if (!on_device) {   // an array the host has to judge
+    if (!on_device) {   // an array for the host to decide about
       on_device = yc::plan_device_repack(nodes, n_node, n_tri, plan, err);
       if (on_device < 0) return fail(YC_E_INVALID, err);
       dev.slots = plan.slots;
