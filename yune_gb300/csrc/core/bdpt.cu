@@ -473,7 +473,7 @@ __device__ __forceinline__ int bdpt_step(const PassParams& pp, const PathState& 
   return emit == 2 ? EMIT_WAIT | (((1 << out.n) - 1) * EMIT_SEG0) : emit;
 }
 
-__global__ void __launch_bounds__(256) k_logic_bdpt(PassParams pp, PathState ps, BdptBuffers bb,
+__global__ void __launch_bounds__(256, 2) k_logic_bdpt(PassParams pp, PathState ps, BdptBuffers bb,
                                                     const int* __restrict__ in_closest, const int* __restrict__ in_wait,
                                                     const RoundCounters* rc_in, int* out_closest, int* out_wait,
                                                     RoundCounters* rc_out, DevStats* st, const int* __restrict__ sorted,

@@ -72,8 +72,10 @@ void launch_raygen_next(const PassParams& pp, const PathState& ps, int* q_closes
   k_raygen_next<<<grid, 256, 0, s>>>(pp, ps, q_closest, rc, st);
 }
 
+// Two blocks per SM: with 129 registers or more, which the compiler otherwise takes for some forms of
+// the step, one block is left and the shading takes 1.4 times as long.
 template <bool TOGETHER, bool MULTI>
-__global__ void __launch_bounds__(LOGIC_TB) k_logic(PassParams pp, PathState ps, const int* __restrict__ in_closest,
+__global__ void __launch_bounds__(LOGIC_TB, 2) k_logic(PassParams pp, PathState ps, const int* __restrict__ in_closest,
                                                     const int* __restrict__ in_wait, const RoundCounters* rc_in,
                                                     int* out_closest, int* out_wait, int* q_any,
                                                     RoundCounters* rc_out,
