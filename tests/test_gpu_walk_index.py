@@ -121,3 +121,21 @@ def test_batch_with_a_scene_that_has_no_index(r, when):
         r.render_passes(sid, ref, seeds, cfg=s.cfg)
         assert np.array_equal(r.read_accum(aid).view(np.int32), r.read_accum(ref).view(np.int32))
     b.close()
+
+
+# Any-hit lists take their steps lane by lane or by vote, spread over half the warps or not, by
+# the list's length and the scene's size: the same answers and distances whatever the list.
+@pytest.mark.parametrize("tris", [0, 1000, 90000])
+@pytest.mark.parametrize("n", [100, 30000, 60000, 262144, 300001])
+def test_any_hit_lists_of_every_length(r, tris, n):
+    s = workloads.mixed_scene(tris, 4, 32, 32, 1) if tris else scenes.c0(32, 32)
+    sid = r.upload(s)
+    rays = _rays(n, -1.0, 1.0, seed=n)
+    tri, light, t = r.trace(sid, rays, any_hit=True)
+    for k in range(0, n, 4096):
+        if n > 60000 and (k // 4096) % 9:
+            continue
+        a, b, c = r.trace(sid, rays[k:k + 4096], any_hit=True)
+        assert np.array_equal(a, tri[k:k + 4096]) and np.array_equal(b, light[k:k + 4096])
+        assert np.array_equal(c.view(np.int32), t[k:k + 4096].view(np.int32))
+    r.release(sid)

@@ -10,6 +10,8 @@
 // the stack is counted in DevStats::stack_overflow instead of writing out of bounds.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "yc_internal.h"
 #include "yc_shade.cuh"
 #include "yc_trace_loop.cuh"
@@ -180,33 +182,47 @@ int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_an
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-// Any-hit queries over two-child nodes take their steps lane by lane where a walk is a few
-// leaves (TINY_SCENE) or the list leaves most lanes of the launch idle: 1,172 segments through
-// the 82K-triangle glass sphere 43.8 us against 49.5 us voted, 20,000 98.8 against 106.3, a
-// million 367 against 315; a million through the 34 triangles of the Cornell box 149 against
-// 162 us.
-constexpr int TINY_SCENE = 512;        // triangles
-constexpr int SHORT_LIST = 1 << 16;    // rays, less than half of the lanes of eight blocks on each of 152 SMs
+// Any-hit queries over two-child nodes take their steps lane by lane, the whole stack in shared
+// memory, except long lists in large scenes, whose steps are voted. Lane by lane / voted, us:
+//   triangles     4,096 rays   100,000     300,000        1M
+//   34             19 / 21     33 / 34     52 / 58     135 / 161
+//   1,000          32 / 38     46 / 53     67 / 75     148 / 170
+//   10,000         45 / 53     80 / 88    118 / 119    273 / 264
+//   30,000         44 / 53     89 / 94    117 / 124    266 / 273
+//   81,954         63 / 74    115 / 122   167 / 163    346 / 315
+//   300,000        72 / 90    135 / 148   186 / 185    407 / 381
+// (Bound by lanes: 3-8 of 32 by lane, but with a third fewer instructions a step.)
+constexpr int VOTE_SCENE = 1 << 16;    // triangles and
+constexpr int VOTE_LIST = 1 << 18;     // segments from which the steps are voted
+constexpr int LANE_STACK = 46;         // entries of a stack at most
 
+static bool lane_steps(const DevScene& sc, bool any_hit, int n) {
+  return any_hit && !sc.wide && stack_cap_for(sc.depth) <= LANE_STACK && (sc.n_tri < VOTE_SCENE || n < VOTE_LIST);
+}
 using RaysKernel = void (*)(DevScene, const float*, int, int*, int*, float*, int, DevStats*, int, int*);
 static RaysKernel rays_kernel(const DevScene& sc, bool any_hit, int n) {
   if (!any_hit) return sc.wide ? k_trace_rays<false, true, false> : k_trace_rays<false, false, false>;
   if (sc.wide) return k_trace_rays<true, true, false>;
-  return sc.n_tri < TINY_SCENE || n < SHORT_LIST ? k_trace_rays<true, false, true> : k_trace_rays<true, false, false>;
+  return lane_steps(sc, any_hit, n) ? k_trace_rays<true, false, true> : k_trace_rays<true, false, false>;
+}
+static int rays_smem_entries(const DevScene& sc, bool any_hit, int n, int n_smem) {
+  const int cap = stack_cap_for(sc.depth);
+  return n_smem > 0 && n_smem < cap && !lane_steps(sc, any_hit, n) ? n_smem : cap;
 }
 
 int trace_rays_grid_blocks(const DevScene& sc, bool any_hit, int n, int n_smem) {
-  const int cap = stack_cap_for(sc.depth);
-  return resident_grid(rays_kernel(sc, any_hit, n), smem_for(n_smem > 0 && n_smem < cap ? n_smem : cap));
+  const int grid = resident_grid(rays_kernel(sc, any_hit, n), smem_for(rays_smem_entries(sc, any_hit, n, n_smem)));
+  // (lists of one ray or two a lane: eight blocks per SM, not nine, share them out better, 1,000
+  // triangles and 100,000 rays 47.3 -> 45.8 us; longer ones gain from the ninth, 152 -> 148 for 1M)
+  const bool short_list = n < (sc.n_tri < 4096 ? 1 << 19 : 1 << 17);
+  return lane_steps(sc, any_hit, n) && short_list && grid > 0 ? std::min(grid, 8 * g_sm_count) : grid;
 }
 
 int launch_trace_rays(const DevScene& sc, bool any_hit, const float* rays9, int n, int* tri_out, float* t_out,
                       int* work, DevStats* st, int grid, cudaStream_t s, int n_smem, int* spill) {
-  const int cap = stack_cap_for(sc.depth);
-  if (!(n_smem > 0 && n_smem < cap && spill)) n_smem = cap;
-  const size_t smem = smem_for(n_smem);
-  const RaysKernel kernel = rays_kernel(sc, any_hit, n);
-  kernel<<<grid, TRACE_TB, smem, s>>>(sc, rays9, n, work, tri_out, t_out, cap, st, n_smem, spill);
+  n_smem = rays_smem_entries(sc, any_hit, n, spill ? n_smem : 0);
+  rays_kernel(sc, any_hit, n)<<<grid, TRACE_TB, smem_for(n_smem), s>>>(sc, rays9, n, work, tri_out, t_out,
+                                                                       stack_cap_for(sc.depth), st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

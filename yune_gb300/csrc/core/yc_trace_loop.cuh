@@ -74,11 +74,13 @@ __device__ __forceinline__ WalkStack thread_stack(int stack_cap, int n_smem, int
 
 // The persistent loop shared by the kernels. Src supplies ray e of the work list and the
 // scene it walks (begin) and stores its result (end). Each thread's stack is thread_stack.
-// LANE: every lane takes its own steps (lane_walk_step) instead of voted ones.
+// LANE (any-hit rays): every lane takes its own steps (any_walk_step) instead of voted ones.
 template <bool ANY, bool WIDE, bool LANE, class Src>
 __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack_cap, DevStats* st,
                                            int n_smem = 1 << 30, int* spill = nullptr) {
+  static_assert(ANY || !LANE, "lane steps are for any-hit rays");
   const WalkStack stack = thread_stack(stack_cap, n_smem, spill);
+  const WholeStack whole{stack.s, stack.stride, stack_cap};   // (LANE: the launch has room for it)
   const int lane = threadIdx.x & 31;
   unsigned long long overflow = 0;
   WalkCount wc;
@@ -93,7 +95,9 @@ __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack
   // there need be (1,172 closest-hit rays through a 300K-triangle scene 147 -> 58 us, 20,000
   // 188 -> 114 us, index included).
   const int warps = (int)(gridDim.x * blockDim.x) >> 6;   // half of them
-  const int quota = min(32, max(1, (n + warps - 1) / warps));
+  // (Lane by lane only below half of that: 50,000 any-hit rays through 34 triangles 30.1 -> 27.6 us.)
+  const int even = min(32, max(1, (n + warps - 1) / warps));
+  const int quota = LANE && even > 16 ? 32 : even;
   const unsigned takers = 0xffffffffu >> (32 - quota);   // the lanes that take rays
   const int refill = quota < 32 ? (quota + 1) / 2 : REFILL_AT;
   auto finish = [&]() {   // hands over the result of this lane's ray
@@ -127,14 +131,11 @@ __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack
         walk_begin(sc, r, w);
         ++rays;
       }
-      continue;
+      if (!LANE) continue;
     }
     bool of = false;
     if (LANE) {
-      if (e_cur >= 0) {
-        lane_walk_step<WIDE>(w, ANY, stack, wc, of);
-        if (!walk_wants_node(w) && !walk_wants_tri(w)) finish();
-      }
+      if (e_cur >= 0 && any_walk_step<WIDE>(w, whole, wc, of)) finish();
     } else {
       warp_walk_step<WIDE>(w, ANY, stack, wc, of, nodes, tris);
     }

@@ -267,6 +267,14 @@ struct WalkStack {
   }
 };
 
+// the same with the whole stack in shared memory
+struct WholeStack {
+  int2* s;
+  int stride, cap;
+  __device__ __forceinline__ void put(int i, int link, float t) const { s[i * stride] = make_int2(link, __float_as_int(t)); }
+  __device__ __forceinline__ int2 at(int i) const { return s[i * stride]; }
+};
+
 // The link of a walk that has to take its next subtree from the stack. Popping is left to
 // the next node step, so that a step has one place where lanes pop, together.
 constexpr int LINK_POP = LINK_NONE - 1;
@@ -283,7 +291,8 @@ __device__ __forceinline__ void load32(const float4* p, ulonglong2& a, ulonglong
 // One interior node of the two-child layout: returns the next node (the nearer child
 // hit, the other one pushed), or pop_link when neither child is hit. LINK_NONE: nothing
 // left to open (or the stack bound was reached).
-__device__ __forceinline__ int visit2(Walk& w, bool any, int link, const WalkStack& st, WalkCount& wc,
+template <class Stack>
+__device__ __forceinline__ int visit2(Walk& w, bool any, int link, const Stack& st, WalkCount& wc,
                                       bool& overflow) {
   const float4* nd = w.nodes + 4 * (size_t)link;
   ulonglong2 nx, ny, nz, links;   // (lo pair, hi pair) of an axis
@@ -338,7 +347,8 @@ __device__ __forceinline__ void cx(float& ta, int& la, float& tb, int& lb) {
 // operation, the hits sorted by entry distance, the nearest returned and the others
 // pushed farthest first (pushed in any order, the walk visited more nodes: 3.97 against
 // 3.59 ms per 1080p pass of a 260K-triangle scene).
-__device__ __forceinline__ int visit4(Walk& w, bool any, int link, const WalkStack& st, WalkCount& wc,
+template <class Stack>
+__device__ __forceinline__ int visit4(Walk& w, bool any, int link, const Stack& st, WalkCount& wc,
                                       bool& overflow) {
   const float INF = __int_as_float(0x7f800000);
   const float4* nd = w.nodes + 8 * (size_t)link;
@@ -476,16 +486,48 @@ __device__ __forceinline__ void warp_walk_step(Walk& w, bool any, const WalkStac
   }
 }
 
-// The while-while loop of Aila and Laine without a vote: every lane with a step to take opens
-// nodes until each of them has a leaf, then tests its leaf's triangles. Any-hit queries use
-// it where the votes cost more than the lanes they bring together (trace.cu, rays_by_lane).
-template <bool WIDE>
-__device__ __forceinline__ void lane_walk_step(Walk& w, bool any, const WalkStack& st, WalkCount& wc, bool& overflow) {
-  while (walk_wants_node(w)) {
-    walk_node_step<WIDE>(w, any, st, wc, overflow);
-    if (!__any_sync(__activemask(), !walk_wants_tri(w))) break;
+// The while-while loop of Aila and Laine without a vote, for any-hit rays: every lane opens nodes
+// until each of them has a leaf, then tests its leaves' triangles; true when the walk has ended.
+// Such a walk keeps its segment's length until it stops, so no entry distance is looked at again.
+// Any-hit queries use it where the votes cost more than the lanes they bring together (trace.cu).
+template <bool WIDE, class Stack>
+__device__ __forceinline__ bool any_walk_step(Walk& w, const Stack& st, WalkCount& wc, bool& overflow) {
+  const auto pop = [&] { return w.sp > 0 ? st.at(--w.sp).x : LINK_NONE; };
+  int link = w.link, leaf = w.leaf;
+  w.leaf = 0;
+  while (link >= 0 && link != LINK_NONE) {
+    link = WIDE ? visit4(w, true, link, st, wc, overflow) : visit2(w, true, link, st, wc, overflow);
+    if (link == LINK_POP) link = pop();
+    if (link < 0 && leaf == 0) {
+      leaf = ~link;
+      link = pop();
+    }
+    if (!__any_sync(__activemask(), leaf == 0)) break;
   }
-  while (walk_wants_tri(w)) walk_leaf(w, any, wc);
+  while (leaf != 0) {
+    const float4* tp = w.tris + 3 * (size_t)(leaf >> 4);
+    int left = leaf & 15;
+    do {
+      const float4 a = __ldg(tp + 0), b = __ldg(tp + 1), c = __ldg(tp + 2);
+      tp += 3;
+      ++wc.tris;
+      TriHit th;
+      if (tri_test(w.ox(), w.oy(), w.oz(), w.dx, w.dy, w.dz, a, b, c, w.best, w.best_rank, th)) {
+        w.best = th.t;
+        w.bu = th.u;
+        w.bv = th.v;
+        w.best_tri = __float_as_int(a.w);
+        return true;
+      }
+    } while (--left);
+    leaf = 0;
+    if (link < 0) {   // a second leaf met on the way
+      leaf = ~link;
+      link = pop();
+    }
+  }
+  w.link = link;
+  return link == LINK_NONE;
 }
 
 }  // namespace yc
