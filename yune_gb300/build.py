@@ -28,15 +28,16 @@ CU_SOURCES = ["core/api.cu", "core/trace.cu", "core/udpt.cu", "core/bench_kernel
               "core/repack_dev.cu", "core/widen.cu"]
 CXX_SOURCES = ["core/repack.cpp", "core/serve.cpp", "core/walk_host.cpp", "core/tune.cpp", "host/yh_bvh.cpp", "host/yh_camera.cpp", "host/yh_scene.cpp", "host/yh_image.cpp",
                "host/yh_cache.cpp", "host/yh_threads.cpp"]
-HEADERS = ["ym_math.h", "core/yc_scene.h", "core/yc_internal.h", "core/yc_traverse.cuh", "core/yc_shade.cuh",
-           "core/yc_repack.h", "core/yc_noalloc.h", "core/yc_bdpt.h", "core/yc_udpt.cuh",
-           "core/yc_trace_loop.cuh", "core/yc_engine.h", "core/yc_sah.h", "host/yh_threads.h"]
 
 
 def _deps():
-    out = [os.path.join(CSRC, h) for h in HEADERS]
-    out += [os.path.join(ROOT, "include", h) for h in ("yune_types.h", "yune_cuda.h", "yune_host.h")]
-    return [p for p in out if os.path.exists(p)]
+    """Every header: a unit is compiled again when any of them changes (a list kept by hand falls
+    behind the includes)."""
+    found = []
+    for top in (CSRC, os.path.join(ROOT, "include")):
+        for d, _, names in os.walk(top):
+            found += [os.path.join(d, n) for n in names if n.endswith((".h", ".cuh"))]
+    return sorted(found)
 
 
 def _obj(src):
