@@ -1,0 +1,60 @@
+"""A call that the device's memory does not hold fails with YC_E_NOMEM and leaves the context as
+usable as before: the buffers that it gave up are made again by the next call that needs them."""
+import numpy as np
+import pytest
+
+import fake_cuda
+from yune_gb300 import _native as N
+from yune_gb300 import scenes, workloads
+from yune_gb300.core import Renderer
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    return fake_cuda.load(tmp_path_factory.mktemp("fake_cuda"))
+
+
+@pytest.fixture
+def r(fake, monkeypatch):
+    monkeypatch.setattr(N, "_lib", fake)
+    fake.fake_limit(fake_cuda.NO_LIMIT)
+    with Renderer(0) as rr:
+        yield rr
+    fake.fake_limit(fake_cuda.NO_LIMIT)
+    assert fake.fake_bytes() == 0   # everything was given back
+
+
+@pytest.mark.parametrize("integrator", [0, 1, 2])
+@pytest.mark.parametrize("tris", [0, 5000])   # 5000: the rays are sorted
+def test_small_frame_after_a_frame_too_large(r, fake, integrator, tris):
+    s = workloads.mixed_scene(tris, 5, 16, 16, 1) if tris else scenes.c0(16, 16)
+    cfg = scenes.default_cfg(integrator=integrator, bdpt_bounces=4)
+    r.set_camera(s.cam)
+
+    def frames(q):
+        q.set_repack(0)   # (on the host: kernels do not run here)
+        sid, small, large = q.upload(s), q.alloc_accum(320, 256), q.alloc_accum(1024, 1024)
+        q.set_camera(s.cam)
+        q.render_passes(sid, small, [1, 2], reset_first=1, cfg=cfg)
+        return sid, small, large
+
+    sid, small, large = frames(r)
+    held = fake.fake_bytes()
+    r.render_passes(sid, large, [1, 2], reset_first=1, cfg=cfg)
+    need = fake.fake_bytes() - held
+    r.close()
+    failed = 0
+    for share in range(20):   # memory ends at one allocation after another
+        with Renderer(0) as q:
+            sid, small, large = frames(q)
+            buffers = fake.fake_allocations()
+            fake.fake_limit(fake.fake_bytes() + need * share // 20)
+            try:
+                q.render_passes(sid, large, [1, 2], reset_first=1, cfg=cfg)
+            except N.YuneError as e:
+                assert e.code == N.YC_E_NOMEM
+                failed += 1
+            fake.fake_limit(fake_cuda.NO_LIMIT)
+            q.render_passes(sid, small, [1, 2], reset_first=1, cfg=cfg)
+            assert fake.fake_allocations() >= buffers   # whichever of them had to go
+    assert failed >= 5

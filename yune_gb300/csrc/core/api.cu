@@ -29,6 +29,7 @@ std::atomic<unsigned long long> g_device_allocs{0};
 
 int fail(int code, const std::string& msg) {
   g_last_error = msg;
+  if (code == YC_E_NOMEM) cudaGetLastError();   // (else the next launch's check would find it)
   return code;
 }
 
@@ -71,6 +72,8 @@ struct DevBuf {
     else p = nullptr;
     return e;
   }
+  // room for count elements, whatever they held (nothing after a failure)
+  cudaError_t need(size_t count) { return count <= n ? cudaSuccess : alloc(count); }
   size_t bytes() const { return n * sizeof(T); }
 };
 
@@ -152,14 +155,11 @@ struct yc_ctx {
   int ss_threshold = 65536;       // YC_OPT_SHADE_SORT_MIN: per-pass shade queues this long are sorted
   DevBuf<int> ss_keys, ss_sorted;
   DevBuf<yc::SortCtl> ss_ctl;
-  size_t ss_cap = 0;
   // ray sort of the per-pass path (raysort.cu)
   DevBuf<unsigned> rs_keys, rs_hist, rs_cursor, rs_blk;
   DevBuf<int> rs_sorted;
   DevBuf<yc::RaySortCtl> rs_ctl;
-  size_t rs_cap = 0;
   // wavefront buffers, sized for the largest image seen
-  size_t cap_paths = 0;
   DevBuf<float4> rec;                // path records, PS_STRIDE float4 per slot
   DevBuf<int> q[4];                  // closest/waiting for two rounds
   DevBuf<int> q_any;                 // a round's any-hit rays
@@ -185,11 +185,10 @@ struct yc_ctx {
   yc_kernel_times ktimes{};
   DevBuf<char> flush_buf;
   // BDPT subpath vertices
-  DevBuf<float4> bd_lv, bd_ev, bd_seg;
+  DevBuf<float4> bd_lv, bd_ev, bd_seg;   // (the MIS tracer has no eye records)
   DevBuf<int> bd_q_any;
   int bd_shift = yc::FAN_SHIFT;       // segments a path sends at once, for frames of bd_paths paths (log2)
   size_t bd_paths = 0;
-  size_t bd_cap = 0, bd_ev_cap = 0;   // light / eye vertex records (the MIS tracer has no eye records)
   // direct queries
   DevBuf<float> q_rays;
   DevBuf<int> q_hits;         // triangle indices, then t
@@ -199,12 +198,12 @@ struct yc_ctx {
 
 namespace {
 
+// (A buffer's own size says whether it is there: an allocation that fails has released what the
+// buffer held.)
 int ensure_paths(yc_ctx* c, size_t n) {
-  if (n <= c->cap_paths) return 0;
-  YC_CUDA(c->rec.alloc(n * yc::PS_STRIDE));
-  for (auto& b : c->q) YC_CUDA(b.alloc(n));
-  YC_CUDA(c->q_any.alloc(2 * n));
-  c->cap_paths = n;
+  YC_CUDA(c->rec.need(n * yc::PS_STRIDE));
+  for (auto& b : c->q) YC_CUDA(b.need(n));
+  YC_CUDA(c->q_any.need(2 * n));
   return 0;
 }
 
@@ -250,13 +249,13 @@ uint64_t layout_digest(const float4* nodes, size_t n_nodes, const float4* tris, 
 
 // the per-pass walks' stack spill area: n ints
 int ensure_pass_spill(yc_ctx* c, size_t n) {
-  if (n > c->pass_spill.n) YC_CUDA(c->pass_spill.alloc(n));
+  YC_CUDA(c->pass_spill.need(n));
   return 0;
 }
 
 // key, histogram and sorted-list buffers of the per-pass ray sort, for n rays
 int ensure_raysort(yc_ctx* c, size_t n) {
-  if (!c->rs_hist.p) {
+  if (!c->rs_ctl.p) {
     const size_t bins = (size_t)yc::raysort_bins(3, 2);   // the largest key allowed (16 bits)
     YC_CUDA(c->rs_hist.alloc(bins));
     YC_CUDA(c->rs_cursor.alloc(bins));
@@ -265,11 +264,8 @@ int ensure_raysort(yc_ctx* c, size_t n) {
     YC_CUDA(cudaMemsetAsync(c->rs_hist.p, 0, c->rs_hist.bytes(), c->stream));
     YC_CUDA(cudaMemsetAsync(c->rs_ctl.p, 0, sizeof(yc::RaySortCtl), c->stream));
   }
-  if (n > c->rs_cap) {
-    YC_CUDA(c->rs_keys.alloc(n));
-    YC_CUDA(c->rs_sorted.alloc(n));
-    c->rs_cap = n;
-  }
+  YC_CUDA(c->rs_keys.need(n));
+  YC_CUDA(c->rs_sorted.need(n));
   return 0;
 }
 
@@ -281,14 +277,10 @@ int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
     const size_t m = n << shift;
     if (shift > 0 && m > ((size_t)1 << 30)) continue;
     cudaError_t e = cudaSuccess;
-    if (c->bd_seg.n < m) e = c->bd_seg.alloc(m);
-    if (e == cudaSuccess && c->bd_q_any.n < m) e = c->bd_q_any.alloc(m);
-    if (e == cudaSuccess && raysort && c->rs_cap < m) {
-      c->rs_cap = 0;
-      e = c->rs_keys.alloc(m);
-      if (e == cudaSuccess) e = c->rs_sorted.alloc(m);
-      if (e == cudaSuccess) c->rs_cap = m;
-    }
+    e = c->bd_seg.need(m);
+    if (e == cudaSuccess) e = c->bd_q_any.need(m);
+    if (e == cudaSuccess && raysort) e = c->rs_keys.need(m);
+    if (e == cudaSuccess && raysort) e = c->rs_sorted.need(m);
     if (e == cudaSuccess) {
       c->bd_shift = shift;
       c->bd_paths = n;
@@ -306,11 +298,8 @@ int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
 // key and sorted-list buffers of the per-pass shade-queue sort, for n paths
 int ensure_shadesort(yc_ctx* c, size_t n) {
   if (!c->ss_ctl.p) YC_CUDA(c->ss_ctl.alloc(1));
-  if (n > c->ss_cap) {
-    YC_CUDA(c->ss_keys.alloc(n));
-    YC_CUDA(c->ss_sorted.alloc(n));
-    c->ss_cap = n;
-  }
+  YC_CUDA(c->ss_keys.need(n));
+  YC_CUDA(c->ss_sorted.need(n));
   return 0;
 }
 
@@ -499,8 +488,8 @@ int run_passes(yc_ctx* c, Scene* sc, Accum* ac, const uint32_t* rands, int n_pas
   yc::PassParams pp = pass_params(c, sc, ac, rands[0], reset, gi_check, cfg, mixed);
   pp.n_pass = n_pass;
   if (n_pass > 1) {
-    if (c->q_restart.n < (size_t)W * H) YC_CUDA(c->q_restart.alloc((size_t)W * H));
-    if (c->seeds.n < (size_t)n_pass) YC_CUDA(c->seeds.alloc(n_pass));
+    YC_CUDA(c->q_restart.need((size_t)W * H));
+    YC_CUDA(c->seeds.need(n_pass));
     YC_CUDA(cudaMemcpyAsync(c->seeds.p, rands, n_pass * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
     pp.seeds = c->seeds.p;
     pp.q_restart = c->q_restart.p;
@@ -510,14 +499,8 @@ int run_passes(yc_ctx* c, Scene* sc, Accum* ac, const uint32_t* rands, int n_pas
   yc::BdptBuffers bb{};
   if (bdpt) {
     const size_t need = (size_t)W * H * 4 * cfg->bdpt_bounces;
-    if (c->bd_cap < need) {
-      YC_CUDA(c->bd_lv.alloc(need));
-      c->bd_cap = need;
-    }
-    if (!bdpt_mis && c->bd_ev_cap < need) {
-      YC_CUDA(c->bd_ev.alloc(need));
-      c->bd_ev_cap = need;
-    }
+    YC_CUDA(c->bd_lv.need(need));
+    if (!bdpt_mis) YC_CUDA(c->bd_ev.need(need));
     bb.lv = c->bd_lv.p;
     bb.ev = c->bd_ev.p;
     bb.N = (size_t)W * H;
@@ -1262,8 +1245,8 @@ int yc_trace(yc_ctx* c, int scene_id, const float* rays, int n, int any_hit, int
   // the device buffers, and for lists of up to kTraceStage rays page-locked memory that takes
   // both results in one copy, are kept from call to call (three allocations, their releases
   // and a copy each were 45 of the 74 us that 4,096 segments through the Cornell box took)
-  if (c->q_rays.n < (size_t)n * 9) YC_CUDA(c->q_rays.alloc((size_t)n * 9));
-  if (c->q_hits.n < 2 * (size_t)n) YC_CUDA(c->q_hits.alloc(2 * (size_t)n));
+  YC_CUDA(c->q_rays.need((size_t)n * 9));
+  YC_CUDA(c->q_hits.need(2 * (size_t)n));
   int* const tri_dev = c->q_hits.p;
   float* const t_dev = reinterpret_cast<float*>(c->q_hits.p + n);
   YC_CUDA(cudaMemcpyAsync(c->q_rays.p, rays, (size_t)n * 9 * sizeof(float), cudaMemcpyHostToDevice, c->stream));
@@ -1388,7 +1371,7 @@ int yc_get_kernel_times(yc_ctx* c, yc_kernel_times* out) {
 
 int yc_flush_l2(yc_ctx* c, size_t bytes) {
   if (!c) return fail(YC_E_INVALID, "ctx is NULL");
-  if (c->flush_buf.n < bytes) YC_CUDA(c->flush_buf.alloc(bytes));
+  YC_CUDA(c->flush_buf.need(bytes));
   YC_CUDA(cudaMemsetAsync(c->flush_buf.p, (int)(c->ktimes.rounds & 0xff), bytes, c->stream));
   return YC_OK;
 }
