@@ -6,6 +6,7 @@ import pytest
 import fake_cuda
 from yune_gb300 import _native as N
 from yune_gb300 import scenes, workloads
+from yune_gb300.batch import Batch
 from yune_gb300.core import Renderer
 
 
@@ -58,3 +59,33 @@ def test_small_frame_after_a_frame_too_large(r, fake, integrator, tris):
             q.render_passes(sid, small, [1, 2], reset_first=1, cfg=cfg)
             assert fake.fake_allocations() >= buffers   # whichever of them had to go
     assert failed >= 5
+
+
+def test_batch_without_memory_for_its_stacks(r, fake):
+    """The walks' spill areas are made when a batch runs and when its walks change to the scenes' own
+    nodes (a scene without an index joins it): no run goes ahead without them."""
+    r.set_repack(0)
+    s = workloads.mixed_scene(5000, 5, 16, 16, 1)
+    sid, aid = r.upload(s), r.alloc_accum(64, 64)
+    r.set_tree_mode(0)
+    plain = r.upload(s)
+    b = Batch(r, pool_paths=4096, stack_cap=64, stack_smem=2)
+    b.add_job(sid, aid, s.cam, [1], s.cfg)
+    made = fake.fake_allocations()
+    fake.fake_limit(fake.fake_bytes() + 4096)
+    with pytest.raises(N.YuneError) as e:
+        b.run(max_launches=1)
+    assert e.value.code == N.YC_E_NOMEM
+    fake.fake_limit(fake_cuda.NO_LIMIT)
+    b.run(max_launches=1)
+    running = fake.fake_allocations()
+    assert running > made
+    fake.fake_limit(1)
+    with pytest.raises(N.YuneError) as e:
+        b.add_job(plain, aid, s.cam, [1], s.cfg)
+    fake.fake_limit(fake_cuda.NO_LIMIT)
+    b.run(max_launches=1)
+    assert e.value.code == N.YC_E_NOMEM and fake.fake_allocations() >= running
+    b.add_job(plain, aid, s.cam, [1], s.cfg)
+    b.run(max_launches=1)
+    assert fake.fake_allocations() > running   # (the job's seeds)

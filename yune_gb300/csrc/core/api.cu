@@ -1464,6 +1464,8 @@ struct yc_batch {
   bool indexed = true;
   int walk_cap = 0, index_cap = 0;   // index_cap: the deepest index of the jobs so far, + 2
   std::vector<yc::DevScene> job_dev;   // each job's scene with its own nodes
+  bool shaped = false;       // the launch shapes and the spill areas are those of the nodes walked
+  bool jobs_stale = false;   // the device's jobs have other nodes than host_jobs
   bool walks_wide() const { return wide == 1 || indexed; }
   int grid_c = 0, grid_a = 0, grid_m = 0, logic_grid = 0;
   bool mixed = true;   // YC_OPT_MIXED_TRACE of the context when the batch was created
@@ -1591,7 +1593,8 @@ int batch_body(yc_batch* b, bool timed) {
   return 0;
 }
 
-// launch shapes and stack spill areas of the traversal kernels for the nodes they walk
+// launch shapes and stack spill areas of the traversal kernels for the nodes they walk; until it
+// has succeeded the batch does not run
 int batch_shape(yc_batch* b) {
   yc_ctx* c = b->ctx;
   const bool wide = b->walks_wide();
@@ -1610,27 +1613,35 @@ int batch_shape(yc_batch* b) {
   if (b->stack_smem < b->walk_cap) {
     const size_t threads = (size_t)std::max({b->grid_c, b->grid_a, b->grid_m}) * b->cfg.trace_block;
     b->spill_slot = threads * 2 * (size_t)(b->walk_cap - b->stack_smem);
-    for (auto& g : b->groups) YC_CUDA(g->spill.alloc(2 * b->spill_slot));
+    for (auto& g : b->groups) YC_CUDA(g->spill.need(2 * b->spill_slot));
   }
+  if (b->jobs_stale && !b->host_jobs.empty()) {
+    YC_CUDA(cudaMemcpyAsync(b->jobs.p, b->host_jobs.data(), b->host_jobs.size() * sizeof(yc::BatchJob),
+                            cudaMemcpyHostToDevice, c->stream));
+    YC_CUDA(cudaStreamSynchronize(c->stream));
+  }
+  b->jobs_stale = false;
+  b->shaped = true;
   return 0;
+}
+
+// the next run shapes its launches anew
+void batch_reshape(yc_batch* b) {
+  b->shaped = false;
+  if (b->exec) cudaGraphExecDestroy(b->exec);
+  if (b->graph) cudaGraphDestroy(b->graph);
+  b->exec = nullptr;
+  b->graph = nullptr;
 }
 
 // From here on the batch walks its scenes' own nodes: a scene without an index was added, one
 // deeper than the stacks of a running batch hold, or one that stack_cap does not hold. Called
 // between launches.
-int batch_unindex(yc_batch* b) {
-  yc_ctx* c = b->ctx;
+void batch_unindex(yc_batch* b) {
   b->indexed = false;
   for (size_t i = 0; i < b->host_jobs.size(); ++i) b->host_jobs[i].pp.sc = b->job_dev[i];
-  if (!b->host_jobs.empty())
-    YC_CUDA(cudaMemcpyAsync(b->jobs.p, b->host_jobs.data(), b->host_jobs.size() * sizeof(yc::BatchJob),
-                            cudaMemcpyHostToDevice, c->stream));
-  YC_CUDA(cudaStreamSynchronize(c->stream));
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
-  b->exec = nullptr;
-  b->graph = nullptr;
-  return b->started ? batch_shape(b) : 0;
+  b->jobs_stale = true;
+  batch_reshape(b);
 }
 
 int batch_launch(yc_batch* b) {
@@ -1776,19 +1787,19 @@ int yc_batch_add_job(yc_batch* b, int scene_id, int accum_id, const yc_cam* cam,
   if (!b->started) b->stack_cap = std::max(b->stack_cap, b->cfg.stack_cap > 0 ? b->cfg.stack_cap : need_cap);
   else if (need_cap > b->stack_cap)
     return fail(YC_E_INVALID, "scene BVH deeper than the running batch's traversal stack");
+  std::unique_ptr<DevBuf<uint32_t>> sd(new DevBuf<uint32_t>);
+  YC_CUDA(sd->alloc(n_pass));
+  YC_CUDA(cudaMemcpyAsync(sd->p, seeds, n_pass * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
   if (b->indexed && sc->dev.wide == 0) {
     // (a scene without interior nodes is walked alike by both kernels)
     const bool has = sc->windex.p || sc->dev.root_link < 0 || sc->dev.root_link == yc::LINK_NONE;
     const int index_cap = sc->windex.p ? yc::trace_stack_cap(sc->windex_depth) : 0;
     if (!has || need_cap > b->stack_cap || (b->started && index_cap > b->walk_cap)) {
-      if (int r = batch_unindex(b)) return r;
+      batch_unindex(b);
     } else if (!b->started) {
       b->index_cap = std::max(b->index_cap, index_cap);
     }
   }
-  std::unique_ptr<DevBuf<uint32_t>> sd(new DevBuf<uint32_t>);
-  YC_CUDA(sd->alloc(n_pass));
-  YC_CUDA(cudaMemcpyAsync(sd->p, seeds, n_pass * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream));
   yc::BatchJob j{};
   j.pp.sc = b->indexed && sc->dev.wide == 0 ? walk_scene(*sc) : sc->dev;
   j.pp.cam = *cam;
@@ -1834,11 +1845,10 @@ int yc_batch_run(yc_batch* b, int max_launches, int* unfinished) {
   if (!b) return fail(YC_E_INVALID, "batch is NULL");
   yc_ctx* c = b->ctx;
   YC_CUDA(cudaSetDevice(c->device));
-  if (!b->started) {
-    if (b->stack_cap <= 0) b->stack_cap = b->cfg.stack_cap > 0 ? b->cfg.stack_cap : 32;
+  if (!b->started && b->stack_cap <= 0) b->stack_cap = b->cfg.stack_cap > 0 ? b->cfg.stack_cap : 32;
+  if (!b->shaped)
     if (int r = batch_shape(b)) return r;
-    b->started = true;
-  }
+  b->started = true;
   if (int r = begin_call_checks(c)) return r;
   YC_CUDA(cudaEventRecord(c->ev0, c->stream));
   int launches = 0;
