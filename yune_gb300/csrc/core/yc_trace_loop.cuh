@@ -74,11 +74,12 @@ __device__ __forceinline__ WalkStack thread_stack(int stack_cap, int n_smem, int
 
 // The persistent loop shared by the kernels. Src supplies ray e of the work list and the
 // scene it walks (begin) and stores its result (end). Each thread's stack is thread_stack.
-// LANE (any-hit rays): every lane takes its own steps (any_walk_step) instead of voted ones.
+// LANE (any-hit rays, two-child nodes): every lane takes its own steps (any_walk_step) instead of
+// voted ones.
 template <bool ANY, bool WIDE, bool LANE, class Src>
 __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack_cap, DevStats* st,
                                            int n_smem = 1 << 30, int* spill = nullptr) {
-  static_assert(ANY || !LANE, "lane steps are for any-hit rays");
+  static_assert((ANY && !WIDE) || !LANE, "lane steps are for any-hit rays over two-child nodes");
   const WalkStack stack = thread_stack(stack_cap, n_smem, spill);
   const WholeStack whole{stack.s, stack.stride, stack_cap};   // (LANE: the launch has room for it)
   const int lane = threadIdx.x & 31;
@@ -135,7 +136,7 @@ __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack
     }
     bool of = false;
     if (LANE) {
-      if (e_cur >= 0 && any_walk_step<WIDE>(w, whole, wc, of)) finish();
+      if (e_cur >= 0 && any_walk_step(w, whole, wc, of)) finish();
     } else {
       warp_walk_step<WIDE>(w, ANY, stack, wc, of, nodes, tris);
     }
