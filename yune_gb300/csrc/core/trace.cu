@@ -182,18 +182,18 @@ int launch_trace_mixed(const DevScene& sc, const int* q_closest, const int* q_an
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
-// Any-hit queries over two-child nodes take their steps lane by lane, the whole stack in shared
-// memory, except long lists in large scenes, whose steps are voted. Lane by lane / voted, us:
-//   triangles     4,096 rays   100,000     300,000        1M
-//   34             19 / 21     33 / 34     52 / 58     135 / 161
-//   1,000          32 / 38     46 / 53     67 / 75     148 / 170
-//   10,000         45 / 53     80 / 88    118 / 119    273 / 264
-//   30,000         44 / 53     89 / 94    117 / 124    266 / 273
-//   81,954         63 / 74    115 / 122   167 / 163    346 / 315
-//   300,000        72 / 90    135 / 148   186 / 185    407 / 381
+// Any-hit queries over two-child nodes take their steps lane by lane, their stacks of links in shared
+// memory, except the longest lists in large scenes, whose steps are voted. Lane by lane / voted, us:
+//   triangles     4,096 rays   100,000     300,000     600,000       1M
+//   34             19 / 20     33 / 34     53 / 58      87 / 99    135 / 161
+//   1,000          32 / 38     46 / 52     66 / 75      99 / 112   148 / 170
+//   10,000         44 / 53     77 / 87    116 / 119    179 / 183   266 / 264
+//   30,000         43 / 54     86 / 93    114 / 125    171 / 187   256 / 273
+//   81,954         62 / 74    111 / 122   163 / 163    226 / 219   325 / 315
+//   300,000        71 / 90    132 / 148   180 / 186    273 / 276   383 / 382
 // (Bound by lanes: 3-8 of 32 by lane, but with a third fewer instructions a step.)
 constexpr int VOTE_SCENE = 1 << 16;    // triangles and
-constexpr int VOTE_LIST = 1 << 18;     // segments from which the steps are voted
+constexpr int VOTE_LIST = 1 << 19;     // segments from which the steps are voted
 constexpr int LANE_STACK = 46;         // entries of a stack at most
 
 static bool lane_steps(const DevScene& sc, bool any_hit, int n) {
@@ -205,24 +205,31 @@ static RaysKernel rays_kernel(const DevScene& sc, bool any_hit, int n) {
   if (sc.wide) return k_trace_rays<true, true, false>;
   return lane_steps(sc, any_hit, n) ? k_trace_rays<true, false, true> : k_trace_rays<true, false, false>;
 }
-static int rays_smem_entries(const DevScene& sc, bool any_hit, int n, int n_smem) {
+static int rays_smem_entries(const DevScene& sc, int n_smem) {
   const int cap = stack_cap_for(sc.depth);
-  return n_smem > 0 && n_smem < cap && !lane_steps(sc, any_hit, n) ? n_smem : cap;
+  return n_smem > 0 && n_smem < cap ? n_smem : cap;
+}
+// lane by lane the whole stack lies in shared memory, a link an entry
+static size_t rays_smem(const DevScene& sc, bool any_hit, int n, int n_smem) {
+  if (lane_steps(sc, any_hit, n)) return (size_t)TRACE_TB * stack_cap_for(sc.depth) * sizeof(int);
+  return smem_for(rays_smem_entries(sc, n_smem));
 }
 
 int trace_rays_grid_blocks(const DevScene& sc, bool any_hit, int n, int n_smem) {
-  const int grid = resident_grid(rays_kernel(sc, any_hit, n), smem_for(rays_smem_entries(sc, any_hit, n, n_smem)));
-  // (lists of one ray or two a lane: eight blocks per SM, not nine, share them out better, 1,000
-  // triangles and 100,000 rays 47.3 -> 45.8 us; longer ones gain from the ninth, 152 -> 148 for 1M)
-  const bool short_list = n < (sc.n_tri < 4096 ? 1 << 19 : 1 << 17);
+  const int grid = resident_grid(rays_kernel(sc, any_hit, n), rays_smem(sc, any_hit, n, n_smem));
+  // (Lists that eight blocks per SM take at one ray a lane, and in scenes of short walks those of up
+  // to three, are shared out better by eight than by nine. Eight / nine, us: 1,000 triangles, 100,000
+  // rays 45.5 / 46.3, 300,000 66 / 67, 1M 150 / 147; 30,000 triangles, 150,000 rays 85 / 88, 200,000
+  // 101 / 99, 600,000 176 / 171.)
+  const bool short_list = n <= 8 * g_sm_count * TRACE_TB || (sc.n_tri < 4096 && n < 1 << 19);
   return lane_steps(sc, any_hit, n) && short_list && grid > 0 ? std::min(grid, 8 * g_sm_count) : grid;
 }
 
 int launch_trace_rays(const DevScene& sc, bool any_hit, const float* rays9, int n, int* tri_out, float* t_out,
                       int* work, DevStats* st, int grid, cudaStream_t s, int n_smem, int* spill) {
-  n_smem = rays_smem_entries(sc, any_hit, n, spill ? n_smem : 0);
-  rays_kernel(sc, any_hit, n)<<<grid, TRACE_TB, smem_for(n_smem), s>>>(sc, rays9, n, work, tri_out, t_out,
-                                                                       stack_cap_for(sc.depth), st, n_smem, spill);
+  n_smem = rays_smem_entries(sc, spill ? n_smem : 0);
+  rays_kernel(sc, any_hit, n)<<<grid, TRACE_TB, rays_smem(sc, any_hit, n, n_smem), s>>>(
+      sc, rays9, n, work, tri_out, t_out, stack_cap_for(sc.depth), st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -81,7 +81,7 @@ __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack
                                            int n_smem = 1 << 30, int* spill = nullptr) {
   static_assert((ANY && !WIDE) || !LANE, "lane steps are for any-hit rays over two-child nodes");
   const WalkStack stack = thread_stack(stack_cap, n_smem, spill);
-  const WholeStack whole{stack.s, stack.stride, stack_cap};   // (LANE: the launch has room for it)
+  const LinkStack links{reinterpret_cast<int*>(stack.s - threadIdx.x) + threadIdx.x, stack.stride, stack_cap};   // (LANE)
   const int lane = threadIdx.x & 31;
   unsigned long long overflow = 0;
   WalkCount wc;
@@ -136,7 +136,7 @@ __device__ __forceinline__ void trace_loop(Src& src, int n, int* work, int stack
     }
     bool of = false;
     if (LANE) {
-      if (e_cur >= 0 && any_walk_step(w, whole, wc, of)) finish();
+      if (e_cur >= 0 && any_walk_step(w, links, wc, of)) finish();
     } else {
       warp_walk_step<WIDE>(w, ANY, stack, wc, of, nodes, tris);
     }
