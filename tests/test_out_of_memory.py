@@ -89,3 +89,27 @@ def test_batch_without_memory_for_its_stacks(r, fake):
     b.add_job(plain, aid, s.cam, [1], s.cfg)
     b.run(max_launches=1)
     assert fake.fake_allocations() > running   # (the job's seeds)
+
+
+def test_upload_indexes_the_scene_when_its_temporaries_are_gone(r, fake):
+    """The least memory that takes an upload takes the scene's walk index too: by then the copies of the
+    caller's arrays have been given back."""
+    s = workloads.mixed_scene(3000, 5, 16, 16, 1)
+    before = fake.fake_bytes()
+    sid = r.upload(s)
+    whole = fake.fake_bytes()
+    assert whole - before > r.scene_bytes(sid)   # (the index is beside the scene's arrays)
+    r.release(sid)
+    low, high = before, before + 64 * (whole - before)
+    while high - low > 256:
+        mid = (low + high) // 2
+        fake.fake_limit(mid)
+        try:
+            r.release(r.upload(s))
+            high = mid
+        except N.YuneError as e:
+            assert e.code == N.YC_E_NOMEM
+            low = mid
+    fake.fake_limit(high)
+    r.upload(s)
+    assert fake.fake_bytes() == whole

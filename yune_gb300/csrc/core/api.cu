@@ -781,7 +781,10 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
   } else if (yc::check_materials(tris, n_tri, n_mat, err)) {
     return fail(YC_E_INVALID, err);
   }
-  if (!on_device && yc::repack_scene(tris, n_tri, nodes, n_node, c->tree_mode, rp, err)) return fail(YC_E_INVALID, err);
+  if (!on_device) {
+    dev.release();
+    if (yc::repack_scene(tris, n_tri, nodes, n_node, c->tree_mode, rp, err)) return fail(YC_E_INVALID, err);
+  }
   const size_t n_node4 = on_device ? 4 * ((size_t)dev.n_leaf - 1) : rp.nodes.size();
   const size_t n_tri4 = on_device ? 3 * dev.slots : rp.tris.size();
   const size_t n_shade4 = on_device ? 4 * (size_t)n_tri : rp.shade.size();
@@ -802,6 +805,7 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
     int depth = 0;
     const int r = yc::repack_device(dev, plan, n_tri, s->nodes.p, s->tris.p, s->shade.p, depth, c->stream, err);
     if (r) return fail(r == -2 ? YC_E_NOMEM : YC_E_LAUNCH, err);
+    dev.release();      // (the scene's walk index may need the room)
     rp.root_link = 0;   // the root is the first node (two leaves or more)
     rp.root_test = 1;
     rp.depth = depth;

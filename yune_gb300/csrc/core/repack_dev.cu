@@ -982,10 +982,13 @@ __global__ void __launch_bounds__(ITEM_TB) k_list_leaves(int n_node, const int* 
 
 }  // namespace
 
-DevRepack::~DevRepack() {
+void DevRepack::release() {
   cudaFree(tris);
   cudaFree(nodes);
   cudaFree(work);
+  tris = nullptr;
+  nodes = nullptr;
+  work = leaf = first = nullptr;
 }
 
 cudaError_t first_bad_material(const yc_triangle* tris, int n, int n_mat, int* first, int& bad, cudaStream_t s) {

@@ -66,7 +66,8 @@ struct DevRepack {
   DevRepack() = default;
   DevRepack(const DevRepack&) = delete;
   DevRepack& operator=(const DevRepack&) = delete;
-  ~DevRepack();
+  ~DevRepack() { release(); }
+  void release();   // the device arrays
 };
 int repack_copy(const yc_triangle* tris_host, int n_tri, int n_mat, const yc_bvh_node* nodes_host, int n_node,
                 bool check, DevRepack& d, cudaStream_t s, std::string& err);
