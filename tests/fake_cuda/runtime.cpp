@@ -11,7 +11,7 @@
 namespace {
 std::map<void*, size_t> g_live;
 size_t g_bytes = 0, g_peak = 0, g_limit = ~(size_t)0;
-long long g_launches = 0;
+long long g_launches = 0, g_mallocs = 0;
 cudaError_t g_last = cudaSuccess;
 int g_handle;   // what streams, events and graphs point to
 
@@ -34,11 +34,13 @@ unsigned long long fake_bytes(void) { return g_bytes; }
 unsigned long long fake_peak(void) { return g_peak; }
 void fake_reset_peak(void) { g_peak = g_bytes; }
 long long fake_launches(void) { return g_launches; }
+long long fake_mallocs(void) { return g_mallocs; }   // calls so far
 int fake_allocations(void) { return (int)g_live.size(); }   // in place now
 
 // ---- memory ----
 cudaError_t cudaMalloc(void** p, size_t n) {
   *p = nullptr;
+  ++g_mallocs;
   if (g_bytes + n > g_limit) return error(cudaErrorMemoryAllocation);
   *p = std::calloc(n ? n : 1, 1);
   g_live[*p] = n;

@@ -113,3 +113,11 @@ def test_upload_indexes_the_scene_when_its_temporaries_are_gone(r, fake):
     fake.fake_limit(high)
     r.upload(s)
     assert fake.fake_bytes() == whole
+
+
+def test_small_upload_makes_few_allocations(r, fake):
+    """An allocation and its release are a twentieth of the Cornell box's upload: the scene's six arrays
+    and its index, and two blocks of temporaries."""
+    n = fake.fake_mallocs()
+    r.upload(scenes.c0(16, 16))
+    assert fake.fake_mallocs() - n <= 9

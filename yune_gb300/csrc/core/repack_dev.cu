@@ -920,6 +920,16 @@ struct Tmp {
   cudaError_t alloc(size_t n) { return cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)); }
 };
 
+// a part of a block: n elements at the next multiple of 256 bytes
+template <class T>
+struct Part {
+  T* p = nullptr;
+  void put(char* base, size_t& at, size_t n) {
+    if (base) p = reinterpret_cast<T*>(base + at);
+    at += (n * sizeof(T) + 255) / 256 * 256;
+  }
+};
+
 // The first triangle without a material, a thread per triangle (bound by the stride of the read;
 // starting and joining the host's threads took 1 ms for 330K triangles).
 __global__ void __launch_bounds__(ITEM_TB) k_check_materials(const yc_triangle* tris, int n, int n_mat, int* first) {
@@ -983,12 +993,11 @@ __global__ void __launch_bounds__(ITEM_TB) k_list_leaves(int n_node, const int* 
 }  // namespace
 
 void DevRepack::release() {
-  cudaFree(tris);
-  cudaFree(nodes);
-  cudaFree(work);
+  cudaFree(block);
+  block = nullptr;
   tris = nullptr;
   nodes = nullptr;
-  work = leaf = first = nullptr;
+  leaf = first = nullptr;
 }
 
 cudaError_t first_bad_material(const yc_triangle* tris, int n, int n_mat, int* first, int& bad, cudaStream_t s) {
@@ -1015,10 +1024,13 @@ int repack_copy(const yc_triangle* tris_host, int n_tri, int n_mat, const yc_bvh
   } while (0)
   // (the scans take whole tiles of 1024)
   const size_t N = (size_t)n_node, tiles = (N + 1023) / 1024;
-  YC_COPY_CUDA(cudaMalloc(&d.tris, (size_t)n_tri * sizeof(yc_triangle)));
-  YC_COPY_CUDA(cudaMalloc(&d.nodes, N * sizeof(yc_bvh_node)));
-  YC_COPY_CUDA(cudaMalloc(&d.work, (7 * N + tiles) * sizeof(int) + sizeof(CopyCtl)));
-  d.leaf = d.work;
+  // (one block of memory: an allocation and its release are 5-10 us, which a small upload notices)
+  static_assert(sizeof(yc_triangle) % 16 == 0 && sizeof(yc_bvh_node) % 16 == 0, "the arrays follow each other");
+  YC_COPY_CUDA(cudaMalloc(&d.block, (size_t)n_tri * sizeof(yc_triangle) + N * sizeof(yc_bvh_node) +
+                                        (7 * N + tiles) * sizeof(int) + sizeof(CopyCtl)));
+  d.tris = reinterpret_cast<yc_triangle*>(d.block);
+  d.nodes = reinterpret_cast<yc_bvh_node*>(d.tris + n_tri);
+  d.leaf = reinterpret_cast<int*>(d.nodes + N);
   d.first = d.leaf + N;
   int* child = d.first + N;
   int *flag = child + N, *len = flag + N, *at = len + N, *slot = at + N, *sums = slot + N;
@@ -1065,15 +1077,21 @@ int repack_device(DevRepack& d, const DevRepackPlan& plan, int n_tri, float4* no
   } while (0)
   const size_t cap_large = (size_t)n_leaf / (SMALL_MAX + 1) + 1;   // disjoint ranges of more than SMALL_MAX
   const size_t cap_small = (size_t)n_leaf / 2 + 1;                 // disjoint ranges of two leaves or more
-  Tmp<SahItem> d_items, d_tmp;
-  Tmp<SahTask> d_ta, d_tb, d_small;
-  Tmp<SahCtl> d_ctl;
-  YC_REPACK_CUDA(d_items.alloc(n_leaf), "allocation");
-  YC_REPACK_CUDA(d_tmp.alloc(n_leaf), "allocation");
-  YC_REPACK_CUDA(d_ta.alloc(cap_large), "allocation");
-  YC_REPACK_CUDA(d_tb.alloc(cap_large), "allocation");
-  YC_REPACK_CUDA(d_small.alloc(cap_small), "allocation");
-  YC_REPACK_CUDA(d_ctl.alloc(1), "allocation");
+  Part<SahItem> d_items, d_tmp;
+  Part<SahTask> d_ta, d_tb, d_small;
+  Part<SahCtl> d_ctl;
+  Tmp<char> block;   // (all in one, as in repack_copy)
+  for (char* base = nullptr;; base = block.p) {
+    size_t at = 0;
+    d_items.put(base, at, n_leaf);
+    d_tmp.put(base, at, n_leaf);
+    d_ta.put(base, at, cap_large);
+    d_tb.put(base, at, cap_large);
+    d_small.put(base, at, cap_small);
+    d_ctl.put(base, at, 1);
+    if (base) break;
+    YC_REPACK_CUDA(block.alloc(at), "allocation");
+  }
   if (!plan.leaf_node.empty()) {
     YC_REPACK_CUDA(cudaMemcpyAsync(d.leaf, plan.leaf_node.data(), (size_t)n_leaf * sizeof(int), cudaMemcpyHostToDevice, s),
                    "copy");

@@ -56,11 +56,11 @@ int check_materials(const yc_triangle* tris, int n_tri, int n_mat, std::string& 
 // and lists (plan_device_repack); -1 (-2: out of memory) with err when a call failed. With `check`
 // false it copies only, and returns 0.
 struct DevRepack {
+  char* block = nullptr;       // what follows lies in it
   yc_triangle* tris = nullptr;
   yc_bvh_node* nodes = nullptr;
   int* leaf = nullptr;         // the leaves and their first slots (room for a leaf a node)
   int* first = nullptr;
-  int* work = nullptr;
   int n_leaf = 0, bad_tri = 0;
   size_t slots = 0;
   DevRepack() = default;
