@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) k_raygen_bdpt(PassParams pp, int n, int r
     // light vertex 0 on light 0 (createLightPath, bdpt.cl:435-456)
     const yc_quad_light& L = sc.lights[0];
     seed = ym::xor_shift(seed);
-    const float lr1 = (float)divided((double)seed, 4294967295.0, 1.0 / 4294967295.0);   // seed / (double)UINT_MAX
+    const float lr1 = ym::u01_inclusive(seed);
     const float lr2 = draw(seed);
     const f4 A = ld4(L.edge_l) * lr2;
     const f4 B = ld4(L.edge_w) * lr1;

@@ -36,13 +36,6 @@ struct LogicCounts {
   unsigned rays = 0, ext = 0, shadow = 0, conn = 0, trav = 0, samples = 0, prim = 0;
 };
 
-// a / b rounded to nearest, from r = 1 / b rounded to nearest: the quotient a * r is within one
-// unit of the last place, and one step along its remainder gives the division's own result
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990).
-__device__ __forceinline__ double divided(double a, double b, double r) {
-  const double q = a * r;
-  return ::fma(::fma(-q, b, a), r, q);
-}
 // The pathtracer prologue and createRay (udpt.cl:158-189, 213-238): the seed of pixel (px, py) of
 // a pass and the direction of its camera ray. Double precision runs at a small fraction of the
 // other rates: the step of the batch engine that starts paths between its shading with a
@@ -56,8 +49,8 @@ __device__ __forceinline__ f4 camera_direction(const PassParams& pp, int px, int
   const float r2 = draw(seed);
   const float fx = ym::add((float)px, r1), fy = ym::add((float)py, r2);
   f4 dir;
-  dir.x = (float)(pp.aspect * (divided(2.0 * (double)fx, pp.w, pp.inv_w) - 1.0));
-  dir.y = (float)(divided(2.0 * (double)fy, pp.h, pp.inv_h) - 1.0);
+  dir.x = (float)(pp.aspect * (ym::divided(2.0 * (double)fx, pp.w, pp.inv_w) - 1.0));
+  dir.y = (float)(ym::divided(2.0 * (double)fy, pp.h, pp.inv_h) - 1.0);
   dir.z = -pp.cam.view_plane_dist;
   dir.w = 0.0f;
   f4 d;

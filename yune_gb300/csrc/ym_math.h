@@ -222,6 +222,24 @@ YM_HD void sincos(float x, float& sn, float& cs) {
   cs = ((q + 1) & 2) ? -b : b;
 }
 
+// ---- double-precision division by a number whose reciprocal is at hand -----------
+// a / b rounded to nearest, for an integer b of up to 32 bits, an a of up to 32 significant bits
+// and r = 1 / b rounded to nearest, nothing near underflow or overflow: a product and one step
+// along its remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990). The rounded product of a and r is off by less than 1.5 units in the last
+// place (a relative 2^-53 from r, half a unit from the product), its remainder a - q * b has few
+// enough bits to be exact, and the corrected value before its one rounding is off by less than 1.5 *
+// 2^-53 units. No quotient of these a and b lies that near to a midpoint of two doubles: scaled to
+// [2^52, 2^53), a / b - (M + 1/2) = (2^k a' - b (2M + 1)) / (2b) with integers k > 0, a' < 2^32 and M,
+// an integer over 2b, and not 0, for 2M + 1 is odd and above 2^53 and would have to divide a'. So
+// it is at least 2^-33 units away, and both round to the same side.
+YM_HD double divided(double a, double b, double r) {
+  const double q = a * r;
+  return ::fma(::fma(-q, b, a), r, q);
+}
+// seed / (double)UINT_MAX as a float: [0, 1] with both ends
+YM_HD float u01_inclusive(uint32_t seed) { return (float)divided((double)seed, 4294967295.0, 1.0 / 4294967295.0); }
+
 // ---- log2 / exp2 / pow ------------------------------------------------------------
 // log2(x) = e + 2*atanh(s)/ln2 with s = (m-1)/(m+1), m in [sqrt(1/2), sqrt(2)).
 YM_HD float log2_pos(float x) {      // x finite, > 0
