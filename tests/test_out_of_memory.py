@@ -121,3 +121,27 @@ def test_small_upload_makes_few_allocations(r, fake):
     n = fake.fake_mallocs()
     r.upload(scenes.c0(16, 16))
     assert fake.fake_mallocs() - n <= 9
+
+
+SEGMENT = 16 + 4 + 8   # bytes of a segment: its ray, its queue entry and the sort's two lists
+
+
+def _sorted_bdpt(q, s):
+    q.set_repack(0)
+    sid, aid = q.upload(s), q.alloc_accum(320, 256)
+    q.set_camera(s.cam)
+    return lambda: q.render(sid, aid, 1, reset=1, cfg=scenes.default_cfg(integrator=2, bdpt_bounces=4)), aid
+
+
+def test_bidirectional_pass_with_room_for_one_segment_a_path(r, fake):
+    s = workloads.mixed_scene(5000, 5, 16, 16, 1)
+    n = 320 * 256
+    render, _ = _sorted_bdpt(r, s)
+    render()
+    room = fake.fake_bytes() - 7 * SEGMENT * n   # eight a path where memory allows
+    r.close()
+    with Renderer(0) as q:
+        render, _ = _sorted_bdpt(q, s)
+        fake.fake_limit(room)
+        render()
+        assert fake.fake_bytes() <= room

@@ -253,7 +253,7 @@ int ensure_pass_spill(yc_ctx* c, size_t n) {
   return 0;
 }
 
-// key, histogram and sorted-list buffers of the per-pass ray sort, for n rays
+// key, histogram and sorted-list buffers of the per-pass ray sort, for n rays in a round
 int ensure_raysort(yc_ctx* c, size_t n) {
   if (!c->rs_ctl.p) {
     const size_t bins = (size_t)yc::raysort_bins(3, 2);   // the largest key allowed (16 bits)
@@ -270,8 +270,8 @@ int ensure_raysort(yc_ctx* c, size_t n) {
 }
 
 // The segments of a bidirectional pass over n paths, and the ray sort's lists for them: 2^FAN_SHIFT
-// a path (180 bytes with the sort's), fewer where an entry would not fit the queues' 32 bits or
-// the device's memory.
+// a path (20 bytes each, 28 with the sort's), fewer where an entry would not fit the queues' 32 bits
+// or the device's memory.
 int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
   for (int shift = c->bd_paths == n ? c->bd_shift : yc::FAN_SHIFT;; --shift) {
     const size_t m = n << shift;
@@ -521,7 +521,9 @@ int run_passes(yc_ctx* c, Scene* sc, Accum* ac, const uint32_t* rands, int n_pas
                        (size_t)W * H >= (size_t)c->rs_threshold && dsc.n_tri >= kRaySortMinTris;
   yc::RaySortBufs rsb{};
   if (raysort) {
-    if (int e = ensure_raysort(c, (size_t)W * H * 3)) return e;   // a closest-hit ray and two segments a path
+    // (a closest-hit ray and a segment, or two segments a path; a bidirectional path sends the one or
+    // the others: ensure_segments)
+    if (int e = ensure_raysort(c, bdpt ? 0 : (size_t)W * H * 2)) return e;
   }
   // shade-queue sort by phase and material class before the logic kernel (unidirectional
   // passes whose frame can fill a sorted queue, in scenes with a mirror or dielectric:

@@ -8,7 +8,7 @@
 //                   any-hit queue (NEE shadow rays and MIS BRDF rays, (d))
 //   logic        -> advances each path whose rays are answered until it needs new ones
 //                   (shading (c), light sampling and MIS (d), Russian roulette), up to
-//                   three at once (logic_path); the new rays are appended to the next
+//                   two at once (logic_path); the new rays are appended to the next
 //                   round's queues with warp prefixes and one atomic per warp and queue
 //                   (e), so finished paths drop out and the queues stay dense.
 // A path that finishes writes its colour into the running-mean accumulator
