@@ -487,10 +487,15 @@ enum {
    * (the caller's triangle and node arrays are copied over and the SAH hierarchy above the
    * reference leaves, the leaves' triangle stream and the shading records are built by
    * kernels), 0 on the host. Both give the same bytes (yc_scene_digest equals
-   * yc_scene_layout's digest). The node checks and the list of reachable leaves stay on
-   * the host; tree modes 0 and 2, and scenes with fewer than two reachable leaves, are
-   * repacked on the host either way. */
-  YC_OPT_REPACK = 10
+   * yc_scene_layout's digest). Scenes of 4096 triangles or more have their materials and nodes
+   * checked and their leaves listed there too (arrays that are not regular go to the host); tree
+   * modes 0 and 2, and scenes with fewer than two reachable leaves, are repacked on the host
+   * either way. */
+  YC_OPT_REPACK = 10,
+  /* Segments (shadow rays) that an eye vertex of a bidirectional pass sends in one round: 8
+   * (default), 4, 2 or 1. A path takes 20 to 28 bytes for each; where the device has no room for
+   * them, fewer are sent. Same results whatever the number. */
+  YC_OPT_SEGMENTS = 11
 };
 int yc_set_option(yc_ctx* ctx, int option, int value);
 

@@ -145,3 +145,21 @@ def test_bidirectional_pass_with_room_for_one_segment_a_path(r, fake):
         fake.fake_limit(room)
         render()
         assert fake.fake_bytes() <= room
+        fake.fake_limit(fake_cuda.NO_LIMIT)
+        q.free_accum(q.alloc_accum(16, 16))   # memory came back: eight again
+        render()
+        assert fake.fake_bytes() == room + 7 * SEGMENT * n
+
+
+def test_segments_option(r, fake):
+    render, _ = _sorted_bdpt(r, workloads.mixed_scene(5000, 5, 16, 16, 1))
+    for bad in (0, 3, 5, 16, -1):
+        with pytest.raises(N.YuneError) as e:
+            r.set_segments(bad)
+        assert e.value.code == N.YC_E_INVALID
+    took = []
+    for k in (1, 2, 4, 8):
+        r.set_segments(k)
+        render()
+        took.append(fake.fake_bytes())
+    assert np.array_equal(np.diff(took), 320 * 256 * SEGMENT * np.array([1, 2, 4]))

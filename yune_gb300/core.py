@@ -212,14 +212,20 @@ class Renderer:
 
     def set_stack_smem(self, n):
         """Walk-stack entries the per-pass traversal keeps in shared memory (YC_OPT_STACK_SMEM;
-        the deeper ones go to a spill area in global memory; 0 = 12, the default; 64 or any
-        value at or above the scene's stack depth = the whole stack)."""
+        the deeper ones go to a spill area in global memory; 0 = 12, the default; a value at or
+        above the entries a walk can need, up to half as many again as scene_depth + 2 over a
+        scene's walk index, = the whole stack)."""
         N.check(self.L.yc_set_option(self.h, 9, int(n)), "yc_set_option")
 
     def set_repack(self, on_device):
         """Where later uploads repack a tree-mode-1 scene (YC_OPT_REPACK): 1 on the device
         (default), 0 on the host; the bytes are the same."""
         N.check(self.L.yc_set_option(self.h, 10, int(on_device)), "yc_set_option")
+
+    def set_segments(self, n):
+        """Segments an eye vertex of a bidirectional pass sends in one round (YC_OPT_SEGMENTS): 8
+        (default), 4, 2 or 1; the images are the same."""
+        N.check(self.L.yc_set_option(self.h, 11, int(n)), "yc_set_option")
 
     def set_tail_paths(self, n):
         """Paths left at which a pass finishes in the tail kernel (-1 auto, 0 off)."""

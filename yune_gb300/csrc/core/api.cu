@@ -187,6 +187,7 @@ struct yc_ctx {
   // BDPT subpath vertices
   DevBuf<float4> bd_lv, bd_ev, bd_seg;   // (the MIS tracer has no eye records)
   DevBuf<int> bd_q_any;
+  int fan_shift = yc::FAN_SHIFT;      // YC_OPT_SEGMENTS (log2)
   int bd_shift = yc::FAN_SHIFT;       // segments a path sends at once, for frames of bd_paths paths (log2)
   size_t bd_paths = 0;
   // direct queries
@@ -270,10 +271,11 @@ int ensure_raysort(yc_ctx* c, size_t n) {
 }
 
 // The segments of a bidirectional pass over n paths, and the ray sort's lists for them: 2^FAN_SHIFT
-// a path (20 bytes each, 28 with the sort's), fewer where an entry would not fit the queues' 32 bits
-// or the device's memory.
+// a path (20 bytes each, 28 with the sort's; YC_OPT_SEGMENTS), fewer where an entry would not fit the
+// queues' 32 bits or the device's memory. What did fit is kept for frames of this size until the
+// context gives memory back.
 int ensure_segments(yc_ctx* c, size_t n, bool raysort) {
-  for (int shift = c->bd_paths == n ? c->bd_shift : yc::FAN_SHIFT;; --shift) {
+  for (int shift = c->bd_paths == n ? c->bd_shift : c->fan_shift;; --shift) {
     const size_t m = n << shift;
     if (shift > 0 && m > ((size_t)1 << 30)) continue;
     cudaError_t e = cudaSuccess;
@@ -1051,6 +1053,7 @@ int yc_release_scene(yc_ctx* c, int scene_id) {
   if (it == c->scenes.end()) return fail(YC_E_NOTFOUND, "unknown scene");
   cudaStreamSynchronize(c->stream);
   c->scenes.erase(it);
+  c->bd_paths = 0;   // (memory came back: ensure_segments asks for the most again)
   return YC_OK;
 }
 
@@ -1114,6 +1117,7 @@ int yc_free_accum(yc_ctx* c, int accum_id) {
   if (it == c->accums.end()) return fail(YC_E_NOTFOUND, "unknown accumulator");
   cudaStreamSynchronize(c->stream);
   c->accums.erase(it);
+  c->bd_paths = 0;
   return YC_OK;
 }
 
@@ -1356,6 +1360,14 @@ int yc_set_option(yc_ctx* c, int option, int value) {
       if (value != 0 && value != 1) return fail(YC_E_INVALID, "repack is 0 (host) or 1 (device)");
       c->repack_device = value;
       return YC_OK;
+    case YC_OPT_SEGMENTS: {
+      int shift = 0;
+      while (shift < yc::FAN_SHIFT && 1 << shift < value) ++shift;
+      if (value != 1 << shift) return fail(YC_E_INVALID, "segments are 1, 2, 4 or 8");
+      c->fan_shift = shift;
+      c->bd_paths = 0;
+      return YC_OK;
+    }
     default:
       return fail(YC_E_INVALID, "unknown option");
   }
@@ -1915,6 +1927,7 @@ int yc_batch_destroy(yc_batch* b) {
   if (b->ctx) {
     auto& v = b->ctx->batches;
     v.erase(std::remove(v.begin(), v.end(), b), v.end());
+    b->ctx->bd_paths = 0;
   }
   free_batch(b);
   return YC_OK;
