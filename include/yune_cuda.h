@@ -279,8 +279,10 @@ typedef struct yc_batch_cfg {
   int32_t stack_smem;          /* entries of each walk's stack kept in shared memory; deeper
                                   entries go to a global spill area of the batch (allocated
                                   when it first runs). Fewer entries leave more of the SM's L1
-                                  to the node and triangle fetches; a value at or above the
-                                  stack depth keeps the whole stack in shared memory; 0 = 12 */
+                                  to the node and triangle fetches; a value at or above
+                                  stack_cap keeps stack_cap entries there, the whole stack of
+                                  walks over the scenes' own nodes (walks over their indexes
+                                  can be up to half as deep again); 0 = 12 */
   int32_t trace_share;         /* percent of the traversal blocks that fit on an SM that the
                                   persistent traversal grid launches (10..100): below 100 each
                                   SM keeps room for the other slot groups' kernels (ray sort,

@@ -23,7 +23,8 @@ def load(out_dir):
         fn.restype, fn.argtypes = res, args
     for name, res, args in (("fake_limit", None, [C.c_uint64]), ("fake_bytes", C.c_uint64, []),
                             ("fake_peak", C.c_uint64, []), ("fake_reset_peak", None, []),
-                            ("fake_launches", C.c_longlong, []), ("fake_mallocs", C.c_longlong, []), ("fake_allocations", C.c_int, [])):
+                            ("fake_launches", C.c_longlong, []), ("fake_mallocs", C.c_longlong, []), ("fake_allocations", C.c_int, []),
+                            ("fake_store", None, [C.c_uint64, C.c_int, C.c_int])):
         fn = getattr(L, name)
         fn.restype, fn.argtypes = res, args
     return L

@@ -37,6 +37,12 @@ long long fake_launches(void) { return g_launches; }
 long long fake_mallocs(void) { return g_mallocs; }   // calls so far
 int fake_allocations(void) { return (int)g_live.size(); }   // in place now
 
+// what kernels would have left: int `at` of every allocation of exactly this many bytes
+void fake_store(unsigned long long bytes, int at, int value) {
+  for (const auto& a : g_live)
+    if (a.second == bytes) static_cast<int*>(a.first)[at] = value;
+}
+
 // ---- memory ----
 cudaError_t cudaMalloc(void** p, size_t n) {
   *p = nullptr;

@@ -163,3 +163,62 @@ def test_segments_option(r, fake):
         render()
         took.append(fake.fake_bytes())
     assert np.array_equal(np.diff(took), 320 * 256 * SEGMENT * np.array([1, 2, 4]))
+
+
+def _indexed(r, fake, need, tris=5000):
+    """A scene whose index walks of `need` entries take (the upload reads it from its two control words)."""
+    fake.fake_store(8, 0, need)
+    return r.upload(workloads.mixed_scene(tris, 5, 16, 16, 1))
+
+
+def _stack_bytes(fake, run):
+    before = fake.fake_bytes()
+    run()
+    return fake.fake_bytes() - before
+
+
+def test_batch_stacks_are_as_deep_as_its_scenes_need(r, fake):
+    r.set_repack(0)
+    s = workloads.mixed_scene(5000, 5, 16, 16, 1)
+    sid, aid = _indexed(r, fake, 22), r.alloc_accum(64, 64)
+    took = []
+    for cap in (0, 64, 200):   # (the scene's own, a server's bound, a generous one)
+        b = Batch(r, pool_paths=4096, stack_cap=cap, stack_smem=12)
+        b.add_job(sid, aid, s.cam, [1], s.cfg)
+        took.append(_stack_bytes(fake, lambda: b.run(max_launches=1)))
+        b.close()
+    # two launches of a group, an entry beyond the 12 in shared memory 8 bytes for each of 152 * 4 * 128
+    # threads, two groups: the bound given, or what the index needs
+    assert took == [2 * 2 * (n - 12) * 8 * 152 * 4 * 128 for n in (24, 64, 200)]
+
+
+@pytest.mark.parametrize("need", [22, 118])
+def test_batch_with_its_whole_stacks_in_shared_memory(r, fake, need):
+    """Stacks that fit a block's shared memory over the scenes' own nodes are not refused over an index."""
+    r.set_repack(0)
+    s = workloads.mixed_scene(5000, 5, 16, 16, 1)
+    sid, aid = _indexed(r, fake, need), r.alloc_accum(64, 64)
+    b = Batch(r, pool_paths=4096, stack_cap=100, stack_smem=120, trace_block=256)
+    b.add_job(sid, aid, s.cam, [1], s.cfg)
+    b.run(max_launches=1)
+
+
+def test_batch_joined_by_a_scene_with_a_deeper_index(r, fake):
+    r.set_repack(0)
+    s = workloads.mixed_scene(5000, 5, 16, 16, 1)
+    sid, aid = _indexed(r, fake, 22), r.alloc_accum(64, 64)
+    per_entry = 2 * 2 * 8 * 152 * 4 * 128
+
+    def started():
+        b = Batch(r, pool_paths=4096, stack_cap=30, stack_smem=12)
+        b.add_job(sid, aid, s.cam, [1], s.cfg)
+        b.run(max_launches=1)
+        return b
+
+    a, b = started(), started()
+    deep = _indexed(r, fake, 58)
+    b.add_job(deep, aid, s.cam, [1], s.cfg)
+    assert _stack_bytes(fake, lambda: b.run(max_launches=1)) == (60 - 30) * per_entry
+    a.add_job(deep, aid, s.cam, [1], s.cfg)
+    fake.fake_limit(fake.fake_bytes() + 4096)   # no room for its stacks: the scenes' own nodes
+    assert _stack_bytes(fake, lambda: a.run(max_launches=1)) == 0

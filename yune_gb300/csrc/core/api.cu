@@ -1616,9 +1616,15 @@ int batch_body(yc_batch* b, bool timed) {
 int batch_shape(yc_batch* b) {
   yc_ctx* c = b->ctx;
   const bool wide = b->walks_wide();
-  // (walks over indexes: room for scenes added later, as deep as stack_cap admits)
-  b->walk_cap = b->indexed && b->wide != 1 ? std::max(b->index_cap, b->stack_cap + b->stack_cap / 2) : b->stack_cap;
-  b->stack_smem = std::min(b->walk_cap, b->cfg.stack_smem);
+  b->walk_cap = b->stack_cap;
+  if (b->indexed && b->wide != 1) {   // and what the indexes of the jobs need, and of the scenes that may come next
+    b->walk_cap = std::max(b->walk_cap, b->index_cap);
+    for (const auto& s : c->scenes)
+      if (s.second->windex.p && s.second->dev.depth + 2 <= b->stack_cap)
+        b->walk_cap = std::max(b->walk_cap, yc::trace_stack_cap(s.second->windex_depth));
+  }
+  // (never more shared memory than the walks over the scenes' own nodes would have)
+  b->stack_smem = std::min({b->walk_cap, b->stack_cap, b->cfg.stack_smem});
   b->grid_c = yc::batch_trace_grid(false, b->stack_smem, wide, b->cfg.trace_block);
   b->grid_a = yc::batch_trace_grid(true, b->stack_smem, wide, b->cfg.trace_block);
   b->grid_m = yc::batch_trace_mixed_grid(b->stack_smem, wide, b->cfg.trace_block);
@@ -1652,9 +1658,8 @@ void batch_reshape(yc_batch* b) {
   b->graph = nullptr;
 }
 
-// From here on the batch walks its scenes' own nodes: a scene without an index was added, one
-// deeper than the stacks of a running batch hold, or one that stack_cap does not hold. Called
-// between launches.
+// From here on the batch walks its scenes' own nodes: a scene without an index was added or one that
+// stack_cap does not hold, or there is no memory for the indexes' stacks. Called between launches.
 void batch_unindex(yc_batch* b) {
   b->indexed = false;
   for (size_t i = 0; i < b->host_jobs.size(); ++i) b->host_jobs[i].pp.sc = b->job_dev[i];
@@ -1812,10 +1817,11 @@ int yc_batch_add_job(yc_batch* b, int scene_id, int accum_id, const yc_cam* cam,
     // (a scene without interior nodes is walked alike by both kernels)
     const bool has = sc->windex.p || sc->dev.root_link < 0 || sc->dev.root_link == yc::LINK_NONE;
     const int index_cap = sc->windex.p ? yc::trace_stack_cap(sc->windex_depth) : 0;
-    if (!has || need_cap > b->stack_cap || (b->started && index_cap > b->walk_cap)) {
+    if (!has || need_cap > b->stack_cap) {
       batch_unindex(b);
-    } else if (!b->started) {
+    } else {
       b->index_cap = std::max(b->index_cap, index_cap);
+      if (b->shaped && index_cap > b->walk_cap) batch_reshape(b);   // deeper stacks
     }
   }
   yc::BatchJob j{};
@@ -1864,8 +1870,14 @@ int yc_batch_run(yc_batch* b, int max_launches, int* unfinished) {
   yc_ctx* c = b->ctx;
   YC_CUDA(cudaSetDevice(c->device));
   if (!b->started && b->stack_cap <= 0) b->stack_cap = b->cfg.stack_cap > 0 ? b->cfg.stack_cap : 32;
-  if (!b->shaped)
-    if (int r = batch_shape(b)) return r;
+  if (!b->shaped) {
+    int r = batch_shape(b);
+    if (r == YC_E_NOMEM && b->indexed && b->wide != 1) {   // walks over the scenes' own nodes stack less
+      batch_unindex(b);
+      r = batch_shape(b);
+    }
+    if (r) return r;
+  }
   b->started = true;
   if (int r = begin_call_checks(c)) return r;
   YC_CUDA(cudaEventRecord(c->ev0, c->stream));
