@@ -147,7 +147,7 @@ int yc_release_scene(yc_ctx* ctx, int scene_id);
 /* bytes of the scene's arrays on the device (yc_scene_layout). Workspaces made from them
  * beside these are not counted: a refit's, and the walk index of a tree-mode-1 scene (at most
  * 128 bytes per interior node, usually 57; made when memory allows, the scene renders the same
- * without it). */
+ * without it; YC_OPT_WALK_INDEX). */
 int yc_scene_bytes(yc_ctx* ctx, int scene_id, uint64_t* bytes);
 /* interior levels of the uploaded hierarchy (a traversal stack needs depth + 2 slots) */
 int yc_scene_depth(yc_ctx* ctx, int scene_id, int* depth);
@@ -497,7 +497,11 @@ enum {
   /* Segments (shadow rays) that an eye vertex of a bidirectional pass sends in one round: 8
    * (default), 4, 2 or 1. A path takes 20 to 28 bytes for each; where the device has no room for
    * them, fewer are sent. Same results whatever the number. */
-  YC_OPT_SEGMENTS = 11
+  YC_OPT_SEGMENTS = 11,
+  /* Whether later uploads in tree mode 1 make a walk index beside the scene's arrays: 1 (default),
+   * 0 = no, for a host that has counted their bytes to the last (yc_scene_bytes). Same results; the
+   * traversal of a 1920x1080 pass of 260K triangles takes a quarter longer without. */
+  YC_OPT_WALK_INDEX = 12
 };
 int yc_set_option(yc_ctx* ctx, int option, int value);
 

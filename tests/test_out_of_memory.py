@@ -5,7 +5,7 @@ import pytest
 
 import fake_cuda
 from yune_gb300 import _native as N
-from yune_gb300 import scenes, workloads
+from yune_gb300 import scenes, serve, workloads
 from yune_gb300.batch import Batch
 from yune_gb300.core import Renderer
 
@@ -222,3 +222,21 @@ def test_batch_joined_by_a_scene_with_a_deeper_index(r, fake):
     a.add_job(deep, aid, s.cam, [1], s.cfg)
     fake.fake_limit(fake.fake_bytes() + 4096)   # no room for its stacks: the scenes' own nodes
     assert _stack_bytes(fake, lambda: a.run(max_launches=1)) == 0
+
+
+def test_server_keeps_its_scene_budget(r, fake):
+    """A scene budget bounds what the resident scenes take on the device, walk indexes included: they get
+    none where it holds their arrays alone."""
+    r.set_repack(0)
+    resident = [scenes.c0(16, 16), workloads.mixed_scene(5000, 5, 16, 16, 1)]
+    layouts = [scenes.layout(s) for s in resident]
+    need = sum(lay["device_bytes"] for lay in layouts)
+    whole = need + sum(scenes.index_bound(lay) for lay in layouts)
+    for budget, took in ((need, need), (whole - 1, need), (whole, whole), (None, whole)):
+        before = fake.fake_bytes()
+        srv = serve.Server(r, resident, hbm_budget=1 << 20, scene_budget=budget, pool_paths=1024)
+        srv.close()   # (its batch goes, the scenes stay)
+        assert fake.fake_bytes() - before == took
+        for sid in srv.sids:
+            r.release(sid)
+    assert r.walk_index

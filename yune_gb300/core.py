@@ -49,6 +49,7 @@ class Renderer:
         self._accum_shape = {}
         self._children = weakref.WeakSet()   # batches: the context releases them
         self.tree_mode = 1                   # YC_OPT_TREE of later uploads
+        self.walk_index = True               # YC_OPT_WALK_INDEX of later uploads
 
     def close(self):
         if getattr(self, "h", None):
@@ -104,7 +105,7 @@ class Renderer:
         N.check(self.L.yc_refit_scene(self.h, sid, ptr(t), len(t)), "yc_refit_scene")
 
     def scene_bytes(self, sid):
-        """Bytes the scene holds on the device."""
+        """Bytes of the scene's arrays on the device (without its walk index, scenes.index_bound)."""
         b = C.c_uint64()
         N.check(self.L.yc_scene_bytes(self.h, sid, C.byref(b)), "yc_scene_bytes")
         return int(b.value)
@@ -226,6 +227,12 @@ class Renderer:
         """Segments an eye vertex of a bidirectional pass sends in one round (YC_OPT_SEGMENTS): 8
         (default), 4, 2 or 1; the images are the same."""
         N.check(self.L.yc_set_option(self.h, 11, int(n)), "yc_set_option")
+
+    def set_walk_index(self, on):
+        """Whether later tree-mode-1 uploads make a walk index beside the scene's arrays
+        (YC_OPT_WALK_INDEX); the images are the same."""
+        N.check(self.L.yc_set_option(self.h, 12, int(on)), "yc_set_option")
+        self.walk_index = bool(on)
 
     def set_tail_paths(self, n):
         """Paths left at which a pass finishes in the tail kernel (-1 auto, 0 off)."""

@@ -172,6 +172,7 @@ struct yc_ctx {
   int max_rounds = 1000000;   // YC_OPT_MAX_ROUNDS: rounds one pass may take
   int stack_limit = 0;        // YC_OPT_STACK_LIMIT: traversal stack entries allowed (0 = any)
   int stack_smem = 12;        // YC_OPT_STACK_SMEM: per-pass walk-stack entries in shared memory
+  int walk_index = 1;         // YC_OPT_WALK_INDEX: uploads in tree mode 1 make a walk index
   int repack_device = 1;      // YC_OPT_REPACK: the upload's repack of tree mode 1 on the device
   DevBuf<int> pass_spill;     // the deeper entries of the per-pass walks (with stack_smem)
   int logic_grid = 0;
@@ -832,7 +833,7 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
   const std::vector<yc_quad_light> dev_lights = prepared_lights(lights, n_light);
   YC_CUDA(cudaMemcpyAsync(s->lights.p, dev_lights.data(), n_light * sizeof(yc_quad_light), cudaMemcpyHostToDevice,
                           c->stream));
-  const bool index = c->tree_mode == yc::TREE_SAH_OVER_LEAVES && rp.root_link == 0 && rp.root_test != 0;
+  const bool index = c->walk_index && c->tree_mode == yc::TREE_SAH_OVER_LEAVES && rp.root_link == 0 && rp.root_test != 0;
   if (index)
     if (int r = queue_walk_index(c, s.get())) return r;
   YC_CUDA(cudaStreamSynchronize(c->stream));
@@ -1359,6 +1360,10 @@ int yc_set_option(yc_ctx* c, int option, int value) {
     case YC_OPT_REPACK:
       if (value != 0 && value != 1) return fail(YC_E_INVALID, "repack is 0 (host) or 1 (device)");
       c->repack_device = value;
+      return YC_OK;
+    case YC_OPT_WALK_INDEX:
+      if (value != 0 && value != 1) return fail(YC_E_INVALID, "walk index is 0 or 1");
+      c->walk_index = value;
       return YC_OK;
     case YC_OPT_SEGMENTS: {
       int shift = 0;

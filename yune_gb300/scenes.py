@@ -186,6 +186,12 @@ def device_bytes(s, tree_mode=1):
     return layout(s, tree_mode)["device_bytes"]
 
 
+def index_bound(lay, tree_mode=1):
+    """The most bytes the walk index of a scene with this layout() takes beside its arrays: 128 for
+    each of its interior nodes (64 bytes), in tree mode 1."""
+    return 2 * lay["node_bytes"] if tree_mode == 1 else 0
+
+
 def walk_counts(s, rays9, any_hit=False, tree_mode=1):
     """The traversal's algorithmic work on explicit rays, replayed on the host
     (yc_walk_counts): (child boxes tested, triangles tested, per-ray triangle, per-ray t)."""

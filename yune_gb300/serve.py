@@ -69,20 +69,25 @@ class Server:
         """scene_budget: device bytes the resident scenes may take together (None: no
         limit); checked on the host before anything is uploaded, as CLManager checks each
         buffer against the device's global memory before creating it
-        (src/CLManager.cpp:428-429, 452-453). shape: an autotune.BatchShape for the
+        (src/CLManager.cpp:428-429, 452-453). A budget that holds the scenes' arrays but not
+        their walk indexes too is kept: the scenes are uploaded without (YC_OPT_WALK_INDEX;
+        `indexed` says whether they have them). shape: an autotune.BatchShape for the
         server's batch (its fields replace pool_paths, rounds_per_launch,
         logic_blocks_per_sm and sort_threshold). sids: the resident scenes' ids when
         they are uploaded already (else they are uploaded here)."""
         self.r = renderer
         self.scenes = resident
         self.scene_bytes = None
+        self.indexed = True
         if scene_budget is not None:
             mode = getattr(renderer, "tree_mode", 1)   # the layout the uploads below will build
-            self.scene_bytes = sum(scenes.device_bytes(s, tree_mode=mode) for s in resident)
+            layouts = [scenes.layout(s, tree_mode=mode) for s in resident]
+            self.scene_bytes = sum(lay["device_bytes"] for lay in layouts)
             if self.scene_bytes > scene_budget:
                 raise ValueError("resident scenes need %d device bytes, above the scene budget of %d"
                                  % (self.scene_bytes, scene_budget))
-        self.sids = list(sids) if sids is not None else [renderer.upload(s) for s in resident]
+            self.indexed = self.scene_bytes + sum(scenes.index_bound(lay, mode) for lay in layouts) <= scene_budget
+        self.sids = list(sids) if sids is not None else self._upload(resident)
         self.budget = int(hbm_budget)
         self.keep = keep_results
         self.cfg = cfg or scenes.default_cfg(max_depth=16)
@@ -102,6 +107,15 @@ class Server:
         self.in_use = 0          # accumulator bytes of the requests in flight
         self.max_in_flight = 0   # most requests admitted at once, and most accumulator bytes
         self.max_in_use = 0
+
+    def _upload(self, resident):
+        if self.indexed or not self.r.walk_index:
+            return [self.r.upload(s) for s in resident]
+        self.r.set_walk_index(False)
+        try:
+            return [self.r.upload(s) for s in resident]
+        finally:
+            self.r.set_walk_index(True)
 
     def info(self, q):
         i = N.RequestInfo()
