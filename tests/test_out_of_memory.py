@@ -240,3 +240,15 @@ def test_server_keeps_its_scene_budget(r, fake):
         for sid in srv.sids:
             r.release(sid)
     assert r.walk_index
+
+
+def test_ray_queries_give_the_buffers_of_long_lists_back(r, fake):
+    """Short lists' buffers are kept from call to call, those of a list of millions until the next."""
+    sid = r.upload(scenes.c0(16, 16))
+    rays = scenes.box_rays(3 << 20, 1)
+    r.trace(sid, rays[:1])
+    before, per_ray = fake.fake_bytes(), (9 + 2) * 4
+    for n, held in ((5000, 5000), (100, 5000), (1 << 20, 1 << 20), (5000, 1 << 20), (3 << 20, 3 << 20),
+                    (2 << 20, 2 << 20), (10, 10)):
+        r.trace(sid, rays[:n])
+        assert fake.fake_bytes() - before == (held - 1) * per_ray

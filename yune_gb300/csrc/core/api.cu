@@ -210,6 +210,7 @@ int ensure_paths(yc_ctx* c, size_t n) {
 }
 
 constexpr int kTraceStage = 1 << 16;
+constexpr int kTraceKeep = 1 << 20;   // 44 MB
 
 // scenes with fewer triangles are traced in queue order by yc_render_pass
 constexpr int kRaySortMinTris = 4096;
@@ -1256,6 +1257,11 @@ int yc_trace(yc_ctx* c, int scene_id, const float* rays, int n, int any_hit, int
   // the device buffers, and for lists of up to kTraceStage rays page-locked memory that takes
   // both results in one copy, are kept from call to call (three allocations, their releases
   // and a copy each were 45 of the 74 us that 4,096 segments through the Cornell box took)
+  // (the buffers of a list of more than kTraceKeep rays go with the next shorter call)
+  if (c->q_rays.n > 9 * (size_t)std::max(n, kTraceKeep)) {
+    c->q_rays.release();
+    c->q_hits.release();
+  }
   YC_CUDA(c->q_rays.need((size_t)n * 9));
   YC_CUDA(c->q_hits.need(2 * (size_t)n));
   int* const tri_dev = c->q_hits.p;
