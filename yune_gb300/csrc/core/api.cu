@@ -582,7 +582,7 @@ int run_passes(yc_ctx* c, Scene* sc, Accum* ac, const uint32_t* rands, int n_pas
   int cur = 0;
   // The host looks at the queues every six rounds, or when the tail can have ended the call: a look
   // leaves the GPU idle for 10-15 us, a round launched in vain costs 10-25 us (256x256 frame of the
-  // Cornell box 0.69 ms with a look at every sixth round, now 0.63; 96x64 with MIS 0.82, now 0.71).
+  // Cornell box 0.69 ms with a look at every sixth round, now 0.63; 96x64 with MIS 0.78, now 0.71).
   const size_t n_paths = (size_t)W * H;
   long long check_at = n_paths <= (size_t)tail_at ? 1 : n_pass == 1 && n_paths <= 2 * (size_t)tail_at ? 2 : 6;
   bool finished = false;
@@ -776,7 +776,8 @@ int yc_upload_scene(yc_ctx* c, const yc_triangle* tris, int n_tri, const yc_mate
     if (!device_checks && yc::check_materials(tris, n_tri, n_mat, err)) return fail(YC_E_INVALID, err);
     const int r = yc::repack_copy(tris, n_tri, n_mat, nodes, n_node, device_checks, dev, c->stream, err);
     if (r < 0) return fail(r == -2 ? YC_E_NOMEM : YC_E_LAUNCH, err);
-    if (dev.bad_tri < n_tri) return fail(YC_E_INVALID, "triangle " + std::to_string(dev.bad_tri) + " has matID out of range");
+    if (dev.bad_tri < n_tri)
+      return fail(YC_E_INVALID, "triangle " + std::to_string(dev.bad_tri) + " has matID out of range");
     on_device = r && dev.n_leaf >= 2 && dev.slots < (size_t)(1 << 27);
     if (!on_device) {   // an array for the host to decide about
       on_device = yc::plan_device_repack(nodes, n_node, n_tri, plan, err);
@@ -1163,8 +1164,8 @@ int yc_render_passes(yc_ctx* c, int scene_id, int accum_id, const uint32_t* rand
   YC_CUDA(cudaEventRecord(c->ev0, c->stream));
   // Unidirectional passes run together, except in large frames of scenes whose rays are not sorted:
   // there a round of one pass's equal rays is worth more than one end for all of them (Cornell
-  // box, ms with passes apart / together: 4 of 128x96 1.89 / 1.57, 4 of 512x512 3.96 / 3.93, 3 of
-  // 1024x1024 9.74 / 10.28; 150K triangles, 3 of 640x480: 7.69 / 6.50, 400K, 2 of 1280x720: 11.7 /
+  // box, ms with passes apart / together: 4 of 128x96 1.40 / 1.15, 2 of 384x384 1.47 / 1.38, 3 of
+  // 1024x1024 8.21 / 8.52; 150K triangles, 3 of 640x480: 7.24 / 6.25, 400K, 2 of 1280x720: 11.6 /
   // 10.3). Bidirectional passes hardly shorten (two of 512x512 with MIS 4.77 / 5.20).
   const bool apart = cfg->integrator != YC_UDPT ||
                      (s->dev.n_tri < kRaySortMinTris && (size_t)a->w * a->h >= kShadeSortMinPixels);
@@ -1588,8 +1589,8 @@ int batch_round(yc_batch* b, BatchGroup& g, int cur, bool timed, bool serial) {
   {
     KTimer kt(c, K_LOGIC, timed);
     yc::launch_batch_logic(b->jobs.p, b->tasks.p, g.ctl.p, ps, batch_state(b).job, g.free_stack.p, in_c, in_w, rin, out_c,
-                           out_w, g.q_any.p, rout, c->stats.p, b->job_done.p, g.sorted.p, g.sctl.p, rs_produce(b, g), b->logic_grid,
-                           sm);
+                           out_w, g.q_any.p, rout, c->stats.p, b->job_done.p, g.sorted.p, g.sctl.p, rs_produce(b, g),
+                           b->logic_grid, sm);
   }
   c->ktimes.rounds++;
   YC_CUDA(cudaPeekAtLastError());

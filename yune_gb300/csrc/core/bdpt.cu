@@ -542,15 +542,17 @@ struct BdptStep {
 };
 
 // The tail kernel (yc_tail.cuh), which spares a pass its last rounds of few paths (each ten launches,
-// most of them empty, and the latency of a walk): a 1280x720 pass over 820K triangles 9.54 -> 9.10 ms, a 160x120 pass over 60K 2.40 -> 1.51.
-// Two blocks per SM: the shading and the walk hold 200-226 registers.
+// most of them empty, and the latency of a walk): a 1280x720 pass over 820K triangles 9.54 -> 9.10
+// ms, a 160x120 pass over 60K 2.40 -> 1.51. Two blocks per SM: the shading and the walk hold 198
+// registers.
 template <bool WIDE>
 __global__ void __launch_bounds__(TAIL_TB, 2) k_tail_bdpt(PassParams pp, PathState ps, BdptBuffers bb,
                                                          const int* __restrict__ in_closest,
                                                          const int* __restrict__ in_wait, RoundCounters* rc_in,
                                                          int threshold, int stack_cap, DevStats* st, int n_smem,
                                                          int* spill) {
-  tail_loop<WIDE>(BdptStep{pp, ps, bb}, pp.sc, ps, bb.sg, in_closest, in_wait, rc_in, threshold, stack_cap, st, n_smem, spill);
+  tail_loop<WIDE>(BdptStep{pp, ps, bb}, pp.sc, ps, bb.sg, in_closest, in_wait, rc_in, threshold, stack_cap, st, n_smem,
+                  spill);
 }
 
 int tail_bdpt_grid(const PassParams& pp, int n_smem) {

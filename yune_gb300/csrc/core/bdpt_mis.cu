@@ -225,7 +225,7 @@ void launch_raygen_bdpt_mis(const PassParams& pp, const PathState& ps, const Bdp
 }
 
 // ---- logic: advance each path to its next ray ----
-// Bound by the latency of a long dependent chain at few warps: 163 registers in three blocks
+// Bound by the latency of a long dependent chain at few warps: 168 registers in three blocks
 // of 128 per SM measured best (unbounded, 210 in two: 2.98 ms per two 512x512 passes; three:
 // 2.70; four, 386 B spilled: 2.87; five, 768 B: 3.22).
 constexpr int MIS_TB = 128;
@@ -667,15 +667,17 @@ struct BdptMisStep {
 };
 
 // The tail kernel (yc_tail.cuh), which spares a pass its last rounds of few paths (each ten launches,
-// most of them empty, and the latency of a walk): a 1280x720 pass over 820K triangles 7.69 -> 6.90 ms, a 96x64 pass of the Cornell box 1.21 -> 0.78.
-// Two blocks per SM: the shading and the walk hold 200-226 registers.
+// most of them empty, and the latency of a walk): a 1280x720 pass over 820K triangles 7.69 -> 6.90
+// ms, a 96x64 pass of the Cornell box 1.21 -> 0.78. Two blocks per SM: the shading and the walk hold
+// 231 registers.
 template <bool WIDE>
 __global__ void __launch_bounds__(TAIL_TB, 2) k_tail_bdpt_mis(PassParams pp, PathState ps, BdptBuffers bb,
                                                          const int* __restrict__ in_closest,
                                                          const int* __restrict__ in_wait, RoundCounters* rc_in,
                                                          int threshold, int stack_cap, DevStats* st, int n_smem,
                                                          int* spill) {
-  tail_loop<WIDE>(BdptMisStep{pp, ps, bb}, pp.sc, ps, bb.sg, in_closest, in_wait, rc_in, threshold, stack_cap, st, n_smem, spill);
+  tail_loop<WIDE>(BdptMisStep{pp, ps, bb}, pp.sc, ps, bb.sg, in_closest, in_wait, rc_in, threshold, stack_cap, st, n_smem,
+                  spill);
 }
 
 int tail_bdpt_mis_grid(const PassParams& pp, int n_smem) {

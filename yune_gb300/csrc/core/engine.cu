@@ -249,8 +249,9 @@ void launch_batch_logic(const BatchJob* jobs, BatchTasks* tasks, BatchCtl* ctl, 
                         unsigned long long* job_done,
                         const int* sorted, const SortCtl* sctl, const RsProduce& rsp, int grid, cudaStream_t s) {
   // (grid counts blocks of ENGINE_TB)
-  k_batch_logic<<<grid * (ENGINE_TB / BATCH_LOGIC_TB), BATCH_LOGIC_TB, 0, s>>>(jobs, tasks, ctl, ps, job_pass, free_stack, in_closest, in_wait, rc_in,
-                                           out_closest, out_wait, q_any, rc_out, st, job_done, sorted, sctl, rsp);
+  k_batch_logic<<<grid * (ENGINE_TB / BATCH_LOGIC_TB), BATCH_LOGIC_TB, 0, s>>>(
+      jobs, tasks, ctl, ps, job_pass, free_stack, in_closest, in_wait, rc_in, out_closest, out_wait, q_any, rc_out, st,
+      job_done, sorted, sctl, rsp);
 }
 
 // ---- shade-queue sort (counting sort over SORT_KEYS keys) ----
@@ -502,34 +503,22 @@ int batch_trace_mixed_grid(int n_smem, bool wide, int tb) {
 }
 
 int launch_batch_trace_mixed(bool wide, const BatchJob* jobs, SF<int4> job_pass, const int* q_closest,
-                             const int* q_any, RoundCounters* rc, const PathState& ps, DevStats* st, int stack_cap, int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s,
-                             const int* sorted, const RaySortCtl* rs) {
-  const size_t smem = batch_smem(n_smem, tb);
-  if (wide)
-    k_batch_trace_mixed<true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit, record_segments(ps),
-                                                            stack_cap, st, sorted, rs, n_smem, spill);
-  else
-    k_batch_trace_mixed<false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit, record_segments(ps),
-                                                             stack_cap, st, sorted, rs, n_smem, spill);
+                             const int* q_any, RoundCounters* rc, const PathState& ps, DevStats* st, int stack_cap,
+                             int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s, const int* sorted,
+                             const RaySortCtl* rs) {
+  const auto kernel = wide ? k_batch_trace_mixed<true> : k_batch_trace_mixed<false>;
+  kernel<<<grid_blocks, tb, batch_smem(n_smem, tb), s>>>(jobs, job_pass, q_closest, q_any, rc, ps.ro, ps.rd, ps.hit,
+                                                         record_segments(ps), stack_cap, st, sorted, rs, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch_batch_trace(bool any_hit, bool wide, const BatchJob* jobs, SF<int4> job_pass, const int* queue,
                        const int* count, int* work, const PathState& ps, DevStats* st,
                        int stack_cap, int n_smem, int* spill, int grid_blocks, int tb, cudaStream_t s) {
-  const size_t smem = batch_smem(n_smem, tb);
-  if (any_hit && wide)
-    k_batch_trace<true, true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
-                                                            stack_cap, st, n_smem, spill);
-  else if (any_hit)
-    k_batch_trace<true, false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
-                                                             stack_cap, st, n_smem, spill);
-  else if (wide)
-    k_batch_trace<false, true><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
-                                                             stack_cap, st, n_smem, spill);
-  else
-    k_batch_trace<false, false><<<grid_blocks, tb, smem, s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit, record_segments(ps),
-                                                              stack_cap, st, n_smem, spill);
+  const auto kernel = any_hit ? (wide ? k_batch_trace<true, true> : k_batch_trace<true, false>)
+                              : (wide ? k_batch_trace<false, true> : k_batch_trace<false, false>);
+  kernel<<<grid_blocks, tb, batch_smem(n_smem, tb), s>>>(jobs, job_pass, queue, count, work, ps.ro, ps.rd, ps.hit,
+                                                         record_segments(ps), stack_cap, st, n_smem, spill);
   return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
 

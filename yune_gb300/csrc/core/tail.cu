@@ -33,7 +33,8 @@ __global__ void __launch_bounds__(TAIL_TB, 3) k_tail(PassParams pp, PathState ps
                   n_smem, spill);
 }
 
-using TailKernel = void (*)(PassParams, PathState, Segments, const int*, const int*, RoundCounters*, int, int, DevStats*, int, int*);
+using TailKernel = void (*)(PassParams, PathState, Segments, const int*, const int*, RoundCounters*, int, int, DevStats*,
+                            int, int*);
 template <bool WIDE>
 static TailKernel tail_kernel_of(bool together, bool multi) {
   if (together) return multi ? k_tail<WIDE, true, true> : k_tail<WIDE, true, false>;

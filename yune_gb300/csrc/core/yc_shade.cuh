@@ -63,8 +63,8 @@ __device__ __forceinline__ f4 camera_direction(const PassParams& pp, int px, int
 
 // The power function and the normalisation, called. A shading step holds six of one and ten of
 // the other; inlined they were a fifth of its code, and with two or three warps a scheduler in
-// different places of it the kernels wait for instructions (5.2 of 10 stalls per issue in the
-// tail): a 256x256 frame of the Cornell box 0.62 -> 0.55 ms, four 512x512 passes 3.87 -> 3.53, the
+// different places of it the kernels wait for instructions (5.0-5.2 stalls per issue in the
+// tail of a 256x256 frame of the Cornell box, 2.9 now): a 256x256 frame of the Cornell box 0.62 -> 0.55 ms, four 512x512 passes 3.87 -> 3.53, the
 // 1024x1024 glass sphere 5.35 -> 5.15, two MIS passes 4.17 -> 4.05. (Fresnel, refraction, the
 // Oren-Nayar term, the light loops, the surface point, sine, root or reciprocal called as well:
 // slower or alike.)

@@ -8,14 +8,18 @@
 // (Step) -- until the path writes its pixel. A warp's lanes walk together, the kind of
 // step more of them can take at a time, and run their state machines together once every
 // lane's ray is answered: the state machine's time is that of its code, whose phases a warp
-// runs one after another whatever the lanes in them (25-65 thousand cycles a step), so the
-// fewer runs the better (run when half the lanes wait: 1.65 ms against 1.40 ms on the glass
+// runs one after another whatever the lanes in them (34-48 thousand cycles a run in the
+// mean), so the fewer runs the better (run when half the lanes wait: 1.65 ms against 1.40 ms on the glass
 // sphere). With each lane on its own the kernel ran 3.5 lanes per instruction: 1.74 ms
 // there against 1.10 ms (one ray at a time), and for a 256x256 frame of the Cornell box 1.10
-// against 0.57 ms, 0.44 ms with its rays sent together. What bounds it is the longest chain
-// of rays in a warp (12-25), at 600-1600 cycles a step of a walk. Every path computes exactly
-// what the round-by-round wavefront computes (same state, same operations), so the pass's
-// result is unchanged; paths no longer wait for each other between rays.
+// against 0.57 ms, 0.44 ms with its rays sent together. What bounds it is the longest chain of a
+// warp: 13-17 runs, and the walks between them, at 1,800-2,900 cycles a step while its warps share
+// their scheduler. (Counted with the clock on both sides of the two, in 256x256 and 256x192
+// frames of the Cornell box and of 90K triangles; there the slowest warp takes two to three times
+// the mean, half of it in the state machine in the box, three quarters in walks of 90K
+// triangles.) Every path computes exactly what the round-by-round wavefront computes (same state,
+// same operations), so the pass's result is unchanged; paths no longer wait for each other between
+// rays.
 // The kernel is launched after every round's logic kernel on that round's output
 // queues: above the threshold it returns at once; at or below it, it finishes the pass
 // and its last block to exit empties the queues, so the remaining round launches find
@@ -164,9 +168,9 @@ __device__ __forceinline__ void tail_loop(const Step& step, const DevScene& sc, 
   if (lc.prim) atomicAdd(&s_cnt[13], (unsigned long long)lc.prim);
   __syncthreads();
   if (threadIdx.x == 0) {
-    unsigned long long* dst[14] = {&st->rays, &st->extension, &st->shadow, Step::BDPT ? &st->connection : &st->mis, &st->traversed, &st->samples,
-                                   &st->ext_rays, &st->ext_boxes, &st->ext_tris, &st->any_rays, &st->any_boxes,
-                                   &st->any_tris, &st->stack_overflow, &st->primary};
+    unsigned long long* dst[14] = {&st->rays, &st->extension, &st->shadow, Step::BDPT ? &st->connection : &st->mis,
+                                   &st->traversed, &st->samples, &st->ext_rays, &st->ext_boxes, &st->ext_tris,
+                                   &st->any_rays, &st->any_boxes, &st->any_tris, &st->stack_overflow, &st->primary};
     for (int q = 0; q < 14; ++q)
       if (s_cnt[q]) atomicAdd(dst[q], s_cnt[q]);
     if (s_cnt[12]) atomicAdd(&st->call_overflow, s_cnt[12]);

@@ -71,8 +71,8 @@ __device__ __forceinline__ void start_udpt(const PassParams& pp, const PathState
 // ---- calls of several passes (MULTI) ----
 // They run in one wavefront: a path that ends pass k of its pixel starts pass k + 1 in the next
 // round (launch_raygen, or at once in the tail), so the rounds stay full and the call has one
-// end with few paths, not one for each pass. Every pixel still adds its passes in order. Two
-// 1003x565 passes over 21K triangles 5.29 -> 4.80 ms, four of 160x120 4.22 -> 3.12 ms.
+// end with few paths, not one for each pass. Every pixel still adds its passes in order. Four
+// 160x120 passes over 20K triangles 3.65 ms apart, 2.70 together, four of 800x600 over 60K 14.5 and 12.4.
 __device__ __forceinline__ bool has_next_pass(const PassParams& pp, const PathState& ps, int p) {
   return ps.job[p].w + 1 < pp.n_pass;
 }
@@ -261,7 +261,7 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
   // the lanes of every phase share is worth the loop: a shadow result that goes on to
   // a MIS ray and a path that samples its next bounce run the same instructions). Most
   // paths leave after one pass; a MIS ray that misses the light takes a second one, and a shadow
-// ray sent with the next ray one or two more.
+  // ray sent with the next ray one or two more.
   // Measured against one copy per phase (a switch over the phases): 2.16 -> 1.69 ms of
   // shading per four 512x512 passes of the Cornell box, whose queue is not sorted, 1.11 ->
   // 0.97 ms per 1024x1024 pass of the glass sphere, whose queue is. The warp barriers keep
@@ -336,7 +336,8 @@ __device__ __forceinline__ int logic_path(const PassParams& pp, int reset, const
           if (mis) {
             if (glossy) flags |= F_NEE_GLOSSY; else flags &= ~F_NEE_GLOSSY;
             brdf_pdf = glossy ? phong_pdf(w_i, wo, V, m) : cos_pdf(w_i, V.n);
-            const float weight = ym::div(ym::mul(mw, mw), ym::add(ym::mul(light_pdf, light_pdf), ym::mul(brdf_pdf, brdf_pdf)));
+            const float weight =
+                ym::div(ym::mul(mw, mw), ym::add(ym::mul(light_pdf, light_pdf), ym::mul(brdf_pdf, brdf_pdf)));
             ls = ls * weight;
             if (TOGETHER && !(weight < INF)) flags |= F_OCC_NAN;
             brdf_pdf = pdf;
