@@ -1034,7 +1034,7 @@ int yc_refit_scene(yc_ctx* c, int scene_id, const yc_triangle* tris, int n_tri) 
   plan.level_off = s->refit_levels;
   // a scene without a BVH walks a chain of unbounded boxes: nothing to refit there
   const bool refit_nodes = s->dev.root_test != 0;
-  const int n_slots = (int)(s->tris.n / 3);
+  const int n_slots = (int)(s->n_tri4 / 3);   // (an empty stream's array has room for one, which holds nothing)
   if (yc::launch_refit(plan, s->refit_tris.p, n_tri, s->nodes.p, s->tris.p, n_slots, s->shade.p, s->dev.wide != 0,
                        s->dev.root_link, refit_nodes, s->refit_root.p, c->stream))
     return fail(YC_E_LAUNCH, std::string("refit: ") + cudaGetErrorString(cudaGetLastError()));
